@@ -13,9 +13,8 @@
 //   32) consecutive chunks form a group whose chunk sums are added in ascending
 //   order; the (at most 32) group sums are added in ascending order.
 //
-// Two kernels follow that order.  The tiled one (any number of tokens) lets every
-// thread carry its outputs through all of K and folds the running chain into the
-// group and total sums at the boundaries.  The one for up to 16 tokens (decoding)
+// Two kernels follow that order.  The tiled one (any number of tokens) cuts the groups among
+// four slices of a block and adds their sums in order.  The one for up to 16 tokens (decoding)
 // is bound by reading the weights once: a block owns eight features and all of K,
 // each of its 32 (warp, slot) pairs owns one group of chunks for those features,
 // a thread fetches its 64 weights of a chunk as 16-byte pieces that are all in
@@ -38,106 +37,240 @@ __host__ __device__ inline int chunks_per_group(int K) {
     return (chunks + kGroups - 1) / kGroups;
 }
 
-template <typename TI, typename TO, int BM, int BN, int BK, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gemm_ffma_kernel(const TI* __restrict__ A, int64_t lda, const TI* __restrict__ W, int64_t ldw,
-                 const float* __restrict__ bias, const float* residual, int64_t ldr, TO* out, int64_t ldo, int M,
-                 int N, int K, int act) {
-    constexpr int THREADS = (BM / TM) * (BN / TN);
-    __shared__ float As[BK][BM + 1];
-    __shared__ float Ws[BK][BN + 1];
+// ---- more than 16 tokens: 64 x 64 outputs a block, four slices of K side by side -------------------------------
+//
+// Bound by the FMA units.  A thread makes 8 x 8 outputs, so a tile of 64 x 64 is the work of two warps, and an SM wants at least eight:
+// four slices of the block (two warps each) take four consecutive groups of chunks at a time, put their group sums into shared
+// memory, and every thread adds them to its sixteen running totals in ascending order.  That keeps the order of the sums and the
+// small tile, which the narrow products need to fill the SMs (590 tokens x 768 features: 120 blocks).  Products come in pairs along
+// the features (fma.rn.f32x2, which rounds each half as fmaf does), half as many instructions as single ones, so that the loads
+// from shared memory and the copies of a token's value into both halves find issue slots beside them.
+// Measured (GPT-2 small in float32, three prompts of 590 tokens together): the step's products took 8.5 of 12.9 ms with 4 x 4 outputs a
+// thread and operands loaded element by element (8 TFLOP/s); with this kernel and the attention of runs the step takes 4.1 ms.  590 x 3072
+// x 768 alone, on the way: 210 us before; 115 us with two pieces of a row a warp (23 TFLOP/s; 123 us with single products, 139 us with
+// a second copy of W in shared memory instead of the copies into both halves), the load unit 80 % busy with uncoalesced rows.
+constexpr int kTile = 64;            // tokens and features of a block
+constexpr int kSlices = 4;           // slices of K
+constexpr int kSliceThreads = 64;
+constexpr int kStepK = 32;           // products between two synchronisations of a slice: 128 bytes of a float32 row
+constexpr int kOperandFloats = kStepK * kTile;      // [k][token or feature], its pieces of four permuted by k / 4
+constexpr size_t kTiledSmem = (size_t)kSlices * (4 * kOperandFloats + kTile * kTile) * sizeof(float);
+
+__device__ __forceinline__ uint64_t both_halves(float v) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float2 halves(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+// The four elements at `at` as floats, of which the first `left` belong to the row; zeros for the others (and for a row that is not there).
+// VECTORS: K and the strides are whole pieces of four and the bases are aligned to them, so a piece is either whole or not there.
+template <typename T, bool VECTORS>
+__device__ __forceinline__ float4 four_of(const T* __restrict__ at, int left, bool live) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (!live || left <= 0) return v;
+    if constexpr (VECTORS && sizeof(T) == 4) {
+        v = *reinterpret_cast<const float4*>(at);
+    } else if constexpr (VECTORS) {
+        const uint2 u = *reinterpret_cast<const uint2*>(at);
+        v = make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+    } else {
+        v.x = lb_to_float(at[0]);
+        if (left > 1) v.y = lb_to_float(at[1]);
+        if (left > 2) v.z = lb_to_float(at[2]);
+        if (left > 3) v.w = lb_to_float(at[3]);
+    }
+    return v;
+}
+
+// GROUPED: a group has more than one chunk (K > 2048).
+template <typename TI, typename TO, bool VECTORS, bool GROUPED>
+__global__ void __launch_bounds__(kSlices* kSliceThreads, 1)
+gemm_ffma_kernel(const TI* __restrict__ A, int64_t lda, const TI* __restrict__ W, int64_t ldw, const float* __restrict__ bias, const float* residual,
+                 int64_t ldr, TO* out, int64_t ldo, int M, int N, int K, int act) {
+    extern __shared__ __align__(16) float tiled_smem[];
     lb_wait_for_predecessor();
     lb_dependents_may_launch();
-    const int tid = threadIdx.x;
-    const int tx = tid % (BN / TN), ty = tid / (BN / TN);
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    // acc: the running chain of the current chunk of 64; grp: the current group's chunk sums; tot: the group sums.
-    float acc[TM][TN], grp[TM][TN], tot[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = grp[i][j] = tot[i][j] = 0.0f;
-    static_assert(kChunk % BK == 0, "a chunk is a whole number of k-tiles");
-    const int group_len = chunks_per_group(K) * kChunk;
+    const int slice = threadIdx.x / kSliceThreads, tid = threadIdx.x % kSliceThreads;
+    const int tx = tid % 8, ty = tid / 8;
+    const int m0 = blockIdx.y * kTile, n0 = blockIdx.x * kTile;
+    float* operands = tiled_smem + (size_t)slice * 4 * kOperandFloats;          // two buffers of A's and W's [32][64]
+    float* sums = tiled_smem + (size_t)kSlices * 4 * kOperandFloats;            // [slice][64][64] group sums
+    const int n_chunks = (K + kChunk - 1) / kChunk, G = chunks_per_group(K);
+    const int n_groups = (n_chunks + G - 1) / G, rounds = (n_groups + kSlices - 1) / kSlices;
 
-    // A thread's pieces of the next tiles wait in registers while the current ones are multiplied: the loads of
-    // step i + 1 travel under the arithmetic of step i.
-    constexpr int LA = BM * BK / THREADS, LW = BN * BK / THREADS;
-    static_assert(LA * THREADS == BM * BK && LW * THREADS == BN * BK, "the tiles divide among the threads");
-    float ra[LA], rw[LW];
-    auto fetch = [&](int k0) {
+    // A thread fetches eight pieces of four of an operand a step: rows row0, row0 + 8, .. and the k piece kq of eight, so that eight lanes
+    // read 128 bytes of a row in one go (two pieces of a row a warp instead took 31 passes of the load unit an instruction, as
+    // many as all the rest together).  Row r of k lies at column r ^ (4 (k / 4 mod 8)): the lanes of a store fall into 32 banks and a
+    // piece of four rows stays one.
+    const int kq = tid & 7, row0 = (tid >> 5) * 4 + ((tid >> 3) & 3);
+    const TI* a_row = A + (size_t)(m0 + row0) * lda + 4 * kq;
+    const TI* w_row = W + (size_t)(n0 + row0) * ldw + 4 * kq;
+    const int a_rows = M - m0 - row0, w_rows = N - n0 - row0;          // rows 8 i below these are there
+    float4 piece[8];
+    auto fetch = [&](const TI* rows, int64_t ld, int n_rows, int k) {
 #pragma unroll
-        for (int i = 0; i < LA; ++i) {
-            const int idx = tid + i * THREADS, r = idx / BK, k = idx % BK;
-            const int gm = m0 + r, gk = k0 + k;
-            ra[i] = (gm < M && gk < K) ? lb_to_float(A[(size_t)gm * lda + gk]) : 0.0f;
-        }
+        for (int i = 0; i < 8; ++i) piece[i] = four_of<TI, VECTORS>(rows + 8 * i * ld + k, K - k - 4 * kq, 8 * i < n_rows);
+    };
+    auto keep = [&](float* operand) {
+        float* to = operand + 4 * kq * kTile;
 #pragma unroll
-        for (int i = 0; i < LW; ++i) {
-            const int idx = tid + i * THREADS, r = idx / BK, k = idx % BK;
-            const int gn = n0 + r, gk = k0 + k;
-            rw[i] = (gn < N && gk < K) ? lb_to_float(W[(size_t)gn * ldw + gk]) : 0.0f;
+        for (int i = 0; i < 8; ++i) {
+            const int column = (row0 + 8 * i) ^ (4 * kq);
+            to[column] = piece[i].x;
+            to[column + kTile] = piece[i].y;
+            to[column + 2 * kTile] = piece[i].z;
+            to[column + 3 * kTile] = piece[i].w;
         }
     };
-    fetch(0);
-    for (int k0 = 0; k0 < K; k0 += BK) {
+
+    // This thread's share of the block's totals: 16-byte pieces threadIdx.x + 256 i of the tile's [64][16 pieces].
+    float4 tot[4];
 #pragma unroll
-        for (int i = 0; i < LA; ++i) {
-            const int idx = tid + i * THREADS;
-            As[idx % BK][idx / BK] = ra[i];
-        }
+    for (int i = 0; i < 4; ++i) tot[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+
+    // Half a step's products run between the loads of an operand's next step and its stores: A's under the first half, W's under the second.
+    const int group_k = G * kChunk;
+    int turn = 0;
+    if (slice < n_groups) {
+        fetch(a_row, lda, a_rows, slice * group_k);
+        keep(operands);
+        fetch(w_row, ldw, w_rows, slice * group_k);
+        keep(operands + kOperandFloats);
+    }
+    for (int round = 0; round < rounds; ++round) {
+        const int group = round * kSlices + slice;
+        uint64_t grp[8][4];
+        if (group < n_groups) {
+            const int k_begin = group * group_k, k_end = min(K, k_begin + group_k);
+            uint64_t acc[8][4];
 #pragma unroll
-        for (int i = 0; i < LW; ++i) {
-            const int idx = tid + i * THREADS;
-            Ws[idx % BK][idx / BK] = rw[i];
-        }
-        __syncthreads();
-        if (k0 + BK < K) fetch(k0 + BK);
+            for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[TM], b[TN];
+                for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+            for (int k0 = k_begin; k0 < k_end; k0 += kStepK) {
+                const float* buffer = operands + turn * 2 * kOperandFloats;
+                turn ^= 1;
+                float* coming = operands + turn * 2 * kOperandFloats;
+                // The slice's two warps: this step's operands are there, and nobody reads the buffer that the next step's go to.
+                asm volatile("bar.sync %0, 64;" ::"r"(slice + 1) : "memory");
+                const int next = k0 + kStepK < k_end ? k0 + kStepK : (group + kSlices) * group_k;      // from K on: zeros
+                auto products = [&](int half) {
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+                    for (int kk = half * (kStepK / 2); kk < (half + 1) * (kStepK / 2); ++kk) {
+                        const int turned = 4 * (kk / 4 % 8);
+                        const float* a_s = buffer + kk * kTile + ((4 * ty) ^ turned);
+                        const float* w_s = buffer + kOperandFloats + kk * kTile + ((4 * tx) ^ turned);
+                        const float4 a0 = *reinterpret_cast<const float4*>(a_s), a1 = *reinterpret_cast<const float4*>(a_s + 32);
+                        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(w_s), w1 = *reinterpret_cast<const ulonglong2*>(w_s + 32);
+                        const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = Ws[kk][tx * TN + j];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        const int k_end = k0 + BK;              // the chunk, the group or K itself may end with this tile
-        const bool last = k_end >= K;
-        if (k_end % kChunk == 0 || last) {
-            const bool first_chunk = (k_end - 1) / kChunk * kChunk % group_len == 0;
-            const bool group_ends = k_end % group_len == 0 || last;
-            const bool first_group = (k_end - 1) / group_len == 0;
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    grp[i][j] = first_chunk ? acc[i][j] : grp[i][j] + acc[i][j];
-                    acc[i][j] = 0.0f;
-                    if (group_ends) tot[i][j] = first_group ? grp[i][j] : tot[i][j] + grp[i][j];
+                        for (int i = 0; i < 8; ++i) {
+                            const uint64_t aa = both_halves(a[i]);
+                            acc[i][0] = fma_pair(aa, w0.x, acc[i][0]);
+                            acc[i][1] = fma_pair(aa, w0.y, acc[i][1]);
+                            acc[i][2] = fma_pair(aa, w1.x, acc[i][2]);
+                            acc[i][3] = fma_pair(aa, w1.y, acc[i][3]);
+                        }
+                    }
+                };
+                if (next < K) fetch(a_row, lda, a_rows, next);
+                products(0);
+                if (next < K) {
+                    keep(coming);
+                    fetch(w_row, ldw, w_rows, next);
                 }
+                products(1);
+                if (next < K) keep(coming + kOperandFloats);
+                const int done = k0 + kStepK;
+                if constexpr (GROUPED) {
+                    if (done % kChunk == 0 || done >= k_end) {                     // a chunk ends: into the group's sum
+                        const bool first = (done - 1) / kChunk * kChunk == k_begin;
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                if (first) {
+                                    grp[i][j] = acc[i][j];
+                                } else {
+                                    const float2 g = halves(grp[i][j]), c = halves(acc[i][j]);
+                                    asm("mov.b64 %0, {%1, %2};" : "=l"(grp[i][j]) : "f"(g.x + c.x), "f"(g.y + c.y));
+                                }
+                                acc[i][j] = 0;
+                            }
+                    }
+                }
+            }
+            if constexpr (!GROUPED) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) grp[i][j] = acc[i][j];
+            }
+        }
+        if (round > 0) __syncthreads();              // the sums of the round before have been read
+        if (group < n_groups) {
+            float* mine = sums + (size_t)slice * kTile * kTile;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float* row = mine + (size_t)((i < 4 ? 0 : 32) + ty * 4 + (i & 3)) * kTile + tx * 4;
+                *reinterpret_cast<ulonglong2*>(row) = make_ulonglong2(grp[i][0], grp[i][1]);
+                *reinterpret_cast<ulonglong2*>(row + 32) = make_ulonglong2(grp[i][2], grp[i][3]);
+            }
         }
         __syncthreads();
+        for (int s2 = 0; s2 < kSlices && round * kSlices + s2 < n_groups; ++s2) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 g = reinterpret_cast<const float4*>(sums + (size_t)s2 * kTile * kTile)[threadIdx.x + 256 * i];
+                if (round == 0 && s2 == 0) {
+                    tot[i] = g;
+                } else {
+                    tot[i].x += g.x;
+                    tot[i].y += g.y;
+                    tot[i].z += g.z;
+                    tot[i].w += g.w;
+                }
+            }
+        }
     }
     const lb_act_pair act_pair = lb_act_load(bias, N, act);
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + ty * TM + i;
+    for (int i = 0; i < 4; ++i) {
+        const int piece = threadIdx.x + 256 * i, gm = m0 + piece / 16;
         if (gm >= M) continue;
+        const float t[4] = {tot[i].x, tot[i].y, tot[i].z, tot[i].w};
 #pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int gn = n0 + tx * TN + j;
+        for (int j = 0; j < 4; ++j) {
+            const int gn = n0 + (piece % 16) * 4 + j;
             if (gn >= N) continue;
-            float v = tot[i][j];
+            float v = t[j];
             if (bias != nullptr) v += bias[gn];
             v = lb_activate(v, act, act_pair);
             if (residual != nullptr) v += residual[(size_t)gm * ldr + gn];
             out[(size_t)gm * ldo + gn] = lb_from_float<TO>(v);
         }
     }
+}
+
+template <typename TI, typename TO, bool VECTORS, bool GROUPED>
+int launch_tiled(const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out, int64_t ldo,
+                 int M, int N, int K, int act, cudaStream_t s) {
+    LB_CHECK_CUDA(cudaFuncSetAttribute(gemm_ffma_kernel<TI, TO, VECTORS, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTiledSmem));
+    const dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
+    LB_CHECK_CUDA(lb_launch_overlapped(gemm_ffma_kernel<TI, TO, VECTORS, GROUPED>, grid, dim3(kSlices * kSliceThreads), kTiledSmem, s, (const TI*)A, lda,
+                                       (const TI*)W, ldw, bias, residual, ldr, (TO*)out, ldo, M, N, K, act));
+    LB_CHECK_LAUNCH();
+    return LB_OK;
 }
 
 // ---- up to 16 tokens: the weights are read once, everything else is arranged around that -----------------
@@ -284,6 +417,9 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
            int64_t ldr, void* out, int64_t ldo, int M, int N, int K, int act, cudaStream_t s) {
     constexpr int VEC = 16 / (int)sizeof(TI);
     const bool vectors = K % VEC == 0 && lda % VEC == 0 && ldw % VEC == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)W & 15) == 0;
+    // The tiled kernel loads four elements at a time where no such piece crosses a row's end and all are aligned.
+    const uintptr_t quad_mask = 4 * sizeof(TI) - 1;
+    const bool quads = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & quad_mask) == 0;
     if (M <= kSkinnyTokens && vectors) {
         // Few tokens: bound by reading the weights once (see the head of the file).  A warp serves four groups of
         // chunks, so a short reduction length makes small blocks, of which several share an SM.
@@ -312,9 +448,11 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
                                                                               (TO*)out, ldo, M, N, K, act));
         }
     } else {
-        dim3 grid((N + 63) / 64, (M + 63) / 64);
-        LB_CHECK_CUDA(lb_launch_overlapped(gemm_ffma_kernel<TI, TO, 64, 64, 16, 4, 4>, dim3(grid), dim3(256), 0, s, (const TI*)A, lda, (const TI*)W, ldw, bias,
-                                                                      residual, ldr, (TO*)out, ldo, M, N, K, act));
+        const bool grouped = chunks_per_group(K) > 1;
+        if (quads) return grouped ? launch_tiled<TI, TO, true, true>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, s)
+                                  : launch_tiled<TI, TO, true, false>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, s);
+        return grouped ? launch_tiled<TI, TO, false, true>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, s)
+                       : launch_tiled<TI, TO, false, false>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, s);
     }
     LB_CHECK_LAUNCH();
     return LB_OK;

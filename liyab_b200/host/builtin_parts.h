@@ -135,7 +135,7 @@ inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView
         return;
     }
     kernels::attention_generic(ctx.stream(), ctx.runtime.dtype, q, cache, ctx.tok_seq, ctx.positions, view.block_table,
-                               view.table_width, att, T, a);
+                               view.table_width, att, T, ctx.n_seq, a);
 }
 
 // ---- causal self-attention over the paged cache, one fused projection of queries, keys and values -----

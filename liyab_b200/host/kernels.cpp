@@ -257,9 +257,15 @@ int decode_splits(int n_seq, int n_kv_head, int max_context, bool tensor_cores) 
 }
 
 void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* cache, const int32_t* tok_seq,
-                       const int32_t* positions, const int32_t* block_table, int table_width, const Rows& out, int n_tokens,
+                       const int32_t* positions, const int32_t* block_table, int table_width, const Rows& out, int n_tokens, int n_seq,
                        const AttentionShape& a) {
     if (q.dtype != dtype || out.dtype != dtype) throw invalid_argument("attention: q, cache and out must have one element type");
+    if (dtype == DType::F32 && a.distance == nullptr && a.soft_cap == 0.0f &&
+        lb_paged_attention_f32_runs_supports(cache, n_tokens, n_seq, a.n_head, a.n_kv_head, a.head_dim, a.mask()) != 0) {
+        check(lb_paged_attention_f32_runs(q.f32(), q.stride, static_cast<const float*>(cache), tok_seq, positions, block_table, table_width, out.f32(),
+                                          out.stride, n_tokens, a.n_head, a.n_kv_head, a.page_size, a.scale, a.mask(), a.sink, s), "paged_attention_f32_runs");
+        return;
+    }
     check(lb_paged_attention_generic_capped(code(dtype, "cache"), q.data, q.stride, cache, tok_seq, positions, block_table, table_width,
                                           out.data, out.stride, n_tokens, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale,
                                           a.mask(), a.distance, a.sink, a.soft_cap, s), "paged_attention_generic");

@@ -59,6 +59,7 @@ _SIGNATURES = {
     "lb_decode_attention_mma_capped": [_p, _l, _p, _i, _p, _p, _i, _p, _l, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _p, _p, _f, _f, _p],
     "lb_prefill_attention_capped": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _p],
     "lb_prefill_attention_tc_capped": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _p],
+    "lb_paged_attention_f32_runs": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _f, _i, _p, _p],
     "lb_qkv_rotary_store_scaled": [_i, _p, _l, _i, _i, _i, _p, _p, _p, _l, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p, _i, _p, _p, _l, _p, _i, _f, _p],
     "lb_row_norm_gate": [_i, _p, _l, _p, _l, _p, _p, _l, _i, _i, _i, _f, _p],
     "lb_activate_columns": [_p, _l, _i, _i, _i, _p],
@@ -373,6 +374,19 @@ def paged_attention_generic(q: torch.Tensor, cache: torch.Tensor, tok_seq: torch
         _dev(block_table, "block_table", torch.int32), block_table.stride(0), _dev(out, "out"), out.stride(0),
         n_tokens, n_head, n_kv_head, head_dim, page_size, float(scale), int(window), _distance(distance, n_head), _sink(sink, n_head), float(soft_cap), stream_ptr()),
         "paged_attention_generic")
+    return out
+
+
+def paged_attention_f32_runs(q: torch.Tensor, cache: torch.Tensor, tok_seq: torch.Tensor, positions: torch.Tensor, block_table: torch.Tensor,
+                             out: torch.Tensor, n_tokens: int, n_head: int, n_kv_head: int, page_size: int, scale: float, window: int = 0,
+                             sink: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """`paged_attention_generic` for float32 heads of 64 without a moving window: a tile is read once for sixteen neighbouring tokens."""
+    if q.stride(1) != 1 or out.stride(1) != 1:
+        raise invalid_argument("attention: q and out must be dense within a row")
+    check(lib().lb_paged_attention_f32_runs(
+        _dev(q, "q", torch.float32), q.stride(0), _dev(cache, "cache", torch.float32), _dev(tok_seq, "tok_seq", torch.int32),
+        _dev(positions, "positions", torch.int32), _dev(block_table, "block_table", torch.int32), block_table.stride(0), _dev(out, "out", torch.float32),
+        out.stride(0), n_tokens, n_head, n_kv_head, page_size, float(scale), int(window), _sink(sink, n_head), stream_ptr()), "paged_attention_f32_runs")
     return out
 
 
