@@ -408,97 +408,97 @@ paged_attention_f32_runs_kernel(const float* __restrict__ q, int64_t q_stride, c
 
     // `pos` stands for the position that the block's first token would have in the run's request: query u is at pos + u throughout.
     for (int run = 0, run_end; run < n_here; run = run_end) {
-      run_end = min(n_here, run + __ffs(starts >> (run + 1)));            // the lanes from n_here on start runs of their own
-      const int first = __shfl_sync(0xffffffffu, my_first, run), pos = __shfl_sync(0xffffffffu, my_pos, run) - run, last = pos + run_end - 1;
-      const int32_t* table = block_table + (size_t)__shfl_sync(0xffffffffu, my_seq, run) * table_stride;
-      for (int j0 = first + warp * kTile; j0 <= last; j0 += kRunWarps * kTile) {
-        const int j = j0 + lane;
-        long long base = -1;
-        if (j <= last) base = (long long)table[j / page_size] * 2 * (long long)plane + ((long long)kvh * page_size + (j % page_size)) * kRunDim;
-        const int u0 = max(run, j0 - pos);                  // the run's first queries may lie before the tile
-        {
-            float4 key[kRunDim / 4];
-#pragma unroll
-            for (int c = 0; c < kRunDim / 4; ++c)
-                key[c] = base >= 0 ? __ldg(reinterpret_cast<const float4*>(cache + base) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int u = u0 & ~3; u < run_end; u += 4) {
-                float dot[4] = {0.f, 0.f, 0.f, 0.f};
+        run_end = min(n_here, run + __ffs(starts >> (run + 1)));            // the lanes from n_here on start runs of their own
+        const int first = __shfl_sync(0xffffffffu, my_first, run), pos = __shfl_sync(0xffffffffu, my_pos, run) - run, last = pos + run_end - 1;
+        const int32_t* table = block_table + (size_t)__shfl_sync(0xffffffffu, my_seq, run) * table_stride;
+        for (int j0 = first + warp * kTile; j0 <= last; j0 += kRunWarps * kTile) {
+            const int j = j0 + lane;
+            long long base = -1;
+            if (j <= last) base = (long long)table[j / page_size] * 2 * (long long)plane + ((long long)kvh * page_size + (j % page_size)) * kRunDim;
+            const int u0 = max(run, j0 - pos);                  // the run's first queries may lie before the tile
+            {
+                float4 key[kRunDim / 4];
 #pragma unroll
                 for (int c = 0; c < kRunDim / 4; ++c)
+                    key[c] = base >= 0 ? __ldg(reinterpret_cast<const float4*>(cache + base) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int u = u0 & ~3; u < run_end; u += 4) {
+                    float dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int c = 0; c < kRunDim / 4; ++c)
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float4 qq = *reinterpret_cast<const float4*>(q_s + (u + e) * kRunDim + 4 * c);
+                            dot[e] = fmaf(qq.x, key[c].x, dot[e]);
+                            dot[e] = fmaf(qq.y, key[c].y, dot[e]);
+                            dot[e] = fmaf(qq.z, key[c].z, dot[e]);
+                            dot[e] = fmaf(qq.w, key[c].w, dot[e]);
+                        }
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        const float4 qq = *reinterpret_cast<const float4*>(q_s + (u + e) * kRunDim + 4 * c);
-                        dot[e] = fmaf(qq.x, key[c].x, dot[e]);
-                        dot[e] = fmaf(qq.y, key[c].y, dot[e]);
-                        dot[e] = fmaf(qq.z, key[c].z, dot[e]);
-                        dot[e] = fmaf(qq.w, key[c].w, dot[e]);
-                    }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int n_keys = min(kTile, pos + u + e + 1 - j0);
-                    const float s = lane < n_keys ? dot[e] * scale : -CUDART_INF_F;
-                    float* state = mine + (u + e) * kRunAcc;
-                    const float m = state[0];
-                    float l = state[1];
-                    const float m_new = fmaxf(m, lb_warp_max(s));
-                    const float p = lane < n_keys ? expf(s - m_new) : 0.0f;
-                    const float corr = expf(m - m_new);      // exp(-inf) = 0 on the first tile
-                    l = l * corr + lb_warp_sum(p);
-                    if (u + e >= u0 && u + e < run_end) {    // the others' states are not this run's, or see none of the tile
-                        p_s[(u + e) * kTile + lane] = p;
-                        if (lane == 0) {
-                            state[0] = m_new;
-                            state[1] = l;
-                            corr_s[u + e] = corr;
+                        const int n_keys = min(kTile, pos + u + e + 1 - j0);
+                        const float s = lane < n_keys ? dot[e] * scale : -CUDART_INF_F;
+                        float* state = mine + (u + e) * kRunAcc;
+                        const float m = state[0];
+                        float l = state[1];
+                        const float m_new = fmaxf(m, lb_warp_max(s));
+                        const float p = lane < n_keys ? expf(s - m_new) : 0.0f;
+                        const float corr = expf(m - m_new);      // exp(-inf) = 0 on the first tile
+                        l = l * corr + lb_warp_sum(p);
+                        if (u + e >= u0 && u + e < run_end) {    // the others' states are not this run's, or see none of the tile
+                            p_s[(u + e) * kTile + lane] = p;
+                            if (lane == 0) {
+                                state[0] = m_new;
+                                state[1] = l;
+                                corr_s[u + e] = corr;
+                            }
                         }
                     }
                 }
             }
-        }
-        __syncwarp();
-        {
-            float v0[kTile], v1[kTile];
-            const int n_rows = min(kTile, last + 1 - j0);
+            __syncwarp();
+            {
+                float v0[kTile], v1[kTile];
+                const int n_rows = min(kTile, last + 1 - j0);
 #pragma unroll
-            for (int k = 0; k < kTile; ++k) {
-                const long long b = __shfl_sync(0xffffffffu, base, k);
-                v0[k] = k < n_rows ? __ldg(cache + b + plane + lane) : 0.0f;
-                v1[k] = k < n_rows ? __ldg(cache + b + plane + 32 + lane) : 0.0f;
-            }
-#pragma unroll 2
-            for (int u = u0; u < run_end; ++u) {
-                const int n_keys = min(kTile, pos + u + 1 - j0);
-                float* state = mine + u * kRunAcc + 2;
-                const float corr = corr_s[u];
-                float o0 = state[lane] * corr, o1 = state[lane + 32] * corr;
-                const float4* weights = reinterpret_cast<const float4*>(p_s + u * kTile);
-                if (n_keys == kTile) {
-#pragma unroll
-                    for (int k = 0; k < kTile / 4; ++k) {
-                        const float4 p = weights[k];
-                        o0 = fmaf(p.x, v0[4 * k], o0);
-                        o1 = fmaf(p.x, v1[4 * k], o1);
-                        o0 = fmaf(p.y, v0[4 * k + 1], o0);
-                        o1 = fmaf(p.y, v1[4 * k + 1], o1);
-                        o0 = fmaf(p.z, v0[4 * k + 2], o0);
-                        o1 = fmaf(p.z, v1[4 * k + 2], o1);
-                        o0 = fmaf(p.w, v0[4 * k + 3], o0);
-                        o1 = fmaf(p.w, v1[4 * k + 3], o1);
-                    }
-                } else {                                      // the keys after the query are no terms of its sums
-#pragma unroll
-                    for (int k = 0; k < kTile; ++k) {
-                        const float p = p_s[u * kTile + k];
-                        o0 = k < n_keys ? fmaf(p, v0[k], o0) : o0;
-                        o1 = k < n_keys ? fmaf(p, v1[k], o1) : o1;
-                    }
+                for (int k = 0; k < kTile; ++k) {
+                    const long long b = __shfl_sync(0xffffffffu, base, k);
+                    v0[k] = k < n_rows ? __ldg(cache + b + plane + lane) : 0.0f;
+                    v1[k] = k < n_rows ? __ldg(cache + b + plane + 32 + lane) : 0.0f;
                 }
-                state[lane] = o0;
-                state[lane + 32] = o1;
+#pragma unroll 2
+                for (int u = u0; u < run_end; ++u) {
+                    const int n_keys = min(kTile, pos + u + 1 - j0);
+                    float* state = mine + u * kRunAcc + 2;
+                    const float corr = corr_s[u];
+                    float o0 = state[lane] * corr, o1 = state[lane + 32] * corr;
+                    const float4* weights = reinterpret_cast<const float4*>(p_s + u * kTile);
+                    if (n_keys == kTile) {
+#pragma unroll
+                        for (int k = 0; k < kTile / 4; ++k) {
+                            const float4 p = weights[k];
+                            o0 = fmaf(p.x, v0[4 * k], o0);
+                            o1 = fmaf(p.x, v1[4 * k], o1);
+                            o0 = fmaf(p.y, v0[4 * k + 1], o0);
+                            o1 = fmaf(p.y, v1[4 * k + 1], o1);
+                            o0 = fmaf(p.z, v0[4 * k + 2], o0);
+                            o1 = fmaf(p.z, v1[4 * k + 2], o1);
+                            o0 = fmaf(p.w, v0[4 * k + 3], o0);
+                            o1 = fmaf(p.w, v1[4 * k + 3], o1);
+                        }
+                    } else {                                      // the keys after the query are no terms of its sums
+#pragma unroll
+                        for (int k = 0; k < kTile; ++k) {
+                            const float p = p_s[u * kTile + k];
+                            o0 = k < n_keys ? fmaf(p, v0[k], o0) : o0;
+                            o1 = k < n_keys ? fmaf(p, v1[k], o1) : o1;
+                        }
+                    }
+                    state[lane] = o0;
+                    state[lane + 32] = o1;
+                }
             }
+            __syncwarp();
         }
-        __syncwarp();
-      }
     }
     __syncthreads();
     for (int i = threadIdx.x; i < n_here * kRunDim; i += blockDim.x) {

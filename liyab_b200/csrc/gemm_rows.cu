@@ -1,7 +1,7 @@
 // out[M, N] = epilogue(A[M, K] . W[N, K]^T) for 1 to 64 tokens (bfloat16
 // operands): the products of a decode step, too small to fill a tcgen05 tile row,
 // whose reduction is short enough (the host takes it for K up to 1024, and for up
-// to 16 tokens up to 4096 where one pass covers a block's features).
+// to 16 tokens up to 8192: gemm_stream_kernel below).
 //
 // At these sizes a product reads a few MB of weights and does next to no
 // arithmetic; what it costs is latency.  The tcgen05 kernel needs K split over
@@ -58,6 +58,18 @@ struct KvScatter {
     const int32_t* slot_mapping;
     int q_dim, n_kv_head, head_dim, page_size;
 };
+
+// Feature f >= q_dim of token r's fused projection: also into the token's slot of its cache page.
+__device__ __forceinline__ void keep_key_or_value(const KvScatter& kv, int r, int f, float y) {
+    const int kvf = f - kv.q_dim, kv_dim = kv.n_kv_head * kv.head_dim;
+    const int which = kvf >= kv_dim ? 1 : 0, within = kvf - which * kv_dim;
+    const int head = within / kv.head_dim, dd = within - head * kv.head_dim;
+    const int slot = __ldg(kv.slot_mapping + r);
+    if (slot < 0) return;
+    const int page = slot / kv.page_size, off = slot - page * kv.page_size;
+    const size_t plane = (size_t)kv.n_kv_head * kv.page_size * kv.head_dim;
+    kv.cache[(size_t)page * 2 * plane + (size_t)which * plane + ((size_t)head * kv.page_size + off) * kv.head_dim + dd] = __float2bfloat16_rn(y);
+}
 
 // Activations made in the kernel from the float32 residual rows by a LayerNorm (two-pass 32-bit statistics,
 // (x - mean) / sqrt(var + eps) * gain + offset, as the separate kernel computes them): for up to 16 tokens and a
@@ -289,19 +301,7 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bf
                 float y = lb_activate(v + early[e].x, act, act_pair);
                 if (residual != nullptr) y += early[e].y;
                 out[(size_t)r * ldo + f] = lb_from_float<TO>(y);
-                if (kv.cache != nullptr && f >= kv.q_dim) {
-                    // A key or value feature of a fused projection: also into the token's slot of its cache page.
-                    const int kvf = f - kv.q_dim, kv_dim = kv.n_kv_head * kv.head_dim;
-                    const int which = kvf >= kv_dim ? 1 : 0, within = kvf - which * kv_dim;
-                    const int head = within / kv.head_dim, dd = within - head * kv.head_dim;
-                    const int slot = __ldg(kv.slot_mapping + r);
-                    if (slot >= 0) {
-                        const int page = slot / kv.page_size, off = slot - page * kv.page_size;
-                        const size_t plane = (size_t)kv.n_kv_head * kv.page_size * kv.head_dim;
-                        kv.cache[(size_t)page * 2 * plane + (size_t)which * plane + ((size_t)head * kv.page_size + off) * kv.head_dim + dd] =
-                            __float2bfloat16_rn(y);
-                    }
-                }
+                if (kv.cache != nullptr && f >= kv.q_dim) keep_key_or_value(kv, r, f, y);
             }
         }
         __syncthreads();
@@ -334,26 +334,289 @@ int launch_by_k(const void* A, int64_t lda, const void* W, int64_t ldw, const fl
     return launch<MT, 1, TO, STAGE>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s);
 }
 
+// ---- up to 16 tokens, a slice of weights that does not fit a pass's registers -----------------------------------------
+//
+// gemm_rows_kernel asks for the weights of a pass at its start and for the next pass's after it, a round trip to memory a pass; the
+// split tcgen05 product that served longer reductions before needs a second launch to add its parts, and a third where the rows
+// have to be normalised first.  Here the block's weights run through a ring in shared memory instead: a lane copies by cp.async the
+// very 16 bytes that it will feed to its products and reads them back itself, so the ring needs no barrier, and it is kept full from
+// before the wait for the kernel before until the last chunk is asked for.  The activations of a chunk travel with its weights, or
+// (NORMED) are made here from the float32 rows as gemm_rows_kernel makes them.  Bound by the weights' way from memory:
+// 148 blocks with some 64 KB in flight each, no more than 113 KB of shared memory a block for up to 8 tokens, so that the next
+// launch's blocks fit beside it and ask for their weights early.
+// Measured (GPT-2 XL, 8 requests, contexts of 360 to 880): the step's 243 launches took 483 before; 2.38 -> 2.31 ms with its logits'
+// copy.  Alone with cold caches, 8 tokens: 1600 -> 6400 normed 9.9 us (before: norm 3.6, split product 9.2 and second half 4.1), 6400 -> 1600 7.5 us
+// (9.2 and 3.6), of which 4.9 us of the first are the rows' norm, which waits behind the weights in flight.
+constexpr int kStreamGroups = 8;       // the most feature groups of eight a block takes
+constexpr int kStreamMaxK = 8192;
+constexpr int kStreamNormedMaxK = 2048;
+// Chunks in flight: GB groups of weights (and the activations' one or two pieces) of 4 KB each a chunk.
+constexpr int stream_depth(int gb, bool normed, bool wide) {
+    const int pieces = normed ? 19 : 24, a = normed ? 0 : wide ? 2 : 1, d = pieces / (gb + a);
+    return d < 2 ? 2 : d > 12 ? 12 : d;
+}
+
+// The rows' norm with gains and offsets in shared memory (gain_s, offset_s), for K up to kStreamNormedMaxK; one warp a row.
+__device__ void stream_norm_rows(const RowNorm& n, int M, int K, __nv_bfloat16* act, int ld, int k_pad, int rows, const float* gain_s, const float* offset_s) {
+    constexpr int kVecs = kStreamNormedMaxK / 128;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n_vec = K / 4;
+    for (int r = warp; r < rows; r += kWarps) {
+        __nv_bfloat16* dst = act + r * ld;
+        if (r >= M) {
+            for (int i = lane * 8; i < k_pad; i += 256) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
+            continue;
+        }
+        const float* row = n.x + (size_t)r * n.ldx;
+        float4 v[kVecs];
+#pragma unroll
+        for (int j = 0; j < kVecs; ++j) {
+            const int i = lane + 32 * j;
+            v[j] = i < n_vec ? __ldcg(reinterpret_cast<const float4*>(row) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kVecs; ++j) sum += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+        const float mean = n.rms ? 0.0f : lb_warp_sum(sum) / (float)K;
+        float ss = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kVecs; ++j) {
+            if (lane + 32 * j < n_vec) {
+                const float d0 = v[j].x - mean, d1 = v[j].y - mean, d2 = v[j].z - mean, d3 = v[j].w - mean;
+                ss = fmaf(d0, d0, ss);
+                ss = fmaf(d1, d1, ss);
+                ss = fmaf(d2, d2, ss);
+                ss = fmaf(d3, d3, ss);
+            }
+        }
+        const float inv = 1.0f / sqrtf(lb_warp_sum(ss) / (float)K + n.eps);
+#pragma unroll
+        for (int j = 0; j < kVecs; ++j) {
+            const int i = lane + 32 * j;
+            if (i < n_vec) {
+                float4 g = make_float4(1.f, 1.f, 1.f, 1.f), o = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (n.gain != nullptr) {
+                    g = reinterpret_cast<const float4*>(gain_s)[i];
+                    g.x += n.gain_offset;
+                    g.y += n.gain_offset;
+                    g.z += n.gain_offset;
+                    g.w += n.gain_offset;
+                }
+                if (n.offset != nullptr) o = reinterpret_cast<const float4*>(offset_s)[i];
+                const __nv_bfloat162 lo = __floats2bfloat162_rn((v[j].x - mean) * inv * g.x + o.x, (v[j].y - mean) * inv * g.y + o.y);
+                const __nv_bfloat162 hi = __floats2bfloat162_rn((v[j].z - mean) * inv * g.z + o.z, (v[j].w - mean) * inv * g.w + o.w);
+                uint2 packed;
+                packed.x = *reinterpret_cast<const uint32_t*>(&lo);
+                packed.y = *reinterpret_cast<const uint32_t*>(&hi);
+                *reinterpret_cast<uint2*>(dst + 4 * i) = packed;
+            }
+        }
+        for (int i = K + lane; i < k_pad; i += 32) dst[i] = __float2bfloat16_rn(0.0f);
+    }
+}
+
+// GB: the most groups a block has.  WIDE: more than 8 tokens.  K, the row strides and the bases as for gemm_rows_kernel.
+template <int GB, bool NORMED, bool WIDE, typename TO>
+__global__ void __launch_bounds__(kThreads, 2)
+gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bfloat16* __restrict__ W, int64_t ldw, const float* __restrict__ bias,
+                   const float* residual, int64_t ldr, TO* out, int64_t ldo, int M, int N, int K, int act, KvScatter kv, RowNorm norm) {
+    constexpr int DEPTH = stream_depth(GB, NORMED, WIDE), ROWS = WIDE ? 16 : 8, APIECES = NORMED ? 0 : WIDE ? 2 : 1;
+    extern __shared__ __align__(16) uint8_t smem_bytes[];
+    uint4* ring = reinterpret_cast<uint4*>(smem_bytes);                      // [DEPTH][GB + APIECES][256 lanes]; at the end the warps' sums
+    float* red_s = reinterpret_cast<float*>(smem_bytes);                     // [kWarps][GB][ROWS][8]
+    static_assert((size_t)kWarps * GB * ROWS * 8 * sizeof(float) <= (size_t)DEPTH * (GB + APIECES) * kThreads * 16, "the sums fit the ring");
+    float* gain_s = reinterpret_cast<float*>(ring + DEPTH * (GB + APIECES) * kThreads);     // NORMED: gains and offsets, then the rows
+    float* offset_s = gain_s + K;
+    const int ld = (K + kChunk - 1) / kChunk * kChunk + 32;                  // 64 bytes mod 128
+    __nv_bfloat16* act_s = reinterpret_cast<__nv_bfloat16*>(offset_s + K);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int n_groups = (N + 7) / 8, n_chunks = (K + kChunk - 1) / kChunk;
+    const int share = n_groups / (int)gridDim.x, more = n_groups % (int)gridDim.x;      // the first `more` blocks have a group more
+    const int g_begin = (int)blockIdx.x * share + min((int)blockIdx.x, more), ng = share + ((int)blockIdx.x < more ? 1 : 0);
+    const int k_lane = warp * 32 + t * 8;
+    const __nv_bfloat16* w_lane = W + (size_t)(g_begin * 8 + g) * ldw + k_lane;
+
+    auto weights = [&](int c) {                                              // chunk c's weights -> its place in the ring
+        uint4* to = ring + (c % DEPTH) * (GB + APIECES) * kThreads + threadIdx.x;
+        const bool there = c * kChunk + k_lane < K;
+#pragma unroll
+        for (int gi = 0; gi < GB; ++gi)
+            if (gi < ng) {
+                const bool valid = there && (g_begin + gi) * 8 + g < N;
+                cp_async16(to + gi * kThreads, valid ? w_lane + (size_t)gi * 8 * ldw + c * kChunk : W, valid);
+            }
+    };
+    auto activations = [&](int c) {
+        uint4* to = ring + ((c % DEPTH) * (GB + APIECES) + GB) * kThreads + threadIdx.x;
+        const int k = c * kChunk + k_lane;
+#pragma unroll
+        for (int p = 0; p < APIECES; ++p) {
+            const bool valid = k < K && g + 8 * p < M;
+            cp_async16(to + p * kThreads, valid ? A + (size_t)(g + 8 * p) * lda + k : A, valid);
+        }
+    };
+
+    // Before the wait: what does not depend on the kernel before.
+    if constexpr (NORMED) {
+        for (int i = threadIdx.x; i < K / 4; i += kThreads) {
+            if (norm.gain != nullptr) cp_async16(gain_s + 4 * i, norm.gain + 4 * i, true);
+            if (norm.offset != nullptr) cp_async16(offset_s + 4 * i, norm.offset + 4 * i, true);
+        }
+        cp_async_commit();
+    }
+#pragma unroll
+    for (int c = 0; c < DEPTH; ++c) {
+        if (c < n_chunks) weights(c);
+        cp_async_commit();
+    }
+    if constexpr (NORMED) cp_async_wait<DEPTH>();
+    const lb_act_pair act_pair = lb_act_load(bias, N, act);
+    lb_wait_for_predecessor();
+    lb_dependents_may_launch();
+    if constexpr (NORMED) {
+        __syncthreads();                                                     // every thread's gains and offsets
+        stream_norm_rows(norm, M, K, act_s, ld, n_chunks * kChunk, ROWS, gain_s, offset_s);
+        __syncthreads();
+    } else {
+#pragma unroll
+        for (int c = 0; c < DEPTH; ++c) {
+            if (c < n_chunks) activations(c);
+            cp_async_commit();
+        }
+    }
+    // The elements this thread will finish: their bias and residual travel under the products.
+    constexpr int kElements = GB * ROWS * 8, kEarly = (kElements + kThreads - 1) / kThreads;
+    float2 early[kEarly];
+#pragma unroll
+    for (int e = 0; e < kEarly; ++e) {
+        early[e] = make_float2(0.f, 0.f);
+        const int idx = threadIdx.x + e * kThreads, gi = idx / (ROWS * 8), r = idx / 8 % ROWS, f = (g_begin + gi) * 8 + (idx & 7);
+        if (gi < ng && r < M && f < N)
+            early[e] = make_float2(bias != nullptr ? __ldg(bias + f) : 0.0f, residual != nullptr ? __ldcg(residual + (size_t)r * ldr + f) : 0.0f);
+    }
+    float acc[GB][4];
+#pragma unroll
+    for (int gi = 0; gi < GB; ++gi) acc[gi][0] = acc[gi][1] = acc[gi][2] = acc[gi][3] = 0.0f;
+    // Groups of copies are counted alike in both forms: DEPTH - 1 later chunks may be on their way when chunk c is used.
+    for (int c = 0; c < n_chunks; ++c) {
+        cp_async_wait<DEPTH - 1>();
+        const uint4* from = ring + (c % DEPTH) * (GB + APIECES) * kThreads + threadIdx.x;
+        uint4 lo, hi = make_uint4(0, 0, 0, 0);
+        if constexpr (NORMED) {
+            const __nv_bfloat16* row = act_s + g * ld + c * kChunk + k_lane;
+            lo = *reinterpret_cast<const uint4*>(row);
+            if constexpr (WIDE) hi = *reinterpret_cast<const uint4*>(row + 8 * ld);
+        } else {
+            lo = from[GB * kThreads];
+            if constexpr (WIDE) hi = from[(GB + 1) * kThreads];
+        }
+#pragma unroll
+        for (int gi = 0; gi < GB; ++gi)
+            if (gi < ng) {
+                const uint4 w = from[gi * kThreads];
+                mma_bf16(acc[gi], lo.x, hi.x, lo.y, hi.y, w.x, w.y);
+                mma_bf16(acc[gi], lo.z, hi.z, lo.w, hi.w, w.z, w.w);
+            }
+        // The pieces are in the products: the chunk DEPTH further on may take their place.
+        if (c + DEPTH < n_chunks) {
+            weights(c + DEPTH);
+            if constexpr (!NORMED) activations(c + DEPTH);
+        }
+        cp_async_commit();
+    }
+    cp_async_wait<0>();
+    __syncthreads();                                                         // the ring turns into the warps' sums
+#pragma unroll
+    for (int gi = 0; gi < GB; ++gi)
+        if (gi < ng) {
+            float* tile = red_s + (size_t)(warp * GB + gi) * ROWS * 8;
+            *reinterpret_cast<float2*>(tile + g * 8 + 2 * t) = make_float2(acc[gi][0], acc[gi][1]);
+            if constexpr (WIDE) *reinterpret_cast<float2*>(tile + (g + 8) * 8 + 2 * t) = make_float2(acc[gi][2], acc[gi][3]);
+        }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < kEarly; ++e) {
+        const int idx = threadIdx.x + e * kThreads, gi = idx / (ROWS * 8), r = idx / 8 % ROWS, f = (g_begin + gi) * 8 + (idx & 7);
+        if (gi >= ng || r >= M || f >= N) continue;
+        float v = 0.0f;
+#pragma unroll
+        for (int wp = 0; wp < kWarps; ++wp) v += red_s[(size_t)(wp * GB) * ROWS * 8 + idx];
+        float y = lb_activate(v + early[e].x, act, act_pair);
+        if (residual != nullptr) y += early[e].y;
+        out[(size_t)r * ldo + f] = lb_from_float<TO>(y);
+        if (kv.cache != nullptr && f >= kv.q_dim) keep_key_or_value(kv, r, f, y);
+    }
+}
+
+template <int GB, bool NORMED, bool WIDE, typename TO>
+int launch_stream(const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out, int64_t ldo,
+                  int M, int N, int K, int act, KvScatter kv, RowNorm norm, int grid, cudaStream_t s) {
+    size_t smem = (size_t)stream_depth(GB, NORMED, WIDE) * (GB + (NORMED ? 0 : WIDE ? 2 : 1)) * kThreads * 16;
+    if (NORMED) smem += (size_t)2 * K * sizeof(float) + (size_t)(WIDE ? 16 : 8) * ((K + kChunk - 1) / kChunk * kChunk + 32) * sizeof(__nv_bfloat16);
+    static size_t configured = 0;
+    if (smem > configured) {
+        LB_CHECK_CUDA(cudaFuncSetAttribute(gemm_stream_kernel<GB, NORMED, WIDE, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured = smem;
+    }
+    LB_CHECK_CUDA(lb_launch_overlapped(gemm_stream_kernel<GB, NORMED, WIDE, TO>, dim3(grid), dim3(kThreads), smem, s, (const __nv_bfloat16*)A, lda,
+                                       (const __nv_bfloat16*)W, ldw, bias, residual, ldr, (TO*)out, ldo, M, N, K, act, kv, norm));
+    return LB_OK;
+}
+
+template <bool NORMED, bool WIDE, typename TO>
+int stream_by_groups(const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out, int64_t ldo,
+                     int M, int N, int K, int act, KvScatter kv, RowNorm norm, int n_sm, cudaStream_t s) {
+    const int n_groups = (N + 7) / 8, grid = n_groups < n_sm ? n_groups : n_sm, most = (n_groups + grid - 1) / grid;
+#define LB_GO(GB) return launch_stream<GB, NORMED, WIDE, TO>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, grid, s)
+    if (most <= 1) LB_GO(1);
+    if (most <= 2) LB_GO(2);
+    if (most <= 4) LB_GO(4);
+    if (most <= 6) LB_GO(6);
+    if (most <= kStreamGroups) LB_GO(8);
+#undef LB_GO
+    return lb_fail(LB_ERR_UNSUPPORTED, "gemm_rows: %d features are too many for one launch", N);
+}
+
+template <bool NORMED>
+int stream(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out,
+           int64_t ldo, int M, int N, int K, int act, KvScatter kv, RowNorm norm, int n_sm, cudaStream_t s) {
+    if (out_dtype == LB_F32)
+        return M > 8 ? stream_by_groups<NORMED, true, float>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s)
+                     : stream_by_groups<NORMED, false, float>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s);
+    return M > 8 ? stream_by_groups<NORMED, true, __nv_bfloat16>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s)
+                 : stream_by_groups<NORMED, false, __nv_bfloat16>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s);
+}
+
+// Whether the ring takes a product of up to 16 tokens: where one pass of gemm_rows_kernel's registers does not hold a block's weights.
+bool rows_streams(int M, int N, int K, int n_sm, bool normed) {
+    if (M > 16 || K > (normed ? kStreamNormedMaxK : kStreamMaxK)) return false;
+    const int n_groups = (N + 7) / 8, grid = n_groups < n_sm ? n_groups : n_sm, most = (n_groups + grid - 1) / grid;
+    if (most > kStreamGroups) return false;
+    const int pass = K <= 4 * kChunk ? 4 : K <= 8 * kChunk ? 2 : K <= 16 * kChunk ? 1 : 0;
+    return (normed && K > 4 * kChunk) || most > pass;
+}
+
 }  // namespace
 
-// Whether the kernel takes the product: 1 to 64 tokens, a reduction length of up to 4096, K and the row strides of
+// Whether the kernels take the product: 1 to 64 tokens, a reduction length of up to 4096 (up to 16 tokens: 8192), K and the row strides of
 // A and W multiples of 8, 16-byte aligned bases, and at most four passes over the feature groups of a block (the
 // head's vocabulary is left to the tcgen05 kernel, whose tiles suit it).
 extern "C" int lb_gemm_rows_supports(const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N, int K) {
     if (M <= 0 || M > kMaxRows || N <= 0 || K <= 0) return 0;
     if (K % 8 != 0 || lda % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)A & 15) != 0 || ((uintptr_t)W & 15) != 0) return 0;
+    if (M <= 16 && (N + 7) / 8 <= 148 * kStreamGroups && K <= kStreamMaxK) return 1;
     if (K > kWRegs * kChunk) return 0;
     const int ng = K <= 4 * kChunk ? 4 : K <= 8 * kChunk ? 2 : 1;
     return (N + 7) / 8 <= 148 * 4 * ng;
 }
 
-// The same product for up to 16 tokens and a reduction length of up to 1024 with the activations made in the kernel:
+// The same product for up to 16 tokens and a reduction length of up to 2048 with the activations made in the kernel:
 // LayerNorm (two-pass 32-bit statistics, eps, gain and offset or null) of the float32 rows x, normalised by every
 // block for itself.  lb_gemm_rows_normed_supports says whether the kernel takes the operands.
 extern "C" int lb_gemm_rows_normed_supports(const void* x, int64_t ldx, const void* W, int64_t ldw, int M, int N, int K) {
-    if (M <= 0 || M > 16 || N <= 0 || K <= 0 || K > 4 * kChunk) return 0;
+    if (M <= 0 || M > 16 || N <= 0 || K <= 0 || K > kStreamNormedMaxK) return 0;
     if (K % 8 != 0 || ldx % 4 != 0 || ldw % 8 != 0 || ((uintptr_t)x & 15) != 0 || ((uintptr_t)W & 15) != 0) return 0;
-    return (N + 7) / 8 <= 148 * 4 * 4;
+    return (N + 7) / 8 <= 148 * (K <= 4 * kChunk ? 4 * 4 : kStreamGroups);
 }
 
 extern "C" int lb_gemm_rows_normed(int out_dtype, const float* x, int64_t ldx, const float* gain, const float* offset, float eps,
@@ -369,10 +632,10 @@ extern "C" int lb_gemm_rows_normed(int out_dtype, const float* x, int64_t ldx, c
 extern "C" int lb_gemm_rows_normed_kind(int out_dtype, const float* x, int64_t ldx, const float* gain, const float* offset, float eps, int rms,
                                         float gain_offset, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr,
                                         void* out, int64_t ldo, int M, int N, int K, int act, void* kv_cache, const int32_t* slot_mapping,
-                                        int q_dim, int n_kv_head, int head_dim, int page_size, void* stream) {
+                                        int q_dim, int n_kv_head, int head_dim, int page_size, void* stream_handle) {
     LB_CHECK_ARG(out_dtype == LB_BF16 || out_dtype == LB_F32, "gemm_rows_normed: unknown output dtype %d", out_dtype);
     if (!lb_gemm_rows_normed_supports(x, ldx, W, ldw, M, N, K) || ((uintptr_t)gain & 15) != 0 || ((uintptr_t)offset & 15) != 0)
-        return lb_fail(LB_ERR_UNSUPPORTED, "gemm_rows_normed: takes 1 to 16 tokens, K up to 1024 and a multiple of 8, 16-byte aligned bases "
+        return lb_fail(LB_ERR_UNSUPPORTED, "gemm_rows_normed: takes 1 to 16 tokens, K up to 2048 and a multiple of 8, 16-byte aligned bases "
                        "(M=%d N=%d K=%d ldx=%lld ldw=%lld)", M, N, K, (long long)ldx, (long long)ldw);
     LB_CHECK_ARG(ldx >= K && ldw >= K && ldo >= N, "gemm_rows_normed: a row stride is shorter than the row");
     static int n_sm = 0;
@@ -388,7 +651,8 @@ extern "C" int lb_gemm_rows_normed_kind(int out_dtype, const float* x, int64_t l
                      "gemm_rows_normed: the cache destination needs N = q_dim + 2 * n_kv_head * head_dim (N=%d q_dim=%d heads %d x %d)", N,
                      q_dim, n_kv_head, head_dim);
     const RowNorm norm{x, ldx, gain, offset, eps, rms, gain_offset};
-    auto s = static_cast<cudaStream_t>(stream);
+    auto s = static_cast<cudaStream_t>(stream_handle);
+    if (rows_streams(M, N, K, n_sm, true)) return stream<true>(out_dtype, nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s);
     if (out_dtype == LB_F32)
         return launch<1, 4, float, 2>(nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s, norm);
     return launch<1, 4, __nv_bfloat16, 2>(nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s, norm);
@@ -397,7 +661,7 @@ extern "C" int lb_gemm_rows_normed_kind(int out_dtype, const float* x, int64_t l
 extern "C" int lb_gemm_rows(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias,
                             const float* residual, int64_t ldr, void* out, int64_t ldo, int M, int N, int K, int act,
                             void* kv_cache, const int32_t* slot_mapping, int q_dim, int n_kv_head, int head_dim, int page_size,
-                            void* stream) {
+                            void* stream_handle) {
     LB_CHECK_ARG(out_dtype == LB_BF16 || out_dtype == LB_F32, "gemm_rows: unknown output dtype %d", out_dtype);
     if (!lb_gemm_rows_supports(A, lda, W, ldw, M, N, K))
         return lb_fail(LB_ERR_UNSUPPORTED, "gemm_rows: takes 1 to 64 tokens, K and row strides multiples of 8 and 16-byte aligned "
@@ -415,7 +679,8 @@ extern "C" int lb_gemm_rows(int out_dtype, const void* A, int64_t lda, const voi
                          q_dim + 2 * n_kv_head * head_dim == N,
                      "gemm_rows: the cache destination needs N = q_dim + 2 * n_kv_head * head_dim (N=%d q_dim=%d heads %d x %d)", N,
                      q_dim, n_kv_head, head_dim);
-    auto s = static_cast<cudaStream_t>(stream);
+    auto s = static_cast<cudaStream_t>(stream_handle);
+    if (rows_streams(M, N, K, n_sm, false)) return stream<false>(out_dtype, A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, RowNorm{}, n_sm, s);
     const int mt = (M + 15) / 16;
 #define LB_GO(MT)                                                                                                          \
     return out_dtype == LB_F32 ? launch_by_k<MT, float>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s)   \

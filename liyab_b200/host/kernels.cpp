@@ -133,9 +133,9 @@ void gemm_rows_normed(cudaStream_t s, const Rows& x, const float* gain, const fl
 bool gemm_rows_takes(int m, int n, int k, int sm_count) {
     if (m < 1 || m > 64) return false;
     if (k <= kRowsMaxK) return true;
-    if (m > 16 || k > 4096) return false;
-    const int groups = (n + 7) / 8, blocks = std::min(groups, std::max(1, sm_count)), per_block = (groups + blocks - 1) / blocks;
-    return per_block <= (k <= 2048 ? 2 : 1);          // the groups a block holds in its registers at that K
+    // Up to 16 tokens: eight groups of eight features a block at most (see gemm_stream_kernel).
+    const int groups = (n + 7) / 8, blocks = std::min(groups, std::max(1, sm_count));
+    return m <= 16 && k <= 8192 && (groups + blocks - 1) / blocks <= 8;
 }
 
 int gemm_splits(int m, int n, int k) {

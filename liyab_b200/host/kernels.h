@@ -59,13 +59,13 @@ void gemm_tcgen05(cudaStream_t s, const Rows& a, const Tensor& w, const float* b
 // activations: a reduction length of up to 1024 (measured: with K = 1600 or 3072 the tcgen05 kernel with K split over
 // blocks and a second half wins, at 8 tokens as at 64).
 inline constexpr int kRowsMaxK = 1024;
-// Up to 16 tokens the kernel keeps all columns of the activations, so a longer reduction (up to 4096) is worth it too
-// where a block then asks for all its weights at once: one pass over its feature groups (GPT-2 small's and medium's
-// down projections; GPT-2 XL's projections would take three passes and stay with the split product: 2.30 against 2.16 ms).
+// Up to 16 tokens a longer reduction (up to 8192) is worth it too while a block has at most eight groups of eight features: in one pass where
+// its registers hold the weights (up to 4096), else through a ring in shared memory (GPT-2 XL's projections; 2.31 against 2.38 ms a step of 8
+// with the split product).
 bool gemm_rows_takes(int m, int n, int k, int sm_count);
 bool gemm_rows_supports(const Rows& a, const Tensor& w, int m);
 // The same product with the rows of the float32 matrix x normalised inside the kernel (LayerNorm: gain, offset or
-// null, eps; with `rms` no mean is taken off and gain_offset is added to every gain): up to 16 tokens, K up to 1024,
+// null, eps; with `rms` no mean is taken off and gain_offset is added to every gain): up to 16 tokens, K up to 2048,
 // bfloat16 weights.
 bool gemm_rows_normed_supports(const Runtime& rt, const Rows& x, const Tensor& w, int m);
 void gemm_rows_normed(cudaStream_t s, const Rows& x, const float* gain, const float* offset, float eps, const Tensor& w, const float* bias,

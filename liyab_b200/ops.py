@@ -275,7 +275,7 @@ def gemm_rows(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
 def gemm_rows_normed(x: torch.Tensor, gain: Optional[torch.Tensor], offset: Optional[torch.Tensor], eps: float, w: torch.Tensor,
                      bias: Optional[torch.Tensor], out: torch.Tensor, m: int, activation: str = "none",
                      residual: Optional[torch.Tensor] = None, kv: Optional[tuple] = None) -> torch.Tensor:
-    """out[:m] = act(LayerNorm(x[:m]) @ w.T + bias) + residual for up to 16 tokens and K up to 1024: the rows are
+    """out[:m] = act(LayerNorm(x[:m]) @ w.T + bias) + residual for up to 16 tokens and K up to 2048: the rows are
     normalised inside the product's kernel.  `kv` as for gemm_rows."""
     n, k = w.shape
     cache, slots, q_dim, n_kv_head, head_dim, page_size = _kv_args(kv)
