@@ -71,8 +71,8 @@ template <int HD, int kWarps, int kStages, bool TMA>
 __global__ void __launch_bounds__(kWarps * 32)
 decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, int kv_rows, int* status,
                             const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_bfloat16* __restrict__ cache,
-                            const int32_t* __restrict__ positions, const int32_t* __restrict__ block_table, int table_stride,
-                            __nv_bfloat16* __restrict__ out, int64_t out_stride, float* __restrict__ partial,
+                            const int32_t* __restrict__ q_start, const int32_t* __restrict__ positions, const int32_t* __restrict__ block_table,
+                            int table_stride, __nv_bfloat16* __restrict__ out, int64_t out_stride, float* __restrict__ partial,
                             int* __restrict__ counters, int n_head, int n_kv_head, int page_shift, float scale, int window,
                             int n_splits, int cluster_merge, const float* __restrict__ distance, const float* __restrict__ sink,
                             float soft_cap, float bound) {
@@ -93,6 +93,13 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, int kv_r
     __shared__ uint64_t bars[kWarps][kStages];
 
     const int split = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z;
+    // A mixed step (q_start given): request seq's tokens start at q_start[seq], and only requests of one token are served here.
+    const int token = q_start != nullptr ? q_start[seq] : seq;
+    if (q_start != nullptr && q_start[seq + 1] - token != 1) {       // the same for all blocks of a cluster
+        lb_wait_for_predecessor();
+        lb_dependents_may_launch();
+        return;
+    }
     // Every block of the cluster has started before one of them writes into another's shared memory: arrive now, wait
     // just before those writes.
     if (cluster_merge) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
@@ -100,7 +107,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, int kv_r
     const int G = n_head / n_kv_head;           // query heads of this key/value head: the tile's valid rows
     const int page_size = 1 << page_shift;
     const size_t plane = (size_t)n_kv_head * page_size * HD;
-    const int pos = positions[seq];
+    const int pos = positions[token];
     const int first = lb_first_visible(pos, window);
     const int n_keys = pos + 1 - first;
     const int chunk = (n_keys + n_splits - 1) / n_splits;
@@ -112,7 +119,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, int kv_r
     // Q as the A operand: row r = query head kvh * G + r (rows past G are zero).  Filled after the wait below.
     uint32_t qf[KS][4];
     auto load_queries = [&]() {
-        const __nv_bfloat16* q_seq = q + (size_t)seq * q_stride + (size_t)kvh * G * HD;
+        const __nv_bfloat16* q_seq = q + (size_t)token * q_stride + (size_t)kvh * G * HD;
 #pragma unroll
         for (int kk = 0; kk < KS; ++kk) {
             const int c = kk * 16 + 2 * t;
@@ -338,7 +345,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, int kv_r
         }
         if (n_splits == 1) {
             if (sink != nullptr) a *= lb_sink_join_exp2(sink[kvh * G + r] * kLbLog2e, mm, ll);
-            out[(size_t)seq * out_stride + (size_t)(kvh * G + r) * HD + d] = __float2bfloat16_rn(a / ll);
+            out[(size_t)token * out_stride + (size_t)(kvh * G + r) * HD + d] = __float2bfloat16_rn(a / ll);
         } else if (cluster_merge) {
             const uint32_t at = first_block + (uint32_t)(r * STATE) * 4u;
             asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at + (uint32_t)(2 + d) * 4u), "f"(a) : "memory");
@@ -375,7 +382,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, int kv_r
                 a += st[2 + d] * f;
             }
             if (sink != nullptr) a *= lb_sink_join_exp2(sink[kvh * G + r] * kLbLog2e, mm, ll);      // once, where the ranges meet
-            out[(size_t)seq * out_stride + (size_t)(kvh * G + r) * HD + d] = __float2bfloat16_rn(a / ll);
+            out[(size_t)token * out_stride + (size_t)(kvh * G + r) * HD + d] = __float2bfloat16_rn(a / ll);
         }
         return;
     }
@@ -402,7 +409,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, int kv_r
             a += __ldcg(st + 2 + d) * f;
         }
         if (sink != nullptr) a *= lb_sink_join_exp2(sink[kvh * G + r] * kLbLog2e, mm, ll);      // once, where the ranges meet
-        out[(size_t)seq * out_stride + (size_t)(kvh * G + r) * HD + d] = __float2bfloat16_rn(a / ll);
+        out[(size_t)token * out_stride + (size_t)(kvh * G + r) * HD + d] = __float2bfloat16_rn(a / ll);
     }
 }
 
@@ -435,7 +442,7 @@ struct Variant {
         return LB_OK;
     }
 
-    static int launch(const CUtensorMap& map_kv, int kv_rows, int* status, const void* q, int64_t q_stride, const void* cache, const int32_t* positions, const int32_t* block_table,
+    static int launch(const CUtensorMap& map_kv, int kv_rows, int* status, const void* q, int64_t q_stride, const void* cache, const int32_t* q_start, const int32_t* positions, const int32_t* block_table,
                       int table_stride, void* out, int64_t out_stride, float* partial, int* counters, int n_seq, int n_head,
                       int n_kv_head, int page_shift, float scale, int window, int n_splits, const float* distance, const float* sink, float soft_cap,
                       float bound, cudaStream_t s) {
@@ -449,7 +456,7 @@ struct Variant {
         if (rc != LB_OK) return rc;
         LB_CHECK_CUDA(lb_launch_overlapped_cluster(3, cluster ? n_splits : 1, decode_attention_mma_kernel<HD, kWarps, kStages, TMA>, grid,
                                                    dim3(kWarps * 32), smem + inbox, s, map_kv, kv_rows, status, (const __nv_bfloat16*)q,
-                                                   q_stride, (const __nv_bfloat16*)cache, positions, block_table, table_stride,
+                                                   q_stride, (const __nv_bfloat16*)cache, q_start, positions, block_table, table_stride,
                                                    (__nv_bfloat16*)out, out_stride, partial, counters, n_head, n_kv_head, page_shift,
                                                    scale, window, n_splits, cluster ? 1 : 0, distance, sink, soft_cap, bound));
         return LB_OK;
@@ -461,7 +468,7 @@ struct Variant {
 // then fit in one).  A choice by the launch's shape only; it changes the order in which tiles are merged, which
 // is rounding.
 template <int HD, bool TMA>
-int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* q, int64_t q_stride, const void* cache, const int32_t* positions, const int32_t* block_table,
+int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* q, int64_t q_stride, const void* cache, const int32_t* q_start, const int32_t* positions, const int32_t* block_table,
                int table_stride, void* out, int64_t out_stride, float* partial, int* counters, int n_seq, int n_head,
                int n_kv_head, int page_shift, float scale, int window, int n_splits, const float* distance, const float* sink, float soft_cap,
                       float bound, cudaStream_t s) {
@@ -482,9 +489,9 @@ int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* 
     // fill = blocks / (waves * slots); compared without division
     const bool narrow = blocks > slots_wide && waves_wide * slots_wide >= waves_narrow * slots_narrow;
     if (narrow)
-        return Narrow::launch(map_kv, kv_rows, status, q, q_stride, cache, positions, block_table, table_stride, out, out_stride, partial, counters,
+        return Narrow::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride, partial, counters,
                               n_seq, n_head, n_kv_head, page_shift, scale, window, n_splits, distance, sink, soft_cap, bound, s);
-    return Wide::launch(map_kv, kv_rows, status, q, q_stride, cache, positions, block_table, table_stride, out, out_stride, partial, counters, n_seq,
+    return Wide::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride, partial, counters, n_seq,
                         n_head, n_kv_head, page_shift, scale, window, n_splits, distance, sink, soft_cap, bound, s);
 }
 
@@ -528,6 +535,15 @@ extern "C" int lb_decode_attention_mma_capped(const void* q, int64_t q_stride, c
                                               const int32_t* block_table, int table_stride, void* out, int64_t out_stride, float* partial, int* counters,
                                               int n_seq, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window, int n_splits,
                                               const float* distance, const float* sink, float soft_cap, float bound, void* stream) {
+    return lb_decode_attention_mma_mixed(q, q_stride, cache, n_pages, nullptr, positions, block_table, table_stride, out, out_stride, partial, counters, n_seq,
+                                         n_head, n_kv_head, head_dim, page_size, scale, window, n_splits, distance, sink, soft_cap, bound, stream);
+}
+
+extern "C" int lb_decode_attention_mma_mixed(const void* q, int64_t q_stride, const void* cache, int n_pages, const int32_t* q_start,
+                                             const int32_t* positions, const int32_t* block_table, int table_stride, void* out, int64_t out_stride,
+                                             float* partial, int* counters, int n_seq, int n_head, int n_kv_head, int head_dim, int page_size, float scale,
+                                             int window, int n_splits, const float* distance, const float* sink, float soft_cap, float bound,
+                                             void* stream) {
     LB_CHECK_ARG(soft_cap >= 0.0f && (soft_cap == 0.0f || distance == nullptr), "decode attention: a soft cap is positive and goes without a penalty by distance");
     LB_CHECK_ARG(n_seq >= 0 && n_splits >= 1, "decode attention: bad sizes n_seq=%d n_splits=%d", n_seq, n_splits);
     if (!lb_decode_attention_mma_supports(n_head, n_kv_head, head_dim, page_size))
@@ -550,13 +566,13 @@ extern "C" int lb_decode_attention_mma_capped(const void* q, int64_t q_stride, c
             int rc = lb_tensor_map_2d(&map_kv, cache, 2, (int)kv_rows, 64, 64, kTile);
             if (rc == LB_OK) rc = lb_tc_status_word(&status);
             if (rc != LB_OK) return rc;
-            return launch_for<64, true>(map_kv, (int)kv_rows, status, q, q_stride, cache, positions, block_table, table_stride,
+            return launch_for<64, true>(map_kv, (int)kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride,
                                         out, out_stride, partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window,
                                         n_splits, distance, sink, soft_cap, bound, s);
         }
-        return launch_for<64, false>(none, 0, nullptr, q, q_stride, cache, positions, block_table, table_stride, out, out_stride,
+        return launch_for<64, false>(none, 0, nullptr, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride,
                                      partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, n_splits, distance, sink, soft_cap, bound, s);
     }
-    return launch_for<128, false>(none, 0, nullptr, q, q_stride, cache, positions, block_table, table_stride, out, out_stride,
+    return launch_for<128, false>(none, 0, nullptr, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride,
                                   partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, n_splits, distance, sink, soft_cap, bound, s);
 }

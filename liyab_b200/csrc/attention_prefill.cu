@@ -73,7 +73,7 @@ prefill_attention_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, 
                          const int32_t* __restrict__ q_start, const int32_t* __restrict__ n_past,
                          const int32_t* __restrict__ block_table, int table_stride, __nv_bfloat16* __restrict__ out,
                          int64_t out_stride, int n_head, int n_kv_head, int page_shift, float scale, int window,
-                         const float* __restrict__ distance, const float* __restrict__ sink, float soft_cap, float bound) {
+                         const float* __restrict__ distance, const float* __restrict__ sink, float soft_cap, float bound, int min_len) {
     constexpr int LD = HD + 8;                  // padded row of a tile in shared memory (elements)
     constexpr int CH = HD / 8;                  // 16-byte chunks per row
     constexpr int KS = HD / 16;                 // k-steps of Q K^T
@@ -90,7 +90,7 @@ prefill_attention_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, 
     // ones fill the gaps at the end.
     const int seq = blockIdx.z, head = blockIdx.y, tile_q = (int)gridDim.x - 1 - (int)blockIdx.x;
     const int row0 = q_start[seq], q_len = q_start[seq + 1] - row0;
-    if (tile_q * kBM >= q_len) return;
+    if (tile_q * kBM >= q_len || q_len < min_len) return;
     const int past = n_past[seq];
     const int kvh = head / (n_head / n_kv_head);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -271,7 +271,7 @@ prefill_attention_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_stride, 
 template <int HD>
 int launch(const void* q, int64_t q_stride, const void* cache, const int32_t* q_start, const int32_t* n_past,
            const int32_t* block_table, int table_stride, void* out, int64_t out_stride, int n_seq, int max_q_len,
-           int n_head, int n_kv_head, int page_shift, float scale, int window, const float* distance, const float* sink, float soft_cap, float bound,
+           int n_head, int n_kv_head, int page_shift, float scale, int window, const float* distance, const float* sink, float soft_cap, float bound, int min_len,
            cudaStream_t s) {
     constexpr size_t smem = (size_t)(kBM + 2 * kStages * kBN) * (HD + 8) * sizeof(__nv_bfloat16);
     static bool configured = false;
@@ -282,7 +282,7 @@ int launch(const void* q, int64_t q_stride, const void* cache, const int32_t* q_
     dim3 grid((max_q_len + kBM - 1) / kBM, n_head, n_seq);
     LB_CHECK_CUDA(lb_launch_overlapped(prefill_attention_kernel<HD>, dim3(grid), dim3(kThreads), smem, s, 
         (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)cache, q_start, n_past, block_table, table_stride,
-        (__nv_bfloat16*)out, out_stride, n_head, n_kv_head, page_shift, scale, window, distance, sink, soft_cap, bound));
+        (__nv_bfloat16*)out, out_stride, n_head, n_kv_head, page_shift, scale, window, distance, sink, soft_cap, bound, min_len));
     LB_CHECK_LAUNCH();
     return LB_OK;
 }
@@ -322,6 +322,14 @@ extern "C" int lb_prefill_attention_capped(const void* q, int64_t q_stride, cons
                                            const int32_t* block_table, int table_stride, void* out, int64_t out_stride, int n_seq, int max_q_len,
                                            int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window, const float* distance,
                                            const float* sink, float soft_cap, float bound, void* stream) {
+    return lb_prefill_attention_portions(q, q_stride, cache, q_start, n_past, block_table, table_stride, out, out_stride, n_seq, max_q_len, n_head, n_kv_head,
+                                         head_dim, page_size, scale, window, distance, sink, soft_cap, bound, 1, stream);
+}
+
+extern "C" int lb_prefill_attention_portions(const void* q, int64_t q_stride, const void* cache, const int32_t* q_start, const int32_t* n_past,
+                                           const int32_t* block_table, int table_stride, void* out, int64_t out_stride, int n_seq, int max_q_len,
+                                           int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window, const float* distance,
+                                           const float* sink, float soft_cap, float bound, int min_len, void* stream) {
     LB_CHECK_ARG(soft_cap >= 0.0f && (soft_cap == 0.0f || distance == nullptr), "prefill attention: a soft cap is positive and goes without a penalty by distance");
     LB_CHECK_ARG(n_seq >= 0 && max_q_len >= 0, "prefill attention: bad sizes");
     if (!lb_prefill_attention_supports(n_head, n_kv_head, head_dim, page_size))
@@ -337,7 +345,7 @@ extern "C" int lb_prefill_attention_capped(const void* q, int64_t q_stride, cons
 #define LB_HD(HD)                                                                                                        \
     case HD:                                                                                                             \
         return launch<HD>(q, q_stride, cache, q_start, n_past, block_table, table_stride, out, out_stride, n_seq, max_q_len, \
-                          n_head, n_kv_head, page_shift, scale, window, distance, sink, soft_cap, bound, s)
+                          n_head, n_kv_head, page_shift, scale, window, distance, sink, soft_cap, bound, min_len, s)
     switch (head_dim) {
         LB_HD(16);
         LB_HD(32);

@@ -108,7 +108,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const int32_t* __restrict__ block_table, int table_stride, __nv_bfloat16* __restrict__ out,
                             int64_t out_stride, int n_head, int n_kv_head, int page_shift, int kv_rows, float scale, int window,
                             const float* __restrict__ distance, const float* __restrict__ sink,
-                            float soft_cap, float bound, int* status) {
+                            float soft_cap, float bound, int min_len, int* status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     lb_wait_for_predecessor();            // queries, keys and values come from the kernel before this one
@@ -124,7 +124,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // The last query tiles of a request see the most keys: blocks are numbered so that all of those start first.
     const int head = blockIdx.x % n_head, seq = blockIdx.x / n_head, tile_q = (int)gridDim.y - 1 - (int)blockIdx.y;
     const int row0 = q_start[seq], q_len = q_start[seq + 1] - row0;
-    if (tile_q * kBM >= q_len) return;
+    if (tile_q * kBM >= q_len || q_len < min_len) return;
     const int past = n_past[seq];
     const int kvh = head / (n_head / n_kv_head);
     const int page_size = 1 << page_shift;
@@ -464,6 +464,14 @@ extern "C" int lb_prefill_attention_tc_capped(const void* q, int64_t q_stride, i
                                               const int32_t* n_past, const int32_t* block_table, int table_stride, void* out, int64_t out_stride,
                                               int n_seq, int max_q_len, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window,
                                               const float* distance, const float* sink, float soft_cap, float bound, void* stream) {
+    return lb_prefill_attention_tc_portions(q, q_stride, n_tokens, cache, n_pages, q_start, n_past, block_table, table_stride, out, out_stride, n_seq, max_q_len,
+                                            n_head, n_kv_head, head_dim, page_size, scale, window, distance, sink, soft_cap, bound, 1, stream);
+}
+
+extern "C" int lb_prefill_attention_tc_portions(const void* q, int64_t q_stride, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
+                                              const int32_t* n_past, const int32_t* block_table, int table_stride, void* out, int64_t out_stride,
+                                              int n_seq, int max_q_len, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window,
+                                              const float* distance, const float* sink, float soft_cap, float bound, int min_len, void* stream) {
     LB_CHECK_ARG(soft_cap >= 0.0f && (soft_cap == 0.0f || distance == nullptr), "prefill attention (tcgen05): a soft cap is positive and goes without a penalty by distance");
     LB_CHECK_ARG(distance == nullptr || scale != 0.0f, "prefill attention (tcgen05): a penalty by distance needs a factor on the scores that is not zero");
     LB_CHECK_ARG(n_seq >= 0 && max_q_len >= 0 && n_tokens >= 0 && n_pages > 0, "prefill attention: bad sizes");
@@ -495,7 +503,7 @@ extern "C" int lb_prefill_attention_tc_capped(const void* q, int64_t q_stride, i
     dim3 grid(n_head * n_seq, (max_q_len + kBM - 1) / kBM);
     LB_CHECK_CUDA(lb_launch_overlapped(prefill_attention_tc_kernel, dim3(grid), dim3(kThreads), smem, static_cast<cudaStream_t>(stream), 
         map_q, map_kv, q_start, n_past, block_table, table_stride, (__nv_bfloat16*)out, out_stride, n_head, n_kv_head, page_shift,
-        (int)kv_rows, scale, window, distance, sink, soft_cap, bound, status));
+        (int)kv_rows, scale, window, distance, sink, soft_cap, bound, min_len, status));
     LB_CHECK_LAUNCH();
     return LB_OK;
 }

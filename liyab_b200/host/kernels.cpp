@@ -271,7 +271,7 @@ void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* c
                                           a.mask(), a.distance, a.sink, a.soft_cap, s), "paged_attention_generic");
 }
 
-void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* positions,
+void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,
                       const int32_t* block_table, int table_width, const Rows& out, float* partial, int* counters, int n_seq,
                       const AttentionShape& a, int n_splits) {
     if (q.dtype != DType::BF16 || out.dtype != DType::BF16) throw invalid_argument("decode attention takes bfloat16 only");
@@ -279,8 +279,9 @@ void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const vo
         throw invalid_argument("decode attention: q rows must be 16-byte aligned and a multiple of 8 elements apart");
     if (n_splits > 1 && (partial == nullptr || counters == nullptr))
         throw invalid_argument("decode attention: scratch buffers are missing");
+    if (q_start != nullptr && !tensor_cores) throw invalid_argument("decode attention: the scalar kernel takes steps of single tokens only");
     if (tensor_cores)
-        check(lb_decode_attention_mma_capped(q.data, q.stride, cache, n_pages, positions, block_table, table_width, out.data, out.stride,
+        check(lb_decode_attention_mma_mixed(q.data, q.stride, cache, n_pages, q_start, positions, block_table, table_width, out.data, out.stride,
                                            partial, counters, n_seq, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale, a.mask(),
                                            n_splits, a.distance, a.sink, a.soft_cap, a.score_bound, s), "decode_attention_mma");
     else
@@ -291,21 +292,22 @@ void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const vo
 
 void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                        const int32_t* n_past, const int32_t* block_table, int table_width, const Rows& out, int n_seq,
-                       int max_q_len, const AttentionShape& a) {
+                       int max_q_len, bool singles_apart, const AttentionShape& a) {
     if (q.dtype != DType::BF16 || out.dtype != DType::BF16) throw invalid_argument("prefill attention takes bfloat16 only");
-    // Measured on B200: the tcgen05 kernel walks a long tile's keys about 1.4x faster, but runs one block per SM,
-    // so it wins while the launch is bound by its longest blocks (up to four blocks per SM) and loses to the
-    // mma.sync kernel's several blocks per SM beyond that.
-    const int64_t blocks = static_cast<int64_t>(n_seq) * a.n_head * ((max_q_len + 127) / 128);
-    const bool tc = prefill_tc_supports(a) && q.stride % 8 == 0 && out.stride % 8 == 0 && aligned16(q.data) &&
-                    aligned16(out.data) && blocks <= 4 * static_cast<int64_t>(rt.sm_count) && a.scale > 0;     // it takes the maximum of the raw scores
+    // The tcgen05 kernel takes 128 rows and keys at a time, one block an SM; it wins up to about four blocks an SM and is level with the
+    // mma.sync kernel's several blocks an SM beyond that (XL, 5 prompts of 220 to 580 tokens: 11.95 against 12.18 ms a step; taken
+    // always, 12.00).  Tiles are counted as they can occur: no more than the tokens fill, and one more a request.
+    const int64_t tiles = std::min<int64_t>(static_cast<int64_t>(n_seq) * ((max_q_len + 127) / 128), n_tokens / 128 + n_seq);
+    const bool tc = prefill_tc_supports(a) && q.stride % 8 == 0 && out.stride % 8 == 0 && aligned16(q.data) && aligned16(out.data) &&
+                    tiles * a.n_head <= 4 * static_cast<int64_t>(rt.sm_count) && a.scale > 0;     // it takes the maximum of the raw scores
+    const int min_len = singles_apart ? 2 : 1;
     if (tc)
-        check(lb_prefill_attention_tc_capped(q.data, q.stride, n_tokens, cache, n_pages, q_start, n_past, block_table, table_width,
+        check(lb_prefill_attention_tc_portions(q.data, q.stride, n_tokens, cache, n_pages, q_start, n_past, block_table, table_width,
                                            out.data, out.stride, n_seq, max_q_len, a.n_head, a.n_kv_head, a.head_dim, a.page_size,
-                                           a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, rt.stream), "prefill_attention_tc");
+                                           a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, rt.stream), "prefill_attention_tc");
     else
-        check(lb_prefill_attention_capped(q.data, q.stride, cache, q_start, n_past, block_table, table_width, out.data, out.stride, n_seq,
-                                        max_q_len, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, rt.stream),
+        check(lb_prefill_attention_portions(q.data, q.stride, cache, q_start, n_past, block_table, table_width, out.data, out.stride, n_seq,
+                                        max_q_len, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, rt.stream),
               "prefill_attention");
 }
 

@@ -107,12 +107,14 @@ int decode_splits(int n_seq, int n_kv_head, int max_context, bool tensor_cores);
 void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* cache, const int32_t* tok_seq,
                        const int32_t* positions, const int32_t* block_table, int table_width, const Rows& out, int n_tokens, int n_seq,
                        const AttentionShape& a);
-void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* positions,
+// q_start: null in steps of single tokens; in a mixed step (tensor cores only) where each request's tokens start: its single tokens are served.
+void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,
                       const int32_t* block_table, int table_width, const Rows& out, float* partial, int* counters, int n_seq,
                       const AttentionShape& a, int n_splits);
+// singles_apart: requests that bring one token are left to decode_attention.
 void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                        const int32_t* n_past, const int32_t* block_table, int table_width, const Rows& out, int n_seq,
-                       int max_q_len, const AttentionShape& a);
+                       int max_q_len, bool singles_apart, const AttentionShape& a);
 
 // ---- row-wise pieces between the products: RMS norm in groups, token shift, xIELU, gated side input ----
 // out[r] = x[rows ? rows[r] : r] cut into `groups` equal parts, each over its own root mean square, times weight.

@@ -59,6 +59,9 @@ _SIGNATURES = {
     "lb_decode_attention_mma_capped": [_p, _l, _p, _i, _p, _p, _i, _p, _l, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _p, _p, _f, _f, _p],
     "lb_prefill_attention_capped": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _p],
     "lb_prefill_attention_tc_capped": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _p],
+    "lb_decode_attention_mma_mixed": [_p, _l, _p, _i, _p, _p, _p, _i, _p, _l, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _p, _p, _f, _f, _p],
+    "lb_prefill_attention_portions": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
+    "lb_prefill_attention_tc_portions": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
     "lb_paged_attention_f32_runs": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _f, _i, _p, _p],
     "lb_qkv_rotary_store_scaled": [_i, _p, _l, _i, _i, _i, _p, _p, _p, _l, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p, _i, _p, _p, _l, _p, _i, _f, _p],
     "lb_row_norm_gate": [_i, _p, _l, _p, _l, _p, _p, _l, _i, _i, _i, _f, _p],
@@ -430,8 +433,10 @@ def decode_attention(q: torch.Tensor, cache: torch.Tensor, positions: torch.Tens
                      out: torch.Tensor, partial: Optional[torch.Tensor], counters: Optional[torch.Tensor], n_seq: int,
                      n_head: int, n_kv_head: int, head_dim: int, page_size: int, scale: float, window: int,
                      n_splits: int, tensor_cores: Optional[bool] = None, distance: Optional[torch.Tensor] = None,
-                     sink: Optional[torch.Tensor] = None, soft_cap: float = 0.0, score_bound: float = 0.0) -> torch.Tensor:
-    """Attention of one new token per request over its pages (bfloat16), keys split `n_splits` ways.
+                     sink: Optional[torch.Tensor] = None, soft_cap: float = 0.0, score_bound: float = 0.0,
+                     q_start: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Attention of one new token per request over its pages (bfloat16), keys split `n_splits` ways.  `q_start` (n_seq + 1 numbers, tensor cores
+    only): where each request's tokens start in a mixed step, of which the requests of one token are served.
     `tensor_cores`: None picks the tensor-core kernel where it takes the shape, else the scalar one.  `distance`: as for
     paged_attention_generic.  `score_bound`: the largest |score| before the cap that can occur, 0 when unknown."""
     if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
@@ -444,8 +449,8 @@ def decode_attention(q: torch.Tensor, cache: torch.Tensor, positions: torch.Tens
             raise invalid_argument("decode attention: scratch buffers are missing or too small")
     if tensor_cores is None:
         tensor_cores = decode_attention_kernels(n_head, n_kv_head, head_dim, page_size)[1]
-    cache_args = (_dev(cache, "cache"), cache.shape[0]) if tensor_cores else (_dev(cache, "cache"),)
-    fn = lib().lb_decode_attention_mma_capped if tensor_cores else lib().lb_decode_attention_capped
+    cache_args = (_dev(cache, "cache"), cache.shape[0], _opt(q_start, "q_start", torch.int32)) if tensor_cores else (_dev(cache, "cache"),)
+    fn = lib().lb_decode_attention_mma_mixed if tensor_cores else lib().lb_decode_attention_capped
     check(fn(
         _dev(q, "q"), q.stride(0), *cache_args, _dev(positions, "positions", torch.int32),
         _dev(block_table, "block_table", torch.int32), block_table.stride(0), _dev(out, "out"), out.stride(0),
@@ -477,8 +482,8 @@ def prefill_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tenso
                       block_table: torch.Tensor, out: torch.Tensor, n_seq: int, max_q_len: int, n_head: int,
                       n_kv_head: int, head_dim: int, page_size: int, scale: float, window: int = 0,
                       tcgen05: Optional[bool] = None, distance: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None,
-                      soft_cap: float = 0.0, score_bound: float = 0.0) -> torch.Tensor:
-    """Attention of the step's prompt portions over their pages (bfloat16, tensor cores).  `tcgen05`: None picks
+                      soft_cap: float = 0.0, score_bound: float = 0.0, min_len: int = 1) -> torch.Tensor:
+    """Attention of the step's prompt portions of at least `min_len` tokens over their pages (bfloat16, tensor cores).  `tcgen05`: None picks
     the tcgen05 kernel where it takes the shape and the rows are 16-byte aligned, else the mma.sync one.  `distance`: as for
     paged_attention_generic; `score_bound`: as for decode_attention."""
     if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
@@ -494,19 +499,19 @@ def prefill_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tenso
                    and out.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
                    and blocks <= 4 * _sm_count(q.device))
     if tcgen05:
-        check(lib().lb_prefill_attention_tc_capped(
+        check(lib().lb_prefill_attention_tc_portions(
             _dev(q, "q"), q.stride(0), q.shape[0], _dev(cache, "cache"), cache.shape[0],
             _dev(q_start, "q_start", torch.int32), _dev(n_past, "n_past", torch.int32),
             _dev(block_table, "block_table", torch.int32), block_table.stride(0), _dev(out, "out"), out.stride(0), n_seq,
             max_q_len, n_head, n_kv_head, head_dim, page_size, float(scale), int(window), _distance(distance, n_head), _sink(sink, n_head), float(soft_cap), float(score_bound),
-            stream_ptr()), "prefill_attention_tc")
+            min_len, stream_ptr()), "prefill_attention_tc")
         return out
-    check(lib().lb_prefill_attention_capped(
+    check(lib().lb_prefill_attention_portions(
         _dev(q, "q"), q.stride(0), _dev(cache, "cache"), _dev(q_start, "q_start", torch.int32),
         _dev(n_past, "n_past", torch.int32), _dev(block_table, "block_table", torch.int32), block_table.stride(0),
         _dev(out, "out"), out.stride(0), n_seq, max_q_len, n_head, n_kv_head, head_dim, page_size, float(scale),
-        int(window), _distance(distance, n_head), _sink(sink, n_head), float(soft_cap), float(score_bound), stream_ptr()),
-        "prefill_attention")
+        int(window), _distance(distance, n_head), _sink(sink, n_head), float(soft_cap), float(score_bound), min_len,
+        stream_ptr()), "prefill_attention")
     return out
 
 
