@@ -62,6 +62,8 @@ _SIGNATURES = {
     "lb_decode_attention_mma_mixed": [_p, _l, _p, _i, _p, _p, _p, _i, _p, _l, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _p, _p, _f, _f, _p],
     "lb_prefill_attention_portions": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
     "lb_prefill_attention_tc_portions": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
+    "lb_gemm_pair": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
+    "lb_gemm_pair_tile": [_i, _i, _i, _i, _p],
     "lb_paged_attention_f32_runs": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _f, _i, _p, _p],
     "lb_qkv_rotary_store_scaled": [_i, _p, _l, _i, _i, _i, _p, _p, _p, _l, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p, _i, _p, _p, _l, _p, _i, _f, _p],
     "lb_row_norm_gate": [_i, _p, _l, _p, _l, _p, _p, _l, _i, _i, _i, _f, _p],
@@ -288,6 +290,20 @@ def gemm_rows_normed(x: torch.Tensor, gain: Optional[torch.Tensor], offset: Opti
                                     residual.stride(0) if residual is not None else 0, _dev(out, "out"), out.stride(0), m, n, k,
                                     ACTIVATIONS[activation], cache, slots, q_dim, n_kv_head, head_dim, page_size, stream_ptr()),
           "gemm_rows_normed")
+    return out
+
+
+def gemm_pair(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, m: int, activation: str = "none",
+              residual: Optional[torch.Tensor] = None, feature_tile: int = 256, kv: Optional[tuple] = None) -> torch.Tensor:
+    """out[:m] = act(a[:m] @ w.T + bias) + residual with tiles of 256 tokens that two SMs make together.  `kv` as for gemm_persistent."""
+    n, k = w.shape
+    if a.shape[1] != k or out.stride(1) != 1 or out.shape[1] != n or not tcgen05_accepts(a, w):
+        raise invalid_argument(f"gemm: shapes do not fit: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    cache, slots, q_dim, n_kv_head, head_dim, page_size = _kv_args(kv)
+    check(lib().lb_gemm_pair(_code(out.dtype, "out"), _dev(a, "a"), a.stride(0), _dev(w, "w"), w.stride(0), _opt(bias, "bias", torch.float32),
+                             _opt(residual, "residual", torch.float32), residual.stride(0) if residual is not None else 0, _dev(out, "out"), out.stride(0),
+                             m, n, k, ACTIVATIONS[activation], feature_tile, cache, slots, q_dim, n_kv_head, head_dim, max(0, page_size.bit_length() - 1), stream_ptr()),
+          "gemm_pair")
     return out
 
 
