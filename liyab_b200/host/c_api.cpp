@@ -37,7 +37,6 @@ struct lb_replayer {
     std::unique_ptr<Replayer> replayer;
     lb_cache cache_handle;
     std::unique_ptr<Event> t0, t1;
-    std::vector<float> host_logits;
 };
 
 namespace {
@@ -707,14 +706,30 @@ int32_t lb_replayer_step(lb_replayer* r, size_t n_entries, const int64_t* reques
             t_at += static_cast<size_t>(n_tokens[i]);
             w_at += static_cast<size_t>(n_want[i]);
         }
-        const StepOutput out = r->replayer->step(entries, logits != nullptr ? &r->host_logits : nullptr);
+        const StepOutput out = r->replayer->step(entries, logits, logits_capacity);
         if (n_rows != nullptr) *n_rows = static_cast<int32_t>(out.rows.size());
-        if (logits != nullptr) {
-            if (logits_capacity < r->host_logits.size())
-                throw invalid_argument("the step's logits need {} floats, the buffer holds {}", r->host_logits.size(), logits_capacity);
-            std::memcpy(logits, r->host_logits.data(), r->host_logits.size() * 4);
-        }
+        const size_t floats = out.rows.size() * static_cast<size_t>(r->replayer->loaded->model->spec.vocab_size());
+        if (logits != nullptr && logits_capacity < floats)
+            throw invalid_argument("the step's logits need {} floats, the buffer holds {}", floats, logits_capacity);
     });
+}
+
+int32_t lb_host_buffer_create(int32_t device, size_t bytes, void** out) {
+    return guarded([&] {
+        need(out, "out");
+        *out = nullptr;
+        LIYAB_CUDA(cudaSetDevice(device));
+        void* p = nullptr;
+        if (const cudaError_t err = cudaMallocHost(&p, bytes); err != cudaSuccess) {
+            cudaGetLastError();          // the caller may go on without the buffer: no launch is to find this error
+            cuda_check(err, "cudaMallocHost");
+        }
+        *out = p;
+    });
+}
+
+void lb_host_buffer_destroy(void* buffer) {
+    if (buffer != nullptr) cudaFreeHost(buffer);
 }
 
 int32_t lb_replayer_set(lb_replayer* r, const char* option, int32_t value) {

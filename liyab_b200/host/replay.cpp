@@ -19,16 +19,14 @@ Replayer::Replayer(const std::string& model_dir, const std::string& dtype, int64
     stepper = std::make_unique<Stepper>(model, *cache, so);
 }
 
-StepOutput Replayer::step(const std::vector<StepEntry>& entries, std::vector<float>* host) {
+StepOutput Replayer::step(const std::vector<StepEntry>& entries, float* host, size_t capacity) {
     LIYAB_CUDA(cudaSetDevice(loaded->runtime.device));
     StepOutput out = stepper->step(entries);
     const size_t rows = out.rows.size(), vocab = static_cast<size_t>(loaded->model->spec.vocab_size());
-    if (host != nullptr) {
-        host->resize(rows * vocab);
-        if (rows > 0)
-            LIYAB_CUDA(cudaMemcpy2DAsync(host->data(), vocab * 4, out.logits.data, static_cast<size_t>(out.logits.stride) * 4, vocab * 4, rows,
-                                         cudaMemcpyDeviceToHost, loaded->runtime.stream));
-    }
+    const bool fits = rows * vocab <= capacity;
+    if (host != nullptr && fits && rows > 0)
+        LIYAB_CUDA(cudaMemcpy2DAsync(host, vocab * 4, out.logits.data, static_cast<size_t>(out.logits.stride) * 4, vocab * 4, rows,
+                                     cudaMemcpyDeviceToHost, loaded->runtime.stream));
     LIYAB_CUDA(cudaStreamSynchronize(loaded->runtime.stream));
     return out;
 }
@@ -78,7 +76,10 @@ int replay_stream(const std::string& model_dir, const std::string& dtype, const 
                 }
             }
             if (!entries.empty()) {
-                const StepOutput out = replayer.step(entries, &logits);
+                size_t wanted = 0;
+                for (const auto& e : entries) wanted += static_cast<size_t>(e.n_want);
+                logits.resize(wanted * static_cast<size_t>(replayer.loaded->model->spec.vocab_size()));
+                const StepOutput out = replayer.step(entries, logits.data(), logits.size());
                 if (!out.rows.empty()) {
                     const std::string tmp = out_dir + "/." + step_name + ".f32.tmp", path = out_dir + "/" + step_name + ".f32";
                     std::FILE* f = std::fopen(tmp.c_str(), "wb");

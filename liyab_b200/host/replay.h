@@ -41,7 +41,8 @@ public:
     std::unique_ptr<Stepper> stepper;
 
     // Runs one step; the logits at the wanted places are copied to `host` (resized to rows * vocab).
-    StepOutput step(const std::vector<StepEntry>& entries, std::vector<float>* host);
+    // The wanted rows' logits go to `host` ([rows, vocab], room for `capacity` floats; null, or too little room: they stay on the device).
+    StepOutput step(const std::vector<StepEntry>& entries, float* host, size_t capacity);
 };
 
 // Reads steps from `in` until it ends; returns the process's exit code.

@@ -271,6 +271,10 @@ LB_API int32_t lb_replayer_describe(const lb_replayer* r, char* buffer, size_t s
 LB_API int32_t lb_replayer_step(lb_replayer* r, size_t n_entries, const int64_t* requests, const int32_t* n_tokens,
                                 const int32_t* tokens, const int32_t* n_want, const int32_t* want, float* logits,
                                 size_t logits_capacity, int32_t* n_rows);
+/* Host memory that the device copies to by itself (page-locked): a `logits` buffer made of it takes a step's rows at the link's rate, any
+ * other one at a fraction of it.  Making one costs as much as many steps: keep it. */
+LB_API int32_t lb_host_buffer_create(int32_t device, size_t bytes, void** out);
+LB_API void lb_host_buffer_destroy(void* buffer);
 /* Options at run time: "cuda_graphs" 0/1, "fused_decode" 0 (cannot be switched back on). */
 LB_API int32_t lb_replayer_set(lb_replayer* r, const char* option, int32_t value);
 /* {"steps", "graph_steps", "fused_steps", "eager_steps", "graphs_captured", "tokens_run", "kernel_launches"} */

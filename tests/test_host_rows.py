@@ -1,0 +1,96 @@
+"""The host memory that steps' logits arrive in: kept within its limit, given back by the arrays, whole after its owner is closed."""
+from __future__ import annotations
+
+import ctypes as C
+import gc
+import threading
+
+import numpy as np
+import pytest
+
+from liyab_b200.engine import _HostRows
+
+PIECE = 65536
+
+
+class FakeLib:
+    """Buffers of ordinary memory, counted; `refuse` stands for an allocation that fails."""
+
+    def __init__(self):
+        self.live, self.made, self.refuse = {}, 0, False
+
+    def lb_host_buffer_create(self, device, size, out):
+        if self.refuse:
+            return 8
+        memory = (C.c_char * size)()
+        self.live[C.addressof(memory)] = memory
+        self.made += 1
+        out._obj.value = C.addressof(memory)
+        return 0
+
+    def lb_host_buffer_destroy(self, address):
+        del self.live[address]
+
+
+@pytest.fixture
+def lib():
+    return FakeLib()
+
+
+def test_buffers_come_back_with_the_last_view(lib):
+    rows = _HostRows(limit=4 * PIECE, lib=lib)
+    a = rows.array(3, 100)
+    a[:] = np.arange(300).reshape(3, 100)
+    view = a[1:, ::2]
+    del a
+    b = rows.array(3, 100)
+    assert lib.made == 2 and b.ctypes.data not in (view.ctypes.data, view.base.ctypes.data)
+    b[:] = -1.0
+    assert (view == np.arange(300).reshape(3, 100)[1:, ::2]).all()
+    del view, b
+    gc.collect()
+    for _ in range(5):
+        c = rows.array(3, 100)
+        del c
+    assert lib.made == 2
+
+
+def test_limit_and_refusals_give_ordinary_arrays(lib):
+    rows = _HostRows(limit=2 * PIECE, lib=lib)
+    held = [rows.array(1, PIECE // 4) for _ in range(4)]
+    assert lib.made == 2 and all(a.shape == (1, PIECE // 4) and a.flags.writeable for a in held)
+    del held
+    big = rows.array(2, PIECE // 4)                  # two free buffers make room for one of twice their size
+    assert lib.made == 3 and len(lib.live) == 1
+    del big
+    lib.refuse = True
+    assert rows.array(1, 10).shape == (1, 10) and len(lib.live) == 1
+
+
+def test_arrays_outlive_their_owner(lib):
+    rows = _HostRows(limit=4 * PIECE, lib=lib)
+    a, b = rows.array(1, 10), rows.array(1, 10)
+    a[:] = 3.0
+    del b
+    rows.close()
+    assert len(lib.live) == 1 and (a == 3.0).all()
+    assert rows.array(1, 10).shape == (1, 10) and len(lib.live) == 1
+    del a
+    gc.collect()
+    assert not lib.live
+
+
+def test_threads_never_share_a_buffer(lib):
+    rows, wrong = _HostRows(limit=64 * PIECE, lib=lib), []
+
+    def work(k):
+        for i in range(200):
+            a = rows.array(1, 50)
+            a[:] = k
+            if (a != k).any():
+                wrong.append((k, i))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(8)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not wrong and len(lib.live) <= 9
