@@ -134,7 +134,7 @@ inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView
     if (ctx.runtime.dtype == DType::BF16 && kernels::prefill_supports(a)) {
         // Single tokens beside prompt portions have a launch of their own: a tile of 64 or 128 rows would be spent on each of them (XL, 12 such tokens
         // beside a portion of 453 on 300: 44 us a layer in one launch, 41 us in two, 5.84 -> 5.66 ms a step).
-        const bool apart = ctx.has_singles && kernels::decode_mma_supports(a);
+        const bool apart = ctx.singles_apart && kernels::decode_mma_supports(a);
         kernels::prefill_attention(ctx.runtime, q, T, cache, n_pages, ctx.q_start, ctx.n_past, view.block_table, view.table_width, att, S, ctx.max_q_len,
                                    apart, a);
         if (apart) decode(true, ctx.q_start);

@@ -147,7 +147,7 @@ struct StepContext {
     int max_q_len = 0;
     int max_kv_len = 0;
     bool decode_only = false;
-    bool has_singles = false;        // some requests of a step with prompt portions bring one token
+    bool singles_apart = false;      // a long portion beside requests of a few tokens: those of one token have a launch of their own
     int max_positions = 0;          // the longest sequence the engine serves (fixes split counts and table widths)
     const TapFn* tap_fn = nullptr;  // when set, parts' outputs are shown to it (tests)
     PhaseTimer* phases = nullptr;   // when set, phase boundaries are recorded

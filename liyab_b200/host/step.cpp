@@ -114,9 +114,7 @@ Stepper::ShapeKey Stepper::shape_key(const std::vector<StepEntry>& entries, cons
         longest = std::max(longest, q_len[i]);
     }
     const int S = static_cast<int>(entries.size());
-    // Steps with single tokens beside their prompt portions launch one kernel more in every attention.
-    const bool singles = T != S && std::any_of(q_len.begin(), q_len.end(), [](int64_t n) { return n == 1; });
-    return {S, T, R, T != S ? static_cast<int>((longest + 63) / 64 * 64) : 1, singles};
+    return {S, T, R, T != S ? static_cast<int>((longest + 63) / 64 * 64) : 1};
 }
 
 bool Stepper::worth_capturing(const std::vector<StepEntry>& entries, const std::vector<int64_t>& q_len) {
@@ -132,7 +130,7 @@ bool Stepper::worth_capturing(const std::vector<StepEntry>& entries, const std::
 Rows Stepper::graph_step(const std::vector<StepEntry>& entries, const std::vector<int>& rows, const std::vector<int64_t>& q_len,
                          const DeviceTokens* dt, Layout* layout) {
     // A graph fits every step with the same number of requests, tokens and wanted rows whose longest portion
-    // falls into the same bucket of 64 tokens, with or without single tokens beside portions; everything else about the step (tokens, positions, where portions
+    // falls into the same bucket of 64 tokens; everything else about the step (tokens, positions, where portions
     // start, block tables, slots) is data the graph reads from its own layout buffer.
     const ShapeKey key = shape_key(entries, q_len);
     const int bucket = std::get<3>(key);
@@ -310,7 +308,12 @@ void Stepper::lay_out(const std::vector<StepEntry>& entries, const std::vector<i
     ctx.max_q_len = max_q_len > 0 ? max_q_len : longest;
     ctx.max_kv_len = max_kv;
     ctx.decode_only = T == S;
-    ctx.has_singles = !ctx.decode_only && std::any_of(q_len.begin(), q_len.end(), [](int64_t n) { return n == 1; });
+    // Single tokens beside one long portion are served apart from it.  A captured step goes by what its replays have in common (requests, tokens, the
+    // bucket of the longest portion) and launches for single tokens that a replay may not have; any other step looks.  The launch costs 2 to
+    // 3 us an attention where it finds none: short portions, and few requests beside a long one, keep to one launch.
+    const int bucket = (longest + 63) / 64 * 64;
+    ctx.singles_apart = !ctx.decode_only && S >= 4 && bucket >= 256 && T - bucket <= 8 * (S - 1) &&
+                        (fixed != nullptr || std::any_of(q_len.begin(), q_len.end(), [](int64_t n) { return n == 1; }));
     ctx.max_positions = max_positions;
 }
 

@@ -86,7 +86,7 @@ public:
     uint64_t steps = 0, graph_steps = 0, fused_steps = 0, eager_steps = 0, tokens_run = 0, graphs_captured = 0;
 
 private:
-    using ShapeKey = std::tuple<int, int, int, int, bool>;  // requests, tokens, wanted rows, bucket of the longest portion, single tokens beside portions
+    using ShapeKey = std::tuple<int, int, int, int>;        // requests, tokens, wanted rows, bucket of the longest portion
     struct CapturedStep {
         DeviceBuffer layout;
         size_t layout_ints = 0;
