@@ -114,16 +114,15 @@ __device__ __forceinline__ void sts4(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// The activation inside the epilogue.  Results that are rounded to bfloat16 take tanh as 1 - 2 / (1 + exp(2u)) with
-// the fast exponential and division (relative error about 1e-6, far below bfloat16's rounding), a few
+// The activation inside the epilogue.  Results that are rounded to bfloat16 take x/2 (1 + tanh u) as x / (1 + exp(-2u)) with
+// the fast exponential and division (relative error about 1e-6, far below bfloat16's rounding), seven
 // instructions instead of dozens; float32 results take the library functions.
 template <int ACT, bool FAST>
 __device__ __forceinline__ float activate(float x, const lb_act_pair& p) {
     if constexpr (ACT == LB_ACT_GELU_TANH) {
         if constexpr (FAST) {
-            const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-            const float t = 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * u));
-            return 0.5f * x * (1.0f + t);
+            // x / (1 + exp(-2u)), 2u = x (1.5957... + 0.0713... x^2).
+            return __fdividef(x, 1.0f + __expf(x * fmaf(-0.07135481282553524f * x, x, -1.5957691216057308f)));
         } else {
             return lb_gelu_tanh(x);
         }
