@@ -342,11 +342,11 @@ int launch_by_k(const void* A, int64_t lda, const void* W, int64_t ldw, const fl
 // very 16 bytes that it will feed to its products and reads them back itself, so the ring needs no barrier, and it is kept full from
 // before the wait for the kernel before until the last chunk is asked for.  The activations of a chunk travel with its weights, or
 // (NORMED) are made here from the float32 rows as gemm_rows_kernel makes them.  Bound by the weights' way from memory:
-// 148 blocks with some 64 KB in flight each, no more than 113 KB of shared memory a block for up to 8 tokens, so that the next
+// 148 blocks with some 64 KB in flight each, some 100 to 136 KB of shared memory a block for up to 8 tokens, so that the next
 // launch's blocks fit beside it and ask for their weights early.
 // Measured (GPT-2 XL, 8 requests, contexts of 360 to 880): the step's 243 launches took 483 before; 2.38 -> 2.31 ms with its logits'
-// copy.  Alone with cold caches, 8 tokens: 1600 -> 6400 normed 9.9 us (before: norm 3.6, split product 9.2 and second half 4.1), 6400 -> 1600 7.5 us
-// (9.2 and 3.6), of which 4.9 us of the first are the rows' norm, which waits behind the weights in flight.
+// copy, 1.98 ms since the norm is short code.  Alone with cold caches, 8 tokens: 1600 -> 6400 normed 10 us (before: norm 3.6, split product 9.2 and
+// second half 4.1), 6400 -> 1600 7.5 us (9.2 and 3.6).
 constexpr int kStreamGroups = 8;       // the most feature groups of eight a block takes
 constexpr int kStreamMaxK = 8192;
 constexpr int kStreamNormedMaxK = 2048;
@@ -356,62 +356,75 @@ constexpr int stream_depth(int gb, bool normed, bool wide) {
     return d < 2 ? 2 : d > 12 ? 12 : d;
 }
 
-// The rows' norm with gains and offsets in shared memory (gain_s, offset_s), for K up to kStreamNormedMaxK; one warp a row.
-__device__ void stream_norm_rows(const RowNorm& n, int M, int K, __nv_bfloat16* act, int ld, int k_pad, int rows, const float* gain_s, const float* offset_s) {
+// Bytes between the rows that are normalised: room for a float32 row, and 64 bytes mod 128 for the bfloat16 one that takes its place.
+__host__ __device__ constexpr int stream_row_bytes(int K) {
+    const int whole = 4 * K, padded = 2 * ((K + kChunk - 1) / kChunk * kChunk), most = whole > padded ? whole : padded;
+    return (most - 64 + 127) / 128 * 128 + 64;
+}
+
+// The rows' norm with gains and offsets in shared memory (gain_s, offset_s), for K up to kStreamNormedMaxK; one warp a row.  A launch
+// runs this code once, among other kernels, so the code is kept short: a lane puts its pieces of the row into shared memory as they come and
+// walks them there in loops.  Unrolled over registers it was half a microsecond faster launched again and again by itself, and
+// slower in a step, where its instructions came from memory each time: GPT-2 XL, 8 requests, 2.08 -> 1.98 ms a step.
+__device__ void stream_norm_rows(const RowNorm& n, int M, int K, uint8_t* rows_s, int k_pad, int rows, const float* gain_s, const float* offset_s) {
     constexpr int kVecs = kStreamNormedMaxK / 128;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_vec = K / 4;
+    const int n_vec = K / 4, stride = stream_row_bytes(K);
     for (int r = warp; r < rows; r += kWarps) {
-        __nv_bfloat16* dst = act + r * ld;
+        float4* x_s = reinterpret_cast<float4*>(rows_s + (size_t)r * stride);
+        uint8_t* dst = rows_s + (size_t)r * stride;
         if (r >= M) {
-            for (int i = lane * 8; i < k_pad; i += 256) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
+            for (int i = lane * 16; i < 2 * k_pad; i += 512) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
             continue;
         }
-        const float* row = n.x + (size_t)r * n.ldx;
-        float4 v[kVecs];
-#pragma unroll
-        for (int j = 0; j < kVecs; ++j) {
-            const int i = lane + 32 * j;
-            v[j] = i < n_vec ? __ldcg(reinterpret_cast<const float4*>(row) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        const float4* row = reinterpret_cast<const float4*>(n.x + (size_t)r * n.ldx);
         float sum = 0.0f;
+        {
+            float4 v[kVecs];
 #pragma unroll
-        for (int j = 0; j < kVecs; ++j) sum += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+            for (int j = 0; j < kVecs; ++j) v[j] = lane + 32 * j < n_vec ? __ldcg(row + lane + 32 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < kVecs; ++j) {
+                if (lane + 32 * j < n_vec) x_s[lane + 32 * j] = v[j];
+                sum += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+            }
+        }
         const float mean = n.rms ? 0.0f : lb_warp_sum(sum) / (float)K;
         float ss = 0.0f;
-#pragma unroll
-        for (int j = 0; j < kVecs; ++j) {
-            if (lane + 32 * j < n_vec) {
-                const float d0 = v[j].x - mean, d1 = v[j].y - mean, d2 = v[j].z - mean, d3 = v[j].w - mean;
-                ss = fmaf(d0, d0, ss);
-                ss = fmaf(d1, d1, ss);
-                ss = fmaf(d2, d2, ss);
-                ss = fmaf(d3, d3, ss);
-            }
+#pragma unroll 4
+        for (int i = lane; i < n_vec; i += 32) {                         // the lane's own pieces
+            const float4 v = x_s[i];
+            const float d0 = v.x - mean, d1 = v.y - mean, d2 = v.z - mean, d3 = v.w - mean;
+            ss = fmaf(d0, d0, ss);
+            ss = fmaf(d1, d1, ss);
+            ss = fmaf(d2, d2, ss);
+            ss = fmaf(d3, d3, ss);
         }
         const float inv = 1.0f / sqrtf(lb_warp_sum(ss) / (float)K + n.eps);
-#pragma unroll
-        for (int j = 0; j < kVecs; ++j) {
-            const int i = lane + 32 * j;
-            if (i < n_vec) {
-                float4 g = make_float4(1.f, 1.f, 1.f, 1.f), o = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (n.gain != nullptr) {
-                    g = reinterpret_cast<const float4*>(gain_s)[i];
-                    g.x += n.gain_offset;
-                    g.y += n.gain_offset;
-                    g.z += n.gain_offset;
-                    g.w += n.gain_offset;
-                }
-                if (n.offset != nullptr) o = reinterpret_cast<const float4*>(offset_s)[i];
-                const __nv_bfloat162 lo = __floats2bfloat162_rn((v[j].x - mean) * inv * g.x + o.x, (v[j].y - mean) * inv * g.y + o.y);
-                const __nv_bfloat162 hi = __floats2bfloat162_rn((v[j].z - mean) * inv * g.z + o.z, (v[j].w - mean) * inv * g.w + o.w);
-                uint2 packed;
-                packed.x = *reinterpret_cast<const uint32_t*>(&lo);
-                packed.y = *reinterpret_cast<const uint32_t*>(&hi);
-                *reinterpret_cast<uint2*>(dst + 4 * i) = packed;
+#pragma unroll 2
+        for (int i0 = 0; i0 < n_vec; i0 += 32) {
+            const int i = i0 + lane;
+            const bool in = i < n_vec;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f), g = make_float4(1.f, 1.f, 1.f, 1.f), o = v;
+            if (in) v = x_s[i];
+            if (in && n.gain != nullptr) {
+                g = reinterpret_cast<const float4*>(gain_s)[i];
+                g.x += n.gain_offset;
+                g.y += n.gain_offset;
+                g.z += n.gain_offset;
+                g.w += n.gain_offset;
             }
+            if (in && n.offset != nullptr) o = reinterpret_cast<const float4*>(offset_s)[i];
+            const __nv_bfloat162 lo = __floats2bfloat162_rn((v.x - mean) * inv * g.x + o.x, (v.y - mean) * inv * g.y + o.y);
+            const __nv_bfloat162 hi = __floats2bfloat162_rn((v.z - mean) * inv * g.z + o.z, (v.w - mean) * inv * g.w + o.w);
+            uint2 packed;
+            packed.x = *reinterpret_cast<const uint32_t*>(&lo);
+            packed.y = *reinterpret_cast<const uint32_t*>(&hi);
+            __syncwarp();                                                // all have read: the 256 bytes of these 32 pieces lie over pieces read by now
+            if (in) *reinterpret_cast<uint2*>(dst + 8 * i) = packed;
         }
-        for (int i = K + lane; i < k_pad; i += 32) dst[i] = __float2bfloat16_rn(0.0f);
+        __syncwarp();
+        for (int i = 2 * K + 2 * lane; i < 2 * k_pad; i += 64) *reinterpret_cast<uint16_t*>(dst + i) = 0;
     }
 }
 
@@ -427,7 +440,7 @@ gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_
     static_assert((size_t)kWarps * GB * ROWS * 8 * sizeof(float) <= (size_t)DEPTH * (GB + APIECES) * kThreads * 16, "the sums fit the ring");
     float* gain_s = reinterpret_cast<float*>(ring + DEPTH * (GB + APIECES) * kThreads);     // NORMED: gains and offsets, then the rows
     float* offset_s = gain_s + K;
-    const int ld = (K + kChunk - 1) / kChunk * kChunk + 32;                  // 64 bytes mod 128
+    const int ld = stream_row_bytes(K) / 2;
     __nv_bfloat16* act_s = reinterpret_cast<__nv_bfloat16*>(offset_s + K);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int n_groups = (N + 7) / 8, n_chunks = (K + kChunk - 1) / kChunk;
@@ -475,7 +488,7 @@ gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_
     lb_dependents_may_launch();
     if constexpr (NORMED) {
         __syncthreads();                                                     // every thread's gains and offsets
-        stream_norm_rows(norm, M, K, act_s, ld, n_chunks * kChunk, ROWS, gain_s, offset_s);
+        stream_norm_rows(norm, M, K, reinterpret_cast<uint8_t*>(act_s), n_chunks * kChunk, ROWS, gain_s, offset_s);
         __syncthreads();
     } else {
 #pragma unroll
@@ -552,7 +565,7 @@ template <int GB, bool NORMED, bool WIDE, typename TO>
 int launch_stream(const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out, int64_t ldo,
                   int M, int N, int K, int act, KvScatter kv, RowNorm norm, int grid, cudaStream_t s) {
     size_t smem = (size_t)stream_depth(GB, NORMED, WIDE) * (GB + (NORMED ? 0 : WIDE ? 2 : 1)) * kThreads * 16;
-    if (NORMED) smem += (size_t)2 * K * sizeof(float) + (size_t)(WIDE ? 16 : 8) * ((K + kChunk - 1) / kChunk * kChunk + 32) * sizeof(__nv_bfloat16);
+    if (NORMED) smem += (size_t)2 * K * sizeof(float) + (size_t)(WIDE ? 16 : 8) * stream_row_bytes(K);
     static size_t configured = 0;
     if (smem > configured) {
         LB_CHECK_CUDA(cudaFuncSetAttribute(gemm_stream_kernel<GB, NORMED, WIDE, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
