@@ -37,6 +37,22 @@ def test_tiled_products(dev, dtypes, M, N, K):
         assert torch.equal(part, out[lo:hi])
 
 
+@pytest.mark.parametrize("M", [9, 13, 16])
+@pytest.mark.parametrize("N,K", [(1, 4), (70, 68), (17, 4160), (2367, 768), (2368, 768), (2377, 3072), (2370, 6400)])
+def test_products_of_nine_to_sixteen_rows(dev, M, N, K):
+    """Sixteen features a block or eight, one chunk a group or several, remainders: the bits of eight rows and one, which another kernel multiplies."""
+    from liyab_b200 import ops
+    a, w, bias, res = _rand((M, K + 4), 65, dev)[:, :K], _rand((N, K), 66, dev), _rand((N,), 67, dev), _rand((M, N), 68, dev)
+    out = res.clone()
+    ops.gemm_ffma(a, w, bias, out, M, "none", residual=out)
+    ref = a.double() @ w.double().t() + bias.double() + res.double()
+    assert ((out.double() - ref).abs() <= EPS * (64 + 32 + K / 2048 + 3) * (a.double().abs() @ w.double().abs().t() + bias.double().abs() + res.double().abs())).all()
+    for lo, hi in ((0, 8), (8, M), (M - 1, M)):
+        part = res[lo:hi].clone()
+        ops.gemm_ffma(a[lo:hi], w, bias, part, hi - lo, "none", residual=part)
+        assert torch.equal(part, out[lo:hi])
+
+
 @pytest.mark.parametrize("M,N,K,pad", [(40, 70, 128, 1), (40, 70, 130, 2), (70, 64, 68, 4)])
 def test_tiled_products_of_strided_rows(dev, M, N, K, pad):
     """Rows that lie K + pad apart, so that they are aligned to whole pieces of four or not."""
