@@ -69,7 +69,7 @@ int lb_gemm_tcgen05_splits(int M, int K, int n_splits);
 int lb_gemm_tcgen05_kv(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, void* out,
                        int64_t ldo, int M, int N, int K, float* partial, int n_splits, void* kv_cache,
                        const int32_t* slot_mapping, int q_dim, int n_kv_head, int head_dim, int page_size, void* stream);
-/* lb_gemm_rows for up to 16 tokens and K up to 1024 with the activations made in the kernel: every block normalises the
+/* lb_gemm_rows for up to 16 tokens and K up to 2048 with the activations made in the kernel: every block normalises the
  * float32 rows x itself (LayerNorm with two-pass 32-bit statistics, eps, gain and offset or null), which saves the
  * LayerNorm's launch.  Everything else as lb_gemm_rows. */
 int lb_gemm_rows_normed_supports(const void* x, int64_t ldx, const void* W, int64_t ldw, int M, int N, int K);

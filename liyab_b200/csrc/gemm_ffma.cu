@@ -13,14 +13,15 @@
 //   32) consecutive chunks form a group whose chunk sums are added in ascending
 //   order; the (at most 32) group sums are added in ascending order.
 //
-// Two kernels follow that order.  The tiled one (any number of tokens) cuts the groups among
+// Three kernels follow that order.  The tiled one (any number of tokens) cuts the groups among
 // four slices of a block and adds their sums in order.  The one for up to 16 tokens (decoding)
 // is bound by reading the weights once: a block owns eight features and all of K,
 // each of its 32 (warp, slot) pairs owns one group of chunks for those features,
 // a thread fetches its 64 weights of a chunk as 16-byte pieces that are all in
 // flight together and multiplies them with the tokens' activations from the warp's
 // buffer in shared memory; the group sums meet in shared memory and are added in
-// order.
+// order.  The third takes 9 to 16 tokens in float32: the weights come into shared
+// memory by whole rows of a chunk as well.
 //
 // Epilogue, in the reference's order (src/core/transformer.cpp:111-118, 4903-4912,
 // 5526-5532): + bias[n], activation, + residual[m, n].
