@@ -258,7 +258,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         lb_wait_for_predecessor();           // before anything this block stores, and before a cache page is written
         lb_dependents_may_launch();
         int it = 0;
-        uint32_t turn = 0;                                             // strips of this group so far: slot and parity
+        uint32_t turn = 0;                                             // strips that this group has stored so far: slot and parity
         for (int tile = pair; tile < total; tile += n_pairs, ++it) {
             const int m0 = (tile % m_tiles) * 2 * kLaneTile + (int)rank * kLaneTile, n0 = (tile / m_tiles) * BN;
             const int buf = it & 1;
@@ -281,7 +281,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const uint32_t bias_u32 = smem_u32(bias_here);
             int slot = -1;                                             // where this thread's token lies in the cache
             if constexpr (KV) slot = m0 + row < M ? __ldg(kv.slot_mapping + m0 + row) : -1;
-            for (int sp = group; sp < n_strips; sp += 2, ++turn) {
+            for (int sp = group; sp < n_strips; sp += 2) {
                 const uint32_t strip = row_u32 + (turn & 1) * kStripBytes;
                 const uint32_t b = bias_u32 + (uint32_t)((sp >> 1) * kStripCols) * 4u;
                 // A strip of keys or values goes straight from the registers to its page, a strip of queries to `out`.
@@ -308,7 +308,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                     }
                     if (!mbar_wait(&c->res_full[group][turn & 1], (turn >> 1) & 1, abort_flag)) give_up(c, status, 4, quarter, rank);
                 } else if (!to_cache) {
-                    // The slot's last store but one has read it.
+                    // The slot's last store but one has read it: one group of stores a turn, and a strip that goes to the cache takes no turn (a turn
+                    // without a store would let the slot be written while that store still reads it).
                     if (elected) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                     named_barrier(2 + group, 128);
                 }
@@ -361,6 +362,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         if (m0 < M) tma_store_2d(&map_out, slots + (turn & 1) * kStripBytes, n0 + sp * kStripCols, m0);
                         bulk_commit();
                     }
+                    ++turn;
                 }
             }
             // The accumulator has been read: the products of the tile after next may overwrite it.

@@ -35,9 +35,13 @@ def test_products(dev, M, N, K, tile):
     assert ops.device_status() == 0
 
 
-def test_keys_and_values_go_to_their_pages(dev):
+@pytest.mark.parametrize("M,n_head,n_kv_head,K", [(300, 6, 2, 136), (2500, 25, 25, 136), (19300, 1, 1, 64), (37988, 3, 1, 72)])
+def test_keys_and_values_go_to_their_pages(dev, M, n_head, n_kv_head, K):
+    """One tile a pair of SMs; several, in other columns; several in the same column, with strips of queries and of keys in one tile: a strip that
+    goes to the cache must not let the next tile overwrite queries that are still on their way out."""
     from liyab_b200 import ops
-    M, n_head, n_kv_head, head_dim, page_size, n_pages, K = 300, 6, 2, 64, 16, 24, 136
+    head_dim, page_size = 64, 16
+    n_pages = -(-M // page_size) + 5
     q_dim, kv_dim = n_head * head_dim, n_kv_head * head_dim
     a, w = _rand((M, K), 94, dev, torch.bfloat16), _rand((q_dim + 2 * kv_dim, K), 95, dev, torch.bfloat16, 0.2)
     bias = _rand((q_dim + 2 * kv_dim,), 96, dev)
