@@ -77,6 +77,9 @@ int lb_gemm_rows_normed(int out_dtype, const float* x, int64_t ldx, const float*
                         int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out, int64_t ldo, int M, int N,
                         int K, int act, void* kv_cache, const int32_t* slot_mapping, int q_dim, int n_kv_head, int head_dim,
                         int page_size, void* stream);
+/* Which of the two kernels for few tokens takes a product of these sizes on n_sm SMs: 2 the one whose weights run through a ring in shared memory, 1 the
+ * one that holds them in registers, 0 none. */
+int lb_gemm_rows_kind(int M, int N, int K, int n_sm, int normed);
 /* The same product for 1 to 64 tokens in one launch on mma.sync (weights streamed once, no split of K over blocks,
  * no second kernel): lb_gemm_rows_supports tells whether it takes the product.  With kv_cache given (bfloat16 pages
  * of one layer), features from q_dim on are the keys and values of a fused projection and are also written to the

@@ -600,36 +600,42 @@ int stream(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw
                  : stream_by_groups<NORMED, false, __nv_bfloat16>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s);
 }
 
-// Whether the ring takes a product of up to 16 tokens: where one pass of gemm_rows_kernel's registers does not hold a block's weights.
-bool rows_streams(int M, int N, int K, int n_sm, bool normed) {
-    if (M > 16 || K > (normed ? kStreamNormedMaxK : kStreamMaxK)) return false;
-    const int n_groups = (N + 7) / 8, grid = n_groups < n_sm ? n_groups : n_sm, most = (n_groups + grid - 1) / grid;
-    if (most > kStreamGroups) return false;
-    const int pass = K <= 4 * kChunk ? 4 : K <= 8 * kChunk ? 2 : K <= 16 * kChunk ? 1 : 0;
-    return (normed && K > 4 * kChunk) || most > pass;
+int sm_count() {
+    static int n_sm = 0;
+    if (n_sm == 0) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n_sm = 148;
+    }
+    return n_sm;
 }
 
 }  // namespace
 
-// Whether the kernels take the product: 1 to 64 tokens, a reduction length of up to 4096 (up to 16 tokens: 8192), K and the row strides of
-// A and W multiples of 8, 16-byte aligned bases, and at most four passes over the feature groups of a block (the
-// head's vocabulary is left to the tcgen05 kernel, whose tiles suit it).
+// The kernel that takes a product of these sizes on n_sm SMs: 2 the ring (gemm_stream_kernel), 1 the one that holds a pass's weights in registers
+// (gemm_rows_kernel), 0 none.  Up to 16 tokens the ring takes over where one pass of registers does not hold a block's weights, while
+// a block has at most eight groups; the register kernel takes reductions of up to 4096 (normed: 1024) and at most four passes over the feature groups of
+// 148 blocks (the head's vocabulary is left to the tcgen05 kernel, whose tiles suit it).
+extern "C" int lb_gemm_rows_kind(int M, int N, int K, int n_sm, int normed) {
+    if (M <= 0 || N <= 0 || K <= 0 || n_sm <= 0 || M > (normed ? 16 : kMaxRows)) return 0;
+    const int n_groups = (N + 7) / 8, grid = n_groups < n_sm ? n_groups : n_sm, most = (n_groups + grid - 1) / grid;
+    const int pass = K <= 4 * kChunk ? 4 : K <= 8 * kChunk ? 2 : K <= 16 * kChunk ? 1 : 0;       // groups whose weights a pass's registers hold
+    const bool registers = normed ? pass == 4 : pass != 0;
+    if (M <= 16 && K <= (normed ? kStreamNormedMaxK : kStreamMaxK) && most <= kStreamGroups && (!registers || most > pass)) return 2;
+    return registers && n_groups <= 148 * 4 * pass ? 1 : 0;
+}
+
+// Whether the kernels take the product: sizes as above, K and the row strides of A and W multiples of 8, 16-byte aligned bases.
 extern "C" int lb_gemm_rows_supports(const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N, int K) {
-    if (M <= 0 || M > kMaxRows || N <= 0 || K <= 0) return 0;
     if (K % 8 != 0 || lda % 8 != 0 || ldw % 8 != 0 || ((uintptr_t)A & 15) != 0 || ((uintptr_t)W & 15) != 0) return 0;
-    if (M <= 16 && (N + 7) / 8 <= 148 * kStreamGroups && K <= kStreamMaxK) return 1;
-    if (K > kWRegs * kChunk) return 0;
-    const int ng = K <= 4 * kChunk ? 4 : K <= 8 * kChunk ? 2 : 1;
-    return (N + 7) / 8 <= 148 * 4 * ng;
+    return lb_gemm_rows_kind(M, N, K, sm_count(), 0) != 0;
 }
 
 // The same product for up to 16 tokens and a reduction length of up to 2048 with the activations made in the kernel:
 // LayerNorm (two-pass 32-bit statistics, eps, gain and offset or null) of the float32 rows x, normalised by every
 // block for itself.  lb_gemm_rows_normed_supports says whether the kernel takes the operands.
 extern "C" int lb_gemm_rows_normed_supports(const void* x, int64_t ldx, const void* W, int64_t ldw, int M, int N, int K) {
-    if (M <= 0 || M > 16 || N <= 0 || K <= 0 || K > kStreamNormedMaxK) return 0;
     if (K % 8 != 0 || ldx % 4 != 0 || ldw % 8 != 0 || ((uintptr_t)x & 15) != 0 || ((uintptr_t)W & 15) != 0) return 0;
-    return (N + 7) / 8 <= 148 * (K <= 4 * kChunk ? 4 * 4 : kStreamGroups);
+    return lb_gemm_rows_kind(M, N, K, sm_count(), 1) != 0;
 }
 
 extern "C" int lb_gemm_rows_normed(int out_dtype, const float* x, int64_t ldx, const float* gain, const float* offset, float eps,
@@ -651,12 +657,7 @@ extern "C" int lb_gemm_rows_normed_kind(int out_dtype, const float* x, int64_t l
         return lb_fail(LB_ERR_UNSUPPORTED, "gemm_rows_normed: takes 1 to 16 tokens, K up to 2048 and a multiple of 8, 16-byte aligned bases "
                        "(M=%d N=%d K=%d ldx=%lld ldw=%lld)", M, N, K, (long long)ldx, (long long)ldw);
     LB_CHECK_ARG(ldx >= K && ldw >= K && ldo >= N, "gemm_rows_normed: a row stride is shorter than the row");
-    static int n_sm = 0;
-    if (n_sm == 0) {
-        int dev = 0;
-        LB_CHECK_CUDA(cudaGetDevice(&dev));
-        LB_CHECK_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-    }
+    const int n_sm = sm_count();
     KvScatter kv{static_cast<__nv_bfloat16*>(kv_cache), slot_mapping, q_dim, n_kv_head, head_dim, page_size};
     if (kv_cache != nullptr)
         LB_CHECK_ARG(slot_mapping != nullptr && q_dim >= 0 && n_kv_head > 0 && head_dim > 0 && page_size > 0 &&
@@ -665,7 +666,7 @@ extern "C" int lb_gemm_rows_normed_kind(int out_dtype, const float* x, int64_t l
                      q_dim, n_kv_head, head_dim);
     const RowNorm norm{x, ldx, gain, offset, eps, rms, gain_offset};
     auto s = static_cast<cudaStream_t>(stream_handle);
-    if (rows_streams(M, N, K, n_sm, true)) return stream<true>(out_dtype, nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s);
+    if (lb_gemm_rows_kind(M, N, K, n_sm, 1) == 2) return stream<true>(out_dtype, nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s);
     if (out_dtype == LB_F32)
         return launch<1, 4, float, 2>(nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s, norm);
     return launch<1, 4, __nv_bfloat16, 2>(nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s, norm);
@@ -680,12 +681,7 @@ extern "C" int lb_gemm_rows(int out_dtype, const void* A, int64_t lda, const voi
         return lb_fail(LB_ERR_UNSUPPORTED, "gemm_rows: takes 1 to 64 tokens, K and row strides multiples of 8 and 16-byte aligned "
                        "bases (M=%d N=%d K=%d lda=%lld ldw=%lld)", M, N, K, (long long)lda, (long long)ldw);
     LB_CHECK_ARG(lda >= K && ldw >= K && ldo >= N, "gemm_rows: a row stride is shorter than the row");
-    static int n_sm = 0;
-    if (n_sm == 0) {
-        int dev = 0;
-        LB_CHECK_CUDA(cudaGetDevice(&dev));
-        LB_CHECK_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-    }
+    const int n_sm = sm_count();
     KvScatter kv{static_cast<__nv_bfloat16*>(kv_cache), slot_mapping, q_dim, n_kv_head, head_dim, page_size};
     if (kv_cache != nullptr)
         LB_CHECK_ARG(slot_mapping != nullptr && q_dim >= 0 && n_kv_head > 0 && head_dim > 0 && page_size > 0 &&
@@ -693,7 +689,7 @@ extern "C" int lb_gemm_rows(int out_dtype, const void* A, int64_t lda, const voi
                      "gemm_rows: the cache destination needs N = q_dim + 2 * n_kv_head * head_dim (N=%d q_dim=%d heads %d x %d)", N,
                      q_dim, n_kv_head, head_dim);
     auto s = static_cast<cudaStream_t>(stream_handle);
-    if (rows_streams(M, N, K, n_sm, false)) return stream<false>(out_dtype, A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, RowNorm{}, n_sm, s);
+    if (lb_gemm_rows_kind(M, N, K, n_sm, 0) == 2) return stream<false>(out_dtype, A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, RowNorm{}, n_sm, s);
     const int mt = (M + 15) / 16;
 #define LB_GO(MT)                                                                                                          \
     return out_dtype == LB_F32 ? launch_by_k<MT, float>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s)   \

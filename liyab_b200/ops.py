@@ -64,6 +64,7 @@ _SIGNATURES = {
     "lb_prefill_attention_tc_portions": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
     "lb_gemm_pair": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
     "lb_gemm_pair_tile": [_i, _i, _i, _i, _p],
+    "lb_gemm_rows_kind": [_i, _i, _i, _i, _i],
     "lb_paged_attention_f32_runs": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _f, _i, _p, _p],
     "lb_qkv_rotary_store_scaled": [_i, _p, _l, _i, _i, _i, _p, _p, _p, _l, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p, _i, _p, _p, _l, _p, _i, _f, _p],
     "lb_row_norm_gate": [_i, _p, _l, _p, _l, _p, _p, _l, _i, _i, _i, _f, _p],
@@ -258,6 +259,11 @@ def gemm_rows_supports(a: torch.Tensor, w: torch.Tensor, m: int) -> bool:
     if not tcgen05_accepts(a, w):
         return False
     return bool(lib().lb_gemm_rows_supports(_dev(a, "a"), a.stride(0), _dev(w, "w"), w.stride(0), m, w.shape[0], w.shape[1]))
+
+
+def gemm_rows_kind(m: int, n: int, k: int, n_sm: int = 148, normed: bool = False) -> int:
+    """Which kernel of the one-launch product takes these sizes on n_sm SMs: 2 weights through a ring in shared memory, 1 in registers, 0 none."""
+    return int(lib().lb_gemm_rows_kind(m, n, k, n_sm, int(normed)))
 
 
 def gemm_rows(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, m: int,

@@ -59,3 +59,28 @@ def test_cache_destination_of_the_projection():
     assert not f(bf16, 288, none, 0, 96, 1, 96, 16)                         # head size 96
     assert not f(bf16, 2304, none, 0, 768, 12, 64, 24)                      # a page that is no power of two
     assert not f(bf16, 2300, none, 0, 768, 12, 64, 16)                      # not [q | k | v]
+
+
+@pytest.mark.parametrize("n_sm", [148, 132, 100, 74, 20, 1])
+def test_products_of_few_tokens_go_to_a_kernel_that_holds_them(n_sm):
+    """On any number of SMs: the ring has at most eight groups of eight features a block and reductions of up to 8192 (normed rows: 2048); the kernel
+    that holds a pass's weights in registers reductions of up to 4096 (normed: 1024); everything else is refused."""
+    seen = set()
+    for normed in (False, True):
+        for M in (0, 1, 8, 9, 16, 17, 64, 65):
+            for N in (8, 40, 1184, 1192, 2368, 4736, 4744, 6400, 9472, 9480, 18944, 18952, 50257):
+                for K in (64, 1024, 1032, 1600, 2048, 2056, 4096, 4104, 8192, 8200):
+                    kind = ops.gemm_rows_kind(M, N, K, n_sm, normed)
+                    groups = -(-N // 8)
+                    if kind == 2:
+                        assert 1 <= M <= 16 and K <= (2048 if normed else 8192) and -(-groups // min(groups, n_sm)) <= 8
+                    elif kind == 1:
+                        assert 1 <= M <= (16 if normed else 64) and K <= (1024 if normed else 4096)
+                    else:
+                        assert kind == 0
+                    if 1 <= M <= (16 if normed else 64) and K <= (1024 if normed else 4096) and groups <= 148 * 4 * (4 if K <= 1024 else 2 if K <= 2048 else 1):
+                        assert kind != 0                                     # what registers hold is taken on any GPU
+                    seen.add(kind)
+    assert seen == {0, 1, 2}
+    assert (ops.gemm_rows_kind(8, 6400, 1600, n_sm, True) == 2) == (n_sm >= 100)      # 800 groups
+    assert ops.gemm_rows_kind(8, 6400, 1600, n_sm, False) == (2 if n_sm >= 100 else 1)
