@@ -108,12 +108,12 @@ int lb_gemm_persistent(int out_dtype, const void* A, int64_t lda, const void* W,
 int lb_gemm_persistent_kv_supports(int out_dtype, int N, int act, int has_residual, int q_dim, int n_kv_head, int head_dim,
                                    int page_size);
 /* The same product with tiles of 256 tokens x feature_tile (128, 192 or 256) features that two SMs make together.  Operands as lb_gemm_persistent
- * takes them; page_shift is log2 of the page size where kv_cache is given.  lb_gemm_pair_tile: the feature tile it would take and its estimated
+ * takes them, with the same checks.  lb_gemm_pair_tile: the feature tile it would take and its estimated
  * time on n_sm SMs; lb_gemm_persistent asks it and hands the product over where that estimate is the lower one. */
 int lb_gemm_pair_tile(int M, int N, int K, int n_sm, int* cost_ns);
 int lb_gemm_pair(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out,
                  int64_t ldo, int M, int N, int K, int act, int feature_tile, void* kv_cache, const int32_t* slot_mapping, int q_dim, int n_kv_head,
-                 int head_dim, int page_shift, void* stream);
+                 int head_dim, int page_size, void* stream);
 /* Reads and clears the status word that a bounded wait sets when it runs out
  * (0: none did).  Synchronises the device. */
 int lb_gemm_tcgen05_status(int* status);

@@ -421,13 +421,25 @@ extern "C" int lb_gemm_pair_tile(int M, int N, int K, int n_sm, int* cost_ns) {
     return best;
 }
 
-// Operands as lb_gemm_persistent takes them (its caller has checked them); feature_tile 128, 192 or 256.
+// Operands as lb_gemm_persistent takes them; feature_tile 128, 192 or 256.
 extern "C" int lb_gemm_pair(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr,
                             void* out, int64_t ldo, int M, int N, int K, int act, int feature_tile, void* kv_cache, const int32_t* slot_mapping, int q_dim,
-                            int n_kv_head, int head_dim, int page_shift, void* stream) {
+                            int n_kv_head, int head_dim, int page_size, void* stream) {
     LB_CHECK_ARG(M > 0 && N > 0 && K > 0 && (out_dtype == LB_BF16 || out_dtype == LB_F32), "gemm_pair: bad sizes or type M=%d N=%d K=%d", M, N, K);
     LB_CHECK_ARG(feature_tile == 128 || feature_tile == 192 || feature_tile == 256, "gemm_pair: feature tile %d", feature_tile);
-    LB_CHECK_ARG(residual == nullptr || out_dtype == LB_F32, "gemm_pair: a residual goes with a float32 output");
+    LB_CHECK_ARG(lda >= K && ldw >= K && ldo >= N, "gemm_pair: a row stride is shorter than the row");
+    if (lb_gemm_persistent_tile(out_dtype, A, lda, W, ldw, residual, ldr, out, ldo, M, N, K) == 0)
+        return lb_fail(LB_ERR_UNSUPPORTED, "gemm_pair: needs more than 64 tokens, K and all row strides on 16-byte boundaries, and float32 output where a residual "
+                       "is given (M=%d K=%d lda=%lld ldw=%lld ldo=%lld ldr=%lld)", M, K, (long long)lda, (long long)ldw, (long long)ldo, (long long)ldr);
+    KvTarget kv{static_cast<__nv_bfloat16*>(kv_cache), slot_mapping, q_dim, n_kv_head, head_dim, 0};
+    if (kv_cache != nullptr) {
+        if (!lb_gemm_persistent_kv_supports(out_dtype, N, act, residual != nullptr, q_dim, n_kv_head, head_dim, page_size))
+            return lb_fail(LB_ERR_UNSUPPORTED, "gemm_pair: keys and values go to the cache only from a bfloat16 product without activation or residual, with q_dim "
+                           "and head_dim multiples of 64 and a power-of-two page (N=%d q_dim=%d kv_heads=%d head_dim=%d page_size=%d)", N, q_dim, n_kv_head,
+                           head_dim, page_size);
+        LB_CHECK_ARG(slot_mapping != nullptr, "gemm_pair: the slot mapping is missing");
+        while ((1 << kv.page_shift) < page_size) ++kv.page_shift;
+    }
     const int elem = out_dtype == LB_F32 ? 4 : 2, bn = feature_tile, n_stages = stages_for(bn);
     CUtensorMap map_a, map_w, map_res, map_out;
     int rc = lb_tensor_map_2d(&map_a, A, 2, M, K, lda, kLaneTile);
@@ -444,7 +456,6 @@ extern "C" int lb_gemm_pair(int out_dtype, const void* A, int64_t lda, const voi
     LB_CHECK_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
     const long tiles = (long)((M + 2 * kLaneTile - 1) / (2 * kLaneTile)) * ((N + bn - 1) / bn);
     const int grid = 2 * (int)(tiles < n_sm / 2 ? tiles : n_sm / 2);
-    const KvTarget kv{static_cast<__nv_bfloat16*>(kv_cache), slot_mapping, q_dim, n_kv_head, head_dim, page_shift};
     const size_t smem = kSmemLimit;                  // a block has its SM, and all of its tensor memory, to itself
     auto s = static_cast<cudaStream_t>(stream);
 #define LB_GO(TO, ACT, RES, KV)                                                                                                                    \

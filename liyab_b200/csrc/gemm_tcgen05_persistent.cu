@@ -627,7 +627,7 @@ extern "C" int lb_gemm_persistent(int out_dtype, const void* A, int64_t lda, con
         const int bn_shared = lb_gemm_pair_tile(M, N, K, n_sm, &shared);
         if (8 * (long)shared < 7 * here)
             return lb_gemm_pair(out_dtype, A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, bn_shared, kv_cache, slot_mapping, q_dim, n_kv_head,
-                                head_dim, kv.page_shift, stream);
+                                head_dim, page_size, stream);
     }
     return launch_persistent(out_dtype, A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, bn_used, pair, kv, n_sm, stream);
 }

@@ -305,11 +305,11 @@ def gemm_pair(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     n, k = w.shape
     if a.shape[1] != k or out.stride(1) != 1 or out.shape[1] != n or not tcgen05_accepts(a, w):
         raise invalid_argument(f"gemm: shapes do not fit: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
-    cache, slots, q_dim, n_kv_head, head_dim, page_size = _kv_args(kv)
+    if residual is not None and (residual.shape[1] != n or residual.stride(1) != 1):
+        raise invalid_argument("gemm: residual has the wrong shape")
     check(lib().lb_gemm_pair(_code(out.dtype, "out"), _dev(a, "a"), a.stride(0), _dev(w, "w"), w.stride(0), _opt(bias, "bias", torch.float32),
                              _opt(residual, "residual", torch.float32), residual.stride(0) if residual is not None else 0, _dev(out, "out"), out.stride(0),
-                             m, n, k, ACTIVATIONS[activation], feature_tile, cache, slots, q_dim, n_kv_head, head_dim, max(0, page_size.bit_length() - 1), stream_ptr()),
-          "gemm_pair")
+                             m, n, k, ACTIVATIONS[activation], feature_tile, *_kv_args(kv), stream_ptr()), "gemm_pair")
     return out
 
 

@@ -84,3 +84,19 @@ def test_products_of_few_tokens_go_to_a_kernel_that_holds_them(n_sm):
     assert seen == {0, 1, 2}
     assert (ops.gemm_rows_kind(8, 6400, 1600, n_sm, True) == 2) == (n_sm >= 100)      # 800 groups
     assert ops.gemm_rows_kind(8, 6400, 1600, n_sm, False) == (2 if n_sm >= 100 else 1)
+
+
+@pytest.mark.parametrize("change", ["float32", "activation", "page", "q_dim", "head_dim", "slots", "rows", "stride", "alignment"])
+def test_shared_tiles_refuse_what_the_persistent_product_refuses(change):
+    """The product whose tiles two SMs make together, asked directly: refused before anything is launched (there is no memory behind these addresses)."""
+    f = ops.lib().lb_gemm_pair
+    at = 1 << 20
+    a = dict(out=ops.BF16, A=at, lda=768, M=300, N=2304, K=768, act=ops.ACTIVATIONS["none"], ldo=2304, cache=at, slots=at, q_dim=768, heads=12, dim=64, page=16)
+    a.update({"float32": dict(out=ops.F32), "activation": dict(act=ops.ACTIVATIONS["gelu_tanh"]), "page": dict(page=24), "q_dim": dict(q_dim=800, N=2336, ldo=2336),
+              "head_dim": dict(dim=32, heads=24), "slots": dict(slots=None), "rows": dict(M=64, cache=None), "stride": dict(ldo=2296, cache=None),
+              "alignment": dict(A=at + 2, cache=None)}[change])
+    rc = f(a["out"], a["A"], a["lda"], at, a["K"], None, None, 0, at, a["ldo"], a["M"], a["N"], a["K"], a["act"], 256, a["cache"], a["slots"], a["q_dim"],
+           a["heads"], a["dim"], a["page"], None)
+    with pytest.raises(Exception) as e:
+        ops.check(rc, "gemm_pair")
+    assert "gemm_pair" in str(e.value) and "CUDA" not in str(e.value), str(e.value)
