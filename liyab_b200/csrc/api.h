@@ -72,6 +72,8 @@ int lb_gemm_tcgen05_kv(int out_dtype, const void* A, int64_t lda, const void* W,
 /* lb_gemm_rows for up to 16 tokens and K up to 2048 with the activations made in the kernel: every block normalises the
  * float32 rows x itself (LayerNorm with two-pass 32-bit statistics, eps, gain and offset or null), which saves the
  * LayerNorm's launch.  Everything else as lb_gemm_rows. */
+/* lb_gemm_rows_normed_pays: whether that is faster than a LayerNorm launch and lb_gemm_rows. */
+int lb_gemm_rows_normed_pays(int M, int K);
 int lb_gemm_rows_normed_supports(const void* x, int64_t ldx, const void* W, int64_t ldw, int M, int N, int K);
 int lb_gemm_rows_normed(int out_dtype, const float* x, int64_t ldx, const float* gain, const float* offset, float eps, const void* W,
                         int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out, int64_t ldo, int M, int N,

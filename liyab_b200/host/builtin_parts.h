@@ -180,7 +180,7 @@ public:
     bool capturable() const override { return true; }
     std::optional<KvNeed> kv_need() const override { return KvNeed{shape.n_kv_head, shape.head_dim, shape.window}; }
 
-    // A step of up to 16 tokens in bfloat16 with rows of up to 2048 values: the projection normalises the rows inside
+    // A step of up to 16 tokens in bfloat16 with rows of up to 1024 values (up to 8 with 2048): the projection normalises the rows inside
     // its kernel (and fills the cache from its epilogue), so the LayerNorm before the mixer is not launched.
     bool forward_from(StepContext& ctx, const Rows& x_in, const NormRecipe& norm, const Rows& x, CacheUnit unit) override {
         const int T = ctx.n_tokens;

@@ -117,7 +117,7 @@ bool tcgen05_accepts(const Rows& a, const Tensor& w) {
 
 bool gemm_rows_normed_supports(const Runtime& rt, const Rows& x, const Tensor& w, int m) {
     return rt.dtype == DType::BF16 && x.dtype == DType::F32 && w.dtype == DType::BF16 && x.cols == w.dim(1) &&
-           lb_gemm_rows_normed_supports(x.data, x.stride, w.data, w.dim(1), m, static_cast<int>(w.dim(0)), static_cast<int>(w.dim(1))) != 0;
+           lb_gemm_rows_normed_pays(m, static_cast<int>(w.dim(1))) != 0 && lb_gemm_rows_normed_supports(x.data, x.stride, w.data, w.dim(1), m, static_cast<int>(w.dim(0)), static_cast<int>(w.dim(1))) != 0;
 }
 
 void gemm_rows_normed(cudaStream_t s, const Rows& x, const float* gain, const float* offset, float eps, const Tensor& w, const float* bias,

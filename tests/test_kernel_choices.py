@@ -100,3 +100,11 @@ def test_shared_tiles_refuse_what_the_persistent_product_refuses(change):
     with pytest.raises(Exception) as e:
         ops.check(rc, "gemm_pair")
     assert "gemm_pair" in str(e.value) and "CUDA" not in str(e.value), str(e.value)
+
+
+def test_long_rows_of_many_tokens_are_normalised_by_a_launch_of_their_own():
+    """Up to 16 tokens the projection normalises rows of up to 1024 values itself, longer ones (as GPT-2 XL's 1600) up to 8 tokens: with more, every block
+    would spend more time on them than the launch takes."""
+    pays = ops.lib().lb_gemm_rows_normed_pays
+    assert all(pays(m, 768) and pays(m, 1024) for m in (1, 8, 9, 16))
+    assert all(pays(m, 1600) for m in (1, 8)) and not any(pays(m, k) for m in (9, 12, 16) for k in (1032, 1600, 2048))
