@@ -615,13 +615,22 @@ int sm_count() {
 // (gemm_rows_kernel), 0 none.  Up to 16 tokens the ring takes over where one pass of registers does not hold a block's weights, while
 // a block has at most eight groups; the register kernel takes reductions of up to 4096 (normed: 1024) and at most four passes over the feature groups of
 // 148 blocks (the head's vocabulary is left to the tcgen05 kernel, whose tiles suit it).
+// Where either could take 9 to 16 tokens with K up to 1024, the ring's two pieces of activations (or its norm, which walks shared memory) leave less
+// to gain.  Measured with cold weights, registers / ring in us: 12 tokens, normed, 4744 x 512 6.9 / 6.6, 9472 x 512 7.9 / 8.0, 4744 x 1024 8.1 / 9.1, 9472 x
+// 1024 9.7 / 11.3; not normed, 9472 x 768 7.3 / 6.6, 6400 x 1024 7.0 / 5.9, 8192 x 1024 7.8 / 7.8.
 extern "C" int lb_gemm_rows_kind(int M, int N, int K, int n_sm, int normed) {
     if (M <= 0 || N <= 0 || K <= 0 || n_sm <= 0 || M > (normed ? 16 : kMaxRows)) return 0;
     const int n_groups = (N + 7) / 8, grid = n_groups < n_sm ? n_groups : n_sm, most = (n_groups + grid - 1) / grid;
     const int pass = K <= 4 * kChunk ? 4 : K <= 8 * kChunk ? 2 : K <= 16 * kChunk ? 1 : 0;       // groups whose weights a pass's registers hold
-    const bool registers = normed ? pass == 4 : pass != 0;
-    if (M <= 16 && K <= (normed ? kStreamNormedMaxK : kStreamMaxK) && most <= kStreamGroups && (!registers || most > pass)) return 2;
-    return registers && n_groups <= 148 * 4 * pass ? 1 : 0;
+    const bool registers = (normed ? pass == 4 : pass != 0) && n_groups <= 148 * 4 * pass;
+    const bool ring = M <= 16 && K <= (normed ? kStreamNormedMaxK : kStreamMaxK) && most <= kStreamGroups;
+    if (!registers) return ring ? 2 : 0;
+    bool faster = most > pass;
+    if (M > 8 && K <= 4 * kChunk) {
+        const bool few = most <= 6;
+        faster = faster && (normed ? K <= kChunk || (K <= 2 * kChunk && few) : K <= 3 * kChunk + kChunk / 2 || few);
+    }
+    return ring && faster ? 2 : 1;
 }
 
 // Whether the kernels take the product: sizes as above, K and the row strides of A and W multiples of 8, 16-byte aligned bases.

@@ -108,3 +108,13 @@ def test_long_rows_of_many_tokens_are_normalised_by_a_launch_of_their_own():
     pays = ops.lib().lb_gemm_rows_normed_pays
     assert all(pays(m, 768) and pays(m, 1024) for m in (1, 8, 9, 16))
     assert all(pays(m, 1600) for m in (1, 8)) and not any(pays(m, k) for m in (9, 12, 16) for k in (1032, 1600, 2048))
+
+
+def test_nine_to_sixteen_tokens_keep_to_registers_where_the_ring_is_slower():
+    kind = ops.gemm_rows_kind
+    for m in (9, 12, 16):
+        assert [kind(m, 4744, k, normed=True) for k in (256, 512, 520, 768, 1024)] == [2, 2, 1, 1, 1]
+        assert [kind(m, 9472, k, normed=True) for k in (256, 512, 768, 1024)] == [2, 1, 1, 1]
+        assert [kind(m, 9472, k) for k in (512, 896, 904, 1024, 1032)] == [2, 2, 1, 1, 2]
+        assert [kind(m, 6400, k) for k in (512, 1024, 1600)] == [2, 2, 2]
+    assert [kind(8, 9472, k, normed=normed) for k in (512, 1024) for normed in (False, True)] == [2] * 4
