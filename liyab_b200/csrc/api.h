@@ -46,6 +46,8 @@ int lb_kv_append(int dtype, const void* k, const void* v, int64_t row_stride, co
 int lb_gemm_ffma(int in_dtype, int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias,
                  const float* residual, int64_t ldr, void* out, int64_t ldo, int M, int N, int K, int act,
                  void* stream);
+/* Which of its kernels takes a float32 product of 9 to 16 rows: features a block (16 or 8) of the one whose weights come by whole rows, 0 the other one. */
+int lb_gemm_ffma_row_features(int M, int N, int K);
 
 /* The same product for bfloat16 operands on the tcgen05 tensor cores (TMA-fed,
  * accumulator in tensor memory).  Needs K, lda and ldw to be multiples of 8 and

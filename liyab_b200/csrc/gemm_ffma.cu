@@ -20,8 +20,8 @@
 // a thread fetches its 64 weights of a chunk as 16-byte pieces that are all in
 // flight together and multiplies them with the tokens' activations from the warp's
 // buffer in shared memory; the group sums meet in shared memory and are added in
-// order.  The third takes 9 to 16 tokens in float32: the weights come into shared
-// memory by whole rows of a chunk as well.
+// order.  The third takes some products of 9 to 16 tokens in float32: the weights come into
+// shared memory by whole rows of a chunk as well.
 //
 // Epilogue, in the reference's order (src/core/transformer.cpp:111-118, 4903-4912,
 // 5526-5532): + bias[n], activation, + residual[m, n].
@@ -416,7 +416,8 @@ gemm_ffma_skinny_kernel(const TI* __restrict__ A, int64_t lda, const TI* __restr
 // The same for 9 to 16 tokens in float32, with the weights brought into shared memory by whole rows of a chunk: sixteen lanes copy a chunk's 256 bytes, where the
 // kernel above has every lane read 16 bytes of a chunk of its own (32 lines an instruction) and hold all sixteen pieces of it beside its sixteen sums (214
 // registers: nine warps an SM).  A thread has FPT features, eight apart, so that a piece of the activations that it reads serves FPT times four products.
-// Sums as above, in their order.  GPT-2 small, a decode step of 12 requests: 910 -> 791 us; of 16: 946 -> 858 us.
+// Sums as above, in their order.  Which products take it: lb_gemm_ffma_row_features (all of them have one chunk a group; without the loop over chunks the
+// compiler keeps 72 registers instead of 214, and the kernel is up to a tenth slower).  GPT-2 small, a decode step of 12 requests: 910 -> 791 us; of 16: 946 -> 858 us.
 constexpr int kRowPitch = kChunk + 4;          // floats between the chunks of neighbouring features: eight lanes' pieces fall into 32 banks
 
 constexpr size_t skinny_rows_smem(int warps, int fpt) {
@@ -545,12 +546,11 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
         const int n_chunks = (K + kChunk - 1) / kChunk, per_group = chunks_per_group(K);
         const int n_groups = (n_chunks + per_group - 1) / per_group, warps = (n_groups + 3) / 4;
         if constexpr (sizeof(TI) == 4) {
-            // Sixteen features a block where that fills the GPU and the weights of a chunk of every group fit; eight otherwise.  (Up to eight tokens the
-            // kernel below is the faster one, 615 against 632 us a step of 8 requests: it is bound by latency, and its weights need no barrier.)
-            if (M > 8)
-                return N >= 16 * 148 && skinny_rows_smem(warps, 2) <= 227 * 1024
-                           ? launch_skinny_rows<2>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, warps, s)
-                           : launch_skinny_rows<1>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, warps, s);
+            if (M > 8) {
+                const int features = lb_gemm_ffma_row_features(M, N, K);
+                if (features == 16) return launch_skinny_rows<2>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, warps, s);
+                if (features == 8) return launch_skinny_rows<1>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, warps, s);
+            }
         }
         const dim3 grid((N + kSkinnyFeatures - 1) / kSkinnyFeatures);
         if (M <= 8) {
@@ -563,7 +563,7 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
             }
             LB_CHECK_CUDA(lb_launch_overlapped(gemm_ffma_skinny_kernel<TI, TO, 8>, dim3(grid), dim3(warps * 32), smem, s, (const TI*)A, lda, (const TI*)W, ldw, bias, residual, ldr,
                                                                              (TO*)out, ldo, M, N, K, act));
-        } else if constexpr (sizeof(TI) == 2) {
+        } else {
             const size_t smem = (size_t)warps * 4 * skinny_pitch(16) * sizeof(float);
             static bool configured = false;
             if (!configured) {
@@ -586,6 +586,21 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
 }
 
 }  // namespace
+
+// The features a block has in the kernel whose weights come by whole rows, for float32 products of whole 16-byte pieces: 16, 8, or 0 where the kernel that
+// brings them lane by lane is the faster one.  Measured with cold weights, lane by lane / by rows in us (12 tokens): 9.8 / 8.4 for 3072 x 768, 110 / 91 for
+// 50257 x 768, 15.9 / 12.5 for 4096 x 1024; 4.7 / 5.5 for 768 x 64 and 22.3 / 24.7 for 256 x 6400 (bound by latency: the rows' form has a barrier more), 19.0 /
+// 25.6 for 2304 x 3072 (a block's chunks fill an SM by themselves, as do those of K = 1280).  So: two to four warps (K of 257 to 1024; one warp with 193 to
+// 256 and two rounds of blocks), enough blocks to fill the GPU, and with four warps, whose blocks of sixteen features have an SM each, rounds over the SMs
+// that are at least two thirds full (3072 x 1024: 11.5 / 12.0).  Up to eight tokens the other kernel is the faster one throughout (a step of 8 requests 615 against 632 us).
+extern "C" int lb_gemm_ffma_row_features(int M, int N, int K) {
+    const int n_chunks = (K + kChunk - 1) / kChunk, warps = (n_chunks + 3) / 4;
+    const int round = 16 * 148, rounds = (N + round - 1) / round;
+    if (M <= 8 || M > kSkinnyTokens || n_chunks < 4 || warps > 4) return 0;
+    if (warps == 1) return N >= 2 * round ? 16 : 0;
+    if (N < round) return N >= 1536 && n_chunks > 10 ? 8 : 0;
+    return warps < 4 || 3ll * N >= 2ll * rounds * round ? 16 : 0;
+}
 
 extern "C" int lb_gemm_ffma(int in_dtype, int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw,
                             const float* bias, const float* residual, int64_t ldr, void* out, int64_t ldo, int M, int N,

@@ -38,7 +38,8 @@ def test_tiled_products(dev, dtypes, M, N, K):
 
 
 @pytest.mark.parametrize("M", [9, 13, 16])
-@pytest.mark.parametrize("N,K", [(1, 4), (70, 68), (17, 4160), (2367, 768), (2368, 768), (2377, 3072), (2370, 6400)])
+@pytest.mark.parametrize("N,K", [(1, 4), (70, 68), (17, 4160), (2367, 768), (2368, 768), (2377, 3072), (2370, 6400), (1536, 644), (2375, 260),
+                                 (1541, 1000), (4738, 1024), (4740, 200)])
 def test_products_of_nine_to_sixteen_rows(dev, M, N, K):
     """Sixteen features a block or eight, one chunk a group or several, remainders: the bits of eight rows and one, which another kernel multiplies."""
     from liyab_b200 import ops

@@ -118,3 +118,14 @@ def test_nine_to_sixteen_tokens_keep_to_registers_where_the_ring_is_slower():
         assert [kind(m, 9472, k) for k in (512, 896, 904, 1024, 1032)] == [2, 2, 1, 1, 2]
         assert [kind(m, 6400, k) for k in (512, 1024, 1600)] == [2, 2, 2]
     assert [kind(8, 9472, k, normed=normed) for k in (512, 1024) for normed in (False, True)] == [2] * 4
+
+
+def test_float32_products_of_nine_to_sixteen_rows():
+    """Weights by whole rows where that is the faster kernel: reductions of 193 to 1024, features that fill the GPU."""
+    f = ops.lib().lb_gemm_ffma_row_features
+    for m in (9, 12, 16):
+        assert [f(m, n, 768) for n in (64, 768, 1535, 1536, 2304, 2367, 2368, 3072, 50257)] == [0, 0, 0, 8, 8, 8, 16, 16, 16]
+        assert [f(m, 4096, k) for k in (64, 256, 260, 512, 1024, 1028, 1280, 4096)] == [0, 0, 16, 16, 16, 0, 0, 0]
+        assert [f(m, n, 1024) for n in (1024, 2304, 2368, 3072, 3157, 4096, 4800)] == [0, 8, 16, 0, 0, 16, 16]
+        assert [f(m, 2304, k) for k in (640, 644, 1024, 3072)] == [0, 8, 8, 0] and [f(m, 4736, k) for k in (128, 192, 196, 256)] == [0, 0, 16, 16]
+    assert not any(f(m, 3072, 768) for m in (1, 8, 17))
