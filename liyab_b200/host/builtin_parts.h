@@ -110,6 +110,7 @@ public:
 // single tokens (on the tensor cores where that one takes the shape, else scalar), the tensor-core prefill kernel for
 // steps with prompt portions, where they take the shape.  Else the generic kernel; all of the 32-bit engine runs on it,
 // so that there a position's result has the same bits however the work was cut.  `span`: the most keys a query sees.
+inline AttentionUse attention_use(const kernels::AttentionShape& a) { return {a.n_head, a.n_kv_head, a.head_dim, a.mask()}; }
 inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView& view, const Rows& att, const kernels::AttentionShape& a, int span) {
     const int T = ctx.n_tokens, S = ctx.n_seq;
     const int n_pages = view.group->pool.num_pages();
@@ -131,13 +132,12 @@ inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView
             return;
         }
     }
+    AttentionPlan plan = ctx.attention_plan(attention_use(a));
+    plan.apart = plan.apart && kernels::decode_mma_supports(a);
     if (ctx.runtime.dtype == DType::BF16 && kernels::prefill_supports(a)) {
-        // Single tokens beside prompt portions have a launch of their own: a tile of 64 or 128 rows would be spent on each of them (XL, 12 such tokens
-        // beside a portion of 453 on 300: 44 us a layer in one launch, 41 us in two, 5.84 -> 5.66 ms a step).
-        const bool apart = ctx.singles_apart && kernels::decode_mma_supports(a);
         kernels::prefill_attention(ctx.runtime, q, T, cache, n_pages, ctx.q_start, ctx.n_past, view.block_table, view.table_width, att, S, ctx.max_q_len,
-                                   apart, a);
-        if (apart) decode(true, ctx.q_start);
+                                   plan, a);
+        if (plan.apart) decode(true, ctx.q_start);
         return;
     }
     kernels::attention_generic(ctx.stream(), ctx.runtime.dtype, q, cache, ctx.tok_seq, ctx.positions, view.block_table,
@@ -179,6 +179,7 @@ public:
     }
     bool capturable() const override { return true; }
     std::optional<KvNeed> kv_need() const override { return KvNeed{shape.n_kv_head, shape.head_dim, shape.window}; }
+    std::vector<AttentionUse> attention_uses() const override { return {attention_use(shape)}; }
 
     // A step of up to 16 tokens in bfloat16 with rows of up to 1024 values (up to 8 with 2048): the projection normalises the rows inside
     // its kernel (and fills the cache from its epilogue), so the LayerNorm before the mixer is not launched.

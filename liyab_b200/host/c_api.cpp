@@ -3,6 +3,7 @@
 // message (the reference's pattern: src/c_api/liyab_c_api.cpp:34-58).
 #include "../include/liyab_b200.h"
 
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <unordered_map>
@@ -730,6 +731,25 @@ int32_t lb_host_buffer_create(int32_t device, size_t bytes, void** out) {
 
 void lb_host_buffer_destroy(void* buffer) {
     if (buffer != nullptr) cudaFreeHost(buffer);
+}
+
+int32_t lb_attention_plan(const char* dtype, int32_t n_head, int32_t n_kv_head, int32_t head_dim, int32_t page_size, int32_t mask, int32_t sm_count, int32_t n_seq,
+                          const int32_t* q_start, const int32_t* n_past, int32_t max_q_len, int32_t* bits) {
+    return guarded([&] {
+        need(q_start, "q_start");
+        need(n_past, "n_past");
+        need(bits, "bits");
+        Runtime rt;
+        rt.dtype = compute_dtype_from_name(dtype);
+        rt.sm_count = sm_count;
+        kernels::AttentionShape a;
+        a.n_head = n_head;
+        a.n_kv_head = n_kv_head;
+        a.head_dim = head_dim;
+        a.page_size = page_size;
+        (mask < 0 ? a.chunk : a.window) = std::abs(mask);
+        *bits = kernels::attention_plan(rt, a, q_start, n_past, n_seq, max_q_len).bits();
+    });
 }
 
 int32_t lb_replayer_set(lb_replayer* r, const char* option, int32_t value) {

@@ -124,6 +124,15 @@ std::map<int, KvNeed> DecoderModel::kv_needs() const {
     return out;
 }
 
+std::vector<AttentionUse> DecoderModel::attention_uses() const {
+    std::vector<AttentionUse> out;
+    for (const Layer& l : layers)
+        for (const Mixer* m : l.block->mixers())
+            for (const AttentionUse& u : m->attention_uses())
+                if (std::find(out.begin(), out.end(), u) == out.end()) out.push_back(u);
+    return out;
+}
+
 std::map<int, StateNeed> DecoderModel::state_needs() const {
     std::map<int, StateNeed> out;
     for (size_t i = 0; i < spec.run_order.size(); ++i) {

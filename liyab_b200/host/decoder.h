@@ -46,6 +46,7 @@ public:
     int64_t max_positions() const;
     size_t weight_bytes() const;                     // bytes of all parameters, a tied table counted once
     bool capturable() const;                         // every part may be captured into a CUDA graph
+    std::vector<AttentionUse> attention_uses() const;     // of all mixers, each once
 
     // Runs the step's tokens; returns logits [R, vocab] float32 at ctx.logit_rows (rows == 0 when R = 0).
     Rows forward(StepContext& ctx);

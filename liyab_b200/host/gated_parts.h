@@ -216,6 +216,7 @@ public:
     }
     bool capturable() const override { return true; }
     std::optional<KvNeed> kv_need() const override { return KvNeed{G, shape.head_dim, shape.chunk > 0 ? shape.chunk : shape.window}; }
+    std::vector<AttentionUse> attention_uses() const override { return {attention_use(shape)}; }
 
     void forward(StepContext& ctx, const Rows& h, const Rows& x, CacheUnit unit) override { run(ctx, &h, nullptr, nullptr, x, &x, unit); }
     void forward_into(StepContext& ctx, const Rows& h, const Rows& y, CacheUnit unit) override { run(ctx, &h, nullptr, nullptr, y, nullptr, unit); }
@@ -469,6 +470,12 @@ public:
         for (const auto& b : branches)
             if (!b->capturable()) return false;
         return true;
+    }
+    std::vector<AttentionUse> attention_uses() const override {
+        std::vector<AttentionUse> out;
+        for (const auto& b : branches)
+            for (const AttentionUse& u : b->attention_uses()) out.push_back(u);
+        return out;
     }
     std::optional<KvNeed> kv_need() const override {
         for (const auto& b : branches)

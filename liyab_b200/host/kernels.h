@@ -111,10 +111,14 @@ void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* c
 void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,
                       const int32_t* block_table, int table_width, const Rows& out, float* partial, int* counters, int n_seq,
                       const AttentionShape& a, int n_splits);
-// singles_apart: requests that bring one token are left to decode_attention.
+// plan.apart: requests that bring one token are left to decode_attention.
 void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                        const int32_t* n_past, const int32_t* block_table, int table_width, const Rows& out, int n_seq,
-                       int max_q_len, bool singles_apart, const AttentionShape& a);
+                       int max_q_len, const AttentionPlan& plan, const AttentionShape& a);
+// How a step with prompt portions launches an attention (page_size, sink and so on of `a` are those of its launches): the cheapest of the launches that
+// take it, by estimates from the requests' tokens (q_start, n_past: n_seq + 1 and n_seq numbers on the host) and the longest portion that
+// the launches have room for.
+AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const int32_t* q_start, const int32_t* n_past, int n_seq, int max_q_len);
 
 // ---- row-wise pieces between the products: RMS norm in groups, token shift, xIELU, gated side input ----
 // out[r] = x[rows ? rows[r] : r] cut into `groups` equal parts, each over its own root mean square, times weight.

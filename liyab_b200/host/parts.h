@@ -19,7 +19,8 @@
 // change between replays: a part whose forward reads the host copies of the
 // layout (host_q_start, host_n_past, max_kv_len), copies from the device, or
 // keeps host-side state between steps must leave `capturable()` false (the
-// default); a model with one such part is never captured.
+// default); a model with one such part is never captured.  What the host decides
+// about a step's attention is no such copy: steps that differ in it are captured apart.
 #pragma once
 
 #include <functional>
@@ -58,6 +59,17 @@ struct CacheUnit {
     // keeps one, lives under `read`.
     static constexpr int kExtraStride = 1 << 20;
     int extra_state(int k) const { return entry + (k + 1) * kExtraStride; }
+};
+
+// An attention that `attend` (builtin_parts.h) launches, and how it is launched in a step with prompt portions (see kernels::attention_plan).
+struct AttentionUse {
+    int n_head = 0, n_kv_head = 0, head_dim = 0, mask = 0;
+    auto operator<=>(const AttentionUse&) const = default;
+};
+struct AttentionPlan {
+    bool apart = false;        // bfloat16: requests of one token have a launch of their own, by the decode kernel
+    bool tcgen05 = false;      // bfloat16: portions by the tcgen05 kernel where it takes the shape, else by the mma.sync one
+    int bits() const { return (apart ? 1 : 0) | (tcgen05 ? 2 : 0); }
 };
 
 // One cache group as a step sees it.
@@ -147,7 +159,7 @@ struct StepContext {
     int max_q_len = 0;
     int max_kv_len = 0;
     bool decode_only = false;
-    bool singles_apart = false;      // a long portion beside requests of a few tokens: those of one token have a launch of their own
+    std::vector<std::pair<AttentionUse, AttentionPlan>> attention;      // the model's attentions in this step (empty: single tokens only)
     int max_positions = 0;          // the longest sequence the engine serves (fixes split counts and table widths)
     const TapFn* tap_fn = nullptr;  // when set, parts' outputs are shown to it (tests)
     PhaseTimer* phases = nullptr;   // when set, phase boundaries are recorded
@@ -168,6 +180,11 @@ struct StepContext {
     cudaStream_t stream() const { return runtime.stream; }
     // The unit's pages [page, K|V, kv_head, slot, head_dim] and its group's view.
     void* kv(int unit, const GroupView** view) const;
+    AttentionPlan attention_plan(const AttentionUse& use) const {
+        for (const auto& [u, plan] : attention)
+            if (u == use) return plan;
+        return AttentionPlan{};
+    }
     // The unit's state storage [slot, ...]; index it with `state_slots`.
     void* state(int unit, size_t* slot_bytes = nullptr) const;
     void tap(std::string_view name, const Rows& rows) const {
@@ -220,6 +237,8 @@ class Mixer : public Part {
 public:
     virtual std::optional<KvNeed> kv_need() const { return std::nullopt; }
     virtual std::optional<StateNeed> state_need() const { return std::nullopt; }
+    // The attentions that the mixer launches by `attend`.
+    virtual std::vector<AttentionUse> attention_uses() const { return {}; }
     // Adds the mixer's output for the step's tokens to the residual stream x; `h` is its normalised input.
     virtual void forward(StepContext& ctx, const Rows& h, const Rows& x, CacheUnit unit) = 0;
     // Writes the mixer's output to `out` (float32 [T, width]) instead of adding it to the stream, for a mixer that is one of

@@ -1,6 +1,7 @@
 #include "step.h"
 
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 #include <set>
 
@@ -20,6 +21,8 @@ Stepper::Stepper(DecoderModel& model_, CacheManager& cache_, const StepperOption
     }
     cache.stream = model.runtime.stream;
     model_capturable_ = model.capturable();
+    attention_uses_ = model.attention_uses();
+    if (attention_uses_.size() > 32) attention_uses_.resize(32);       // two bits each in a step's key; others launch in one way
     // Decode steps of a few tokens go to the one-kernel path where the model is made of standard parts.
     if (o.fused_decode) fused_ = FusedDecodeStack::try_build(model, cache);
 }
@@ -67,6 +70,7 @@ StepOutput Stepper::step(const std::vector<StepEntry>& entries, const DeviceToke
     std::vector<int> rows;
     std::vector<int64_t> q_len;
     validate(entries, dt, &rows, &q_len);
+    plan_attention(rows, q_len);
     cache.reserve_rows(rows, q_len);         // all or nothing: throws OutOfPages and takes no page
     Layout layout;
     Rows logits;
@@ -105,6 +109,31 @@ StepOutput Stepper::step(const std::vector<StepEntry>& entries, const DeviceToke
     return StepOutput{logits, std::move(layout.out_rows)};
 }
 
+void Stepper::plan_attention(const std::vector<int>& rows, const std::vector<int64_t>& q_len) {
+    attention_plan_.clear();
+    attention_bits_ = 0;
+    const int64_t longest = *std::max_element(q_len.begin(), q_len.end());
+    std::vector<int32_t> q_start{0}, n_past;
+    for (size_t i = 0; i < rows.size(); ++i) {
+        q_start.push_back(q_start.back() + static_cast<int32_t>(q_len[i]));
+        n_past.push_back(static_cast<int32_t>(cache.length_of_row[static_cast<size_t>(rows[i])]));
+    }
+    for (const AttentionUse& use : attention_uses_) {
+        kernels::AttentionShape a;
+        a.n_head = use.n_head;
+        a.n_kv_head = use.n_kv_head;
+        a.head_dim = use.head_dim;
+        a.page_size = cache.page_size;
+        (use.mask < 0 ? a.chunk : a.window) = std::abs(use.mask);
+        // Steps of single tokens go to the decode kernels where one takes the shape.
+        if (longest == 1 && (model.runtime.dtype == DType::F32 || kernels::decode_mma_supports(a) || kernels::decode_scalar_supports(a))) continue;
+        const AttentionPlan plan = kernels::attention_plan(model.runtime, a, q_start.data(), n_past.data(), static_cast<int>(rows.size()),
+                                                           static_cast<int>((longest + 63) / 64 * 64));
+        attention_bits_ |= static_cast<uint64_t>(plan.bits()) << (2 * attention_plan_.size());
+        attention_plan_.emplace_back(use, plan);
+    }
+}
+
 Stepper::ShapeKey Stepper::shape_key(const std::vector<StepEntry>& entries, const std::vector<int64_t>& q_len) const {
     int T = 0, R = 0;
     int64_t longest = 0;
@@ -114,7 +143,7 @@ Stepper::ShapeKey Stepper::shape_key(const std::vector<StepEntry>& entries, cons
         longest = std::max(longest, q_len[i]);
     }
     const int S = static_cast<int>(entries.size());
-    return {S, T, R, T != S ? static_cast<int>((longest + 63) / 64 * 64) : 1};
+    return {S, T, R, T != S ? static_cast<int>((longest + 63) / 64 * 64) : 1, attention_bits_};
 }
 
 bool Stepper::worth_capturing(const std::vector<StepEntry>& entries, const std::vector<int64_t>& q_len) {
@@ -130,7 +159,7 @@ bool Stepper::worth_capturing(const std::vector<StepEntry>& entries, const std::
 Rows Stepper::graph_step(const std::vector<StepEntry>& entries, const std::vector<int>& rows, const std::vector<int64_t>& q_len,
                          const DeviceTokens* dt, Layout* layout) {
     // A graph fits every step with the same number of requests, tokens and wanted rows whose longest portion
-    // falls into the same bucket of 64 tokens; everything else about the step (tokens, positions, where portions
+    // falls into the same bucket of 64 tokens and whose attentions are launched alike; everything else about the step (tokens, positions, where portions
     // start, block tables, slots) is data the graph reads from its own layout buffer.
     const ShapeKey key = shape_key(entries, q_len);
     const int bucket = std::get<3>(key);
@@ -308,12 +337,7 @@ void Stepper::lay_out(const std::vector<StepEntry>& entries, const std::vector<i
     ctx.max_q_len = max_q_len > 0 ? max_q_len : longest;
     ctx.max_kv_len = max_kv;
     ctx.decode_only = T == S;
-    // Single tokens beside one long portion are served apart from it.  A captured step goes by what its replays have in common (requests, tokens, the
-    // bucket of the longest portion) and launches for single tokens that a replay may not have; any other step looks.  The launch costs 2 to
-    // 3 us an attention where it finds none: short portions, and few requests beside a long one, keep to one launch.
-    const int bucket = (longest + 63) / 64 * 64;
-    ctx.singles_apart = !ctx.decode_only && S >= 4 && bucket >= 256 && T - bucket <= 8 * (S - 1) &&
-                        (fixed != nullptr || std::any_of(q_len.begin(), q_len.end(), [](int64_t n) { return n == 1; }));
+    ctx.attention = attention_plan_;
     ctx.max_positions = max_positions;
 }
 

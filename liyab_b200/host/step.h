@@ -86,7 +86,8 @@ public:
     uint64_t steps = 0, graph_steps = 0, fused_steps = 0, eager_steps = 0, tokens_run = 0, graphs_captured = 0;
 
 private:
-    using ShapeKey = std::tuple<int, int, int, int>;        // requests, tokens, wanted rows, bucket of the longest portion
+    // Requests, tokens, wanted rows, bucket of the longest portion, and how the step launches its attentions.
+    using ShapeKey = std::tuple<int, int, int, int, uint64_t>;
     struct CapturedStep {
         DeviceBuffer layout;
         size_t layout_ints = 0;
@@ -108,6 +109,7 @@ private:
     void lay_out(const std::vector<StepEntry>& entries, const std::vector<int>& rows, const std::vector<int64_t>& q_len,
                  const DeviceTokens* dt, CapturedStep* fixed, int max_q_len, Layout* out);
     void drop_graph(CapturedStep& g);
+    void plan_attention(const std::vector<int>& rows, const std::vector<int64_t>& q_len);
 
     std::unique_ptr<FusedDecodeStack> fused_;
     std::map<ShapeKey, CapturedStep> graphs_;
@@ -120,6 +122,9 @@ private:
     PhaseTimer* phases_ = nullptr;
     double* phase_totals_ = nullptr;
     bool model_capturable_ = false;
+    std::vector<AttentionUse> attention_uses_;                                 // the model's
+    std::vector<std::pair<AttentionUse, AttentionPlan>> attention_plan_;       // in this step
+    uint64_t attention_bits_ = 0;
 };
 
 }  // namespace liyab
