@@ -134,8 +134,8 @@ int lb_paged_attention_generic(int dtype, const void* q, int64_t q_stride, const
 
 /* The same for float32 with head size 64 where neighbouring tokens start at the same key (window <= 0), with a sink a head (or null): a
  * tile of keys and values is read once for sixteen neighbouring tokens.  Bit for bit what lb_paged_attention_generic_sink gives.
- * lb_paged_attention_f32_runs_supports says whether a step of n_tokens tokens of n_seq requests is faster with it. */
-int lb_paged_attention_f32_runs_supports(const void* cache, int n_tokens, int n_seq, int n_head, int n_kv_head, int head_dim, int window);
+ * lb_paged_attention_f32_runs_supports says whether a step of n_tokens tokens can take it. */
+int lb_paged_attention_f32_runs_supports(const void* cache, int n_tokens, int n_head, int n_kv_head, int head_dim, int window);
 int lb_paged_attention_f32_runs(const float* q, int64_t q_stride, const float* cache, const int32_t* tok_seq, const int32_t* positions,
                                 const int32_t* block_table, int table_stride, float* out, int64_t out_stride, int n_tokens, int n_head,
                                 int n_kv_head, int page_size, float scale, int window, const float* sink, void* stream);

@@ -738,11 +738,11 @@ int launch(const void* q, int64_t q_stride, const void* cache, const int32_t* to
 }  // namespace
 
 // Whether float32 launches of these sizes take the kernel that shares a tile among neighbouring tokens: head size 64, keys whose first one does
-// not move with the token (all earlier ones, or those of a chunk), plain scores, more pairs than the few that are bound by latency (that
-// kernel is the faster one up to there), and at least eight tokens a request on average: a block takes single tokens one after another.
-extern "C" int lb_paged_attention_f32_runs_supports(const void* cache, int n_tokens, int n_seq, int n_head, int n_kv_head, int head_dim, int window) {
+// not move with the token (all earlier ones, or those of a chunk), plain scores, and more pairs than the few that are bound by latency (that
+// kernel is the faster one up to there).  A block takes single tokens one after another: whether a step's portions suit it is the host's to say.
+extern "C" int lb_paged_attention_f32_runs_supports(const void* cache, int n_tokens, int n_head, int n_kv_head, int head_dim, int window) {
     return head_dim == kRunDim && warps_for(head_dim) == kRunWarps && window <= 0 && n_head > 0 && n_kv_head > 0 && n_head % n_kv_head == 0 &&
-           (long long)n_tokens * n_head > kFewPairs && (long long)n_tokens * n_head <= 2147483647ll && n_tokens >= 8ll * n_seq && ((uintptr_t)cache & 15) == 0;
+           (long long)n_tokens * n_head > kFewPairs && (long long)n_tokens * n_head <= 2147483647ll && ((uintptr_t)cache & 15) == 0;
 }
 
 extern "C" int lb_paged_attention_f32_runs(const float* q, int64_t q_stride, const float* cache, const int32_t* tok_seq, const int32_t* positions,

@@ -141,7 +141,7 @@ inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView
         return;
     }
     kernels::attention_generic(ctx.stream(), ctx.runtime.dtype, q, cache, ctx.tok_seq, ctx.positions, view.block_table,
-                               view.table_width, att, T, ctx.n_seq, a);
+                               view.table_width, att, T, plan.runs, a);
 }
 
 // ---- causal self-attention over the paged cache, one fused projection of queries, keys and values -----

@@ -257,11 +257,11 @@ int decode_splits(int n_seq, int n_kv_head, int max_context, bool tensor_cores) 
 }
 
 void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* cache, const int32_t* tok_seq,
-                       const int32_t* positions, const int32_t* block_table, int table_width, const Rows& out, int n_tokens, int n_seq,
+                       const int32_t* positions, const int32_t* block_table, int table_width, const Rows& out, int n_tokens, bool runs,
                        const AttentionShape& a) {
     if (q.dtype != dtype || out.dtype != dtype) throw invalid_argument("attention: q, cache and out must have one element type");
-    if (dtype == DType::F32 && a.distance == nullptr && a.soft_cap == 0.0f &&
-        lb_paged_attention_f32_runs_supports(cache, n_tokens, n_seq, a.n_head, a.n_kv_head, a.head_dim, a.mask()) != 0) {
+    if (runs && dtype == DType::F32 && a.distance == nullptr && a.soft_cap == 0.0f &&
+        lb_paged_attention_f32_runs_supports(cache, n_tokens, a.n_head, a.n_kv_head, a.head_dim, a.mask()) != 0) {
         check(lb_paged_attention_f32_runs(q.f32(), q.stride, static_cast<const float*>(cache), tok_seq, positions, block_table, table_width, out.f32(),
                                           out.stride, n_tokens, a.n_head, a.n_kv_head, a.page_size, a.scale, a.mask(), a.sink, s), "paged_attention_f32_runs");
         return;
@@ -319,7 +319,29 @@ AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const i
     AttentionPlan plan;
     const double heads = a.n_head, sms = rt.sm_count;
     const int64_t span = a.chunk > 0 ? a.chunk : a.window;
-    if (rt.dtype != DType::BF16 || !prefill_supports(a)) return plan;
+    if (rt.dtype == DType::F32) {
+        // Blocks of sixteen tokens walk the runs of their tokens one after another (4 us a 256 keys, and 3.1 for every four queries), where the other kernel
+        // has a block a token.  Single tokens beside a prompt are what it is slow at: 24 of 300 to 950 keys beside a prompt of 200 take 338 us against 116,
+        // eight tokens for each of sixteen requests on 500 take 46 against 126.
+        if (a.head_dim != 64 || a.window > 0) return plan;
+        double longest = 0, all = 0, block = 0, keys = 0;
+        for (int i = 0; i < n_seq; ++i)
+            for (int t = q_start[i], end = q_start[i + 1]; t < end;) {
+                const int stop = std::min(end, (t / 16 + 1) * 16), n = stop - t;
+                const int64_t end_key = n_past[i] + (stop - q_start[i]), reach = span > 0 ? std::min(span, end_key) : end_key;
+                block += static_cast<double>((reach + 255) / 256) * (4.0 + 3.1 * ((n + 3) / 4));
+                keys += static_cast<double>(n) * static_cast<double>(reach);
+                if (stop % 16 == 0 || (i + 1 == n_seq && stop == end)) {
+                    longest = std::max(longest, block);
+                    all += block;
+                    block = 0;
+                }
+                t = stop;
+            }
+        plan.runs = std::max(longest, all * heads / (2 * sms)) < 35.0 + keys * heads / 6900.0;
+        return plan;
+    }
+    if (!prefill_supports(a)) return plan;
     Tiles wide[2], narrow[2];          // of the portions; of all requests
     double longest_single = 0, all_single = 0;
     for (int i = 0; i < n_seq; ++i) {

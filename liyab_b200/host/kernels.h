@@ -105,7 +105,7 @@ bool prefill_supports(const AttentionShape& a);
 bool prefill_tc_supports(const AttentionShape& a);
 int decode_splits(int n_seq, int n_kv_head, int max_context, bool tensor_cores);
 void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* cache, const int32_t* tok_seq,
-                       const int32_t* positions, const int32_t* block_table, int table_width, const Rows& out, int n_tokens, int n_seq,
+                       const int32_t* positions, const int32_t* block_table, int table_width, const Rows& out, int n_tokens, bool runs,
                        const AttentionShape& a);
 // q_start: null in steps of single tokens; in a mixed step (tensor cores only) where each request's tokens start: its single tokens are served.
 void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,

@@ -69,7 +69,8 @@ struct AttentionUse {
 struct AttentionPlan {
     bool apart = false;        // bfloat16: requests of one token have a launch of their own, by the decode kernel
     bool tcgen05 = false;      // bfloat16: portions by the tcgen05 kernel where it takes the shape, else by the mma.sync one
-    int bits() const { return (apart ? 1 : 0) | (tcgen05 ? 2 : 0); }
+    bool runs = false;         // float32: a tile of keys is read once for sixteen neighbouring tokens
+    int bits() const { return (apart ? 1 : 0) | (tcgen05 ? 2 : 0) | (runs ? 4 : 0); }
 };
 
 // One cache group as a step sees it.

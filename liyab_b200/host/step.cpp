@@ -22,7 +22,7 @@ Stepper::Stepper(DecoderModel& model_, CacheManager& cache_, const StepperOption
     cache.stream = model.runtime.stream;
     model_capturable_ = model.capturable();
     attention_uses_ = model.attention_uses();
-    if (attention_uses_.size() > 32) attention_uses_.resize(32);       // two bits each in a step's key; others launch in one way
+    if (attention_uses_.size() > 21) attention_uses_.resize(21);       // three bits each in a step's key; others launch in one way
     // Decode steps of a few tokens go to the one-kernel path where the model is made of standard parts.
     if (o.fused_decode) fused_ = FusedDecodeStack::try_build(model, cache);
 }
@@ -129,7 +129,7 @@ void Stepper::plan_attention(const std::vector<int>& rows, const std::vector<int
         if (longest == 1 && (model.runtime.dtype == DType::F32 || kernels::decode_mma_supports(a) || kernels::decode_scalar_supports(a))) continue;
         const AttentionPlan plan = kernels::attention_plan(model.runtime, a, q_start.data(), n_past.data(), static_cast<int>(rows.size()),
                                                            static_cast<int>((longest + 63) / 64 * 64));
-        attention_bits_ |= static_cast<uint64_t>(plan.bits()) << (2 * attention_plan_.size());
+        attention_bits_ |= static_cast<uint64_t>(plan.bits()) << (3 * attention_plan_.size());
         attention_plan_.emplace_back(use, plan);
     }
 }

@@ -8,7 +8,7 @@ import pytest
 
 from liyab_b200 import _capi
 
-APART, TCGEN05 = 1, 2
+APART, TCGEN05, RUNS = 1, 2, 4
 
 
 def plan(requests, n_head, dtype="bfloat16", n_kv_head=None, head_dim=64, page_size=16, mask=0, sms=148):
@@ -49,3 +49,15 @@ def test_only_kernels_that_take_the_shape():
     assert plan(mixed, 12, head_dim=40) == 0 and plan(mixed, 34, n_kv_head=2) & APART == 0
     assert plan(mixed, 12, page_size=8) & APART == 0
     assert plan([(100, 1)], 12) in (0, APART, TCGEN05)           # a launch is chosen for any step
+
+
+@pytest.mark.parametrize("requests,runs", [
+    # us by runs / a block a token, 12 heads: 338 / 117, 252 / 57, 167 / 32, 1261 / 213, 104 / 54
+    (singles(24, 300, 950) + [(0, 200)], False), ([(699, 1)] * 12 + [(0, 100)], False), ([(599, 1)] * 8 + [(0, 64)], False), ([(2999, 1)] * 24 + [(0, 200)], False),
+    ([(99, 1)] * 16 + [(0, 120)], False),
+    # 504 / 831, 529 / 1179, 46 / 126, 34 / 122, 19 / 68, 213 / 1420, 28 / 82
+    ([(899, 1)] * 100 + [(0, 800)], True), ([(999, 1)] * 120 + [(0, 1000)], True), ([(492, 8)] * 16, True), ([(484, 16)] * 8, True), ([(0, 20)] * 10, True),
+    ([(2700, 300)], True), ([(313, 87)], True)])
+def test_float32_runs(requests, runs):
+    assert plan(requests, 12, dtype="float32") == (RUNS if runs else 0)
+    assert plan(requests, 12, dtype="float32", mask=64) == 0 and plan(requests, 12, dtype="float32", head_dim=32) == 0
