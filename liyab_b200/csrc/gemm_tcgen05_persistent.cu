@@ -35,6 +35,8 @@
 #include "gemm_tile.cuh"
 #include "tcgen05.cuh"
 
+#include <cmath>
+
 namespace {
 
 using namespace lb_tc;
@@ -568,6 +570,34 @@ static bool tiles_shared() {
     return on;
 }
 
+// The feature tile of the tiles that two SMs make together where the product takes those, 0 where every tile stays with one SM: where their estimate is
+// the lower one by an eighth.  This kernel's k-blocks cost what best_tile says, or what all active blocks' operands take from L2 at 13.5 TB/s.  The line lies
+// between products like 2048 x 1600 x 6400 (47 us here, 40 us shared) and 2048 x 3072 x 768 (16.9 us here, 17.4 us shared: short reductions leave a
+// tile's epilogue bare).
+// With 16-bit results the two are closer than with float32 ones and those estimates are too rough: of 252 products from 66 to 8192 tokens x 264 to 10240
+// features x 1024 to 6400 that they would share, 20 were 2 to 5 % slower so (2048 x 2560 x 2560 32.5 / 33.9 us, 2343 x 2560 x 1280 19.0 / 20.0).  A second
+// pair of estimates, fitted to those products round by round (the last round of blocks has L2 to itself), keeps the 176 that gain 17 % on average.
+extern "C" int lb_gemm_shared_tile(int out_dtype, int M, int N, int K, int n_sm) {
+    if (K < 1024) return 0;
+    const int elem = out_dtype == LB_F32 ? 4 : 2, bn = best_tile(elem, M, N, K, n_sm, false, nullptr);
+    if (bn <= 0) return 0;
+    const long n_kb = (K + kBlockK - 1) / kBlockK, tiles = (long)((M + kLaneTile - 1) / kLaneTile) * ((N + bn - 1) / bn), rounds = (tiles + n_sm - 1) / n_sm;
+    const long active = tiles < n_sm ? tiles : n_sm, operands = active * (kLaneTile + bn) * 128 / 13500, step_ns = bn > 192 ? 420 : 300;
+    const long here = rounds * (n_kb * (operands > step_ns ? operands : step_ns) + 1000 + 1000 * bn / 256);
+    int shared = 0;
+    const int bn_shared = lb_gemm_pair_tile(M, N, K, n_sm, &shared);
+    if (8 * (long)shared >= 7 * here) return 0;
+    if (elem == 2) {
+        const long pairs = n_sm / 2, shared_tiles = (long)((M + 2 * kLaneTile - 1) / (2 * kLaneTile)) * ((N + bn_shared - 1) / bn_shared);
+        auto one = [&](long act) { return n_kb * fmax((double)act * (kLaneTile + bn) * 128 / 19.0e6, bn > 192 ? 0.44 : 0.345) + 0.8 * bn / 256; };
+        auto two = [&](long act) { return n_kb * fmax(2.0 * act * (kLaneTile + bn_shared / 2) * 128 / 13.9e6, 0.317) + 0.7 * bn_shared / 256; };
+        const double us_one = 4.0 + (tiles / n_sm) * one(n_sm) + (tiles % n_sm != 0 ? one(tiles % n_sm) : 0.0);
+        const double us_two = 5.8 + (shared_tiles / pairs) * two(pairs) + (shared_tiles % pairs != 0 ? two(shared_tiles % pairs) : 0.0);
+        if (us_two >= 0.965 * us_one) return 0;
+    }
+    return bn_shared;
+}
+
 static int launch_persistent(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual,
                              int64_t ldr, void* out, int64_t ldo, int M, int N, int K, int act, int bn, bool pair, const KvTarget& kv,
                              int n_sm, void* stream);
@@ -616,19 +646,10 @@ extern "C" int lb_gemm_persistent(int out_dtype, const void* A, int64_t lda, con
         }
     }
     LB_CHECK_ARG(bn % step == 0 && bn >= step && bn <= 256, "gemm_persistent: feature tile %d (a multiple of %d up to 256)", bn, step);
-    // Tiles that two SMs make together, where their estimate is the lower one by an eighth: both estimates are good to about that.  This one's
-    // k-blocks cost what best_tile says, or what all active blocks' operands take from L2 at 13.5 TB/s.  The line lies between products like 2048 x
-    // 1600 x 6400 (47 us here, 40 us shared) and 2048 x 3072 x 768 (16.9 us here, 17.4 us shared: short reductions leave a tile's epilogue bare).
-    if (feature_tile <= 0 && !pair && K >= 1024 && tiles_shared()) {
-        const long tiles = (long)((M + kLaneTile - 1) / kLaneTile) * ((N + bn - 1) / bn), rounds = (tiles + n_sm - 1) / n_sm;
-        const long active = tiles < n_sm ? tiles : n_sm, operands = active * (kLaneTile + bn) * 128 / 13500, step_ns = bn > 192 ? 420 : 300;
-        const long here = rounds * ((K + kBlockK - 1) / kBlockK * (operands > step_ns ? operands : step_ns) + 1000 + 1000 * bn / 256);
-        int shared = 0;
-        const int bn_shared = lb_gemm_pair_tile(M, N, K, n_sm, &shared);
-        if (8 * (long)shared < 7 * here)
+    if (feature_tile <= 0 && !pair && tiles_shared())
+        if (const int bn_shared = lb_gemm_shared_tile(out_dtype, M, N, K, n_sm); bn_shared > 0)
             return lb_gemm_pair(out_dtype, A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, bn_shared, kv_cache, slot_mapping, q_dim, n_kv_head,
                                 head_dim, page_size, stream);
-    }
     return launch_persistent(out_dtype, A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, bn_used, pair, kv, n_sm, stream);
 }
 

@@ -64,6 +64,7 @@ _SIGNATURES = {
     "lb_prefill_attention_tc_portions": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
     "lb_gemm_pair": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
     "lb_gemm_pair_tile": [_i, _i, _i, _i, _p],
+    "lb_gemm_shared_tile": [_i, _i, _i, _i, _i],
     "lb_gemm_rows_kind": [_i, _i, _i, _i, _i],
     "lb_gemm_rows_normed_pays": [_i, _i],
     "lb_gemm_ffma_row_features": [_i, _i, _i],
