@@ -500,7 +500,8 @@ int lb_prefill_attention_tc_capped(const void* q, int64_t q_stride, int n_tokens
                                    const float* distance, const float* sink, float soft_cap, float bound, void* stream);
 
 /* The three for steps that mix prompt portions with single tokens: the prefill kernels serve the requests that bring at least min_len tokens, the
- * decode kernel those that bring one (request i's tokens start at q_start[i], n_seq + 1 numbers; positions, q and out go by token). */
+ * decode kernel those that bring one (request i's tokens start at q_start[i], n_seq + 1 numbers; positions, q and out go by token; max_keys: the most keys
+ * that a token may see in any step of this shape, 0: as many as the block table holds; it only chooses among launches). */
 int lb_prefill_attention_portions(const void* q, int64_t q_stride, const void* cache, const int32_t* q_start, const int32_t* n_past,
                                   const int32_t* block_table, int table_stride, void* out, int64_t out_stride, int n_seq, int max_q_len, int n_head,
                                   int n_kv_head, int head_dim, int page_size, float scale, int window, const float* distance, const float* sink,
@@ -511,7 +512,7 @@ int lb_prefill_attention_tc_portions(const void* q, int64_t q_stride, int n_toke
                                      const float* distance, const float* sink, float soft_cap, float bound, int min_len, void* stream);
 int lb_decode_attention_mma_mixed(const void* q, int64_t q_stride, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,
                                   const int32_t* block_table, int table_stride, void* out, int64_t out_stride, float* partial, int* counters, int n_seq,
-                                  int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window, int n_splits,
+                                  int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window, int n_splits, int max_keys,
                                   const float* distance, const float* sink, float soft_cap, float bound, void* stream);
 
 /* What attention over latent rows may have besides its sizes.  sink [n_head]: exp(sink[h]) joins the divisor of head h's softmax (no key, no

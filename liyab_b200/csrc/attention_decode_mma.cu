@@ -471,7 +471,7 @@ struct Variant {
 template <int HD, bool TMA>
 int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* q, int64_t q_stride, const void* cache, const int32_t* q_start, const int32_t* positions, const int32_t* block_table,
                int table_stride, void* out, int64_t out_stride, float* partial, int* counters, int n_seq, int n_head,
-               int n_kv_head, int page_shift, float scale, int window, int n_splits, const float* distance, const float* sink, float soft_cap,
+               int n_kv_head, int page_shift, float scale, int window, int n_splits, int max_keys, const float* distance, const float* sink, float soft_cap,
                       float bound, cudaStream_t s) {
     using Wide = Variant<HD, 4, 2, TMA>;
     using Narrow = Variant<HD, 2, 2, TMA>;
@@ -485,8 +485,13 @@ int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* 
     // The warps' states then meet in one merge, without the cluster's two barriers and the way through the first block's memory.  Fewer pairs would
     // leave SMs without a block.  Measured: GPT-2 small, 8 requests 369 -> 359 us a step; XL, 8 requests 1.98 -> 1.95 ms; medium, 9 requests 734 -> 706 us
     // (with eight warps for three and four ranges as well: 385, 1.96 and 715).
+    // Long contexts want the GPU's bandwidth more than short merges, and one wide block an SM leaves some of it idle where the pairs fill the last wave badly:
+    // 150 pairs in two ranges, 2048 keys 1.00 to 1.07 times as fast with the wide block, 4096 0.97, 16384 0.88; 160 to 200 pairs 0.97 from 8192 on;
+    // 144 pairs in three ranges 1.06 at 4096, 1.00 at 8192, 0.98 at 16384; up to 128 pairs 1.02 to 1.1 throughout.
     if constexpr (TMA) {
-        if (n_splits >= 2 && n_splits <= 4 && (long)n_kv_head * n_seq >= 64) {
+        const long pairs = (long)n_kv_head * n_seq, reach = max_keys > 0 ? max_keys : (long)table_stride << page_shift;
+        const long longest = n_splits == 2 ? (pairs < 160 ? 2048 : 6144) : pairs <= 128 ? reach : 8192;
+        if (n_splits >= 2 && n_splits <= 4 && pairs >= 64 && reach <= longest) {
             if (n_splits == 2)
                 return Variant<HD, 8, 2, TMA>::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride,
                                                       partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, 1, distance, sink, soft_cap, bound, s);
@@ -550,13 +555,13 @@ extern "C" int lb_decode_attention_mma_capped(const void* q, int64_t q_stride, c
                                               int n_seq, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window, int n_splits,
                                               const float* distance, const float* sink, float soft_cap, float bound, void* stream) {
     return lb_decode_attention_mma_mixed(q, q_stride, cache, n_pages, nullptr, positions, block_table, table_stride, out, out_stride, partial, counters, n_seq,
-                                         n_head, n_kv_head, head_dim, page_size, scale, window, n_splits, distance, sink, soft_cap, bound, stream);
+                                         n_head, n_kv_head, head_dim, page_size, scale, window, n_splits, 0, distance, sink, soft_cap, bound, stream);
 }
 
 extern "C" int lb_decode_attention_mma_mixed(const void* q, int64_t q_stride, const void* cache, int n_pages, const int32_t* q_start,
                                              const int32_t* positions, const int32_t* block_table, int table_stride, void* out, int64_t out_stride,
                                              float* partial, int* counters, int n_seq, int n_head, int n_kv_head, int head_dim, int page_size, float scale,
-                                             int window, int n_splits, const float* distance, const float* sink, float soft_cap, float bound,
+                                             int window, int n_splits, int max_keys, const float* distance, const float* sink, float soft_cap, float bound,
                                              void* stream) {
     LB_CHECK_ARG(soft_cap >= 0.0f && (soft_cap == 0.0f || distance == nullptr), "decode attention: a soft cap is positive and goes without a penalty by distance");
     LB_CHECK_ARG(n_seq >= 0 && n_splits >= 1, "decode attention: bad sizes n_seq=%d n_splits=%d", n_seq, n_splits);
@@ -582,11 +587,11 @@ extern "C" int lb_decode_attention_mma_mixed(const void* q, int64_t q_stride, co
             if (rc != LB_OK) return rc;
             return launch_for<64, true>(map_kv, (int)kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride,
                                         out, out_stride, partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window,
-                                        n_splits, distance, sink, soft_cap, bound, s);
+                                        n_splits, max_keys, distance, sink, soft_cap, bound, s);
         }
         return launch_for<64, false>(none, 0, nullptr, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride,
-                                     partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, n_splits, distance, sink, soft_cap, bound, s);
+                                     partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, n_splits, max_keys, distance, sink, soft_cap, bound, s);
     }
     return launch_for<128, false>(none, 0, nullptr, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride,
-                                  partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, n_splits, distance, sink, soft_cap, bound, s);
+                                  partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, n_splits, max_keys, distance, sink, soft_cap, bound, s);
 }

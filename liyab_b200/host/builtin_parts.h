@@ -123,7 +123,7 @@ inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView
             counters = static_cast<int*>(ctx.workspace->flat("attn.decode.counters", static_cast<int64_t>(S) * a.n_kv_head, DType::I32, true));
         }
         kernels::decode_attention(ctx.stream(), tensor, q, cache, n_pages, q_start, ctx.positions, view.block_table, view.table_width, att, partial,
-                                  counters, S, a, splits);
+                                  counters, S, a, splits, span);
     };
     if (ctx.runtime.dtype == DType::BF16 && ctx.decode_only) {
         const bool tensor = kernels::decode_mma_supports(a), scalar = kernels::decode_scalar_supports(a);

@@ -273,7 +273,7 @@ void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* c
 
 void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,
                       const int32_t* block_table, int table_width, const Rows& out, float* partial, int* counters, int n_seq,
-                      const AttentionShape& a, int n_splits) {
+                      const AttentionShape& a, int n_splits, int max_keys) {
     if (q.dtype != DType::BF16 || out.dtype != DType::BF16) throw invalid_argument("decode attention takes bfloat16 only");
     if (q.stride % 8 != 0 || !aligned16(q.data))
         throw invalid_argument("decode attention: q rows must be 16-byte aligned and a multiple of 8 elements apart");
@@ -283,7 +283,7 @@ void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const vo
     if (tensor_cores)
         check(lb_decode_attention_mma_mixed(q.data, q.stride, cache, n_pages, q_start, positions, block_table, table_width, out.data, out.stride,
                                            partial, counters, n_seq, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale, a.mask(),
-                                           n_splits, a.distance, a.sink, a.soft_cap, a.score_bound, s), "decode_attention_mma");
+                                           n_splits, max_keys, a.distance, a.sink, a.soft_cap, a.score_bound, s), "decode_attention_mma");
     else
         check(lb_decode_attention_capped(q.data, q.stride, cache, positions, block_table, table_width, out.data, out.stride, partial,
                                        counters, n_seq, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale, a.mask(), n_splits, a.distance, a.sink, a.soft_cap, a.score_bound, s),

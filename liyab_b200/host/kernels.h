@@ -110,7 +110,7 @@ void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* c
 // q_start: null in steps of single tokens; in a mixed step (tensor cores only) where each request's tokens start: its single tokens are served.
 void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,
                       const int32_t* block_table, int table_width, const Rows& out, float* partial, int* counters, int n_seq,
-                      const AttentionShape& a, int n_splits);
+                      const AttentionShape& a, int n_splits, int max_keys);
 // plan.apart: requests that bring one token are left to decode_attention.
 void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                        const int32_t* n_past, const int32_t* block_table, int table_width, const Rows& out, int n_seq,

@@ -59,7 +59,7 @@ _SIGNATURES = {
     "lb_decode_attention_mma_capped": [_p, _l, _p, _i, _p, _p, _i, _p, _l, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _p, _p, _f, _f, _p],
     "lb_prefill_attention_capped": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _p],
     "lb_prefill_attention_tc_capped": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _p],
-    "lb_decode_attention_mma_mixed": [_p, _l, _p, _i, _p, _p, _p, _i, _p, _l, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _p, _p, _f, _f, _p],
+    "lb_decode_attention_mma_mixed": [_p, _l, _p, _i, _p, _p, _p, _i, _p, _l, _p, _p, _i, _i, _i, _i, _i, _f, _i, _i, _i, _p, _p, _f, _f, _p],
     "lb_prefill_attention_portions": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
     "lb_prefill_attention_tc_portions": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
     "lb_gemm_pair": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
@@ -459,9 +459,10 @@ def decode_attention(q: torch.Tensor, cache: torch.Tensor, positions: torch.Tens
                      n_head: int, n_kv_head: int, head_dim: int, page_size: int, scale: float, window: int,
                      n_splits: int, tensor_cores: Optional[bool] = None, distance: Optional[torch.Tensor] = None,
                      sink: Optional[torch.Tensor] = None, soft_cap: float = 0.0, score_bound: float = 0.0,
-                     q_start: Optional[torch.Tensor] = None) -> torch.Tensor:
+                     q_start: Optional[torch.Tensor] = None, max_keys: int = 0) -> torch.Tensor:
     """Attention of one new token per request over its pages (bfloat16), keys split `n_splits` ways.  `q_start` (n_seq + 1 numbers, tensor cores
-    only): where each request's tokens start in a mixed step, of which the requests of one token are served.
+    only): where each request's tokens start in a mixed step, of which the requests of one token are served.  `max_keys`: the most keys a token may see (0: what
+    the block table holds), by which the tensor-core kernel chooses its blocks.
     `tensor_cores`: None picks the tensor-core kernel where it takes the shape, else the scalar one.  `distance`: as for
     paged_attention_generic.  `score_bound`: the largest |score| before the cap that can occur, 0 when unknown."""
     if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
@@ -480,8 +481,8 @@ def decode_attention(q: torch.Tensor, cache: torch.Tensor, positions: torch.Tens
         _dev(q, "q"), q.stride(0), *cache_args, _dev(positions, "positions", torch.int32),
         _dev(block_table, "block_table", torch.int32), block_table.stride(0), _dev(out, "out"), out.stride(0),
         _opt(partial, "partial", torch.float32), _opt(counters, "counters", torch.int32), n_seq, n_head, n_kv_head,
-        head_dim, page_size, float(scale), int(window), int(n_splits), _distance(distance, n_head), _sink(sink, n_head), float(soft_cap), float(score_bound),
-        stream_ptr()), "decode_attention")
+        head_dim, page_size, float(scale), int(window), int(n_splits), *((int(max_keys),) if tensor_cores else ()), _distance(distance, n_head), _sink(sink, n_head),
+        float(soft_cap), float(score_bound), stream_ptr()), "decode_attention")
     return out
 
 

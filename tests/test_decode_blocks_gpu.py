@@ -24,6 +24,11 @@ def test_many_pairs(dev, n_head, n_kv_head, page_size, window, n_seq, with_sink,
     ops.decode_attention(q, cache, positions, table, out, partial, counters, n_seq, n_head, n_kv_head, head_dim, page_size, scale, window, splits,
                          tensor_cores=True, sink=sink)
     assert int(counters.abs().sum()) == 0
+    # Where contexts may be long, two ranges, or more than 128 pairs, go to clusters of blocks again.
+    other = torch.full_like(q, float("nan"))
+    ops.decode_attention(q, cache, positions, table, other, partial, counters, n_seq, n_head, n_kv_head, head_dim, page_size, scale, window, splits,
+                         tensor_cores=True, sink=sink, max_keys=20_000)
+    assert int(counters.abs().sum()) == 0 and (other.float() - out.float()).abs().max().item() < 1.5e-2
     # Probabilities and the result in bfloat16 (2^-9 each), values of order one: as for the blocks of four warps.
     generic = torch.empty_like(q)
     ops.paged_attention_generic(q, cache, tok_seq, positions, table, generic, n_seq, n_head, n_kv_head, head_dim, page_size, scale, window, sink=sink)
