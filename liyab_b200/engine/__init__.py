@@ -204,6 +204,8 @@ class _HostRows:
     its buffer comes back when nothing refers to the array any more.  At most `limit` bytes are held, arrays in use included; what does not fit is an
     ordinary array.  Safe with several threads; closing frees what is not in use, the rest goes with its arrays."""
 
+    REST = 64          # requests between two times that buffers give way to one of another size
+
     class _Lease:
         """What an array keeps alive: gives its buffer back when it dies."""
 
@@ -218,27 +220,36 @@ class _HostRows:
         self._lock = threading.RLock()      # a lease may die, by the garbage collector, inside these methods
         self._free: List[Tuple[int, int]] = []      # (bytes, address)
         self._held, self._closed = 0, False
+        self._requests, self._gave_way = 0, -self.REST
 
     def array(self, rows: int, cols: int) -> np.ndarray:
         need = 4 * rows * cols
         size = -(-need // 65536) * 65536
         with self._lock:
-            fit = min((b for b in self._free if size <= b[0] <= 2 * size), default=None)
-            if fit is not None:
-                self._free.remove(fit)
-            else:
-                while self._free and self._held + size > self._limit:      # room for what is asked for now
-                    self._destroy(self._free.pop(0))
-                if self._closed or self._held + size > self._limit:
-                    return np.empty((rows, cols), dtype=np.float32)
-                out = C.c_void_p()
-                if self._lib.lb_host_buffer_create(self._device, size, C.byref(out)) != 0:
-                    return np.empty((rows, cols), dtype=np.float32)
-                self._held += size
-                fit = (size, out.value)
-        memory = (C.c_float * (rows * cols)).from_address(fit[1])
-        memory.lease = self._Lease(self, fit[1], fit[0])
+            self._requests += 1
+            buffer = self._take(size) if size <= self._limit and not self._closed else None
+        if buffer is None:
+            return np.empty((rows, cols), dtype=np.float32)
+        memory = (C.c_float * (rows * cols)).from_address(buffer[1])
+        memory.lease = self._Lease(self, buffer[1], buffer[0])
         return np.frombuffer(memory, dtype=np.float32).reshape(rows, cols)
+
+    def _take(self, size: int) -> Optional[Tuple[int, int]]:
+        fit = min((b for b in self._free if size <= b[0] <= 2 * size), default=None)
+        if fit is not None:
+            self._free.remove(fit)
+            return fit
+        if self._held + size > self._limit:
+            if self._held - sum(b[0] for b in self._free) + size > self._limit or self._requests - self._gave_way < self.REST:
+                return None
+            self._gave_way = self._requests
+            while self._held + size > self._limit:      # room for what is asked for now
+                self._destroy(self._free.pop(0))
+        out = C.c_void_p()
+        if self._lib.lb_host_buffer_create(self._device, size, C.byref(out)) != 0:
+            return None
+        self._held += size
+        return size, out.value
 
     def _destroy(self, buffer) -> None:
         self._held -= buffer[0]

@@ -94,3 +94,21 @@ def test_threads_never_share_a_buffer(lib):
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not wrong and len(lib.live) <= 9
+
+
+def test_a_request_past_the_limit_leaves_the_buffers(lib):
+    rows = _HostRows(limit=4 * PIECE, lib=lib)
+    a = rows.array(1, PIECE // 4)
+    del a
+    for _ in range(3):
+        assert rows.array(8, PIECE // 4).shape == (8, PIECE // 4) and len(lib.live) == 1
+        rows.array(1, PIECE // 4)
+    assert lib.made == 1
+
+
+def test_sizes_that_do_not_fit_beside_one_another_give_way_seldom(lib):
+    rows = _HostRows(limit=4 * PIECE, lib=lib)
+    for _ in range(200):
+        rows.array(4, PIECE // 4)
+        rows.array(1, PIECE // 4)
+    assert lib.made <= 2 + 400 // rows.REST
