@@ -202,8 +202,10 @@ class _HostRows:
     """Page-locked host memory for steps' logits, kept from step to step: the device copies into it at the link's rate, where a fresh array
     costs its page faults and a copy by the processor (64 rows of 50,257: 2.0 ms a step, 0.25 ms this way).  An array from here is the caller's;
     its buffer comes back when nothing refers to the array any more.  At most `limit` bytes are held, arrays in use included; what does not fit is an
-    ordinary array.  Safe with several threads; closing frees what is not in use, the rest goes with its arrays."""
+    ordinary array, and so is what a caller asks for who keeps IN_USE arrays already (making a buffer takes longer than the copy that it saves).  Safe
+    with several threads; closing frees what is not in use, the rest goes with its arrays."""
 
+    IN_USE = 8
     REST = 64          # requests between two times that buffers give way to one of another size
 
     class _Lease:
@@ -219,7 +221,7 @@ class _HostRows:
         self._lib, self._device, self._limit = lib or _capi.lib(), device, limit
         self._lock = threading.RLock()      # a lease may die, by the garbage collector, inside these methods
         self._free: List[Tuple[int, int]] = []      # (bytes, address)
-        self._held, self._closed = 0, False
+        self._held, self._out, self._closed = 0, 0, False
         self._requests, self._gave_way = 0, -self.REST
 
     def array(self, rows: int, cols: int) -> np.ndarray:
@@ -227,9 +229,10 @@ class _HostRows:
         size = -(-need // 65536) * 65536
         with self._lock:
             self._requests += 1
-            buffer = self._take(size) if size <= self._limit and not self._closed else None
-        if buffer is None:
-            return np.empty((rows, cols), dtype=np.float32)
+            buffer = self._take(size) if size <= self._limit and self._out < self.IN_USE and not self._closed else None
+            if buffer is None:
+                return np.empty((rows, cols), dtype=np.float32)
+            self._out += 1
         memory = (C.c_float * (rows * cols)).from_address(buffer[1])
         memory.lease = self._Lease(self, buffer[1], buffer[0])
         return np.frombuffer(memory, dtype=np.float32).reshape(rows, cols)
@@ -257,6 +260,7 @@ class _HostRows:
 
     def _give(self, address: int, size: int) -> None:
         with self._lock:
+            self._out -= 1
             if self._closed:
                 self._destroy((size, address))
             else:

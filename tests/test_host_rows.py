@@ -112,3 +112,16 @@ def test_sizes_that_do_not_fit_beside_one_another_give_way_seldom(lib):
         rows.array(4, PIECE // 4)
         rows.array(1, PIECE // 4)
     assert lib.made <= 2 + 400 // rows.REST
+
+
+def test_a_caller_who_keeps_its_arrays_soon_gets_ordinary_ones(lib):
+    rows = _HostRows(limit=64 * PIECE, lib=lib)
+    kept = [rows.array(1, 10) for _ in range(50)]
+    assert lib.made == rows.IN_USE
+    kept[3] = None
+    kept.append(rows.array(1, 10))
+    assert lib.made == rows.IN_USE
+    del kept
+    for _ in range(20):
+        rows.array(1, 10)
+    assert lib.made == rows.IN_USE
