@@ -199,7 +199,7 @@ class StepOutput:
 
 
 class _HostRows:
-    """Page-locked host memory for steps' logits, kept from step to step: the device copies into it at the link's rate, where a fresh array
+    """Host memory for steps' logits, kept from step to step: the device copies into it at the link's rate, where a fresh array
     costs its page faults and a copy by the processor (64 rows of 50,257: 2.0 ms a step, 0.25 ms this way).  An array from here is the caller's;
     its buffer comes back when nothing refers to the array any more.  At most `limit` bytes are held, arrays in use included; what does not fit is an
     ordinary array, and so is what a caller asks for who keeps IN_USE arrays already (making a buffer takes longer than the copy that it saves).  Safe

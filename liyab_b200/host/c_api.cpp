@@ -719,18 +719,12 @@ int32_t lb_host_buffer_create(int32_t device, size_t bytes, void** out) {
     return guarded([&] {
         need(out, "out");
         *out = nullptr;
-        LIYAB_CUDA(cudaSetDevice(device));
-        void* p = nullptr;
-        if (const cudaError_t err = cudaMallocHost(&p, bytes); err != cudaSuccess) {
-            cudaGetLastError();          // the caller may go on without the buffer: no launch is to find this error
-            cuda_check(err, "cudaMallocHost");
-        }
-        *out = p;
+        *out = HostRows::create(device, bytes);
     });
 }
 
 void lb_host_buffer_destroy(void* buffer) {
-    if (buffer != nullptr) cudaFreeHost(buffer);
+    if (buffer != nullptr) HostRows::destroy(buffer);
 }
 
 int32_t lb_attention_plan(const char* dtype, int32_t n_head, int32_t n_kv_head, int32_t head_dim, int32_t page_size, int32_t mask, int32_t sm_count, int32_t n_seq,

@@ -1,6 +1,11 @@
 #include "device.h"
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
+#include <map>
+#include <mutex>
 
 namespace liyab {
 
@@ -72,6 +77,89 @@ PinnedBuffer& PinnedBuffer::operator=(PinnedBuffer&& o) noexcept {
         o.ptr_ = nullptr; o.bytes_ = 0;
     }
     return *this;
+}
+
+namespace {
+
+struct HostPages {
+    char* locked = nullptr;
+    size_t bytes = 0;
+    int device = 0;
+};
+std::mutex host_pages_mutex;
+std::map<uintptr_t, HostPages> host_pages;         // by the second address
+
+// Locking and unlocking pages is no work of a stream: it goes on while one is being captured, by this thread or another.
+class OutsideCapture {
+public:
+    explicit OutsideCapture(int device) {
+        cudaThreadExchangeStreamCaptureMode(&mode_);
+        if (cudaGetDevice(&before_) != cudaSuccess) before_ = -1;
+        if (before_ != device) cudaSetDevice(device);
+        else before_ = -1;
+    }
+    ~OutsideCapture() {
+        if (before_ >= 0) cudaSetDevice(before_);
+        cudaThreadExchangeStreamCaptureMode(&mode_);
+    }
+
+private:
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+    int before_ = -1;
+};
+
+}  // namespace
+
+void* HostRows::create(int device, size_t bytes) {
+    const size_t page = static_cast<size_t>(sysconf(_SC_PAGESIZE));
+    bytes = std::max<size_t>(1, (bytes + page - 1) / page) * page;
+    const int fd = memfd_create("liyab_b200.rows", MFD_CLOEXEC);
+    if (fd < 0) throw make_error(Code::OutOfMemory, "no memory file for a buffer of {} bytes", bytes);
+    void* at[2] = {MAP_FAILED, MAP_FAILED};
+    if (ftruncate(fd, static_cast<off_t>(bytes)) == 0)
+        for (void*& a : at) a = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_SHARED | MAP_POPULATE, fd, 0);
+    close(fd);
+    cudaError_t err = cudaErrorMemoryAllocation;
+    if (at[0] != MAP_FAILED && at[1] != MAP_FAILED) {
+        OutsideCapture outside(device);
+        err = cudaHostRegister(at[0], bytes, cudaHostRegisterDefault);
+        if (err != cudaSuccess) cudaGetLastError();          // the caller may go on without the buffer: no launch is to find this error
+    }
+    if (err != cudaSuccess) {
+        for (void* a : at)
+            if (a != MAP_FAILED) munmap(a, bytes);
+        cuda_check(err, "cudaHostRegister");
+    }
+    std::lock_guard<std::mutex> lock(host_pages_mutex);
+    host_pages[reinterpret_cast<uintptr_t>(at[1])] = HostPages{static_cast<char*>(at[0]), bytes, device};
+    return at[1];
+}
+
+void HostRows::destroy(void* rows) noexcept {
+    HostPages pages;
+    {
+        std::lock_guard<std::mutex> lock(host_pages_mutex);
+        const auto it = host_pages.find(reinterpret_cast<uintptr_t>(rows));
+        if (it == host_pages.end()) return;
+        pages = it->second;
+        host_pages.erase(it);
+    }
+    {
+        OutsideCapture outside(pages.device);
+        if (cudaHostUnregister(pages.locked) != cudaSuccess) cudaGetLastError();
+    }
+    munmap(pages.locked, pages.bytes);
+    munmap(rows, pages.bytes);
+}
+
+void* HostRows::device_side(void* p, size_t bytes) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    std::lock_guard<std::mutex> lock(host_pages_mutex);
+    auto it = host_pages.upper_bound(at);
+    if (it == host_pages.begin()) return p;
+    --it;
+    const size_t offset = at - it->first;
+    return offset <= it->second.bytes && bytes <= it->second.bytes - offset ? it->second.locked + offset : p;
 }
 
 Event::Event(bool timing) { LIYAB_CUDA(cudaEventCreateWithFlags(&event_, timing ? cudaEventDefault : cudaEventDisableTiming)); }

@@ -61,6 +61,17 @@ private:
     size_t bytes_ = 0;
 };
 
+// Host memory that a device copies into at the link's rate and that is ordinary memory to everyone else: the same pages at two addresses, of
+// which only the first is page-locked for the device.  With page-locked memory in its hands a program's asynchronous copy out of it would read it
+// some time later, when the buffer may hold another step's rows; from the second address CUDA has read everything when the call returns.
+class HostRows {
+public:
+    static void* create(int device, size_t bytes);       // the second address
+    static void destroy(void* rows) noexcept;
+    // Where the device writes `bytes` that are to appear at `p`: the first address of a buffer that holds them, else p itself.
+    static void* device_side(void* p, size_t bytes);
+};
+
 class Event {
 public:
     explicit Event(bool timing = false);

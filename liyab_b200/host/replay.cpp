@@ -25,7 +25,7 @@ StepOutput Replayer::step(const std::vector<StepEntry>& entries, float* host, si
     const size_t rows = out.rows.size(), vocab = static_cast<size_t>(loaded->model->spec.vocab_size());
     const bool fits = rows * vocab <= capacity;
     if (host != nullptr && fits && rows > 0)
-        LIYAB_CUDA(cudaMemcpy2DAsync(host, vocab * 4, out.logits.data, static_cast<size_t>(out.logits.stride) * 4, vocab * 4, rows,
+        LIYAB_CUDA(cudaMemcpy2DAsync(HostRows::device_side(host, rows * vocab * 4), vocab * 4, out.logits.data, static_cast<size_t>(out.logits.stride) * 4, vocab * 4, rows,
                                      cudaMemcpyDeviceToHost, loaded->runtime.stream));
     LIYAB_CUDA(cudaStreamSynchronize(loaded->runtime.stream));
     return out;

@@ -271,8 +271,8 @@ LB_API int32_t lb_replayer_describe(const lb_replayer* r, char* buffer, size_t s
 LB_API int32_t lb_replayer_step(lb_replayer* r, size_t n_entries, const int64_t* requests, const int32_t* n_tokens,
                                 const int32_t* tokens, const int32_t* n_want, const int32_t* want, float* logits,
                                 size_t logits_capacity, int32_t* n_rows);
-/* Host memory that the device copies to by itself (page-locked): a `logits` buffer made of it takes a step's rows at the link's rate, any
- * other one at a fraction of it.  Making one costs as much as many steps: keep it. */
+/* Host memory for `logits`: a step's rows arrive in it at the link's rate, in any other memory at a fraction of it.  To the caller it is ordinary
+ * memory (CUDA does not count it as page-locked: a copy out of it has read it when the call returns).  Making one costs as much as many steps: keep it. */
 LB_API int32_t lb_host_buffer_create(int32_t device, size_t bytes, void** out);
 LB_API void lb_host_buffer_destroy(void* buffer);
 /* How a step whose request i brings q_start[i + 1] - q_start[i] tokens on n_past[i] launches an attention: 1 single tokens by the decode kernel, 2 portions by
