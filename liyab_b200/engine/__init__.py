@@ -11,7 +11,9 @@ the step function themselves.
 from __future__ import annotations
 
 import ctypes as C
+import os
 import threading
+import weakref
 from dataclasses import dataclass, field
 from typing import Any, Callable, Dict, Hashable, List, Optional, Sequence, Tuple
 
@@ -203,7 +205,7 @@ class _HostRows:
     costs its page faults and a copy by the processor (64 rows of 50,257: 2.0 ms a step, 0.25 ms this way).  An array from here is the caller's;
     its buffer comes back when nothing refers to the array any more.  At most `limit` bytes are held, arrays in use included; what does not fit is an
     ordinary array, and so is what a caller asks for who keeps IN_USE arrays already (making a buffer takes longer than the copy that it saves).  Safe
-    with several threads; closing frees what is not in use, the rest goes with its arrays."""
+    with several threads, and a forked process keeps what its parent was handed; closing frees what is not in use, the rest goes with its arrays."""
 
     IN_USE = 8
     REST = 64          # requests between two times that buffers give way to one of another size
@@ -212,10 +214,10 @@ class _HostRows:
         """What an array keeps alive: gives its buffer back when it dies."""
 
         def __init__(self, rows, address, size):
-            self.rows, self.address, self.size = rows, address, size
+            self.rows, self.address, self.size, self.generation = rows, address, size, rows._generation
 
         def __del__(self):
-            self.rows._give(self.address, self.size)
+            self.rows._give(self)
 
     def __init__(self, device: int = 0, limit: int = 128 << 20, lib=None):
         self._lib, self._device, self._limit = lib or _capi.lib(), device, limit
@@ -223,6 +225,8 @@ class _HostRows:
         self._free: List[Tuple[int, int]] = []      # (bytes, address)
         self._held, self._out, self._closed = 0, 0, False
         self._requests, self._gave_way = 0, -self.REST
+        self._generation: Optional[int] = 0      # counts forks: a child still reads what was handed out before
+        _all_host_rows.add(self)
 
     def array(self, rows: int, cols: int) -> np.ndarray:
         need = 4 * rows * cols
@@ -258,19 +262,34 @@ class _HostRows:
         self._held -= buffer[0]
         self._lib.lb_host_buffer_destroy(buffer[1])
 
-    def _give(self, address: int, size: int) -> None:
+    def _give(self, lease) -> None:
         with self._lock:
+            if self._generation is None:         # a forked child: the buffers are its parent's
+                return
             self._out -= 1
-            if self._closed:
-                self._destroy((size, address))
+            if self._closed or lease.generation != self._generation:
+                self._destroy((lease.size, lease.address))
             else:
-                self._free.append((size, address))
+                self._free.append((lease.size, lease.address))
+
+    def _forked(self, child: bool) -> None:
+        if child:
+            self._lock, self._generation, self._closed = threading.RLock(), None, True
+            self._free.clear()
+        else:
+            with self._lock:
+                self._generation += 1
 
     def close(self) -> None:
         with self._lock:
             self._closed = True
             while self._free:
                 self._destroy(self._free.pop())
+
+
+_all_host_rows: "weakref.WeakSet[_HostRows]" = weakref.WeakSet()
+os.register_at_fork(after_in_parent=lambda: [r._forked(False) for r in list(_all_host_rows)],
+                    after_in_child=lambda: [r._forked(True) for r in list(_all_host_rows)])
 
 
 class Replayer:

@@ -3,6 +3,8 @@ from __future__ import annotations
 
 import ctypes as C
 import gc
+import mmap
+import os
 import threading
 
 import numpy as np
@@ -125,3 +127,37 @@ def test_a_caller_who_keeps_its_arrays_soon_gets_ordinary_ones(lib):
     for _ in range(20):
         rows.array(1, 10)
     assert lib.made == rows.IN_USE
+
+
+class SharedLib(FakeLib):
+    """Buffers that a forked child shares with its parent, as the real ones are."""
+
+    def lb_host_buffer_create(self, device, size, out):
+        pages = mmap.mmap(-1, size)
+        memory = (C.c_char * size).from_buffer(pages)
+        self.live[C.addressof(memory)] = memory
+        self.made += 1
+        out._obj.value = C.addressof(memory)
+        return 0
+
+
+def test_a_forked_child_keeps_what_it_was_handed():
+    lib = SharedLib()
+    rows = _HostRows(limit=8 * PIECE, lib=lib)
+    a = rows.array(1, 10)
+    a[:] = 3.0
+    ready, told = os.pipe()
+    child = os.fork()
+    if child == 0:
+        os.read(ready, 1)
+        good = (a == 3.0).all() and rows.array(1, 10).shape == (1, 10) and lib.made == 1
+        del a
+        os._exit(0 if good else 1)
+    del a
+    gc.collect()
+    for _ in range(5):
+        b = rows.array(1, 10)
+        b[:] = 7.0
+        del b
+    os.write(told, b"x")
+    assert os.waitpid(child, 0)[1] == 0 and lib.made == 2 and len(lib.live) == 1
