@@ -54,9 +54,9 @@ def test_only_kernels_that_take_the_shape():
 @pytest.mark.parametrize("requests,runs", [
     # us by runs / a block a token, 12 heads: 338 / 117, 252 / 57, 167 / 32, 1261 / 213, 104 / 54
     (singles(24, 300, 950) + [(0, 200)], False), ([(699, 1)] * 12 + [(0, 100)], False), ([(599, 1)] * 8 + [(0, 64)], False), ([(2999, 1)] * 24 + [(0, 200)], False),
-    ([(99, 1)] * 16 + [(0, 120)], False),
+    ([(99, 1)] * 16 + [(0, 120)], False), ([(899, 1)] * 24 + [(0, 200)], False), ([(999, 1)] * 24 + [(0, 200)], False),
     # 504 / 831, 529 / 1179, 46 / 126, 34 / 122, 19 / 68, 213 / 1420, 28 / 82
-    ([(899, 1)] * 100 + [(0, 800)], True), ([(999, 1)] * 120 + [(0, 1000)], True), ([(492, 8)] * 16, True), ([(484, 16)] * 8, True), ([(0, 20)] * 10, True),
+    ([(899, 1)] * 100 + [(0, 800)], True), ([(999, 1)] * 120 + [(0, 1000)], True), ([(492, 8)] * 16, True), ([(484, 16)] * 8, True), ([(488, 12)] * 10, True), ([(0, 20)] * 10, True),
     ([(2700, 300)], True), ([(313, 87)], True)])
 def test_float32_runs(requests, runs):
     assert plan(requests, 12, dtype="float32") == (RUNS if runs else 0)

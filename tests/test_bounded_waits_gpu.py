@@ -1,7 +1,7 @@
 """A wait inside a kernel that nothing ends runs to its limit, reports it and lets the kernel return.
 
 The failure is made on the host's order and faults nothing: one launch is told to leave a barrier one signal
-short (the tensor-core product's accumulator-ready barrier; one block's arrival at the fused step's first grid
+short (the tensor-core products' accumulator-ready barriers; one block's arrival at the fused step's first grid
 barrier).  The waiting threads poll to their limit of about two seconds, write the status word and go to the
 kernel's end, where tensor memory is given back.  The tests check the word, that the device still computes right
 results afterwards, and what the engine does with a step that reported one."""
@@ -30,6 +30,7 @@ def no_order_left_behind():
     yield
     withhold_next(0, False)
     withhold_next(1, False)
+    withhold_next(2, False)
     device_status()
 
 
@@ -54,6 +55,33 @@ def test_product_whose_accumulator_is_never_reported_gives_up_and_the_next_one_i
     for _ in range(3):
         out.fill_(float("nan"))
         ops.gemm_tcgen05(a, w, None, out, M)
+        torch.cuda.synchronize()
+        assert (out.double() - want).abs().max().item() <= 1e-5 * max(1.0, want.abs().max().item())
+    assert device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("M,N,K,residual", [(300, 200, 320, True), (9472, 1536, 768, False)])
+def test_two_sm_product_whose_accumulator_is_never_reported_stops_both_blocks(M, N, K, residual):
+    """One tile a pair, with a residual on its way; and three, so that the other roles are found waiting in the middle of their rings."""
+    from liyab_b200 import ops
+    from liyab_b200.engine import device_status, withhold_next
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(6)
+    a = torch.randn((M, K), generator=g).to(torch.bfloat16).to(dev)
+    w = (torch.randn((N, K), generator=g) * 0.2).to(torch.bfloat16).to(dev)
+    res = torch.randn((M, N), generator=g).to(dev) if residual else None
+    want = a.double() @ w.double().t() + (res.double() if residual else 0.0)
+    out = torch.zeros((M, N), dtype=torch.float32, device=dev)
+    assert device_status() == (0, 0)
+    withhold_next(2)
+    ops.gemm_pair(a, w, None, out, M, residual=res)
+    torch.cuda.synchronize()
+    word, barrier = device_status()
+    assert word >> 12 == 0xE and (word >> 8 & 0xF) in (1, 3, 5), f"a role of the two-SM product reports itself: {word:#x}"
+    assert barrier == 0
+    for _ in range(3):
+        out.fill_(float("nan"))
+        ops.gemm_pair(a, w, None, out, M, residual=res)
         torch.cuda.synchronize()
         assert (out.double() - want).abs().max().item() <= 1e-5 * max(1.0, want.abs().max().item())
     assert device_status() == (0, 0)
