@@ -36,7 +36,7 @@ def singles(n, lo, hi):
     # Many blocks without rows: the mma.sync kernel for a short portion (the tcgen05 kernel has 0.82 of its speed there, 0.95 to 0.93 in two launches).
     (12, singles(30, 50, 250) + [(0, 130)], 0), (25, singles(30, 300, 900) + [(0, 130)], APART), (12, singles(60, 900, 1000) + [(0, 130)], APART),
     # Portions alone: the tcgen05 kernel for long ones (0.94 to 0.86 of its speed by the other), the other one for many short ones (0.87 to 0.94).
-    (12, [(0, 1024)], TCGEN05), (12, [(0, 1000)] * 2, TCGEN05), (25, [(0, 1000)] * 2, TCGEN05), (25, [(0, 100)] * 20, 0), (25, [(350, 64)] * 20, 0), (16, [(350, 40)] * 20, 0)])
+    (12, [(0, 1024)], TCGEN05), (12, [(0, 1000)] * 2, TCGEN05), (25, [(0, 1000)] * 2, TCGEN05), (25, [(0, 218), (0, 441), (0, 583), (0, 560), (0, 541)], TCGEN05), (25, [(0, 100)] * 20, 0), (25, [(350, 64)] * 20, 0), (16, [(350, 40)] * 20, 0)])
 def test_choices_that_were_measured(heads, requests, want):
     assert plan(requests, heads) == want
     assert plan(requests[::-1], heads) == want          # whatever their order
