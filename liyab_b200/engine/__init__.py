@@ -204,10 +204,11 @@ class _HostRows:
     """Host memory for steps' logits, kept from step to step: the device copies into it at the link's rate, where a fresh array
     costs its page faults and a copy by the processor (64 rows of 50,257: 2.0 ms a step, 0.25 ms this way).  An array from here is the caller's;
     its buffer comes back when nothing refers to the array any more.  At most `limit` bytes are held, arrays in use included; what does not fit is an
-    ordinary array, and so is what a caller asks for who keeps IN_USE arrays already (making a buffer takes longer than the copy that it saves).  Safe
-    with several threads, and a forked process keeps what its parent was handed; closing frees what is not in use, the rest goes with its arrays."""
+    ordinary array.  A buffer costs more to make than it saves a step (1.6 ms for 1.6 MB, 6.4 ms for 12.9 MB; 0.24 and 1.5 ms): after the first few, one more is
+    made for every time that one is used again, so a caller who keeps its arrays soon gets ordinary ones.  Safe with several threads, and a forked process
+    keeps what its parent was handed; closing frees what is not in use, the rest goes with its arrays."""
 
-    IN_USE = 4         # a buffer takes 1.6 ms to make for 1.6 MB and 6.4 ms for 12.9 MB, and saves a step 0.24 and 1.5 ms: it pays once it is used again
+    FIRST, MOST = 4, 32      # buffers that may be made before any is used again; that earlier use may pay for
     REST = 64          # requests between two times that buffers give way to one of another size
 
     class _Lease:
@@ -223,7 +224,7 @@ class _HostRows:
         self._lib, self._device, self._limit = lib or _capi.lib(), device, limit
         self._lock = threading.RLock()      # a lease may die, by the garbage collector, inside these methods
         self._free: List[Tuple[int, int]] = []      # (bytes, address)
-        self._held, self._out, self._closed = 0, 0, False
+        self._held, self._credit, self._closed = 0, self.FIRST, False
         self._requests, self._gave_way = 0, -self.REST
         self._generation: Optional[int] = 0      # counts forks: a child still reads what was handed out before
         _all_host_rows.add(self)
@@ -233,10 +234,9 @@ class _HostRows:
         size = -(-need // 65536) * 65536
         with self._lock:
             self._requests += 1
-            buffer = self._take(size) if size <= self._limit and self._out < self.IN_USE and not self._closed else None
-            if buffer is None:
-                return np.empty((rows, cols), dtype=np.float32)
-            self._out += 1
+            buffer = self._take(size) if size <= self._limit and not self._closed else None
+        if buffer is None:
+            return np.empty((rows, cols), dtype=np.float32)
         memory = (C.c_float * (rows * cols)).from_address(buffer[1])
         memory.lease = self._Lease(self, buffer[1], buffer[0])
         return np.frombuffer(memory, dtype=np.float32).reshape(rows, cols)
@@ -245,7 +245,10 @@ class _HostRows:
         fit = min((b for b in self._free if size <= b[0] <= 2 * size), default=None)
         if fit is not None:
             self._free.remove(fit)
+            self._credit = min(self._credit + 1, self.MOST)
             return fit
+        if self._credit <= 0:
+            return None
         if self._held + size > self._limit:
             if self._held - sum(b[0] for b in self._free) + size > self._limit or self._requests - self._gave_way < self.REST:
                 return None
@@ -256,6 +259,7 @@ class _HostRows:
         if self._lib.lb_host_buffer_create(self._device, size, C.byref(out)) != 0:
             return None
         self._held += size
+        self._credit -= 1
         return size, out.value
 
     def _destroy(self, buffer) -> None:
@@ -266,7 +270,6 @@ class _HostRows:
         with self._lock:
             if self._generation is None:         # a forked child: the buffers are its parent's
                 return
-            self._out -= 1
             if self._closed or lease.generation != self._generation:
                 self._destroy((lease.size, lease.address))
             else:

@@ -119,14 +119,24 @@ def test_sizes_that_do_not_fit_beside_one_another_give_way_seldom(lib):
 def test_a_caller_who_keeps_its_arrays_soon_gets_ordinary_ones(lib):
     rows = _HostRows(limit=64 * PIECE, lib=lib)
     kept = [rows.array(1, 10) for _ in range(50)]
-    assert lib.made == rows.IN_USE
+    assert lib.made == rows.FIRST
     kept[3] = None
     kept.append(rows.array(1, 10))
-    assert lib.made == rows.IN_USE
+    assert lib.made == rows.FIRST
     del kept
     for _ in range(20):
         rows.array(1, 10)
-    assert lib.made == rows.IN_USE
+    assert lib.made == rows.FIRST
+
+
+def test_a_caller_who_uses_many_at_a_time_soon_has_buffers_for_all(lib):
+    rows = _HostRows(limit=64 * PIECE, lib=lib)
+    made = []
+    for _ in range(5):
+        session = [rows.array(1, 10) for _ in range(17)]
+        made.append(lib.made)
+        del session
+    assert made == [4, 8, 16, 17, 17]
 
 
 class SharedLib(FakeLib):
