@@ -208,7 +208,7 @@ class _HostRows:
     made for every time that one is used again, so a caller who keeps its arrays soon gets ordinary ones.  Safe with several threads, and a forked process
     keeps what its parent was handed; closing frees what is not in use, the rest goes with its arrays."""
 
-    FIRST, MOST = 4, 32      # buffers that may be made before any is used again; that earlier use may pay for
+    FIRST, MOST = 8, 32      # buffers that may be made before any is used again; that earlier use may pay for
     REST = 64          # requests between two times that buffers give way to one of another size
 
     class _Lease:

@@ -136,7 +136,7 @@ def test_a_caller_who_uses_many_at_a_time_soon_has_buffers_for_all(lib):
         session = [rows.array(1, 10) for _ in range(17)]
         made.append(lib.made)
         del session
-    assert made == [4, 8, 16, 17, 17]
+    assert made == [8, 16, 17, 17, 17]
 
 
 class SharedLib(FakeLib):
