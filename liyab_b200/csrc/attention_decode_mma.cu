@@ -414,7 +414,7 @@ decode_attention_mma_kernel(const __grid_constant__ CUtensorMap map_kv, int kv_r
     }
 }
 
-// LIYAB_B200_ATTN_CLUSTER=0 in the environment keeps the merge through global memory at every number of ranges
+// LIYAB_B200_ATTN_CLUSTER=0 in the environment keeps the merge through global memory at every number of ranges (no wide blocks either)
 // (measurements: 8 requests x 12 heads at 650 keys in 3 ranges: 7.3 us that way, 5.8 us inside a cluster).
 bool cluster_merge_enabled() {
     static const bool on = [] { const char* e = getenv("LIYAB_B200_ATTN_CLUSTER"); return e == nullptr || e[0] != '0'; }();
@@ -491,7 +491,7 @@ int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* 
     if constexpr (TMA) {
         const long pairs = (long)n_kv_head * n_seq, reach = max_keys > 0 ? max_keys : (long)table_stride << page_shift;
         const long longest = n_splits == 2 ? (pairs < 160 ? 2048 : 6144) : pairs <= 128 ? reach : 8192;
-        if (n_splits >= 2 && n_splits <= 4 && pairs >= 64 && reach <= longest) {
+        if (n_splits >= 2 && n_splits <= 4 && pairs >= 64 && reach <= longest && cluster_merge_enabled()) {
             if (n_splits == 2)
                 return Variant<HD, 8, 2, TMA>::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride,
                                                       partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, 1, distance, sink, soft_cap, bound, s);
