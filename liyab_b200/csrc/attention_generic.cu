@@ -675,8 +675,8 @@ paged_attention_f32_wide_kernel(const float* __restrict__ q, int64_t q_stride, c
     }
 }
 
-// Whether a launch takes the kernel above: float32, 16-byte rows, few enough pairs that latency and not throughput
-// sets the time, and a block's two tiles per warp fit the shared memory of an SM.
+// What a block of paged_attention_f32_few_kernel needs of an SM's shared memory; launch() takes that kernel for float32, 16-byte rows and few enough pairs that
+// latency and not throughput sets the time, where head size 64 and plain scores do not make it the one with the streams' steps side by side.
 size_t few_smem(int warps, int head_dim) {
     return (size_t)warps * (head_dim + 2 * kTile * (head_dim + 4) + kTile + 2 * kTile + head_dim + 2) * sizeof(float);
 }

@@ -342,8 +342,9 @@ int launch_by_k(const void* A, int64_t lda, const void* W, int64_t ldw, const fl
 // very 16 bytes that it will feed to its products and reads them back itself, so the ring needs no barrier, and it is kept full from
 // before the wait for the kernel before until the last chunk is asked for.  The activations of a chunk travel with its weights, or
 // (NORMED) are made here from the float32 rows as gemm_rows_kernel makes them.  Bound by the weights' way from memory:
-// 148 blocks with some 64 KB in flight each, some 100 to 136 KB of shared memory a block for up to 8 tokens, so that the next
-// launch's blocks fit beside it and ask for their weights early.
+// 148 blocks with some 64 KB in flight each.  A block takes 74 to 138 KB of shared memory for up to 8 tokens (more beyond), so that small launches
+// start beside the one before; GPT-2 XL's do not (138 KB where rows are normalised, 98 KB elsewhere, and an SM has 228), and ask for their weights as
+// the blocks before them leave.
 // Measured (GPT-2 XL, 8 requests, contexts of 360 to 880): the step's 243 launches took 483 before; 2.38 -> 2.31 ms with its logits'
 // copy, 1.98 ms since the norm is short code.  Alone with cold caches, 8 tokens: 1600 -> 6400 normed 10 us (before: norm 3.6, split product 9.2 and
 // second half 4.1), 6400 -> 1600 7.5 us (9.2 and 3.6).

@@ -40,8 +40,7 @@ public:
     std::unique_ptr<CacheManager> cache;
     std::unique_ptr<Stepper> stepper;
 
-    // Runs one step; the logits at the wanted places are copied to `host` (resized to rows * vocab).
-    // The wanted rows' logits go to `host` ([rows, vocab], room for `capacity` floats; null, or too little room: they stay on the device).
+    // Runs one step.  The wanted rows' logits go to `host` ([rows, vocab], room for `capacity` floats; null, or too little room: they stay on the device).
     StepOutput step(const std::vector<StepEntry>& entries, float* host, size_t capacity);
 };
 
