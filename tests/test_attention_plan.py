@@ -33,6 +33,7 @@ def singles(n, lo, hi):
     (12, singles(3, 50, 250) + [(0, 500)], TCGEN05), (12, singles(6, 300, 900) + [(700, 200)], TCGEN05), (12, singles(6, 50, 250) + [(300, 300)], TCGEN05),
     # ... but where they reach further than the portion (1.05 to 1.10), or their blocks would fill the GPU several times (1.15 to 1.6).
     (12, singles(6, 900, 1000) + [(0, 256)], APART | TCGEN05), (25, singles(12, 300, 900) + [(300, 500)], APART | TCGEN05), (12, singles(30, 900, 1000) + [(0, 500)], APART | TCGEN05),
+    (25, singles(16, 100, 300) + [(0, 700)], APART | TCGEN05),
     # Many blocks without rows: the mma.sync kernel for a short portion (the tcgen05 kernel has 0.82 of its speed there, 0.95 to 0.93 in two launches).
     (12, singles(30, 50, 250) + [(0, 130)], 0), (25, singles(30, 300, 900) + [(0, 130)], APART), (12, singles(60, 900, 1000) + [(0, 130)], APART),
     # Portions alone: the tcgen05 kernel for long ones (0.94 to 0.86 of its speed by the other), the other one for many short ones (0.87 to 0.94).
