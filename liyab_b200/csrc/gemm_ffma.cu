@@ -416,8 +416,8 @@ gemm_ffma_skinny_kernel(const TI* __restrict__ A, int64_t lda, const TI* __restr
 // The same for 9 to 16 tokens in float32, with the weights brought into shared memory by whole rows of a chunk: sixteen lanes copy a chunk's 256 bytes, where the
 // kernel above has every lane read 16 bytes of a chunk of its own (32 lines an instruction) and hold all sixteen pieces of it beside its sixteen sums (214
 // registers: nine warps an SM).  A thread has FPT features, eight apart, so that a piece of the activations that it reads serves FPT times four products.
-// Sums as above, in their order.  Which products take it: lb_gemm_ffma_row_features (all of them have one chunk a group; without the loop over chunks the
-// compiler keeps 72 registers instead of 214, and the kernel is up to a tenth slower).  GPT-2 small, a decode step of 12 requests: 910 -> 791 us; of 16: 946 -> 858 us.
+// Sums as above, in their order.  Which products take it: lb_gemm_ffma_row_features.  (Without the loop over chunks, which most of them go
+// through once, the compiler keeps 72 registers instead of 214, and the kernel is up to a tenth slower.)  GPT-2 small, a decode step of 12 requests: 910 -> 791 us; of 16: 946 -> 858 us.
 constexpr int kRowPitch = kChunk + 4;          // floats between the chunks of neighbouring features: eight lanes' pieces fall into 32 banks
 
 constexpr size_t skinny_rows_smem(int warps, int fpt) {
@@ -592,14 +592,16 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
 // 50257 x 768, 15.9 / 12.5 for 4096 x 1024; 4.7 / 5.5 for 768 x 64 and 22.3 / 24.7 for 256 x 6400 (bound by latency: the rows' form has a barrier more), 19.0 /
 // 25.6 for 2304 x 3072 (a block's chunks fill an SM by themselves, as do those of K = 1280).  So: two to four warps (K of 257 to 1024; one warp with 193 to
 // 256 and two rounds of blocks), enough blocks to fill the GPU, and with four warps, whose blocks of sixteen features have an SM each, rounds over the SMs
-// that are at least two thirds full (3072 x 1024: 11.5 / 12.0).  Up to eight tokens the other kernel is the faster one throughout (a step of 8 requests 615 against 632 us).
+// that are at least two thirds full (3072 x 1024: 11.5 / 12.0).  Fewer features than a wave of such blocks go by rows, eight a block, from 768 on, with 11 to 16
+// chunks, or 33 to 48 below 1536 features: alone such a product is level (768 x 3072 13.4 / 13.0), within a step it is not (GPT-2 small, 12
+// requests: 878 / 803 us with its down products by rows; medium, 9 requests: 1677 / 1647 with its output products).  Up to eight tokens the other kernel is the faster one throughout (a step of 8 requests 615 against 632 us).
 extern "C" int lb_gemm_ffma_row_features(int M, int N, int K) {
     const int n_chunks = (K + kChunk - 1) / kChunk, warps = (n_chunks + 3) / 4;
     const int round = 16 * 148, rounds = (N + round - 1) / round;
-    if (M <= 8 || M > kSkinnyTokens || n_chunks < 4 || warps > 4) return 0;
+    if (M <= 8 || M > kSkinnyTokens || n_chunks < 4) return 0;
+    if (N < round) return (N >= 768 && n_chunks > 10 && n_chunks <= 16) || (N >= 768 && N < 1536 && n_chunks > 32 && n_chunks <= 48) ? 8 : 0;
     if (warps == 1) return N >= 2 * round ? 16 : 0;
-    if (N < round) return N >= 1536 && n_chunks > 10 ? 8 : 0;
-    return warps < 4 || 3ll * N >= 2ll * rounds * round ? 16 : 0;
+    return warps < 4 || (warps == 4 && 3ll * N >= 2ll * rounds * round) ? 16 : 0;
 }
 
 extern "C" int lb_gemm_ffma(int in_dtype, int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw,

@@ -575,8 +575,9 @@ static bool tiles_shared() {
 // between products like 2048 x 1600 x 6400 (47 us here, 40 us shared) and 2048 x 3072 x 768 (16.9 us here, 17.4 us shared: short reductions leave a
 // tile's epilogue bare).
 // With 16-bit results the two are closer than with float32 ones and those estimates are too rough: of 252 products from 66 to 8192 tokens x 264 to 10240
-// features x 1024 to 6400 that they would share, 20 were 2 to 5 % slower so (2048 x 2560 x 2560 32.5 / 33.9 us, 2343 x 2560 x 1280 19.0 / 20.0).  A second
-// pair of estimates, fitted to those products round by round (the last round of blocks has L2 to itself), keeps the 176 that gain 17 % on average.
+// features x 1024 to 6400 that they would share, 20 were 2 to 5 % slower so (2343 x 2560 x 1280 19.0 / 20.0 us, 2048 x 3072 x 1024 16.3 / 16.8).  A second
+// pair of estimates, fitted to those products round by round (the last round of blocks has L2 to itself), keeps 212, which gain 14 % on average, and three of
+// the slower ones (2048 x 2560 x 2560 32.5 / 33.9).
 extern "C" int lb_gemm_shared_tile(int out_dtype, int M, int N, int K, int n_sm) {
     if (K < 1024) return 0;
     const int elem = out_dtype == LB_F32 ? 4 : 2, bn = best_tile(elem, M, N, K, n_sm, false, nullptr);
@@ -589,11 +590,11 @@ extern "C" int lb_gemm_shared_tile(int out_dtype, int M, int N, int K, int n_sm)
     if (8 * (long)shared >= 7 * here) return 0;
     if (elem == 2) {
         const long pairs = n_sm / 2, shared_tiles = (long)((M + 2 * kLaneTile - 1) / (2 * kLaneTile)) * ((N + bn_shared - 1) / bn_shared);
-        auto one = [&](long act) { return n_kb * fmax((double)act * (kLaneTile + bn) * 128 / 19.0e6, bn > 192 ? 0.44 : 0.345) + 0.8 * bn / 256; };
-        auto two = [&](long act) { return n_kb * fmax(2.0 * act * (kLaneTile + bn_shared / 2) * 128 / 13.9e6, 0.317) + 0.7 * bn_shared / 256; };
+        auto one = [&](long act) { return n_kb * fmax((double)act * (kLaneTile + bn) * 128 / 16.0e6, bn > 192 ? 0.44 : 0.345) + 0.8 * bn / 256; };
+        auto two = [&](long act) { return n_kb * fmax(2.0 * act * (kLaneTile + bn_shared / 2) * 128 / 13.9e6, 0.317) + 1.1 * bn_shared / 256; };
         const double us_one = 4.0 + (tiles / n_sm) * one(n_sm) + (tiles % n_sm != 0 ? one(tiles % n_sm) : 0.0);
         const double us_two = 5.8 + (shared_tiles / pairs) * two(pairs) + (shared_tiles % pairs != 0 ? two(shared_tiles % pairs) : 0.0);
-        if (us_two >= 0.965 * us_one) return 0;
+        if (us_two >= 0.98 * us_one) return 0;
     }
     return bn_shared;
 }

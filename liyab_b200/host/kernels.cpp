@@ -306,7 +306,7 @@ struct Tiles {
 // Microseconds of a launch of the tcgen05 kernel (128 rows and 128 keys a step, one block an SM), of the mma.sync kernel (64 and 64, several
 // blocks an SM) and of the decode kernel.  A block without rows costs the first a wave's start, half a microsecond, and the second next to nothing.
 // Fitted to 813 steps of GPT-2 small, medium and XL (none to 60 single tokens on 50 to 1000 keys beside portions of 40 to 700 tokens on 0 to 700, and one to
-// twenty portions alone), each timed in all four ways: the cheapest estimate is within 0.3 % of the fastest way on average, and at most 9 % behind it.
+// twenty portions alone), each timed in all four ways: the cheapest estimate is within 0.3 % of the fastest way on average, and at most 6 % behind it.
 double tcgen05_cost(const Tiles& t, double heads, double blocks, double sms) {
     return 3.2 + std::max(1.7 * t.longest, 1.9 * (t.steps + 2.1 * t.count) * heads / sms) + 0.52 * (blocks - t.count * heads) / sms;
 }
