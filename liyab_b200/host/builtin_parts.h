@@ -106,11 +106,12 @@ public:
     int64_t max_;
 };
 
+inline AttentionUse attention_use(const kernels::AttentionShape& a) { return {a.n_head, a.n_kv_head, a.head_dim, a.mask()}; }
+
 // Chooses the attention kernel for queries q over a unit's pages.  bfloat16: a split-key decode kernel for steps of
 // single tokens (on the tensor cores where that one takes the shape, else scalar), the tensor-core prefill kernel for
-// steps with prompt portions, where they take the shape.  Else the generic kernel; all of the 32-bit engine runs on it,
+// steps with prompt portions (and the decode kernel for their single tokens, as the step's plan says), where they take the shape.  Else the generic kernel; all of the 32-bit engine runs on it,
 // so that there a position's result has the same bits however the work was cut.  `span`: the most keys a query sees.
-inline AttentionUse attention_use(const kernels::AttentionShape& a) { return {a.n_head, a.n_kv_head, a.head_dim, a.mask()}; }
 inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView& view, const Rows& att, const kernels::AttentionShape& a, int span) {
     const int T = ctx.n_tokens, S = ctx.n_seq;
     const int n_pages = view.group->pool.num_pages();
@@ -132,7 +133,10 @@ inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView
             return;
         }
     }
-    AttentionPlan plan = ctx.attention_plan(attention_use(a));
+    // An attention that its mixer does not list is planned here; a captured step keeps to the plan of the step that it was recorded from.
+    AttentionPlan plan;
+    if (const AttentionPlan* p = ctx.attention_plan(attention_use(a)); p != nullptr) plan = *p;
+    else if (!ctx.decode_only) plan = kernels::attention_plan(ctx.runtime, a, ctx.host_q_start.data(), ctx.host_n_past.data(), S, ctx.max_q_len);
     plan.apart = plan.apart && kernels::decode_mma_supports(a);
     if (ctx.runtime.dtype == DType::BF16 && kernels::prefill_supports(a)) {
         kernels::prefill_attention(ctx.runtime, q, T, cache, n_pages, ctx.q_start, ctx.n_past, view.block_table, view.table_width, att, S, ctx.max_q_len,

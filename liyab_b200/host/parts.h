@@ -181,10 +181,10 @@ struct StepContext {
     cudaStream_t stream() const { return runtime.stream; }
     // The unit's pages [page, K|V, kv_head, slot, head_dim] and its group's view.
     void* kv(int unit, const GroupView** view) const;
-    AttentionPlan attention_plan(const AttentionUse& use) const {
+    const AttentionPlan* attention_plan(const AttentionUse& use) const {
         for (const auto& [u, plan] : attention)
-            if (u == use) return plan;
-        return AttentionPlan{};
+            if (u == use) return &plan;
+        return nullptr;
     }
     // The unit's state storage [slot, ...]; index it with `state_slots`.
     void* state(int unit, size_t* slot_bytes = nullptr) const;
@@ -238,7 +238,7 @@ class Mixer : public Part {
 public:
     virtual std::optional<KvNeed> kv_need() const { return std::nullopt; }
     virtual std::optional<StateNeed> state_need() const { return std::nullopt; }
-    // The attentions that the mixer launches by `attend`.
+    // The attentions that the mixer launches by `attend`, so that captured steps that launch them in other ways are kept apart.
     virtual std::vector<AttentionUse> attention_uses() const { return {}; }
     // Adds the mixer's output for the step's tokens to the residual stream x; `h` is its normalised input.
     virtual void forward(StepContext& ctx, const Rows& h, const Rows& x, CacheUnit unit) = 0;
