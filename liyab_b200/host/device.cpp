@@ -95,9 +95,10 @@ public:
     explicit OutsideCapture(int device) {
         cudaThreadExchangeStreamCaptureMode(&mode_);
         if (cudaGetDevice(&before_) != cudaSuccess) before_ = -1;
-        if (before_ != device) cudaSetDevice(device);
+        if (before_ != device) status_ = cudaSetDevice(device);
         else before_ = -1;
     }
+    cudaError_t status() const { return status_; }
     ~OutsideCapture() {
         if (before_ >= 0) cudaSetDevice(before_);
         cudaThreadExchangeStreamCaptureMode(&mode_);
@@ -105,6 +106,7 @@ public:
 
 private:
     cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+    cudaError_t status_ = cudaSuccess;
     int before_ = -1;
 };
 
@@ -122,7 +124,8 @@ void* HostRows::create(int device, size_t bytes) {
     cudaError_t err = cudaErrorMemoryAllocation;
     if (at[0] != MAP_FAILED && at[1] != MAP_FAILED) {
         OutsideCapture outside(device);
-        err = cudaHostRegister(at[0], bytes, cudaHostRegisterDefault);
+        err = outside.status();
+        if (err == cudaSuccess) err = cudaHostRegister(at[0], bytes, cudaHostRegisterDefault);
         if (err != cudaSuccess) cudaGetLastError();          // the caller may go on without the buffer: no launch is to find this error
     }
     if (err != cudaSuccess) {

@@ -58,3 +58,11 @@ def test_arrays_may_die_while_a_stream_is_captured(engine):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, x)
+
+
+def test_a_buffer_for_a_device_that_is_not_there_is_refused():
+    import ctypes as C
+    from liyab_b200 import _capi
+    out = C.c_void_p(1)
+    assert _capi.lib().lb_host_buffer_create(99, 1 << 16, C.byref(out)) != 0 and not out.value
+    assert torch.ones(2, device="cuda").sum().item() == 2.0          # no error is left behind, and the device is the one it was
