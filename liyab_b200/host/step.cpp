@@ -22,7 +22,9 @@ Stepper::Stepper(DecoderModel& model_, CacheManager& cache_, const StepperOption
     cache.stream = model.runtime.stream;
     model_capturable_ = model.capturable();
     attention_uses_ = model.attention_uses();
-    if (attention_uses_.size() > 21) attention_uses_.resize(21);       // three bits each in a step's key; others launch in one way
+    if (attention_uses_.size() > 21) attention_uses_.resize(21);       // three bits each in a step's key; others are planned where they run
+    singles_planned_ = false;
+    for (const AttentionUse& use : attention_uses_) singles_planned_ = singles_planned_ || !decode_covers(use);
     // Decode steps of a few tokens go to the one-kernel path where the model is made of standard parts.
     if (o.fused_decode) fused_ = FusedDecodeStack::try_build(model, cache);
 }
@@ -109,25 +111,35 @@ StepOutput Stepper::step(const std::vector<StepEntry>& entries, const DeviceToke
     return StepOutput{logits, std::move(layout.out_rows)};
 }
 
+kernels::AttentionShape Stepper::attention_shape(const AttentionUse& use) const {
+    kernels::AttentionShape a;
+    a.n_head = use.n_head;
+    a.n_kv_head = use.n_kv_head;
+    a.head_dim = use.head_dim;
+    a.page_size = cache.page_size;
+    (use.mask < 0 ? a.chunk : a.window) = std::abs(use.mask);
+    return a;
+}
+
+// Steps of single tokens go to the decode kernels where one takes the shape (float32: to the one that all its steps share).
+bool Stepper::decode_covers(const AttentionUse& use) const {
+    const kernels::AttentionShape a = attention_shape(use);
+    return model.runtime.dtype == DType::F32 || kernels::decode_mma_supports(a) || kernels::decode_scalar_supports(a);
+}
+
 void Stepper::plan_attention(const std::vector<int>& rows, const std::vector<int64_t>& q_len) {
     attention_plan_.clear();
     attention_bits_ = 0;
     const int64_t longest = *std::max_element(q_len.begin(), q_len.end());
+    if (longest == 1 && !singles_planned_) return;
     std::vector<int32_t> q_start{0}, n_past;
     for (size_t i = 0; i < rows.size(); ++i) {
         q_start.push_back(q_start.back() + static_cast<int32_t>(q_len[i]));
         n_past.push_back(static_cast<int32_t>(cache.length_of_row[static_cast<size_t>(rows[i])]));
     }
     for (const AttentionUse& use : attention_uses_) {
-        kernels::AttentionShape a;
-        a.n_head = use.n_head;
-        a.n_kv_head = use.n_kv_head;
-        a.head_dim = use.head_dim;
-        a.page_size = cache.page_size;
-        (use.mask < 0 ? a.chunk : a.window) = std::abs(use.mask);
-        // Steps of single tokens go to the decode kernels where one takes the shape.
-        if (longest == 1 && (model.runtime.dtype == DType::F32 || kernels::decode_mma_supports(a) || kernels::decode_scalar_supports(a))) continue;
-        const AttentionPlan plan = kernels::attention_plan(model.runtime, a, q_start.data(), n_past.data(), static_cast<int>(rows.size()),
+        if (longest == 1 && decode_covers(use)) continue;
+        const AttentionPlan plan = kernels::attention_plan(model.runtime, attention_shape(use), q_start.data(), n_past.data(), static_cast<int>(rows.size()),
                                                            static_cast<int>((longest + 63) / 64 * 64));
         attention_bits_ |= static_cast<uint64_t>(plan.bits()) << (3 * attention_plan_.size());
         attention_plan_.emplace_back(use, plan);

@@ -28,6 +28,7 @@
 
 #include "decoder.h"
 #include "fused_decode.h"
+#include "kernels.h"
 
 namespace liyab {
 
@@ -110,6 +111,8 @@ private:
                  const DeviceTokens* dt, CapturedStep* fixed, int max_q_len, Layout* out);
     void drop_graph(CapturedStep& g);
     void plan_attention(const std::vector<int>& rows, const std::vector<int64_t>& q_len);
+    kernels::AttentionShape attention_shape(const AttentionUse& use) const;
+    bool decode_covers(const AttentionUse& use) const;
 
     std::unique_ptr<FusedDecodeStack> fused_;
     std::map<ShapeKey, CapturedStep> graphs_;
@@ -125,6 +128,7 @@ private:
     std::vector<AttentionUse> attention_uses_;                                 // the model's
     std::vector<std::pair<AttentionUse, AttentionPlan>> attention_plan_;       // in this step
     uint64_t attention_bits_ = 0;
+    bool singles_planned_ = false;                                             // steps of single tokens have an attention to plan too
 };
 
 }  // namespace liyab
