@@ -214,8 +214,10 @@ class _HostRows:
     class _Lease:
         """What an array keeps alive: gives its buffer back when it dies."""
 
-        def __init__(self, rows, address, size):
-            self.rows, self.address, self.size, self.generation = rows, address, size, rows._generation
+        __slots__ = ("rows", "buffer", "generation")
+
+        def __init__(self, rows, buffer):
+            self.rows, self.buffer, self.generation = rows, buffer, rows._generation
 
         def __del__(self):
             self.rows._give(self)
@@ -230,23 +232,28 @@ class _HostRows:
         _all_host_rows.add(self)
 
     def array(self, rows: int, cols: int) -> np.ndarray:
-        need = 4 * rows * cols
-        size = -(-need // 65536) * 65536
+        size = (4 * rows * cols + 65535) & ~65535
         with self._lock:
-            self._requests += 1
-            buffer = self._take(size) if size <= self._limit and not self._closed else None
+            buffer = self._take(size)
         if buffer is None:
             return np.empty((rows, cols), dtype=np.float32)
         memory = (C.c_float * (rows * cols)).from_address(buffer[1])
-        memory.lease = self._Lease(self, buffer[1], buffer[0])
-        return np.frombuffer(memory, dtype=np.float32).reshape(rows, cols)
+        memory.lease = self._Lease(self, buffer)
+        return np.ndarray((rows, cols), dtype=np.float32, buffer=memory)
 
     def _take(self, size: int) -> Optional[Tuple[int, int]]:
-        fit = min((b for b in self._free if size <= b[0] <= 2 * size), default=None)
+        self._requests += 1
+        fit = None
+        for b in self._free:
+            if size <= b[0] <= 2 * size and (fit is None or b < fit):
+                fit = b
         if fit is not None:
             self._free.remove(fit)
-            self._credit = min(self._credit + 1, self.MOST)
+            if self._credit < self.MOST:
+                self._credit += 1
             return fit
+        if size > self._limit or self._closed:
+            return None
         if self._credit <= 0:
             return None
         if self._held + size > self._limit:
@@ -271,9 +278,9 @@ class _HostRows:
             if self._generation is None:         # a forked child: the buffers are its parent's
                 return
             if self._closed or lease.generation != self._generation:
-                self._destroy((lease.size, lease.address))
+                self._destroy(lease.buffer)
             else:
-                self._free.append((lease.size, lease.address))
+                self._free.append(lease.buffer)
 
     def _forked(self, child: bool) -> None:
         if child:
