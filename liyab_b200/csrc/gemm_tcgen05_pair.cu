@@ -5,8 +5,8 @@
 // 128 tokens and half of the tile's features (32 KB a k-block at BN = 256) and keeps the 128 x BN sums of its own tokens, 4.2 MFLOP for
 // those 32 KB.  The float32 results and residuals pass through four strips of shared memory instead of a whole tile, which leaves
 // room for five stages.
-// Measured (B200, back to back, TFLOP/s; one block a tile / here / cuBLAS): 2343 x 6400 x 1600 993 / 1241 / 1182, with GELU 909 / 1064 / -;
-// 2343 x 1600 x 6400 with residual 657 / 1149 / 1148; 2343 x 4800 x 1600 961 / 1194 / 1111.  GPT-2 XL, five prompts of 2,343 tokens: 11.77 -> 9.87 ms
+// Measured (B200, 20 launches a graph, TFLOP/s; one block a tile / here / cuBLAS with bfloat16 results and a bare epilogue): 2343 x 6400 x 1600 1062 / 1246 /
+// 1347, with GELU 983 / 1147 / -; 2343 x 1600 x 6400 with residual 705 / 1183 / 1337; 2343 x 4800 x 1600 997 / 1221 / 1289.  GPT-2 XL, five prompts of 2,343 tokens: 11.77 -> 9.87 ms
 // a step.  A k-block takes 0.31 to 0.34 us whatever the tile's features and however few tiles run (the products alone would take 0.26 us at 256
 // features), and two producer threads instead of one change nothing.
 //
