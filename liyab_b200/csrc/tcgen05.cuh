@@ -114,6 +114,20 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
         : "memory");
 }
 
+// One lane of a converged warp.  tcgen05.mma takes its descriptors and addresses from uniform registers: issued inside a branch on the
+// lane's number, every operand of every instruction is moved there one by one (80 to 90 cycles an instruction, measured by cycle
+// stamps in the attention kernel); where the whole warp walks the loop and one lane is elected for the instruction alone, the
+// operands are made in uniform registers to begin with.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t elected;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(elected));
+    return elected != 0;
+}
+
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");

@@ -303,12 +303,16 @@ struct Tiles {
     }
 };
 
-// Microseconds of a launch of the tcgen05 kernel (128 rows and 128 keys a step, one block an SM), of the mma.sync kernel (64 and 64, several
-// blocks an SM) and of the decode kernel.  A block without rows costs the first a wave's start, half a microsecond, and the second next to nothing.
-// Fitted to 813 steps of GPT-2 small, medium and XL (none to 60 single tokens on 50 to 1000 keys beside portions of 40 to 700 tokens on 0 to 700, and one to
-// twenty portions alone), each timed in all four ways: the cheapest estimate is within 0.3 % of the fastest way on average, and at most 6 % behind it.
-double tcgen05_cost(const Tiles& t, double heads, double blocks, double sms) {
-    return 3.2 + std::max(1.7 * t.longest, 1.9 * (t.steps + 2.1 * t.count) * heads / sms) + 0.52 * (blocks - t.count * heads) / sms;
+// Microseconds of a launch of the tcgen05 kernel (128 rows and 128 keys a step, two blocks an SM), of the mma.sync kernel (64 and 64, several
+// blocks an SM) and of the decode kernel.  The last two were fitted to 813 steps of GPT-2 small, medium and XL (none to 60 single tokens on 50 to 1000 keys
+// beside portions of 40 to 700 tokens on 0 to 700, and one to twenty portions alone), the first to launches of one to sixteen portions of 37 to 1024 tokens on 0 to
+// 896 with 12 and 25 heads (us measured / estimated: 1 x 37 3.9 / 4.1, 16 x 128 6.5 / 6.3, 8 x 180 7.1 / 7.1, 1 x 453 8.8 / 9.0, 453 on 300 12.3 / 12.3,
+// 1 x 1024 15.4 / 15.6, 5 x 469 18.5 / 18.3, 2 x 1024 with 25 heads 22.1 / 21.4; the mma.sync kernel 4.1 to 62 there).
+// Steps of twenty requests and more were not timed again with this kernel: they keep the estimate, and so the choice, of the kernel
+// before it (one block an SM, which a block without rows cost half a microsecond a wave).
+double tcgen05_cost(const Tiles& t, double heads, double grid, double all_tiles, bool many, double sms) {
+    if (many) return 3.2 + std::max(1.7 * t.longest, 1.9 * (t.steps + 2.1 * t.count) * heads / sms) + 0.52 * (all_tiles - t.count * heads) / sms;
+    return 2.4 + std::max(1.65 * t.longest, 1.16 * (t.steps + 1.56 * t.count) * heads / sms) + 0.25 * (grid - t.count * heads) / sms;
 }
 double mma_cost(const Tiles& t, double heads, double sms) { return 1.8 + std::max(2.15 * t.longest, 1.15 * (t.steps + 0.4 * t.count) * heads / sms); }
 double decode_cost(double longest, double all, double heads, double sms) { return 2.5 + std::max(0.35 * longest, 0.6 * all * heads / sms) / 128; }
@@ -356,14 +360,15 @@ AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const i
             all_single += keys;
         }
     }
-    const double never = 1e30, blocks = static_cast<double>(n_seq) * heads * ((max_q_len + 127) / 128);
+    const double never = 1e30, all_tiles = static_cast<double>(n_seq) * heads * ((max_q_len + 127) / 128);
+    const double grid = std::min(all_tiles, heads * (q_start[n_seq] / 128 + n_seq));
     const bool tc = prefill_tc_supports(a), decode = longest_single > 0 && decode_mma_supports(a);
     const double singles = decode ? decode_cost(longest_single, all_single, heads, sms) : never;
     double best = never;
     for (const bool apart : {false, true})
         for (const bool tcgen05 : {true, false}) {
             const int which = apart ? 0 : 1;
-            const double cost = (!tcgen05 ? mma_cost(narrow[which], heads, sms) : tc ? tcgen05_cost(wide[which], heads, blocks, sms) : never) + (apart ? singles : 0);
+            const double cost = (!tcgen05 ? mma_cost(narrow[which], heads, sms) : tc ? tcgen05_cost(wide[which], heads, grid, all_tiles, n_seq >= 20, sms) : never) + (apart ? singles : 0);
             if (cost < best) {
                 best = cost;
                 plan.apart = apart;

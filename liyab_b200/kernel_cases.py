@@ -167,20 +167,21 @@ def case_prefill_attention(args) -> None:
     from . import ops
     dev = torch.device("cuda:0")
     S, L, H, hd, ps = args.seqs, args.length, args.heads, args.head_dim, 16
-    pages_per = -(-L // ps)
+    pages_per = -(-(L + args.past) // ps)
     cache = torch.randn(S * pages_per, 2, H, ps, hd, device=dev).to(torch.bfloat16)
     table = torch.arange(S * pages_per, dtype=torch.int32, device=dev).view(S, pages_per)
     q = torch.randn(S * L, H * hd, device=dev).to(torch.bfloat16)
     out = torch.empty_like(q)
     q_start = torch.arange(0, (S + 1) * L, L, dtype=torch.int32, device=dev)
-    n_past = torch.zeros(S, dtype=torch.int32, device=dev)
+    n_past = torch.full((S,), args.past, dtype=torch.int32, device=dev)
+    torch.cuda.synchronize()
 
     def launch():
         ops.prefill_attention(q, cache, q_start, n_past, table, out, S, L, H, H, hd, ps, hd ** -0.5, 0,
                               tcgen05=False if args.mma_sync else None, soft_cap=args.soft_cap, score_bound=args.score_bound)
 
     ms = _graph_timed(launch, args.reps) if args.graph else _timed(launch, args.reps)
-    flop = S * H * (L * L / 2) * hd * 4
+    flop = S * H * (L * L / 2 + L * args.past) * hd * 4
     print(f"prefill-attention seqs={S} length={L} heads={H} head_dim={hd}{f" soft cap {args.soft_cap:g}" if args.soft_cap else ""}: {ms * 1e3:.1f} us, {flop / ms / 1e9:.1f} TFLOP/s "
           f"(causal half of the square)")
 
@@ -359,6 +360,7 @@ def main(argv=None) -> int:
     a = sub.add_parser("prefill-attention")
     a.add_argument("--seqs", type=int, default=2)
     a.add_argument("--length", type=int, default=1024)
+    a.add_argument("--past", type=int, default=0, help="earlier tokens of every request")
     a.add_argument("--heads", type=int, default=12)
     a.add_argument("--head-dim", type=int, default=64)
     a.add_argument("--reps", type=int, default=20)

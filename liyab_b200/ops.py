@@ -517,9 +517,8 @@ def prefill_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tenso
     if q.stride(1) != 1 or out.stride(1) != 1:
         raise invalid_argument("prefill attention: q and out must be dense within a row")
     if tcgen05 is None:
-        # The tcgen05 kernel walks a long tile's keys about 1.4x faster, but runs one block per SM, so it wins while the launch is bound by its longest
-        # blocks (up to about four blocks per SM).  The engine knows the requests' lengths and estimates both (lb_attention_plan); here they
-        # are on the device.
+        # The tcgen05 kernel is the faster one up to about four blocks per SM.  The engine knows the requests' lengths and estimates both
+        # (lb_attention_plan); here they are on the device.
         blocks = n_seq * n_head * -(-max_q_len // 128)
         tcgen05 = (prefill_attention_tc_supports(n_head, n_kv_head, head_dim, page_size) and q.stride(0) % 8 == 0
                    and out.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
