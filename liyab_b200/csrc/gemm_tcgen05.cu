@@ -87,7 +87,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_lane, const __grid_c
     constexpr uint32_t kTmemCols = BN < 32 ? 32 : BN;
     constexpr uint32_t kStageBytes = (kLaneTile + BN) * kBlockK * sizeof(__nv_bfloat16);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // one number for the warp: see elect_one
     const int n0 = blockIdx.x * (TOKENS_ON_LANES ? BN : kLaneTile);     // first output feature of the tile
     const int m0 = blockIdx.y * (TOKENS_ON_LANES ? kLaneTile : BN);     // first token of the tile
     const int lane_row0 = TOKENS_ON_LANES ? m0 : n0, col_row0 = TOKENS_ON_LANES ? n0 : m0;
@@ -116,59 +116,64 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_lane, const __grid_c
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = s.tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, s.tmem_base, 0);
 
     if (warp == 0) {
-        if (lane == 0) {
-            // The weights of the first ring of stages are asked for before the kernel before this one has ended
-            // (they do not depend on it); the activations of those stages follow once it has.
-            const int ahead = n_kb < STAGES ? n_kb : STAGES;
-            for (int kb = 0; kb < ahead; ++kb) {
+        // The whole warp walks these loops and one lane issues the copies (see elect_one).
+        // The weights of the first ring of stages are asked for before the kernel before this one has ended
+        // (they do not depend on it); the activations of those stages follow once it has.
+        const int ahead = n_kb < STAGES ? n_kb : STAGES;
+        for (int kb = 0; kb < ahead; ++kb) {
+            if (elect_one()) {
                 mbar_expect_tx(&s.full[kb], kStageBytes);
                 if (TOKENS_ON_LANES) tma_load_2d(s.col_tile[kb], &map_col, &s.full[kb], (kb_first + kb) * kBlockK, col_row0);
                 else tma_load_2d(s.lane_tile[kb], &map_lane, &s.full[kb], (kb_first + kb) * kBlockK, lane_row0);
             }
-            lb_wait_for_predecessor();
-            lb_dependents_may_launch();
-            for (int kb = 0; kb < ahead; ++kb) {
+        }
+        lb_wait_for_predecessor();
+        lb_dependents_may_launch();
+        for (int kb = 0; kb < ahead; ++kb) {
+            if (elect_one()) {
                 if (TOKENS_ON_LANES) tma_load_2d(s.lane_tile[kb], &map_lane, &s.full[kb], (kb_first + kb) * kBlockK, lane_row0);
                 else tma_load_2d(s.col_tile[kb], &map_col, &s.full[kb], (kb_first + kb) * kBlockK, col_row0);
             }
-            int issued = ahead;
-            for (int kb = ahead; kb < n_kb; ++kb) {
-                const int st = kb % STAGES;
-                const uint32_t ph = (kb / STAGES) & 1;
-                if (!mbar_wait(&s.empty[st], ph ^ 1, abort_flag)) {
-                    atomicCAS(&g_status, 0, (1 << 8) | st);
-                    s.abort_flag = 1;
-                    break;
-                }
+        }
+        int issued = ahead;
+        for (int kb = ahead; kb < n_kb; ++kb) {
+            const int st = kb % STAGES;
+            const uint32_t ph = (kb / STAGES) & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(&s.empty[st], ph ^ 1, abort_flag))) {
+                atomicCAS(&g_status, 0, (1 << 8) | st);
+                s.abort_flag = 1;
+                break;
+            }
+            if (elect_one()) {
                 mbar_expect_tx(&s.full[st], kStageBytes);
                 tma_load_2d(s.lane_tile[st], &map_lane, &s.full[st], (kb_first + kb) * kBlockK, lane_row0);
                 tma_load_2d(s.col_tile[st], &map_col, &s.full[st], (kb_first + kb) * kBlockK, col_row0);
-                issued = kb + 1;
             }
-            if (s.abort_flag != 0 && issued > 0) {
-                // Leave no copy in flight: the last stage issued signals its full barrier when its bytes landed.
-                const int kb = issued - 1;
-                mbar_wait(&s.full[kb % STAGES], (kb / STAGES) & 1, nullptr);
-            }
+            issued = kb + 1;
+        }
+        if (s.abort_flag != 0 && issued > 0) {
+            // Leave no copy in flight: the last stage issued signals its full barrier when its bytes landed.
+            const int kb = issued - 1;
+            mbar_wait(&s.full[kb % STAGES], (kb / STAGES) & 1, nullptr);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc(kLaneTile, BN);
-            bool ok = true;
-            for (int kb = 0; kb < n_kb && ok; ++kb) {
-                const int st = kb % STAGES;
-                const uint32_t ph = (kb / STAGES) & 1;
-                if (!mbar_wait(&s.full[st], ph, abort_flag)) {
-                    atomicCAS(&g_status, 0, (2 << 8) | st);
-                    s.abort_flag = 1;
-                    ok = false;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t l_addr = smem_u32(s.lane_tile[st]), c_addr = smem_u32(s.col_tile[st]);
+        constexpr uint32_t idesc = umma_idesc(kLaneTile, BN);
+        bool ok = true;
+        for (int kb = 0; kb < n_kb && ok; ++kb) {
+            const int st = kb % STAGES;
+            const uint32_t ph = (kb / STAGES) & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(&s.full[st], ph, abort_flag))) {
+                atomicCAS(&g_status, 0, (2 << 8) | st);
+                s.abort_flag = 1;
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t l_addr = smem_u32(s.lane_tile[st]), c_addr = smem_u32(s.col_tile[st]);
+            if (elect_one()) {
 #pragma unroll
                 for (int k = 0; k < kBlockK / kUmmaK; ++k) {
                     const uint32_t off = k * kUmmaK * sizeof(__nv_bfloat16);
@@ -176,10 +181,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_lane, const __grid_c
                 }
                 umma_commit(&s.empty[st]);      // the stage is free once these MMAs have read it
             }
-            // The accumulator is complete once every MMA retired.  (`withhold_ready`: a test's launch, whose
-            // epilogue then meets a barrier that nothing signals and has to give up at its limit.)
-            if (ok && withhold_ready == 0) umma_commit(&s.acc_ready);
         }
+        // The accumulator is complete once every MMA retired.  (`withhold_ready`: a test's launch, whose
+        // epilogue then meets a barrier that nothing signals and has to give up at its limit.)
+        if (ok && withhold_ready == 0 && elect_one()) umma_commit(&s.acc_ready);
     } else {
         // Epilogue: warp w may touch tensor-memory lanes 32 * (w % 4) .. + 31.
         const int quarter = warp & 3;

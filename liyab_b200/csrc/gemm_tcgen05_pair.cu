@@ -120,7 +120,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     volatile int* abort_flag = &c->abort_flag;
     const uint32_t stages_u32 = smem_u32(base), full_u32 = smem_u32(&c->full[0]), empty_u32 = smem_u32(&c->empty[0]);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // one number for the warp: see elect_one
     uint32_t rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const int m_tiles = (M + 2 * kLaneTile - 1) / (2 * kLaneTile), n_tiles = (N + BN - 1) / BN, total = m_tiles * n_tiles;
@@ -152,66 +152,70 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     __syncthreads();
     cluster_barrier();                          // both blocks' barriers and tensor memory exist
     tc_fence_after();
-    const uint32_t tmem_base = c->tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, c->tmem_base, 0);
 
     if (warp == 0) {
-        if (lane == 0) {
-            const uint32_t lead_full = peer_address(full_u32, 0);
-            uint32_t st = 0, empty_parity = 1;                      // a fresh barrier passes a wait for parity 1
-            bool ok = true, first = true;
-            uint32_t last_stage = 0, last_parity = 0;
-            int issued = 0;
-            for (int tile = pair; tile < total && ok; tile += n_pairs) {
-                const int m0 = (tile % m_tiles) * 2 * kLaneTile + (int)rank * kLaneTile, n0 = (tile / m_tiles) * BN + (int)rank * (BN / 2);
-                int kb = 0;
-                if (first) {
-                    // The first ring: the weights are asked for before the kernel before this one has ended, the activations after.
-                    first = false;
-                    const int ahead = n_kb < n_stages ? n_kb : n_stages;
-                    for (int i = 0; i < ahead; ++i) {
+        // The whole warp walks these loops and one lane issues the copies (see elect_one).
+        const uint32_t lead_full = peer_address(full_u32, 0);
+        uint32_t st = 0, empty_parity = 1;                      // a fresh barrier passes a wait for parity 1
+        bool ok = true, first = true;
+        uint32_t last_stage = 0, last_parity = 0;
+        int issued = 0;
+        for (int tile = pair; tile < total && ok; tile += n_pairs) {
+            const int m0 = (tile % m_tiles) * 2 * kLaneTile + (int)rank * kLaneTile, n0 = (tile / m_tiles) * BN + (int)rank * (BN / 2);
+            int kb = 0;
+            if (first) {
+                // The first ring: the weights are asked for before the kernel before this one has ended, the activations after.
+                first = false;
+                const int ahead = n_kb < n_stages ? n_kb : n_stages;
+                for (int i = 0; i < ahead; ++i) {
+                    if (elect_one()) {
                         if (rank == 0) expect_tx_u32(full_u32 + 8 * i, 2 * stage_bytes);
                         tma_load_pair(stages_u32 + i * stage_bytes + kATileBytes, &map_w, lead_full + 8 * i, i * kBlockK, n0);
                     }
-                    lb_wait_for_predecessor();
-                    lb_dependents_may_launch();
-                    for (int i = 0; i < ahead; ++i) tma_load_pair(stages_u32 + i * stage_bytes, &map_a, lead_full + 8 * i, i * kBlockK, m0);
-                    kb = issued = ahead;
-                    last_stage = (uint32_t)ahead - 1;
-                    st = (uint32_t)ahead;
-                    if (st == (uint32_t)n_stages) {
-                        st = 0;
-                        empty_parity ^= 1;
-                    }
                 }
-                for (; kb < n_kb; ++kb) {
-                    if (!wait_u32(empty_u32 + 8 * st, empty_parity, abort_flag)) {
-                        give_up(c, status, 1, st, rank);
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t dst = stages_u32 + st * stage_bytes, bar = lead_full + 8 * st;
+                lb_wait_for_predecessor();
+                lb_dependents_may_launch();
+                for (int i = 0; i < ahead; ++i)
+                    if (elect_one()) tma_load_pair(stages_u32 + i * stage_bytes, &map_a, lead_full + 8 * i, i * kBlockK, m0);
+                kb = issued = ahead;
+                last_stage = (uint32_t)ahead - 1;
+                st = (uint32_t)ahead;
+                if (st == (uint32_t)n_stages) {
+                    st = 0;
+                    empty_parity ^= 1;
+                }
+            }
+            for (; kb < n_kb; ++kb) {
+                if (!__all_sync(0xffffffffu, wait_u32(empty_u32 + 8 * st, empty_parity, abort_flag))) {
+                    give_up(c, status, 1, st, rank);
+                    ok = false;
+                    break;
+                }
+                const uint32_t dst = stages_u32 + st * stage_bytes, bar = lead_full + 8 * st;
+                if (elect_one()) {
                     if (rank == 0) expect_tx_u32(full_u32 + 8 * st, 2 * stage_bytes);
                     tma_load_pair(dst, &map_a, bar, kb * kBlockK, m0);
                     tma_load_pair(dst + kATileBytes, &map_w, bar, kb * kBlockK, n0);
-                    ++issued;
-                    last_stage = st;
-                    last_parity = empty_parity ^ 1;
-                    if (++st == (uint32_t)n_stages) {
-                        st = 0;
-                        empty_parity ^= 1;
-                    }
+                }
+                ++issued;
+                last_stage = st;
+                last_parity = empty_parity ^ 1;
+                if (++st == (uint32_t)n_stages) {
+                    st = 0;
+                    empty_parity ^= 1;
                 }
             }
-            if (*abort_flag != 0 && issued > 0) {
-                // Leave no copy in flight.  The first block's barrier counts both blocks' copies; the other block, which has none of its own
-                // to ask, gives its last ones a millisecond, hundreds of times what they take.
-                if (rank == 0) mbar_wait(&c->full[last_stage], last_parity, nullptr);
-                const long long t0 = clock64();
-                while (clock64() - t0 < 2000000) {}
-            }
+        }
+        if (*abort_flag != 0 && issued > 0) {
+            // Leave no copy in flight.  The first block's barrier counts both blocks' copies; the other block, which has none of its own
+            // to ask, gives its last ones a millisecond, hundreds of times what they take.
+            if (rank == 0) mbar_wait(&c->full[last_stage], last_parity, nullptr);
+            const long long t0 = clock64();
+            while (clock64() - t0 < 2000000) {}
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t idesc = umma_idesc(2 * kLaneTile, BN);
             const uint32_t desc_hi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
             const uint32_t lo0 = ((stages_u32 & 0x3FFFFu) >> 4) | (1u << 16);
@@ -221,31 +225,33 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             bool ok = true;
             for (int tile = pair; tile < total && ok; tile += n_pairs, ++it) {
                 const int buf = it & 1;
-                if (!wait_cluster(smem_u32(&c->acc_empty[buf]), (uint32_t)(((it >> 1) & 1) ^ 1), abort_flag)) {
+                if (!__all_sync(0xffffffffu, wait_cluster(smem_u32(&c->acc_empty[buf]), (uint32_t)(((it >> 1) & 1) ^ 1), abort_flag))) {
                     give_up(c, status, 5, buf, rank);
                     break;
                 }
                 tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)buf * 256u;
                 for (int kb = 0; kb < n_kb; ++kb) {
-                    if (!wait_u32(full_u32 + 8 * st, full_parity, abort_flag)) {
+                    if (!__all_sync(0xffffffffu, wait_u32(full_u32 + 8 * st, full_parity, abort_flag))) {
                         give_up(c, status, 2, st, rank);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t a_lo = lo0 + st * lo_stage, w_lo = a_lo + lo_w;
-                    umma_pair(d, a_lo, w_lo, desc_hi, idesc, kb != 0 ? 1u : 0u);
+                    if (elect_one()) {
+                        umma_pair(d, a_lo, w_lo, desc_hi, idesc, kb != 0 ? 1u : 0u);
 #pragma unroll
-                    for (uint32_t k = 1; k < kBlockK / kUmmaK; ++k) umma_pair(d, a_lo + 2 * k, w_lo + 2 * k, desc_hi, idesc, 1u);
-                    commit_pair(empty_u32 + 8 * st);
+                        for (uint32_t k = 1; k < kBlockK / kUmmaK; ++k) umma_pair(d, a_lo + 2 * k, w_lo + 2 * k, desc_hi, idesc, 1u);
+                        commit_pair(empty_u32 + 8 * st);
+                    }
                     if (++st == (uint32_t)n_stages) {
                         st = 0;
                         full_parity ^= 1;
                     }
                 }
                 // (`withhold`: a test's launch, whose epilogues find nothing and give up.)
-                if (ok && (withhold == 0 || it != 0)) commit_pair(smem_u32(&c->acc_full[buf]));
+                if (ok && (withhold == 0 || it != 0) && elect_one()) commit_pair(smem_u32(&c->acc_full[buf]));
             }
         }
     } else {

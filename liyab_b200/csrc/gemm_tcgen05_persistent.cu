@@ -106,7 +106,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const uint32_t stages_u32 = smem_u32(base), staging_u32 = smem_u32(staging), bias_u32 = smem_u32(bias_s);
     const uint32_t full_u32 = smem_u32(&c->full[0]), empty_u32 = smem_u32(&c->empty[0]);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;      // one number for the warp: see elect_one
     const int m_tiles = (M + kLaneTile - 1) / kLaneTile, n_tiles = (N + BN - 1) / BN;
     const int total = m_tiles * n_tiles;
     uint32_t rank = 0;
@@ -147,7 +147,7 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = c->tmem_base;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, c->tmem_base, 0);
     if (threadIdx.x == 0) stamp(timing, 1);
     if constexpr (PAIR) {
         // Both blocks' barriers exist before one arrives at the other's.
@@ -156,132 +156,139 @@ gemm_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
 
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t st = 0, empty_parity = 1;                      // a fresh barrier passes a wait for parity 1
-            int issued = 0, last_stage = 0;
-            uint32_t last_parity = 0;
-            bool res_in_flight = false;
-            uint32_t res_parity = 0;
-            int it = 0;
-            bool ok = true;
-            // The residual goes out once the ring is full for the first time in a tile (or after the tile's
-            // last k-block): by then the loads that the MMAs wait for first are under way.
-            const int res_at = (n_kb < n_stages ? n_kb : n_stages) - 1;
-            // The first tile's first ring of stages: the weights are asked for before the kernel before this one has
-            // ended (they do not depend on it); activations and residual follow once it has.
-            const int ahead = res_at + 1;
-            int kb_start = 0;
-            if (cta < total) {
-                const int tile = cta;
-                const int m0 = (tile % m_tiles) * kLaneTile, n0 = (tile / m_tiles) * BN;
-                for (int kb = 0; kb < ahead; ++kb) {
+        // The whole warp walks these loops and one lane issues the copies (see elect_one).
+        uint32_t st = 0, empty_parity = 1;                      // a fresh barrier passes a wait for parity 1
+        int issued = 0, last_stage = 0;
+        uint32_t last_parity = 0;
+        bool res_in_flight = false;
+        uint32_t res_parity = 0;
+        int it = 0;
+        bool ok = true;
+        // The residual goes out once the ring is full for the first time in a tile (or after the tile's
+        // last k-block): by then the loads that the MMAs wait for first are under way.
+        const int res_at = (n_kb < n_stages ? n_kb : n_stages) - 1;
+        // The first tile's first ring of stages: the weights are asked for before the kernel before this one has
+        // ended (they do not depend on it); activations and residual follow once it has.
+        const int ahead = res_at + 1;
+        int kb_start = 0;
+        if (cta < total) {
+            const int tile = cta;
+            const int m0 = (tile % m_tiles) * kLaneTile, n0 = (tile / m_tiles) * BN;
+            for (int kb = 0; kb < ahead; ++kb) {
+                if (elect_one()) {
                     expect_tx_u32(full_u32 + 8 * kb, stage_bytes);
                     tma_load_u32(stages_u32 + kb * stage_bytes + kATileBytes, &map_w, full_u32 + 8 * kb, (kb_lo + kb) * kBlockK, n0);
                 }
-                lb_wait_for_predecessor();
-                lb_dependents_may_launch();
-                for (int kb = 0; kb < ahead; ++kb)
-                    tma_load_u32(stages_u32 + kb * stage_bytes, &map_a, full_u32 + 8 * kb, (kb_lo + kb) * kBlockK, m0);
-                issued = ahead;
-                last_stage = ahead - 1;
-                last_parity = 0;
-                st = (uint32_t)ahead;
-                if (st == (uint32_t)n_stages) {
-                    st = 0;
-                    empty_parity ^= 1;
-                }
-                if (res_here) {                    // the staging buffer is free before the first tile
+            }
+            lb_wait_for_predecessor();
+            lb_dependents_may_launch();
+            for (int kb = 0; kb < ahead; ++kb)
+                if (elect_one()) tma_load_u32(stages_u32 + kb * stage_bytes, &map_a, full_u32 + 8 * kb, (kb_lo + kb) * kBlockK, m0);
+            issued = ahead;
+            last_stage = ahead - 1;
+            last_parity = 0;
+            st = (uint32_t)ahead;
+            if (st == (uint32_t)n_stages) {
+                st = 0;
+                empty_parity ^= 1;
+            }
+            if (res_here) {                    // the staging buffer is free before the first tile
+                if (elect_one()) {
                     mbar_expect_tx(&c->res_full, (uint32_t)((n_strips - res_first + res_step - 1) / res_step) * kStripBytes);
                     for (int sp = res_first; sp < n_strips; sp += res_step)
                         tma_load_2d(staging + (size_t)sp * kStripBytes, &map_res, &c->res_full, n0 + sp * kStripCols, m0);
-                    res_in_flight = true;
-                    res_parity = 0;
                 }
-                kb_start = ahead;
+                res_in_flight = true;
+                res_parity = 0;
             }
-            for (int tile = cta; tile < total && ok; tile += n_cta, ++it) {
-                const int m0 = (tile % m_tiles) * kLaneTile, n0 = (tile / m_tiles) * BN;
-                for (int kb = kb_start; kb < n_kb; ++kb) {
-                    if (!wait_u32(empty_u32 + 8 * st, empty_parity, abort_flag)) {
-                        give_up(c, status, 1, st);
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t dst = stages_u32 + st * stage_bytes, bar = full_u32 + 8 * st;
+            kb_start = ahead;
+        }
+        for (int tile = cta; tile < total && ok; tile += n_cta, ++it) {
+            const int m0 = (tile % m_tiles) * kLaneTile, n0 = (tile / m_tiles) * BN;
+            for (int kb = kb_start; kb < n_kb; ++kb) {
+                if (!__all_sync(0xffffffffu, wait_u32(empty_u32 + 8 * st, empty_parity, abort_flag))) {
+                    give_up(c, status, 1, st);
+                    ok = false;
+                    break;
+                }
+                const uint32_t dst = stages_u32 + st * stage_bytes, bar = full_u32 + 8 * st;
+                if (elect_one()) {
                     expect_tx_u32(bar, stage_bytes);
                     tma_load_u32(dst, &map_a, bar, (kb_lo + kb) * kBlockK, m0);
                     tma_load_u32(dst + kATileBytes, &map_w, bar, (kb_lo + kb) * kBlockK, n0);
-                    ++issued;
-                    last_stage = st;
-                    last_parity = empty_parity ^ 1;
-                    if (++st == (uint32_t)n_stages) {
-                        st = 0;
-                        empty_parity ^= 1;
-                    }
-                    if (res_here && kb == res_at) {
-                        if (!mbar_wait(&c->staging_free, (it & 1) ^ 1, abort_flag)) {
-                            give_up(c, status, 4, 0);
-                            ok = false;
-                            break;
-                        }
-                        mbar_expect_tx(&c->res_full, (uint32_t)((n_strips - res_first + res_step - 1) / res_step) * kStripBytes);
-                        for (int sp = res_first; sp < n_strips; sp += res_step)
-                            tma_load_2d(staging + (size_t)sp * kStripBytes, &map_res, &c->res_full, n0 + sp * kStripCols, m0);
-                        res_in_flight = true;
-                        res_parity = it & 1;
-                    }
                 }
-                kb_start = 0;
-            }
-            stamp(timing, 7);
-            if (*abort_flag != 0) {
-                // Leave no copy in flight: the barriers of the last loads issued complete when their bytes landed.
-                if (issued > 0) mbar_wait(&c->full[last_stage], last_parity, nullptr);
-                if (res_in_flight) mbar_wait(&c->res_full, res_parity, nullptr);
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc(kLaneTile, BN);
-            // Descriptor words: the high one is the same for every tile (stride between 8-row groups 1024 bytes,
-            // version 1, 128-byte swizzle); the low one holds the start address >> 4 and moves with stage and k.
-            const uint32_t desc_hi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
-            const uint32_t lo0 = ((stages_u32 & 0x3FFFFu) >> 4) | (1u << 16);
-            const uint32_t lo_stage = stage_bytes >> 4, lo_w = kATileBytes >> 4;
-            uint32_t st = 0, full_parity = 0;
-            int it = 0;
-            bool ok = true;
-            for (int tile = cta; tile < total && ok; tile += n_cta, ++it) {
-                const int buf = it & 1;
-                if (!mbar_wait(&c->acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag)) {
-                    give_up(c, status, 5, buf);
-                    break;
+                ++issued;
+                last_stage = st;
+                last_parity = empty_parity ^ 1;
+                if (++st == (uint32_t)n_stages) {
+                    st = 0;
+                    empty_parity ^= 1;
                 }
-                tc_fence_after();
-                const uint32_t d = tmem_base + (uint32_t)buf * acc_stride;
-                for (int kb = 0; kb < n_kb; ++kb) {
-                    if (!wait_u32(full_u32 + 8 * st, full_parity, abort_flag)) {
-                        give_up(c, status, 2, st);
+                if (res_here && kb == res_at) {
+                    if (!__all_sync(0xffffffffu, mbar_wait(&c->staging_free, (it & 1) ^ 1, abort_flag))) {
+                        give_up(c, status, 4, 0);
                         ok = false;
                         break;
                     }
-                    tc_fence_after();
-                    if (it == 0 && kb == 0) stamp(timing, 2);
-                    const uint32_t a_lo = lo0 + st * lo_stage, w_lo = a_lo + lo_w;
+                    if (elect_one()) {
+                        mbar_expect_tx(&c->res_full, (uint32_t)((n_strips - res_first + res_step - 1) / res_step) * kStripBytes);
+                        for (int sp = res_first; sp < n_strips; sp += res_step)
+                            tma_load_2d(staging + (size_t)sp * kStripBytes, &map_res, &c->res_full, n0 + sp * kStripCols, m0);
+                    }
+                    res_in_flight = true;
+                    res_parity = it & 1;
+                }
+            }
+            kb_start = 0;
+        }
+        if (lane == 0) stamp(timing, 7);
+        if (*abort_flag != 0) {
+            // Leave no copy in flight: the barriers of the last loads issued complete when their bytes landed.
+            if (issued > 0) mbar_wait(&c->full[last_stage], last_parity, nullptr);
+            if (res_in_flight) mbar_wait(&c->res_full, res_parity, nullptr);
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = umma_idesc(kLaneTile, BN);
+        // Descriptor words: the high one is the same for every tile (stride between 8-row groups 1024 bytes,
+        // version 1, 128-byte swizzle); the low one holds the start address >> 4 and moves with stage and k.
+        const uint32_t desc_hi = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
+        const uint32_t lo0 = ((stages_u32 & 0x3FFFFu) >> 4) | (1u << 16);
+        const uint32_t lo_stage = stage_bytes >> 4, lo_w = kATileBytes >> 4;
+        uint32_t st = 0, full_parity = 0;
+        int it = 0;
+        bool ok = true;
+        for (int tile = cta; tile < total && ok; tile += n_cta, ++it) {
+            const int buf = it & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(&c->acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag))) {
+                give_up(c, status, 5, buf);
+                break;
+            }
+            tc_fence_after();
+            const uint32_t d = tmem_base + (uint32_t)buf * acc_stride;
+            for (int kb = 0; kb < n_kb; ++kb) {
+                if (!__all_sync(0xffffffffu, wait_u32(full_u32 + 8 * st, full_parity, abort_flag))) {
+                    give_up(c, status, 2, st);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                if (it == 0 && kb == 0 && lane == 0) stamp(timing, 2);
+                const uint32_t a_lo = lo0 + st * lo_stage, w_lo = a_lo + lo_w;
+                if (elect_one()) {
                     umma_lo(d, a_lo, w_lo, desc_hi, idesc, kb != 0 ? 1u : 0u);
 #pragma unroll
                     for (uint32_t k = 1; k < kBlockK / kUmmaK; ++k)
                         umma_lo(d, a_lo + 2 * k, w_lo + 2 * k, desc_hi, idesc, 1u);      // 16 elements = 32 bytes further
                     commit_u32(empty_u32 + 8 * st);
-                    if (++st == (uint32_t)n_stages) {
-                        st = 0;
-                        full_parity ^= 1;
-                    }
                 }
-                if (!ok) break;
-                umma_commit(&c->acc_full[buf]);
-                if (it == 0) stamp(timing, 3);
+                if (++st == (uint32_t)n_stages) {
+                    st = 0;
+                    full_parity ^= 1;
+                }
             }
+            if (!ok) break;
+            if (elect_one()) umma_commit(&c->acc_full[buf]);
+            if (it == 0 && lane == 0) stamp(timing, 3);
         }
     } else {
         // Eight warps in two groups of four: group g stages the strips g, g + 2, ...; within a group warp w owns
