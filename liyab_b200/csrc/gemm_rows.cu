@@ -85,7 +85,7 @@ struct RowNorm {
     float gain_offset;
 };
 
-__device__ void layernorm_rows_to_smem(const RowNorm& n, int M, int K, __nv_bfloat16* act, int ld, int k_pad) {
+__device__ void layernorm_rows_to_smem(const RowNorm& n, int M, int K, __nv_bfloat16* act, int ld, int k_pad, int rows) {
     constexpr int kVecs = 8;                       // float4 per lane: rows of up to 1024 values
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_vec = K / 4;
@@ -104,7 +104,7 @@ __device__ void layernorm_rows_to_smem(const RowNorm& n, int M, int K, __nv_bflo
     }
     lb_wait_for_predecessor();
     lb_dependents_may_launch();
-    for (int r = warp; r < 16; r += kWarps) {
+    for (int r = warp; r < rows; r += kWarps) {
         __nv_bfloat16* dst = act + r * ld;
         if (r >= M) {                              // rows past the step's tokens: zeros
             for (int i = lane * 8; i < k_pad; i += 256) *reinterpret_cast<uint4*>(dst + i) = make_uint4(0, 0, 0, 0);
@@ -156,21 +156,25 @@ __device__ void layernorm_rows_to_smem(const RowNorm& n, int M, int K, __nv_bflo
 // STAGE: how the activations reach shared memory.  0: chunk by chunk through two buffers (any number of tokens).
 // 1 (up to 16 tokens): all columns at once, one round trip, kept for all of the block's passes.  2 (up to 16 tokens,
 // K up to 1024): the same, made here from the float32 rows by a LayerNorm.
-template <int MT, int NG, typename TO, int STAGE = 0>
+// FEW (up to 8 tokens, STAGE 1 and 2): two feature groups are the sixteen rows of a product and the tokens its eight columns, where otherwise sixteen
+// rows of tokens, half of them empty, meet eight features: half as many products for the same sums (mma.sync is one product in some 32
+// cycles a scheduler, 0.3 of the 1.0 us that a pass over 2304 x 768 spends in them).
+template <int MT, int NG, typename TO, int STAGE = 0, bool FEW = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bfloat16* __restrict__ W, int64_t ldw,
                  const float* __restrict__ bias, const float* residual, int64_t ldr, TO* out, int64_t ldo, int M, int N, int K,
                  int act, KvScatter kv, RowNorm norm) {
     static_assert(STAGE == 0 || MT == 1, "all columns at once for up to 16 tokens only");
     static_assert(STAGE != 2 || NG == 4, "rows are normalised in the kernel for K up to 1024");
+    static_assert(!FEW || STAGE != 0, "few tokens have all columns at once");
     constexpr bool FULL = STAGE != 0;
-    constexpr int kRows = MT * 16, MC = kWRegs / NG;
+    constexpr int kRows = FEW ? 8 : MT * 16, MC = kWRegs / NG, kTileFloats = FEW ? 64 : 128;
     extern __shared__ __align__(16) uint8_t smem_bytes[];
     // The activations: two buffers of one chunk each, [2][kRows][kChunkLd]; or (FULL) all columns at once, [16][ld_full].
     __nv_bfloat16* act_s = reinterpret_cast<__nv_bfloat16*>(smem_bytes);
     const int ld_full = (K + kChunk - 1) / kChunk * kChunk + 32;        // 64 bytes mod 128 as well
-    const size_t act_bytes = FULL ? (size_t)16 * ld_full * sizeof(__nv_bfloat16) : (size_t)2 * kRows * kChunkLd * sizeof(__nv_bfloat16);
-    float* red_s = reinterpret_cast<float*>(smem_bytes + act_bytes);   // [kWarps][NG][MT][128]
+    const size_t act_bytes = FULL ? (size_t)kRows * ld_full * sizeof(__nv_bfloat16) : (size_t)2 * kRows * kChunkLd * sizeof(__nv_bfloat16);
+    float* red_s = reinterpret_cast<float*>(smem_bytes + act_bytes);   // [kWarps][NG][MT][kTileFloats]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int n_groups = (N + 7) / 8;
     const int per_cta = (n_groups + (int)gridDim.x - 1) / (int)gridDim.x;
@@ -209,13 +213,13 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bf
         if (gp == g_begin) {
             // The first pass's weights are under way; the activations come from the kernel before this one.
             if constexpr (STAGE == 2) {
-                layernorm_rows_to_smem(norm, M, K, act_s, ld_full, n_chunks * kChunk);
+                layernorm_rows_to_smem(norm, M, K, act_s, ld_full, n_chunks * kChunk, kRows);
                 __syncthreads();
             } else if constexpr (STAGE == 1) {
                 lb_wait_for_predecessor();
                 lb_dependents_may_launch();
                 const int pieces = n_chunks * kChunk / 8;
-                for (int idx = threadIdx.x; idx < 16 * pieces; idx += kThreads) {
+                for (int idx = threadIdx.x; idx < kRows * pieces; idx += kThreads) {
                     const int r = idx / pieces, p = idx - r * pieces;
                     const bool valid = r < M && p * 8 < K;
                     cp_async16(act_s + r * ld_full + p * 8, A + (valid ? (size_t)r * lda + p * 8 : 0), valid);
@@ -256,7 +260,19 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bf
                 }
                 const int kLd = FULL ? ld_full : kChunkLd;
                 const __nv_bfloat16* buf = (FULL ? act_s + c * kChunk : act_s + (size_t)(c & 1) * kRows * kChunkLd) + warp * 32 + t * 8;
-                if (c * kChunk + warp * 32 < K) {
+                if constexpr (FEW) {
+                    if (c * kChunk + warp * 32 < K) {
+                        const uint4 x = *reinterpret_cast<const uint4*>(buf + g * kLd);
+#pragma unroll
+                        for (int gi = 0; gi < NG; gi += 2) {
+                            if (gi < ng) {                            // a group that is not there: zeros
+                                const uint4 w0 = w[c * NG + gi], w1 = gi + 1 < NG ? w[c * NG + (gi + 1 < NG ? gi + 1 : gi)] : make_uint4(0, 0, 0, 0);
+                                mma_bf16(acc[gi][0], w0.x, w1.x, w0.y, w1.y, x.x, x.y);
+                                mma_bf16(acc[gi][0], w0.z, w1.z, w0.w, w1.w, x.z, x.w);
+                            }
+                        }
+                    }
+                } else if (c * kChunk + warp * 32 < K) {
 #pragma unroll
                     for (int m = 0; m < MT; ++m) {
                         const uint4 lo = *reinterpret_cast<const uint4*>(buf + (m * 16 + g) * kLd);
@@ -276,7 +292,12 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bf
         // Partial tiles of the eight warps -> shared memory -> summed in warp order -> epilogue.
 #pragma unroll
         for (int gi = 0; gi < NG; ++gi) {
-            if (gi < ng) {
+            if (FEW && gi < ng) {
+                // Feature g of the group, tokens 2t and 2t + 1: a pair's first group has the first half of the sums, its second one the other.
+                float* tile = red_s + (size_t)(warp * NG + gi) * kTileFloats;
+                tile[2 * t * 8 + g] = acc[gi & ~1][0][gi & 1 ? 2 : 0];
+                tile[(2 * t + 1) * 8 + g] = acc[gi & ~1][0][gi & 1 ? 3 : 1];
+            } else if (gi < ng) {
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
                     float* tile = red_s + ((size_t)(warp * NG + gi) * MT + m) * 128;
@@ -297,7 +318,7 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bf
                 const int m = r >> 4, rr = r & 15;
                 float v = 0.0f;
 #pragma unroll
-                for (int wp = 0; wp < kWarps; ++wp) v += red_s[((size_t)(wp * NG + gi) * MT + m) * 128 + rr * 8 + cfeat];
+                for (int wp = 0; wp < kWarps; ++wp) v += red_s[((size_t)(wp * NG + gi) * MT + m) * kTileFloats + rr * 8 + cfeat];
                 float y = lb_activate(v + early[e].x, act, act_pair);
                 if (residual != nullptr) y += early[e].y;
                 out[(size_t)r * ldo + f] = lb_from_float<TO>(y);
@@ -308,30 +329,30 @@ gemm_rows_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_bf
     }
 }
 
-template <int MT, int NG, typename TO, int STAGE = 0>
+template <int MT, int NG, typename TO, int STAGE = 0, bool FEW = false>
 int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr,
            void* out, int64_t ldo, int M, int N, int K, int act, KvScatter kv, int n_sm, cudaStream_t s, RowNorm norm = RowNorm{}) {
     const size_t ld_full = (size_t)(K + kChunk - 1) / kChunk * kChunk + 32;
-    const size_t act_bytes = STAGE != 0 ? 16 * ld_full * sizeof(__nv_bfloat16) : (size_t)2 * MT * 16 * kChunkLd * sizeof(__nv_bfloat16);
-    const size_t smem = act_bytes + (size_t)kWarps * NG * MT * 128 * sizeof(float);
+    const size_t act_bytes = STAGE != 0 ? (FEW ? 8 : 16) * ld_full * sizeof(__nv_bfloat16) : (size_t)2 * MT * 16 * kChunkLd * sizeof(__nv_bfloat16);
+    const size_t smem = act_bytes + (size_t)kWarps * NG * MT * (FEW ? 64 : 128) * sizeof(float);
     static size_t configured = 0;
     if (smem > configured) {
-        LB_CHECK_CUDA(cudaFuncSetAttribute(gemm_rows_kernel<MT, NG, TO, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        LB_CHECK_CUDA(cudaFuncSetAttribute(gemm_rows_kernel<MT, NG, TO, STAGE, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured = smem;
     }
     const int n_groups = (N + 7) / 8;
     const int grid = n_groups < n_sm ? n_groups : n_sm;
-    LB_CHECK_CUDA(lb_launch_overlapped(gemm_rows_kernel<MT, NG, TO, STAGE>, dim3(grid), dim3(kThreads), smem, s, (const __nv_bfloat16*)A, lda,
+    LB_CHECK_CUDA(lb_launch_overlapped(gemm_rows_kernel<MT, NG, TO, STAGE, FEW>, dim3(grid), dim3(kThreads), smem, s, (const __nv_bfloat16*)A, lda,
                                        (const __nv_bfloat16*)W, ldw, bias, residual, ldr, (TO*)out, ldo, M, N, K, act, kv, norm));
     return LB_OK;
 }
 
-template <int MT, typename TO, int STAGE = 0>
+template <int MT, typename TO, int STAGE = 0, bool FEW = false>
 int launch_by_k(const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr,
                 void* out, int64_t ldo, int M, int N, int K, int act, KvScatter kv, int n_sm, cudaStream_t s) {
-    if (K <= 4 * kChunk) return launch<MT, 4, TO, STAGE>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s);
-    if (K <= 8 * kChunk) return launch<MT, 2, TO, STAGE>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s);
-    return launch<MT, 1, TO, STAGE>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s);
+    if (K <= 4 * kChunk) return launch<MT, 4, TO, STAGE, FEW>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s);
+    if (K <= 8 * kChunk) return launch<MT, 2, TO, STAGE, FEW>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s);
+    return launch<MT, 1, TO, STAGE, FEW>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s);
 }
 
 // ---- up to 16 tokens, a slice of weights that does not fit a pass's registers -----------------------------------------
@@ -508,6 +529,7 @@ gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_
         if (gi < ng && r < M && f < N)
             early[e] = make_float2(bias != nullptr ? __ldg(bias + f) : 0.0f, residual != nullptr ? __ldcg(residual + (size_t)r * ldr + f) : 0.0f);
     }
+    // Up to 8 tokens a pair of groups is the sixteen rows of a product, the tokens its columns (see FEW above): acc[gi] has both groups' sums, gi even.
     float acc[GB][4];
 #pragma unroll
     for (int gi = 0; gi < GB; ++gi) acc[gi][0] = acc[gi][1] = acc[gi][2] = acc[gi][3] = 0.0f;
@@ -524,9 +546,20 @@ gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_
             lo = from[GB * kThreads];
             if constexpr (WIDE) hi = from[(GB + 1) * kThreads];
         }
+        if constexpr (!WIDE) {
+#pragma unroll
+            for (int gi = 0; gi < GB; gi += 2)
+                if (gi < ng) {
+                    const uint4 w0 = from[gi * kThreads];
+                    // (The place of a group that the block does not have holds anything: its sums are rows of their own, which nobody reads.)
+                    const uint4 w1 = gi + 1 < GB ? from[(gi + 1 < GB ? gi + 1 : gi) * kThreads] : make_uint4(0, 0, 0, 0);
+                    mma_bf16(acc[gi], w0.x, w1.x, w0.y, w1.y, lo.x, lo.y);
+                    mma_bf16(acc[gi], w0.z, w1.z, w0.w, w1.w, lo.z, lo.w);
+                }
+        }
 #pragma unroll
         for (int gi = 0; gi < GB; ++gi)
-            if (gi < ng) {
+            if (WIDE && gi < ng) {
                 const uint4 w = from[gi * kThreads];
                 mma_bf16(acc[gi], lo.x, hi.x, lo.y, hi.y, w.x, w.y);
                 mma_bf16(acc[gi], lo.z, hi.z, lo.w, hi.w, w.z, w.w);
@@ -544,8 +577,13 @@ gemm_stream_kernel(const __nv_bfloat16* __restrict__ A, int64_t lda, const __nv_
     for (int gi = 0; gi < GB; ++gi)
         if (gi < ng) {
             float* tile = red_s + (size_t)(warp * GB + gi) * ROWS * 8;
-            *reinterpret_cast<float2*>(tile + g * 8 + 2 * t) = make_float2(acc[gi][0], acc[gi][1]);
-            if constexpr (WIDE) *reinterpret_cast<float2*>(tile + (g + 8) * 8 + 2 * t) = make_float2(acc[gi][2], acc[gi][3]);
+            if constexpr (WIDE) {
+                *reinterpret_cast<float2*>(tile + g * 8 + 2 * t) = make_float2(acc[gi][0], acc[gi][1]);
+                *reinterpret_cast<float2*>(tile + (g + 8) * 8 + 2 * t) = make_float2(acc[gi][2], acc[gi][3]);
+            } else {
+                tile[2 * t * 8 + g] = acc[gi & ~1][gi & 1 ? 2 : 0];
+                tile[(2 * t + 1) * 8 + g] = acc[gi & ~1][gi & 1 ? 3 : 1];
+            }
         }
     __syncthreads();
 #pragma unroll
@@ -684,8 +722,8 @@ extern "C" int lb_gemm_rows_normed_kind(int out_dtype, const float* x, int64_t l
     auto s = static_cast<cudaStream_t>(stream_handle);
     if (lb_gemm_rows_kind(M, N, K, n_sm, 1) == 2) return stream<true>(out_dtype, nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, norm, n_sm, s);
     if (out_dtype == LB_F32)
-        return launch<1, 4, float, 2>(nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s, norm);
-    return launch<1, 4, __nv_bfloat16, 2>(nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s, norm);
+        return (M <= 8 ? launch<1, 4, float, 2, true> : launch<1, 4, float, 2>)(nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s, norm);
+    return (M <= 8 ? launch<1, 4, __nv_bfloat16, 2, true> : launch<1, 4, __nv_bfloat16, 2>)(nullptr, 0, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s, norm);
 }
 
 extern "C" int lb_gemm_rows(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias,
@@ -707,6 +745,9 @@ extern "C" int lb_gemm_rows(int out_dtype, const void* A, int64_t lda, const voi
     auto s = static_cast<cudaStream_t>(stream_handle);
     if (lb_gemm_rows_kind(M, N, K, n_sm, 0) == 2) return stream<false>(out_dtype, A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, RowNorm{}, n_sm, s);
     const int mt = (M + 15) / 16;
+    if (M <= 8)
+        return out_dtype == LB_F32 ? launch_by_k<1, float, 1, true>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s)
+                                   : launch_by_k<1, __nv_bfloat16, 1, true>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s);
 #define LB_GO(MT)                                                                                                          \
     return out_dtype == LB_F32 ? launch_by_k<MT, float>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s)   \
                                : launch_by_k<MT, __nv_bfloat16>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, kv, n_sm, s)
