@@ -200,13 +200,33 @@ void gemm_persistent(cudaStream_t s, const Rows& a, const Tensor& w, const float
                              d.page_size, s), "gemm_persistent");
 }
 
+bool gemm_narrow_takes(const Rows& a, const Tensor& w, const Rows& out, int m, const Rows* residual) {
+    return tcgen05_accepts(a, w) && lb_gemm_narrow_pays(code(out.dtype, "out"), m, static_cast<int>(w.dim(0)), static_cast<int>(w.dim(1))) != 0 &&
+           lb_gemm_narrow_supports(code(out.dtype, "out"), a.data, a.stride, w.data, w.dim(1), residual ? residual->f32() : nullptr, residual ? residual->stride : 0,
+                                   out.data, out.stride, m, static_cast<int>(w.dim(0)), static_cast<int>(w.dim(1))) != 0;
+}
+
+bool gemm_narrow_kv_supports(const Tensor& w, const Rows& out, const KvDestination& kv) {
+    return lb_gemm_narrow_kv_supports(code(out.dtype, "out"), static_cast<int>(w.dim(0)), kNone, 0, kv.q_dim, kv.n_kv_head, kv.head_dim, kv.page_size) != 0;
+}
+
+void gemm_narrow(cudaStream_t s, const Rows& a, const Tensor& w, const float* bias, const Rows& out, int m, int act, const Rows* residual, const KvDestination* kv) {
+    check_product(a, w, out, residual);
+    const KvDestination none;
+    const KvDestination& d = kv ? *kv : none;
+    check(lb_gemm_narrow(code(out.dtype, "out"), a.data, a.stride, w.data, w.dim(1), bias, residual ? residual->f32() : nullptr, residual ? residual->stride : 0,
+                         out.data, out.stride, m, static_cast<int>(w.dim(0)), static_cast<int>(w.dim(1)), act, 0, 0, d.cache, d.slot_mapping, d.q_dim,
+                         d.n_kv_head, d.head_dim, d.page_size, s), "gemm_narrow");
+}
+
 void linear(const Runtime& rt, Workspace* ws, const Rows& a, const Tensor& w, const float* bias, const Rows& out, int m,
             int act, const Rows* residual) {
     if (tcgen05_accepts(a, w)) {
         const int n = static_cast<int>(w.dim(0)), k = static_cast<int>(w.dim(1));
+        if (gemm_narrow_takes(a, w, out, m, residual)) return gemm_narrow(rt.stream, a, w, bias, out, m, act, residual, nullptr);
         if (m > 64 && gemm_persistent_tile(a, w, out, m, residual) > 0)
             return gemm_persistent(rt.stream, a, w, bias, out, m, act, residual, nullptr);
-        // Up to 64 tokens: one launch on mma.sync where every block can afford to fetch all activations (measured on
+        // Few tokens, or shapes that the kernel above declines: one launch on mma.sync where every block can afford to fetch all activations (measured on
         // B200, 64 tokens: 6-7 us against 8-9 us for K = 768; for K = 3072 the 393 KB of activations per block cost
         // more than the split of K saves: 13 us against 8 us).
         if (gemm_rows_takes(m, n, k, rt.sm_count) && gemm_rows_supports(a, w, m))

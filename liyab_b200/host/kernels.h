@@ -72,6 +72,11 @@ void gemm_rows_normed(cudaStream_t s, const Rows& x, const float* gain, const fl
                       const Rows& out, int m, int act, const Rows* residual, const KvDestination* kv, bool rms = false, float gain_offset = 0.0f);
 void gemm_rows(cudaStream_t s, const Rows& a, const Tensor& w, const float* bias, const Rows& out, int m, int act,
                const Rows* residual, const KvDestination* kv);
+// Some dozens of tokens, where that kernel is the faster one (lb_gemm_narrow_pays); with `kv` only the queries go to `out`.
+bool gemm_narrow_takes(const Rows& a, const Tensor& w, const Rows& out, int m, const Rows* residual);
+bool gemm_narrow_kv_supports(const Tensor& w, const Rows& out, const KvDestination& kv);
+void gemm_narrow(cudaStream_t s, const Rows& a, const Tensor& w, const float* bias, const Rows& out, int m, int act, const Rows* residual,
+                 const KvDestination* kv);
 int gemm_persistent_tile(const Rows& a, const Tensor& w, const Rows& out, int m, const Rows* residual);
 bool gemm_persistent_kv_supports(const Tensor& w, const Rows& out, const KvDestination& kv);
 void gemm_persistent(cudaStream_t s, const Rows& a, const Tensor& w, const float* bias, const Rows& out, int m, int act,

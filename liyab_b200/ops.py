@@ -63,6 +63,9 @@ _SIGNATURES = {
     "lb_prefill_attention_portions": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
     "lb_prefill_attention_tc_portions": [_p, _l, _i, _p, _i, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _i, _i, _f, _i, _p, _p, _f, _f, _i, _p],
     "lb_gemm_pair": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
+    "lb_gemm_narrow": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
+    "lb_gemm_narrow_pays": [_i, _i, _i, _i],
+    "lb_gemm_narrow_plan": [_i, _i, _i, _i, _p, _p],
     "lb_gemm_pair_tile": [_i, _i, _i, _i, _p],
     "lb_gemm_shared_tile": [_i, _i, _i, _i, _i],
     "lb_gemm_rows_kind": [_i, _i, _i, _i, _i],
@@ -313,6 +316,21 @@ def gemm_pair(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
     check(lib().lb_gemm_pair(_code(out.dtype, "out"), _dev(a, "a"), a.stride(0), _dev(w, "w"), w.stride(0), _opt(bias, "bias", torch.float32),
                              _opt(residual, "residual", torch.float32), residual.stride(0) if residual is not None else 0, _dev(out, "out"), out.stride(0),
                              m, n, k, ACTIVATIONS[activation], feature_tile, *_kv_args(kv), stream_ptr()), "gemm_pair")
+    return out
+
+
+def gemm_narrow(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, m: int, activation: str = "none",
+                residual: Optional[torch.Tensor] = None, features: int = 0, splits: int = 0, kv: Optional[tuple] = None) -> torch.Tensor:
+    """out[:m] = act(a[:m] @ w.T + bias) + residual in tiles of 64 or 128 tokens by `features` features, the reduction in `splits` parts
+    (0: the kernel's plan).  `kv` as for gemm_persistent."""
+    n, k = w.shape
+    if a.shape[1] != k or out.stride(1) != 1 or out.shape[1] != n or not tcgen05_accepts(a, w):
+        raise invalid_argument(f"gemm: shapes do not fit: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+    if residual is not None and (residual.shape[1] != n or residual.stride(1) != 1):
+        raise invalid_argument("gemm: residual has the wrong shape")
+    check(lib().lb_gemm_narrow(_code(out.dtype, "out"), _dev(a, "a"), a.stride(0), _dev(w, "w"), w.stride(0), _opt(bias, "bias", torch.float32),
+                               _opt(residual, "residual", torch.float32), residual.stride(0) if residual is not None else 0, _dev(out, "out"), out.stride(0),
+                               m, n, k, ACTIVATIONS[activation], features, splits, *_kv_args(kv), stream_ptr()), "gemm_narrow")
     return out
 
 
