@@ -13,7 +13,7 @@
 //   32) consecutive chunks form a group whose chunk sums are added in ascending
 //   order; the (at most 32) group sums are added in ascending order.
 //
-// Three kernels follow that order.  The tiled one (any number of tokens) cuts the groups among
+// Four kernels follow that order.  The tiled one (any number of tokens) cuts the groups among
 // four slices of a block and adds their sums in order.  The one for up to 16 tokens (decoding)
 // is bound by reading the weights once: a block owns eight features and all of K,
 // each of its 32 (warp, slot) pairs owns one group of chunks for those features,
@@ -21,12 +21,14 @@
 // flight together and multiplies them with the tokens' activations from the warp's
 // buffer in shared memory; the group sums meet in shared memory and are added in
 // order.  The third takes some products of 9 to 16 tokens in float32: the weights come into
-// shared memory by whole rows of a chunk as well.
+// shared memory by whole rows of a chunk as well.  The fourth takes most of up to 8 tokens in float32: whole rows of
+// weights by bulk copies, the activations once a block.
 //
 // Epilogue, in the reference's order (src/core/transformer.cpp:111-118, 4903-4912,
 // 5526-5532): + bias[n], activation, + residual[m, n].
 #include "api.h"
 #include "common.cuh"
+#include "tcgen05.cuh"
 
 namespace {
 
@@ -532,6 +534,179 @@ int launch_skinny_rows(const void* A, int64_t lda, const void* W, int64_t ldw, c
     return LB_OK;
 }
 
+// ---- up to 8 tokens in float32, whole rows of weights by bulk copies --------------------------------------------
+//
+// Both kernels above bring their weights and, again for every eight or sixteen features, the activations: as many bytes from L2 as the weights are, which
+// is what the logits' product was bound by (76 us for 50257 x 768 at eight tokens, 24 for its bytes), and lane by lane, 32 lines an instruction.  Here the
+// activations of all tokens stay in a block's shared memory, and the block walks groups of eight features whose rows come whole, by one bulk copy each, a ring of
+// them ahead and the first ones before the wait for the kernel before.  A thread has a feature and a group of chunks, as above, and the sums are made in the same order:
+// the same bits.  A long reduction (K = 3072) has a block's eight rows at once instead of a chunk after the other.
+// Bound by shared memory now: a warp reads nine pieces for 32 products, and few warps fit beside the rows.  With 9 to 16 tokens that was slower than the kernel
+// above (50257 x 768 107 us against 89).
+// Measured (us, before / here): 8 tokens 50257 x 768 68 / 48, 4800 x 1600 22.2 / 14.0, 1600 x 1600 8.5 / 7.1, and within a step of GPT-2 small 2304 x 768 6.2 / 4.9,
+// 768 x 3072 11.4 / 8.3, but 768 x 768 3.8 / 4.8 and 3072 x 768 6.6 / 6.9: see stream_takes.
+constexpr int kStreamFeatures = 8, kStreamTokens = 8;
+constexpr int kStreamChunkPitch = kChunk + 8;       // floats between the chunks of a token: the four chunks a warp reads fall into banks 8 apart
+__host__ __device__ constexpr int stream_row_pitch(int K) { return (K + 31) / 32 * 32 + 4; }      // eight features' pieces fall into 32 banks
+
+struct StreamShape {
+    int warps, stages;
+    size_t smem;
+};
+// Stages that fit (up to `most`; 0: not even one), two blocks an SM where that leaves each two stages.
+inline StreamShape stream_shape(int K, int most) {
+    const int n_chunks = (K + kChunk - 1) / kChunk, G = chunks_per_group(K), n_groups = (n_chunks + G - 1) / G;
+    constexpr int kFinishing = kStreamTokens * kStreamFeatures / 32;          // a thread an element at the end
+    StreamShape s{(n_groups + 3) / 4 > kFinishing ? (n_groups + 3) / 4 : kFinishing, 0, 0};
+    const size_t fixed = ((size_t)kStreamTokens * n_chunks * kStreamChunkPitch + (size_t)2 * s.warps * 4 * kStreamTokens * kStreamFeatures) * sizeof(float) + 64;
+    const size_t stage = (size_t)kStreamFeatures * stream_row_pitch(K) * sizeof(float), half = 113 * 1024, whole = 227 * 1024;
+    if (fixed + stage > whole) return s;
+    const int in_half = fixed < half ? (int)((half - fixed) / stage) : 0, in_whole = (int)((whole - fixed) / stage);
+    s.stages = in_half >= 2 || in_half >= most ? in_half : in_whole;
+    if (s.stages > most) s.stages = most;
+    if (s.stages > 8) s.stages = 8;
+    s.smem = fixed + s.stages * stage;
+    return s;
+}
+
+// Whether a product goes that way: a block has at least two stages or no second group of features.  Short reductions (one chunk a group, which the kernel of
+// eight features a block brings in one go as well) stay with that one where they have no more groups than SMs, and where the last round of blocks would be less
+// than two fifths full.
+inline bool stream_takes(int N, int K, StreamShape* shape, int* grid) {
+    static const int n_sm = [] {
+        int dev = 0, n = 0;
+        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 148;
+    }();
+    const int groups = (N + kStreamFeatures - 1) / kStreamFeatures;
+    *shape = stream_shape(K, (groups + n_sm - 1) / n_sm);
+    if (shape->stages < 1 || (shape->stages < 2 && groups > n_sm)) return false;
+    const int slots = n_sm * (shape->smem <= 113 * 1024 ? 2 : 1), last = groups % slots;
+    *grid = groups < slots ? groups : slots;
+    if (K <= 1024 && (groups <= n_sm || (groups > slots && groups < 4 * slots && last != 0 && 5 * last < 2 * slots))) return false;
+    return true;
+}
+
+__device__ __forceinline__ uint32_t ffma_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__global__ void __launch_bounds__(256)
+gemm_ffma_stream_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ W, int64_t ldw, const float* __restrict__ bias,
+                        const float* residual, int64_t ldr, float* out, int64_t ldo, int M, int N, int K, int act, int stages, int* status) {
+    constexpr int TOKENS = kStreamTokens;
+    extern __shared__ __align__(16) float stream_smem[];
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+    const int fi = lane & 7, group = warp * 4 + (lane >> 3);
+    const int n_chunks = (K + kChunk - 1) / kChunk, G = chunks_per_group(K), n_groups = (n_chunks + G - 1) / G;
+    const int w_pitch = stream_row_pitch(K), a_pitch = n_chunks * kStreamChunkPitch;
+    float* w_s = stream_smem;                                            // [stage][8][w_pitch]
+    float* a_s = w_s + (size_t)stages * kStreamFeatures * w_pitch;       // [token][chunk][64 + 8]
+    float* red = a_s + (size_t)TOKENS * a_pitch;                         // [2][group][token][8]
+    const int red_floats = n_warps * 4 * TOKENS * kStreamFeatures;
+    uint64_t* full = reinterpret_cast<uint64_t*>(red + 2 * red_floats);
+    const int n_feature_groups = (N + kStreamFeatures - 1) / kStreamFeatures, step = gridDim.x;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < stages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ffma_smem(full + i)));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    // Eight rows of weights -> a stage (by the first warp).
+    auto rows = [&](int fg, int stage) {
+        const int here = min(kStreamFeatures, N - fg * kStreamFeatures);
+        const uint32_t bar = ffma_smem(full + stage), bytes = (uint32_t)K * 4u;
+        if (lb_tc::elect_one()) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"((uint32_t)here * bytes) : "memory");
+        __syncwarp();
+        for (int i = 0; i < here; ++i)
+            if (lb_tc::elect_one())
+                asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                             ::"r"(ffma_smem(w_s + ((size_t)stage * kStreamFeatures + i) * w_pitch)), "l"(W + (size_t)(fg * kStreamFeatures + i) * ldw), "r"(bytes), "r"(bar)
+                             : "memory");
+        __syncwarp();
+    };
+    if (warp == 0)
+        for (int s = 0; s < stages; ++s)
+            if ((int)blockIdx.x + s * step < n_feature_groups) rows((int)blockIdx.x + s * step, s);
+    const lb_act_pair act_pair = lb_act_load(bias, N, act);
+    lb_wait_for_predecessor();               // the weights are under way; the activations come from the kernel before this one
+    lb_dependents_may_launch();
+    for (int idx = threadIdx.x; idx < M * n_chunks * 16; idx += blockDim.x) {
+        const int q = idx & 15, c = (idx >> 4) % n_chunks, r = (idx >> 4) / n_chunks, k = c * kChunk + 4 * q;
+        cp_async16_zfill(a_s + (size_t)r * a_pitch + c * kStreamChunkPitch + 4 * q, k < K ? A + (size_t)r * lda + k : A, k < K);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int c_begin = min(n_chunks, group * G), c_end = min(n_chunks, c_begin + G);
+    int it = 0;
+    for (int fg = blockIdx.x; fg < n_feature_groups; fg += step, ++it) {
+        const int stage = it % stages;
+        // The element that this thread finishes: its bias and residual travel under the products.
+        const int er = threadIdx.x / kStreamFeatures, ef = fg * kStreamFeatures + threadIdx.x % kStreamFeatures;
+        const bool finishes = threadIdx.x < TOKENS * kStreamFeatures && er < M && ef < N;
+        const float early_b = finishes && bias != nullptr ? __ldg(bias + ef) : 0.0f, early_r = finishes && residual != nullptr ? __ldcg(residual + (size_t)er * ldr + ef) : 0.0f;
+        {
+            // Bounded: a copy that never lands leaves a code in the status word and wrong results instead of a hang.
+            const uint32_t bar = ffma_smem(full + stage), parity = (uint32_t)(it / stages) & 1u;
+            uint32_t ok = 0;
+            const long long t0 = clock64();
+            while (!ok) {
+                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+                if (!ok && clock64() - t0 > 4000000000ll) atomicCAS(status, 0, (0x9 << 12) | 1);
+                if (!ok && clock64() - t0 > 8000000000ll) break;              // the copy has had its time again: the block may leave
+            }
+        }
+        const float* w_row = w_s + ((size_t)stage * kStreamFeatures + fi) * w_pitch;
+        float grp[TOKENS];
+#pragma unroll
+        for (int r = 0; r < TOKENS; ++r) grp[r] = 0.0f;
+        for (int c = c_begin; c < c_end; ++c) {
+            const float* w = w_row + c * kChunk;
+            const float* a = a_s + (size_t)c * kStreamChunkPitch;
+            const int quads = min(kChunk, K - c * kChunk) / 4;
+            float acc[TOKENS];
+#pragma unroll
+            for (int r = 0; r < TOKENS; ++r) acc[r] = 0.0f;
+#pragma unroll 4
+            for (int i = 0; i < quads; ++i) {
+                const float4 wq = *reinterpret_cast<const float4*>(w + 4 * i);
+#pragma unroll
+                for (int r = 0; r < TOKENS; ++r) {
+                    const float4 aq = *reinterpret_cast<const float4*>(a + (size_t)r * a_pitch + 4 * i);
+                    acc[r] = fmaf(aq.x, wq.x, acc[r]);
+                    acc[r] = fmaf(aq.y, wq.y, acc[r]);
+                    acc[r] = fmaf(aq.z, wq.z, acc[r]);
+                    acc[r] = fmaf(aq.w, wq.w, acc[r]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < TOKENS; ++r) grp[r] = c == c_begin ? acc[r] : grp[r] + acc[r];
+        }
+        float* here = red + (it & 1) * red_floats;
+#pragma unroll
+        for (int r = 0; r < TOKENS; ++r) here[(group * TOKENS + r) * kStreamFeatures + fi] = grp[r];
+        __syncthreads();                                                 // the group sums are there, and the stage has been read
+        if (warp == 0 && fg + stages * step < n_feature_groups) rows(fg + stages * step, stage);
+        if (finishes) {
+            float v = here[threadIdx.x];
+            for (int g2 = 1; g2 < n_groups; ++g2) v += here[g2 * TOKENS * kStreamFeatures + threadIdx.x];
+            if (bias != nullptr) v += early_b;
+            v = lb_activate(v, act, act_pair);
+            if (residual != nullptr) v += early_r;
+            out[(size_t)er * ldo + ef] = v;
+        }
+    }
+}
+
+int launch_stream(const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out, int64_t ldo,
+                  int M, int N, int K, int act, const StreamShape& shape, int grid, cudaStream_t s) {
+    int* status = nullptr;
+    const int rc = lb_tc_status_word(&status);
+    if (rc != LB_OK) return rc;
+    LB_CHECK_CUDA(cudaFuncSetAttribute(gemm_ffma_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    LB_CHECK_CUDA(lb_launch_overlapped(gemm_ffma_stream_kernel, dim3(grid), dim3(shape.warps * 32), shape.smem, s, (const float*)A, lda,
+                                       (const float*)W, ldw, bias, residual, ldr, (float*)out, ldo, M, N, K, act, shape.stages, status));
+    LB_CHECK_LAUNCH();
+    return LB_OK;
+}
+
 template <typename TI, typename TO>
 int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual,
            int64_t ldr, void* out, int64_t ldo, int M, int N, int K, int act, cudaStream_t s) {
@@ -545,6 +720,11 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
         // chunks, so a short reduction length makes small blocks, of which several share an SM.
         const int n_chunks = (K + kChunk - 1) / kChunk, per_group = chunks_per_group(K);
         const int n_groups = (n_chunks + per_group - 1) / per_group, warps = (n_groups + 3) / 4;
+        if constexpr (sizeof(TI) == 4 && sizeof(TO) == 4) {
+            StreamShape shape;
+            int grid = 0;
+            if (M <= kStreamTokens && stream_takes(N, K, &shape, &grid)) return launch_stream(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, shape, grid, s);
+        }
         if constexpr (sizeof(TI) == 4) {
             if (M > 8) {
                 const int features = lb_gemm_ffma_row_features(M, N, K);
