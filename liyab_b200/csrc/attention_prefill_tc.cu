@@ -128,7 +128,7 @@ __host__ __device__ constexpr uint32_t umma_idesc_b_mn(int m, int n) { return um
 // The query tile that the block of this number serves: among every 32 requests the last tiles first, which see the most keys.  The grid holds
 // no more blocks than tiles can exist among its tokens (a block that finds none still costs a launch: 0.5 us for every 148 with one block
 // an SM).  False: no such tile.
-__device__ __forceinline__ bool find_tile(const int32_t* __restrict__ q_start, int n_seq, int min_len, int number, int lane, int* seq, int* tile) {
+__device__ __forceinline__ bool find_tile(const int32_t* __restrict__ q_start, int n_seq, int min_len, int& number, int lane, int* seq, int* tile) {
     for (int s0 = 0; s0 < n_seq; s0 += 32) {
         const int s = s0 + lane, len = s < n_seq ? q_start[s + 1] - q_start[s] : 0;
         const int mine = len >= min_len ? (len + kBM - 1) / kBM : 0;
@@ -147,6 +147,163 @@ __device__ __forceinline__ bool find_tile(const int32_t* __restrict__ q_start, i
     return false;
 }
 
+// The number-th request of one token; -1: there is none.
+__device__ __forceinline__ int find_single(const int32_t* __restrict__ q_start, int n_seq, int number, int lane) {
+    for (int s0 = 0; s0 < n_seq; s0 += 32) {
+        const int s = s0 + lane;
+        const bool single = s < n_seq && q_start[s + 1] - q_start[s] == 1;
+        const uint32_t with = __ballot_sync(0xffffffffu, single);
+        if (number < __popc(with)) return s0 + __ffs(__ballot_sync(0xffffffffu, single && __popc(with & ((1u << lane) - 1u)) == number)) - 1;
+        number -= __popc(with);
+    }
+    return -1;
+}
+
+__device__ __forceinline__ void unpack_bf16(const uint4& u, float (&f)[8]) {
+    f[0] = __uint_as_float(u.x << 16); f[1] = __uint_as_float(u.x & 0xffff0000u);
+    f[2] = __uint_as_float(u.y << 16); f[3] = __uint_as_float(u.y & 0xffff0000u);
+    f[4] = __uint_as_float(u.z << 16); f[5] = __uint_as_float(u.z & 0xffff0000u);
+    f[6] = __uint_as_float(u.w << 16); f[7] = __uint_as_float(u.w & 0xffff0000u);
+}
+
+// 16 bytes global -> shared; when `valid` is false nothing is read and the destination is filled with zeros.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
+    const int bytes = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+
+// A request's one token and one head (with a key/value head of its own) by a whole block on the 32-bit units, as the decode kernel does it
+// (attention_decode_mma.cu, SINGLE): a pair of lanes has a key's score, a lane eight dims of four keys of the update.  A lane copies the pieces that it will
+// read itself, two tiles of 16 keys ahead, into places of its own (no barrier); all of a block's shared memory is on its way at once.
+// A step that mixes a portion with single tokens has blocks without a query tile anyway, and the portion's few blocks leave most of the GPU idle, while
+// a launch of their own takes the single tokens as long as the portion: a step of XL with 12 single tokens beside a portion of 453 4.44 -> 4.23 ms (host/kernels.cpp has
+// the launches and where they pay).  Bound by the bytes on their way: the two lanes of a key take its pieces in turn, so that a copy of the warp asks for
+// whole sectors (halves of 32 dims each: 22.7 us for that attention in place of 20.0, 41.5 in place of 29.9 for 4 tokens on 6000 keys); without the ring, straight to
+// registers, that step took 4.68 ms.
+template <bool PLAIN>
+__device__ void serve_single(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* cache, const int32_t* __restrict__ table, __nv_bfloat16* __restrict__ out,
+                             int pos, int head, int n_head, int page_shift, float scale, int window, const float* __restrict__ distance,
+                             const float* __restrict__ sink, float soft_cap, float bound, uint8_t* smem) {
+    constexpr int kWarps = kThreads / 32, kKeysTile = 16, kState = kHD + 2, kRing = 2;
+    static_assert(kWarps * kRing * 8 * 32 * 16 == (1 + 2 * kStages) * kTileBytes, "the rings take the place of the query, key and value tiles");
+    static_assert(kHD * sizeof(float) <= sizeof(Control), "the query lies behind them");
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint4* ring = reinterpret_cast<uint4*>(smem) + (size_t)warp * kRing * 8 * 32 + lane;      // [stage][piece: 4 of a key, 4 of values][lane]
+    float* q_s = reinterpret_cast<float*>(smem + (1 + 2 * kStages) * kTileBytes);               // the query
+    float* red = reinterpret_cast<float*>(smem);                                              // at the end: [warp][maximum, sum, 64 values]
+    const int page_size = 1 << page_shift, key = lane >> 1, half = lane & 1;
+    const int first = lb_first_visible(pos, window), tile0 = first / kKeysTile, n_tiles = pos / kKeysTile + 1 - tile0;
+    const int my_tiles = n_tiles > warp ? (n_tiles - warp + kWarps - 1) / kWarps : 0;
+    const size_t v_plane = (size_t)n_head * page_size * kHD;
+    int page_reg = 0;
+    auto tile_at = [&](int i) { return (tile0 + warp + kWarps * i) * kKeysTile; };
+    auto load = [&](int i) {                    // the page numbers of 32 tiles are read at once
+        if ((i & 31) == 0) page_reg = i + lane < my_tiles ? table[tile_at(i + lane) >> page_shift] : 0;
+        const int page = __shfl_sync(0xffffffffu, page_reg, i & 31), j0 = tile_at(i), j = j0 + key;
+        const __nv_bfloat16* rows = cache + (((size_t)page * 2 * n_head + head) * page_size + (j0 & (page_size - 1))) * kHD;
+        uint4* to = ring + (i % kRing) * 8 * 32;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) cp_async16(to + c * 32, rows + key * kHD + (2 * c + half) * 8, j >= first && j <= pos);
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) {
+            const int vk = (lane >> 3) * 4 + k4;
+            cp_async16(to + (4 + k4) * 32, rows + v_plane + vk * kHD + (lane & 7) * 8, j0 + vk >= first && j0 + vk <= pos);
+        }
+    };
+    // Keys and values of earlier positions are there before the kernel before this one ends; that kernel writes the newest position's.
+    bool asked[kRing];
+#pragma unroll
+    for (int i = 0; i < kRing; ++i) {
+        asked[i] = i >= my_tiles || tile_at(i) + kKeysTile <= pos;
+        if (asked[i] && i < my_tiles) load(i);
+    }
+    lb_wait_for_predecessor();
+    lb_dependents_may_launch();
+#pragma unroll
+    for (int i = 0; i < kRing; ++i) {           // a tile held back is the request's last: those before it are asked for already
+        if (!asked[i]) load(i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (threadIdx.x < kHD) q_s[threadIdx.x] = __bfloat162float(q[threadIdx.x]);
+    __syncthreads();
+    const lb_soft_cap capped(PLAIN ? 0.0f : soft_cap, bound);
+    const bool biased = !PLAIN && distance != nullptr;
+    const float r1 = biased ? distance[head] : 0.0f, r2 = biased ? distance[n_head + head] : 0.0f, sc = scale * kLog2e;
+    float m = -CUDART_INF_F, l = 0.0f, o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int i = 0; i < my_tiles; ++i) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        const uint4* from = ring + (i % kRing) * 8 * 32;
+        float dot[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            float kf[8];
+            unpack_bf16(from[c * 32], kf);
+            const float4 qa = *reinterpret_cast<const float4*>(q_s + (2 * c + half) * 8), qb = *reinterpret_cast<const float4*>(q_s + (2 * c + half) * 8 + 4);
+            dot[0] = fmaf(qa.x, kf[0], dot[0]); dot[1] = fmaf(qa.y, kf[1], dot[1]);
+            dot[2] = fmaf(qa.z, kf[2], dot[2]); dot[3] = fmaf(qa.w, kf[3], dot[3]);
+            dot[0] = fmaf(qb.x, kf[4], dot[0]); dot[1] = fmaf(qb.y, kf[5], dot[1]);
+            dot[2] = fmaf(qb.z, kf[6], dot[2]); dot[3] = fmaf(qb.w, kf[7], dot[3]);
+        }
+        const int j = tile_at(i) + key;
+        float s1 = (dot[0] + dot[1]) + (dot[2] + dot[3]);
+        s1 = (s1 + __shfl_xor_sync(0xffffffffu, s1, 1)) * sc;
+        if (capped.on) s1 = capped(s1);
+        if (biased) s1 -= lb_distance_penalty_log2(r1, r2, max(pos - j, 0));
+        if (j < first || j > pos) s1 = -CUDART_INF_F;
+        if (__any_sync(0xffffffffu, s1 > m)) {                    // a maximum moved: rare after the first tiles
+            float mx = s1;
+#pragma unroll
+            for (int d = 2; d < 32; d *= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+            mx = fmaxf(mx, m);
+            const float corr = exp2f(m - mx);
+            m = mx;
+            l *= corr;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[e] *= corr;
+        }
+        const float p = exp2f(s1 - (m == -CUDART_INF_F ? 0.0f : m));
+        l += half == 0 ? p : 0.0f;
+#pragma unroll
+        for (int k4 = 0; k4 < 4; ++k4) {
+            const float pk = __shfl_sync(0xffffffffu, p, 2 * ((lane >> 3) * 4 + k4));
+            float vf[8];
+            unpack_bf16(from[(4 + k4) * 32], vf);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) o[e] = fmaf(pk, vf[e], o[e]);
+        }
+        if (i + kRing < my_tiles) load(i + kRing);          // its place has been read, by this lane alone
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    l = lb_warp_sum(l);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        o[e] += __shfl_xor_sync(0xffffffffu, o[e], 8);
+        o[e] += __shfl_xor_sync(0xffffffffu, o[e], 16);
+    }
+    __syncthreads();                            // the rings have been read
+    if (lane < 8) {
+        float* st = red + warp * kState;
+        if (lane == 0) { st[0] = m; st[1] = l; }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) st[2 + lane * 8 + e] = o[e];
+    }
+    __syncthreads();
+    if (threadIdx.x < kHD) {
+        const int d = threadIdx.x;
+        float mm = -CUDART_INF_F, ll = 0.0f, a = 0.0f;
+        for (int w = 0; w < kWarps; ++w) mm = fmaxf(mm, red[w * kState]);
+        for (int w = 0; w < kWarps; ++w) {
+            const float* st = red + w * kState;
+            const float f = mm == -CUDART_INF_F ? 0.0f : exp2f(st[0] - mm);
+            ll += st[1] * f;
+            a += st[2 + d] * f;
+        }
+        if (sink != nullptr) a *= lb_sink_join_exp2(sink[head] * kLog2e, mm, ll);
+        out[d] = __float2bfloat16_rn(a / ll);
+    }
+}
+
 // PLAIN: no soft cap on the scores and no penalty by distance.
 template <bool PLAIN>
 __global__ void __launch_bounds__(kThreads, 2)
@@ -155,7 +312,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                             const int32_t* __restrict__ block_table, int table_stride, __nv_bfloat16* __restrict__ out,
                             int64_t out_stride, int n_head, int n_kv_head, int page_shift, int kv_rows, float scale, int window,
                             const float* __restrict__ distance, const float* __restrict__ sink,
-                            float soft_cap, float bound, int n_seq, int min_len, int* status) {
+                            float soft_cap, float bound, int n_seq, int min_len, const __nv_bfloat16* __restrict__ q, int64_t q_stride, const __nv_bfloat16* cache,
+                            int singles, int* status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* q_s = base;                                   // 16 KB
@@ -170,8 +328,17 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
     // before it.  A block without rows ends at once (one of the grid waits all the same, so that this kernel never ends
     // before the one before it).
     const int head = (int)(blockIdx.x % (unsigned)n_head);
-    int seq = 0, tile_q = 0;
-    if (!find_tile(q_start, n_seq, min_len, (int)(blockIdx.x / (unsigned)n_head), lane, &seq, &tile_q)) {
+    int seq = 0, tile_q = 0, number = (int)(blockIdx.x / (unsigned)n_head);
+    if (!find_tile(q_start, n_seq, min_len, number, lane, &seq, &tile_q)) {
+        // The blocks past the last query tile take the single tokens, where they are asked to.
+        const int single = singles != 0 ? find_single(q_start, n_seq, number, lane) : -1;
+        if (single >= 0) {
+            const int token = q_start[single];
+            serve_single<PLAIN>(q + (size_t)token * q_stride + (size_t)head * kHD, cache, block_table + (size_t)single * table_stride,
+                                out + (size_t)token * out_stride + (size_t)head * kHD, n_past[single], head, n_head, page_shift, scale, window, distance, sink,
+                                soft_cap, bound, base);
+            return;
+        }
         if (blockIdx.x == gridDim.x - 1) lb_wait_for_predecessor();
         return;
     }
@@ -565,6 +732,15 @@ extern "C" int lb_prefill_attention_tc_portions(const void* q, int64_t q_stride,
                                               const int32_t* n_past, const int32_t* block_table, int table_stride, void* out, int64_t out_stride,
                                               int n_seq, int max_q_len, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window,
                                               const float* distance, const float* sink, float soft_cap, float bound, int min_len, void* stream) {
+    return lb_prefill_attention_tc_mixed(q, q_stride, n_tokens, cache, n_pages, q_start, n_past, block_table, table_stride, out, out_stride, n_seq, max_q_len,
+                                         n_head, n_kv_head, head_dim, page_size, scale, window, distance, sink, soft_cap, bound, min_len, 0, stream);
+}
+
+extern "C" int lb_prefill_attention_tc_mixed(const void* q, int64_t q_stride, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
+                                              const int32_t* n_past, const int32_t* block_table, int table_stride, void* out, int64_t out_stride,
+                                              int n_seq, int max_q_len, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window,
+                                              const float* distance, const float* sink, float soft_cap, float bound, int min_len, int singles, void* stream) {
+    LB_CHECK_ARG(singles == 0 || (min_len > 1 && n_head == n_kv_head), "prefill attention (tcgen05): single tokens beside the tiles need a key/value head to every query head and min_len above 1");
     LB_CHECK_ARG(soft_cap >= 0.0f && (soft_cap == 0.0f || distance == nullptr), "prefill attention (tcgen05): a soft cap is positive and goes without a penalty by distance");
     LB_CHECK_ARG(distance == nullptr || scale != 0.0f, "prefill attention (tcgen05): a penalty by distance needs a factor on the scores that is not zero");
     LB_CHECK_ARG(n_seq >= 0 && max_q_len >= 0 && n_tokens >= 0 && n_pages > 0, "prefill attention: bad sizes");
@@ -602,7 +778,8 @@ extern "C" int lb_prefill_attention_tc_portions(const void* q, int64_t q_stride,
     auto* kernel = soft_cap == 0.0f && distance == nullptr ? prefill_attention_tc_kernel<true> : prefill_attention_tc_kernel<false>;
     LB_CHECK_CUDA(lb_launch_overlapped(kernel, dim3(grid), dim3(kThreads), smem, static_cast<cudaStream_t>(stream), 
         map_q, map_kv, q_start, n_past, block_table, table_stride, (__nv_bfloat16*)out, out_stride, n_head, n_kv_head, page_shift,
-        (int)kv_rows, scale, window, distance, sink, soft_cap, bound, n_seq, min_len, status));
+        (int)kv_rows, scale, window, distance, sink, soft_cap, bound, n_seq, min_len,
+        (const __nv_bfloat16*)q, q_stride, (const __nv_bfloat16*)cache, singles, status));
     LB_CHECK_LAUNCH();
     return LB_OK;
 }

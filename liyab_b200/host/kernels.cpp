@@ -334,6 +334,14 @@ double tcgen05_cost(const Tiles& t, double heads, double grid, double all_tiles,
     if (many) return 3.2 + std::max(1.7 * t.longest, 1.9 * (t.steps + 2.1 * t.count) * heads / sms) + 0.52 * (all_tiles - t.count * heads) / sms;
     return 2.4 + std::max(1.65 * t.longest, 1.16 * (t.steps + 1.56 * t.count) * heads / sms) + 0.25 * (grid - t.count * heads) / sms;
 }
+// The tcgen05 launch with a block for each single token and head: such a block takes 1.5 us and 1 us for every 217 keys on an SM of its own, 7.5 us and 1 us for
+// every 95 keys where all SMs have two blocks, beside the tiles' work (us measured / estimated, us in two launches: 12 on 100 to 900 beside 453 on 300,
+// 25 heads 20.0 / 20.6, 25.0; 16 on 50 to 900 beside 100, 12 heads 8.5 / 10.8, 14.0; 6 on 300 to 900 beside 300 7.3 / 8.0, 15.2; 4 beside 200, 25 heads 6.9 / 8.0, 13.8;
+// 12 on 1000 beside 2000 on 4000, 16 heads 93.9 / 97, 105.5; not there: 40 on 500 beside 2, 12 heads 24.0 / 23.4, 16.1; 100 on 300 beside 64 44.6 / 45, 29.8; 30 on
+// 800 beside 600, 25 heads 46.4 / 47, 38.2; and by the keys' ranges of eight blocks, 4 on 6000 beside 200 29.9 / 31, 20.2; 1 on 3000 beside 100 15.4 / 17.7, 10.6).
+double joined_cost(const Tiles& t, double singles, double longest, double all, double heads, double sms) {
+    return 2.4 + std::max({1.65 * t.longest, 1.5 + longest / 217, 1.16 * (t.steps + 1.56 * t.count) * heads / sms + (7.5 * singles + all / 95) * heads / (2 * sms)});
+}
 double mma_cost(const Tiles& t, double heads, double sms) { return 1.8 + std::max(2.15 * t.longest, 1.15 * (t.steps + 0.4 * t.count) * heads / sms); }
 double decode_cost(double longest, double all, double heads, double sms) { return 2.5 + std::max(0.35 * longest, 0.6 * all * heads / sms) / 128; }
 
@@ -367,7 +375,7 @@ AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const i
     }
     if (!prefill_supports(a)) return plan;
     Tiles wide[2], narrow[2];          // of the portions; of all requests
-    double longest_single = 0, all_single = 0;
+    double longest_single = 0, all_single = 0, n_single = 0;
     for (int i = 0; i < n_seq; ++i) {
         const int q = q_start[i + 1] - q_start[i];
         for (int which = q == 1 ? 1 : 0; which < 2; ++which) {
@@ -378,6 +386,7 @@ AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const i
             const double keys = static_cast<double>(span > 0 ? std::min<int64_t>(span, n_past[i] + 1) : n_past[i] + 1);
             longest_single = std::max(longest_single, keys);
             all_single += keys;
+            n_single += 1;
         }
     }
     const double never = 1e30, all_tiles = static_cast<double>(n_seq) * heads * ((max_q_len + 127) / 128);
@@ -395,24 +404,30 @@ AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const i
                 plan.tcgen05 = tcgen05;
             }
         }
+    // Behind the tiles the decode kernel's work takes half as long again as in a launch alone.
+    if (plan.tcgen05 && a.n_head == a.n_kv_head && n_single > 0 && wide[0].count > 0)
+        plan.joined = joined_cost(wide[0], n_single, longest_single, all_single, heads, sms) <
+                      tcgen05_cost(wide[plan.apart ? 0 : 1], heads, grid, all_tiles, false, sms) + (plan.apart ? decode_cost(longest_single, 1.5 * all_single, heads, sms) : 0);
     return plan;
 }
 
-void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
+bool prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                        const int32_t* n_past, const int32_t* block_table, int table_width, const Rows& out, int n_seq,
                        int max_q_len, const AttentionPlan& plan, const AttentionShape& a) {
     if (q.dtype != DType::BF16 || out.dtype != DType::BF16) throw invalid_argument("prefill attention takes bfloat16 only");
     const bool tc = plan.tcgen05 && prefill_tc_supports(a) && q.stride % 8 == 0 && out.stride % 8 == 0 && aligned16(q.data) && aligned16(out.data) &&
                     a.scale > 0;     // it takes the maximum of the raw scores
-    const int min_len = plan.apart ? 2 : 1;
+    const bool singles = tc && plan.joined;
+    const int min_len = plan.apart || singles ? 2 : 1;
     if (tc)
-        check(lb_prefill_attention_tc_portions(q.data, q.stride, n_tokens, cache, n_pages, q_start, n_past, block_table, table_width,
+        check(lb_prefill_attention_tc_mixed(q.data, q.stride, n_tokens, cache, n_pages, q_start, n_past, block_table, table_width,
                                            out.data, out.stride, n_seq, max_q_len, a.n_head, a.n_kv_head, a.head_dim, a.page_size,
-                                           a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, rt.stream), "prefill_attention_tc");
+                                           a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, singles ? 1 : 0, rt.stream), "prefill_attention_tc");
     else
         check(lb_prefill_attention_portions(q.data, q.stride, cache, q_start, n_past, block_table, table_width, out.data, out.stride, n_seq,
                                         max_q_len, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, rt.stream),
               "prefill_attention");
+    return singles;
 }
 
 void rms_groups(cudaStream_t s, const Rows& x, const int32_t* rows, const float* weight, const Rows& out, int n_rows, int groups, float eps, float gain_offset) {

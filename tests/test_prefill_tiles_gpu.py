@@ -37,3 +37,27 @@ def test_portions_at_the_edges(dev, new, past, n_head, n_kv_head, window, soft_c
             # Weights and the result in bfloat16 (2^-9 each) on values of order one, as in the kernels' own tests.
             assert (out.float() - want.float())[served].abs().max().item() < 1.5e-2
             assert (out[~served] == 7.0).all()
+
+
+@pytest.mark.parametrize("soft_cap,slopes", [(0.0, False), (20.0, False), (0.0, True)])
+@pytest.mark.parametrize("window", [0, 200])
+@pytest.mark.parametrize("new,past", [
+    ([1, 300, 1, 1, 45, 1, 1, 1], [0, 20, 15, 16, 700, 512, 1, 930]),
+    ([1] * 40 + [200] + [1] * 37, [(53 * i) % 900 for i in range(78)])])
+def test_single_tokens_in_the_launch(dev, new, past, window, soft_cap, slopes):
+    """Contexts that end in every part of a tile and fill some warps or all, more requests than one look finds, beside a portion."""
+    from liyab_b200 import ops
+    n_head, page_size, S = 5, 16, len(new)
+    q, cache, tok_seq, positions, table, _ = _paged_case(dev, torch.bfloat16, n_head, n_head, 64, page_size, [p + n for p, n in zip(past, new)], new, seed=S + window)
+    starts = torch.tensor([sum(new[:i]) for i in range(S + 1)], dtype=torch.int32, device=dev)
+    held = torch.tensor(past, dtype=torch.int32, device=dev)
+    sink = _rand((n_head,), 6, dev)
+    distance = torch.cat([_rand((n_head,), 7, dev).abs() * 0.1, torch.full((n_head,), -1.0, device=dev)]) if slopes else None
+    want, out = torch.empty_like(q), torch.full_like(q, float("nan"))
+    ops.paged_attention_generic(q, cache, tok_seq, positions, table, want, q.shape[0], n_head, n_head, 64, page_size, 0.125, window, sink=sink, soft_cap=soft_cap,
+                                distance=distance)
+    ops.prefill_attention(q, cache, starts, held, table, out, S, max(new), n_head, n_head, 64, page_size, 0.125, window, tcgen05=True, sink=sink, soft_cap=soft_cap,
+                          distance=distance, min_len=2, singles=True)
+    assert ops.device_status() == 0
+    # As above; the single tokens' weights stay in 32 bits, their result has one rounding.
+    assert (out.float() - want.float()).abs().max().item() < 1.5e-2
