@@ -113,7 +113,9 @@ int lb_gemm_persistent_kv_supports(int out_dtype, int N, int act, int has_residu
                                    int page_size);
 /* The same product with tiles of 256 tokens x feature_tile (128, 192 or 256) features that two SMs make together.  Operands as lb_gemm_persistent
  * takes them, with the same checks.  lb_gemm_pair_tile: the feature tile it would take and its estimated
- * time on n_sm SMs.  lb_gemm_shared_tile: that tile where lb_gemm_persistent hands the product over, else 0. */
+ * time on n_sm SMs.  lb_gemm_shared_tile: that tile where lb_gemm_persistent hands the product over, else 0.  lb_gemm_halved_tile: the tile of a product with
+ * float32 results whose reduction lb_gemm_persistent gives to two blocks in halves, else 0. */
+int lb_gemm_halved_tile(int M, int N, int K, int n_sm);
 int lb_gemm_shared_tile(int out_dtype, int M, int N, int K, int n_sm);
 int lb_gemm_pair_tile(int M, int N, int K, int n_sm, int* cost_ns);
 int lb_gemm_pair(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out,

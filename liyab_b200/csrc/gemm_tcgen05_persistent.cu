@@ -577,6 +577,49 @@ static bool tiles_shared() {
     return on;
 }
 
+// Microseconds of a product with float32 results: one block a tile, the halves of a reduction by two blocks, and the tiles of two SMs (the best of their
+// widths).  A round of tiles takes its k-blocks, each what the active blocks' operands take from L2 or what the issue of a step takes, whichever is longer.  Fitted to 90
+// products (200 to 2343 tokens; GPT-2's output and down projections and those of 1280 and 2560 features): of the tiles that were worth taking, half are
+// within 3 % and nineteen of twenty within 12 %.
+static double whole_us(int M, int N, int K, int bn, int n_sm) {
+    const long n_kb = (K + kBlockK - 1) / kBlockK, tiles = (long)((M + kLaneTile - 1) / kLaneTile) * ((N + bn - 1) / bn);
+    auto round = [&](long act) { return n_kb * fmax((double)act * (kLaneTile + bn) * 128 / 15.9e6, bn > 192 ? 0.457 : bn > 128 ? 0.288 : 0.24) + 1.35 * bn / 256; };
+    return 3.15 + (tiles / n_sm) * round(n_sm) + (tiles % n_sm != 0 ? round(tiles % n_sm) : 0.0);
+}
+static double halves_us(int M, int N, int K, int bn) {
+    const long n_kb = (K + kBlockK - 1) / kBlockK, tiles = (long)((M + kLaneTile - 1) / kLaneTile) * ((N + bn - 1) / bn);
+    return 2.86 + (n_kb + 1) / 2 * fmax(2.0 * tiles * (kLaneTile + bn) * 128 / 15.6e6, 0.257) + 8.35 * bn / 256;
+}
+static double shared_us(int M, int N, int K, int n_sm, int* bn_out) {
+    const long n_kb = (K + kBlockK - 1) / kBlockK, pairs = n_sm / 2;
+    const struct { int bn; double tile, rate, step; } widths[] = {{128, 1.59, 18.0e6, 0.202}, {192, 2.48, 14.35e6, 0.25}, {256, 3.85, 13.15e6, 0.322}};
+    double best = 1e30;
+    for (const auto& w : widths) {
+        const long tiles = (long)((M + 2 * kLaneTile - 1) / (2 * kLaneTile)) * ((N + w.bn - 1) / w.bn);
+        auto round = [&](long act) { return w.tile + n_kb * fmax(2.0 * act * (kLaneTile + w.bn / 2) * 128 / w.rate, w.step); };
+        const double us = 3.0 + (tiles / pairs) * round(pairs) + (tiles % pairs != 0 ? round(tiles % pairs) : 0.0);
+        if (us < best) {
+            best = us;
+            *bn_out = w.bn;
+        }
+    }
+    return best;
+}
+
+// The feature tile of a product (float32 results, nothing after the sum but a residual) whose reduction two blocks halve, 0 where they do not.
+// The first estimates alone took it for reductions where the exchange costs more than half of them saves (us halved / in whole tiles: 1024 x 1280 x 1280
+// 11.3 / 9.0, 800 x 1600 x 1600 12.5 / 10.2, 465 x 1600 x 1600 10.5 / 9.5; but 600 x 1600 x 6400 20.6 / 27, 600 x 768 x 3072 11.5 / 14.2) or where tiles of two
+// SMs take less from L2 (1400 x 1280 x 5120 25.2 / 21.5 by those, 2048 x 1024 x 4096 20.7 / 18.7, 465 x 2560 x 2560 15.8 / 13.7).
+extern "C" int lb_gemm_halved_tile(int M, int N, int K, int n_sm) {
+    long whole = 0, halved = 0;
+    const int bn = best_tile(4, M, N, K, n_sm, false, &whole), bn_halved = best_tile(4, M, N, K, n_sm, true, &halved);
+    if (bn <= 0 || bn_halved <= 0 || halved >= whole) return 0;
+    const double us = halves_us(M, N, K, bn_halved);
+    if (us >= whole_us(M, N, K, bn, n_sm)) return 0;
+    int shared = 0;
+    return K >= 1024 && shared_us(M, N, K, n_sm, &shared) < 0.96 * us ? 0 : bn_halved;
+}
+
 // The feature tile of the tiles that two SMs make together where the product takes those, 0 where every tile stays with one SM: where their estimate is
 // the lower one by an eighth.  This kernel's k-blocks cost what best_tile says, or what all active blocks' operands take from L2 at 13.5 TB/s.  The line lies
 // between products like 2048 x 1600 x 6400 (47 us here, 40 us shared) and 2048 x 3072 x 768 (16.9 us here, 17.4 us shared: short reductions leave a
@@ -594,7 +637,12 @@ extern "C" int lb_gemm_shared_tile(int out_dtype, int M, int N, int K, int n_sm)
     const long here = rounds * (n_kb * (operands > step_ns ? operands : step_ns) + 1000 + 1000 * bn / 256);
     int shared = 0;
     const int bn_shared = lb_gemm_pair_tile(M, N, K, n_sm, &shared);
-    if (8 * (long)shared >= 7 * here) return 0;
+    if (8 * (long)shared >= 7 * here) {
+        // The closer estimates for float32 results find more of them (us one block a tile / shared: 1024 x 2560 x 10240 57.0 / 50.6, 2048 x 1280 x 5120
+        // 29.5 / 26.0, 2343 x 1024 x 4096 23.8 / 22.0, 2048 x 1600 x 1600 14.1 / 13.3; one of 90 is slower: 1400 x 1600 x 6400 30.1 / 30.7).
+        int closer = 0;
+        return elem == 4 && shared_us(M, N, K, n_sm, &closer) < 0.96 * whole_us(M, N, K, bn, n_sm) ? closer : 0;
+    }
     if (elem == 2) {
         const long pairs = n_sm / 2, shared_tiles = (long)((M + 2 * kLaneTile - 1) / (2 * kLaneTile)) * ((N + bn_shared - 1) / bn_shared);
         auto one = [&](long act) { return n_kb * fmax((double)act * (kLaneTile + bn) * 128 / 16.0e6, bn > 192 ? 0.44 : 0.345) + 0.8 * bn / 256; };
@@ -645,12 +693,9 @@ extern "C" int lb_gemm_persistent(int out_dtype, const void* A, int64_t lda, con
     bool pair = false;
     int bn_used = bn;
     if (feature_tile <= 0 && elem == 4 && act == LB_ACT_NONE && kv_cache == nullptr && pairs_enabled()) {
-        long single = 0, paired = 0;
-        best_tile(elem, M, N, K, n_sm, false, &single);
-        const int bn_pair = best_tile(elem, M, N, K, n_sm, true, &paired);
-        if (bn_pair > 0 && paired < single) {
+        if (const int bn_halved = lb_gemm_halved_tile(M, N, K, n_sm); bn_halved > 0) {
             pair = true;
-            bn_used = bn_pair;
+            bn_used = bn_halved;
         }
     }
     LB_CHECK_ARG(bn % step == 0 && bn >= step && bn <= 256, "gemm_persistent: feature tile %d (a multiple of %d up to 256)", bn, step);

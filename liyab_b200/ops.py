@@ -69,6 +69,7 @@ _SIGNATURES = {
     "lb_gemm_narrow_plan": [_i, _i, _i, _i, _p, _p],
     "lb_gemm_pair_tile": [_i, _i, _i, _i, _p],
     "lb_gemm_shared_tile": [_i, _i, _i, _i, _i],
+    "lb_gemm_halved_tile": [_i, _i, _i, _i],
     "lb_gemm_rows_kind": [_i, _i, _i, _i, _i],
     "lb_gemm_rows_normed_pays": [_i, _i],
     "lb_gemm_ffma_row_features": [_i, _i, _i],

@@ -139,3 +139,13 @@ def test_tiles_of_two_sms_only_where_they_are_faster():
     assert not any(f(ops.BF16, *s, 148) for s in slower) and all(f(ops.BF16, *s, 148) for s in faster)
     assert all(f(ops.F32, *s, 148) for s in faster + slower[:4])            # float32 results: 1.07 to 1.3 times as fast
     assert not any(f(t, 2048, 3072, k, 148) for t in (ops.BF16, ops.F32) for k in (64, 768, 1016))
+
+
+@pytest.mark.parametrize("shape,halved,shared", [
+    ((1024, 1280, 1280), 0, 0), ((800, 1600, 1600), 0, 0), ((465, 1600, 1600), 0, 0), ((465, 1280, 1280), 0, 0),        # in whole tiles
+    ((600, 1600, 6400), 1, 0), ((600, 768, 3072), 1, 0), ((1024, 768, 3072), 1, 0), ((100, 1600, 6400), 1, 0),     # by halves
+    ((1400, 1280, 5120), 0, 128), ((2048, 1024, 4096), 0, 128), ((465, 2560, 2560), 0, 128), ((1024, 2560, 10240), 0, 192)])       # by tiles of two SMs
+def test_float32_results_in_halves_or_whole(shape, halved, shared):
+    lib = ops.lib()
+    got = lib.lb_gemm_halved_tile(*shape, 148)
+    assert (got > 0) == (halved > 0) and (halved > 0 or lib.lb_gemm_shared_tile(ops.F32, *shape, 148) == shared)
