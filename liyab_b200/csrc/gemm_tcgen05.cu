@@ -1,6 +1,6 @@
 // out[M, N] = epilogue(A[M, K] . W[N, K]^T) for bfloat16 operands on the fifth
 // generation tensor cores: operands staged in shared memory by TMA
-// (cp.async.bulk.tensor, 128-byte swizzle), products issued by one thread with
+// (cp.async.bulk.tensor, 128-byte swizzle), products issued by one elected lane with
 // tcgen05.mma into an accumulator in tensor memory, read back with tcgen05.ld
 // for the epilogue (bias, activation, residual sum, in the reference's order:
 // src/core/transformer.cpp:111-118, 4903-4912, 5526-5532).

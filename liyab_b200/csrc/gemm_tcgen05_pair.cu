@@ -7,8 +7,9 @@
 // room for five stages.
 // Measured (B200, 20 launches a graph, TFLOP/s; one block a tile / here / cuBLAS with bfloat16 results and a bare epilogue): 2343 x 6400 x 1600 1062 / 1246 /
 // 1347, with GELU 983 / 1147 / -; 2343 x 1600 x 6400 with residual 705 / 1183 / 1337; 2343 x 4800 x 1600 997 / 1221 / 1289.  GPT-2 XL, five prompts of 2,343 tokens: 11.77 -> 9.87 ms
-// a step.  A k-block takes 0.31 to 0.34 us whatever the tile's features and however few tiles run (the products alone would take 0.26 us at 256
-// features), and two producer threads instead of one change nothing.
+// a step.  A k-block took 0.31 to 0.34 us whatever the tile's features and however few tiles run while a branch on the lane's number issued products and
+// copies; from an elected lane (elect_one in tcgen05.cuh) it takes 0.20, 0.25 or 0.32 us at 128, 192 or 256 features until the operands of all
+// blocks take longer from L2 (some 13 to 18 TB/s).  Two producer threads instead of one change nothing.
 //
 // Roles of a block's warps:
 //   warp 0      TMA producer of the block's own operands; both blocks' copies count on the first block's barrier.

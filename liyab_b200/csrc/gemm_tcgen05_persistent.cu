@@ -10,7 +10,7 @@
 //               strips of the tile: tcgen05.ld of their 32 lanes, bias, activation,
 //               residual (read from the staging buffer, where TMA put it), result
 //               written back to the same place, then one TMA store per strip.
-// The two single-thread roles run once per k-block while the tensor pipe waits for
+// The two issuing roles (an elected lane of a whole warp) run once per k-block while the tensor pipe waits for
 // them, so their loops are kept to a few dozen instructions (32-bit shared-memory
 // addresses, running stage index, descriptor words advanced by addition).
 // The staging buffer is laid out as TMA's 128-byte swizzle wants it ([strip][128
@@ -545,7 +545,8 @@ extern "C" int lb_gemm_persistent_tile(int out_dtype, const void* A, int64_t lda
     }
     // Cost of a choice, in nanoseconds: rounds over the SMs x (k-blocks x time per k-block + epilogue).  Measured on
     // B200: a tcgen05.mma of 128 rows takes about as long for 32 columns as for 192 (the tensor core walks the rows),
-    // so a k-block costs about 300 ns up to 192 columns and 420 ns at 256; the epilogue of a tile costs about a
+    // so a k-block costs about 300 ns up to 192 columns and 420 ns at 256 (240 up to 128 and 290 at 192 since an elected lane issues them, which moves the
+    // choice of a width by little: of 200 products six had a width 2 to 7 % faster); the epilogue of a tile costs about a
     // microsecond plus one per 256 columns.  Ties go to the wider tile (fewer blocks fetch the same activations).
     return best_tile(elem, M, N, K, n_sm, false, nullptr);
 }

@@ -9,7 +9,7 @@ namespace lb_tile {
 
 using namespace lb_tc;
 
-// The loops of the two single-thread roles run once per k-block while the tensor pipe waits for them: they work on
+// The loops of the two issuing warps (one elected lane of each) run once per k-block while the tensor pipe waits for them: they work on
 // 32-bit shared-memory addresses and a running stage index, with no division and no 64-bit pointer arithmetic.
 __device__ __forceinline__ bool try_wait_u32(uint32_t bar, uint32_t parity) {
     uint32_t ok;
