@@ -123,11 +123,13 @@ int lb_gemm_pair(int out_dtype, const void* A, int64_t lda, const void* W, int64
                  int head_dim, int page_size, void* stream);
 /* The product for some dozens of tokens in one launch: 64 or 128 tokens by `features` (a multiple of 8 * splits, at most 256) a block, the reduction cut between
  * the `splits` (1, 2, 4 or 8) blocks of a cluster; features 0: lb_gemm_narrow_plan's choice (its return value; 0: sizes it does not take; *cost_ns an estimate).
- * lb_gemm_narrow_pays: whether it is the faster kernel for a product.  With kv_cache as lb_gemm_persistent. */
+ * lb_gemm_narrow_pays: whether it is the faster kernel for a product.  lb_gemm_narrow_block: bytes of shared memory and columns of tensor memory of a block.
+ * With kv_cache as lb_gemm_persistent. */
 int lb_gemm_narrow_pays(int out_dtype, int M, int N, int K);
 int lb_gemm_narrow_plan(int M, int N, int K, int n_sm, int* splits, int* cost_ns);
 int lb_gemm_narrow_supports(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* residual, int64_t ldr, const void* out,
                             int64_t ldo, int M, int N, int K);
+int lb_gemm_narrow_block(int M, int K, int features, int splits, int* columns);
 int lb_gemm_narrow_kv_supports(int out_dtype, int N, int act, int has_residual, int q_dim, int n_kv_head, int head_dim, int page_size);
 int lb_gemm_narrow(int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw, const float* bias, const float* residual, int64_t ldr, void* out,
                    int64_t ldo, int M, int N, int K, int act, int features, int splits, void* kv_cache, const int32_t* slot_mapping, int q_dim,

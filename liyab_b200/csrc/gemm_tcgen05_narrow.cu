@@ -291,8 +291,17 @@ Plan stages_for(int rows, int features, int splits, int n_kb) {
     return p;
 }
 
+// Columns of tensor memory for the block's sums.
+int tmem_columns(int features) { return features <= 32 ? 32 : features <= 64 ? 64 : features <= 128 ? 128 : 256; }
+
+// The blocks of a cluster wait for one another while each holds its columns, so one that waited for columns held by a block of another cluster could wait for
+// good, each cluster's other blocks being in the other's place on another SM.  A block that is part of a cluster therefore asks for at least as large a share of
+// the SM's 228 KB (1 KB of each block's is the system's) as of its 512 columns: what fits the one fits the other.  Only short parts of a reduction with many
+// features are below that (K = 128 in two parts of 144 features: 66 KB and half of the columns); the plan makes none.
 size_t smem_bytes(int rows, const Plan& p) {
-    return 1024 + (size_t)p.stages * (rows + p.features) * 128 + behind_bytes(rows, p.features, p.splits, p.alias != 0);
+    const size_t needed = 1024 + (size_t)p.stages * (rows + p.features) * 128 + behind_bytes(rows, p.features, p.splits, p.alias != 0);
+    const size_t share = (size_t)tmem_columns(p.features) * (228 * 1024 / 512) - 1024;
+    return p.splits > 1 && needed < share ? share : needed;
 }
 
 }  // namespace
@@ -355,6 +364,16 @@ extern "C" int lb_gemm_narrow_supports(int out_dtype, const void* A, int64_t lda
            (ldo * elem) % 16 == 0 && (residual == nullptr || (out_dtype == LB_F32 && ((uintptr_t)residual & 15) == 0 && ldr % 4 == 0));
 }
 
+// Shared memory of a block of that launch, and its columns of tensor memory; 0: no such launch.
+extern "C" int lb_gemm_narrow_block(int M, int K, int features, int splits, int* columns) {
+    if (M < 1 || K < 1 || features < 8 || features > kMaxFeatures || splits < 1 || splits > kMaxSplits || features % (8 * splits) != 0) return 0;
+    const int rows = M <= 64 ? 64 : 128, all_kb = (K + kBlockK - 1) / kBlockK, per = (all_kb + splits - 1) / splits;
+    if ((splits - 1) * per >= all_kb) return 0;
+    const Plan plan = stages_for(rows, features, splits, per);
+    if (columns != nullptr) *columns = tmem_columns(features);
+    return plan.stages >= 1 ? (int)smem_bytes(rows, plan) : 0;
+}
+
 // Whether it can put the features from q_dim on into the pages of a cache instead of `out`.
 extern "C" int lb_gemm_narrow_kv_supports(int out_dtype, int N, int act, int has_residual, int q_dim, int n_kv_head, int head_dim, int page_size) {
     return out_dtype == LB_BF16 && act == LB_ACT_NONE && !has_residual && q_dim > 0 && q_dim % 8 == 0 && head_dim > 0 && head_dim % 8 == 0 &&
@@ -400,7 +419,7 @@ extern "C" int lb_gemm_narrow(int out_dtype, const void* A, int64_t lda, const v
     rc = lb_tc_status_word(&status);
     if (rc != LB_OK) return rc;
     const size_t smem = smem_bytes(rows, plan);
-    const int mma_features = (features + 15) / 16 * 16, tmem_cols = mma_features <= 32 ? 32 : mma_features <= 64 ? 64 : mma_features <= 128 ? 128 : 256;
+    const int tmem_cols = tmem_columns(features);
     const dim3 grid((N + features - 1) / features * splits, (M + rows - 1) / rows);
     auto s = static_cast<cudaStream_t>(stream);
 #define LB_GO(ROWS, TO, ACT)                                                                                                                                     \

@@ -66,6 +66,7 @@ _SIGNATURES = {
     "lb_gemm_pair": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
     "lb_gemm_narrow": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
     "lb_gemm_narrow_pays": [_i, _i, _i, _i],
+    "lb_gemm_narrow_block": [_i, _i, _i, _i, _p],
     "lb_gemm_narrow_plan": [_i, _i, _i, _i, _p, _p],
     "lb_gemm_pair_tile": [_i, _i, _i, _i, _p],
     "lb_gemm_shared_tile": [_i, _i, _i, _i, _i],

@@ -4,6 +4,8 @@ These decide whether a size that the configuration allows reaches a specialised 
 clear refusal, so they are pinned here for the sizes the kernels' comments promise."""
 from __future__ import annotations
 
+import ctypes as C
+
 import pytest
 
 from liyab_b200 import ops
@@ -149,3 +151,20 @@ def test_float32_results_in_halves_or_whole(shape, halved, shared):
     lib = ops.lib()
     got = lib.lb_gemm_halved_tile(*shape, 148)
     assert (got > 0) == (halved > 0) and (halved > 0 or lib.lb_gemm_shared_tile(ops.F32, *shape, 148) == shared)
+
+
+@pytest.mark.parametrize("M", [40, 300])
+def test_clusters_of_narrow_products_cannot_run_out_of_tensor_memory(M):
+    """Blocks of a cluster wait for one another: an SM that took more of them than its 512 columns serve could leave two clusters waiting for each other.  With at
+    least as large a share of its 228 KB as of its columns, what fits the one fits the other."""
+    columns, seen = C.c_int(0), set()
+    for splits in (2, 4, 8):
+        for features in range(8 * splits, 257, 8 * splits):
+            for K in [64 * n for n in range(1, 40)] + [6400]:
+                smem = ops.lib().lb_gemm_narrow_block(M, K, features, splits, C.addressof(columns))
+                if smem == 0:
+                    continue
+                assert columns.value >= features and smem <= 227 * 1024
+                assert columns.value * 228 * 1024 <= 512 * (smem + 1024), (K, features, splits)
+                seen.add(columns.value)
+    assert seen == {32, 64, 128, 256}
