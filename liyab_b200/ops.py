@@ -543,7 +543,9 @@ def prefill_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tenso
         blocks = n_seq * n_head * -(-max_q_len // 128)
         tcgen05 = (prefill_attention_tc_supports(n_head, n_kv_head, head_dim, page_size) and q.stride(0) % 8 == 0
                    and out.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
-                   and blocks <= 4 * _sm_count(q.device))
+                   and (singles or blocks <= 4 * _sm_count(q.device)))
+    if singles and not tcgen05:
+        raise invalid_argument("prefill attention: only the tcgen05 launch serves single tokens beside the portions")
     if tcgen05:
         check(lib().lb_prefill_attention_tc_mixed(
             _dev(q, "q"), q.stride(0), q.shape[0], _dev(cache, "cache"), cache.shape[0],

@@ -168,3 +168,15 @@ def test_clusters_of_narrow_products_cannot_run_out_of_tensor_memory(M):
                 assert columns.value * 228 * 1024 <= 512 * (smem + 1024), (K, features, splits)
                 seen.add(columns.value)
     assert seen == {32, 64, 128, 256}
+
+
+@pytest.mark.parametrize("head_dim,tcgen05", [(64, False), (128, None)])
+def test_single_tokens_beside_portions_are_not_left_out(head_dim, tcgen05):
+    """Asked to serve the requests of one token as well, where the launch is not the kernel that does: refused, before anything else (these are no device's)."""
+    import torch
+
+    from liyab_b200.status import LiyabError
+    rows, ints = torch.zeros((8, 2 * head_dim), dtype=torch.bfloat16), torch.zeros(4, dtype=torch.int32)
+    with pytest.raises(LiyabError, match="single tokens"):
+        ops.prefill_attention(rows, torch.zeros((1, 2, 2, 16, head_dim), dtype=torch.bfloat16), ints, ints, ints.view(1, 4), rows, 3, 64, 2, 2, head_dim, 16, 0.125,
+                              tcgen05=tcgen05, min_len=2, singles=True)
