@@ -139,9 +139,9 @@ inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView
     else if (!ctx.decode_only) plan = kernels::attention_plan(ctx.runtime, a, ctx.host_q_start.data(), ctx.host_n_past.data(), S, ctx.max_q_len);
     plan.apart = plan.apart && kernels::decode_mma_supports(a);
     if (ctx.runtime.dtype == DType::BF16 && kernels::prefill_supports(a)) {
-        const bool whole = kernels::prefill_attention(ctx.runtime, q, T, cache, n_pages, ctx.q_start, ctx.n_past, view.block_table, view.table_width, att, S,
-                                                      ctx.max_q_len, plan, a);
-        if (plan.apart && !whole) decode(true, ctx.q_start);
+        kernels::prefill_attention(ctx.runtime, q, T, cache, n_pages, ctx.q_start, ctx.n_past, view.block_table, view.table_width, att, S, ctx.max_q_len,
+                                   plan, a);
+        if (plan.apart) decode(true, ctx.q_start);
         return;
     }
     kernels::attention_generic(ctx.stream(), ctx.runtime.dtype, q, cache, ctx.tok_seq, ctx.positions, view.block_table,

@@ -408,10 +408,11 @@ AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const i
     if (plan.tcgen05 && a.n_head == a.n_kv_head && n_single > 0 && wide[0].count > 0)
         plan.joined = joined_cost(wide[0], n_single, longest_single, all_single, heads, sms) <
                       tcgen05_cost(wide[plan.apart ? 0 : 1], heads, grid, all_tiles, false, sms) + (plan.apart ? decode_cost(longest_single, 1.5 * all_single, heads, sms) : 0);
+    if (plan.joined) plan.apart = false;
     return plan;
 }
 
-bool prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
+void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                        const int32_t* n_past, const int32_t* block_table, int table_width, const Rows& out, int n_seq,
                        int max_q_len, const AttentionPlan& plan, const AttentionShape& a) {
     if (q.dtype != DType::BF16 || out.dtype != DType::BF16) throw invalid_argument("prefill attention takes bfloat16 only");
@@ -427,7 +428,6 @@ bool prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const voi
         check(lb_prefill_attention_portions(q.data, q.stride, cache, q_start, n_past, block_table, table_width, out.data, out.stride, n_seq,
                                         max_q_len, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, rt.stream),
               "prefill_attention");
-    return singles;
 }
 
 void rms_groups(cudaStream_t s, const Rows& x, const int32_t* rows, const float* weight, const Rows& out, int n_rows, int groups, float eps, float gain_offset) {

@@ -116,9 +116,8 @@ void attention_generic(cudaStream_t s, DType dtype, const Rows& q, const void* c
 void decode_attention(cudaStream_t s, bool tensor_cores, const Rows& q, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,
                       const int32_t* block_table, int table_width, const Rows& out, float* partial, int* counters, int n_seq,
                       const AttentionShape& a, int n_splits, int max_keys);
-// Whether the launch served the requests of one token as well: with plan.apart they are left to decode_attention, where plan.joined or the rows'
-// alignment does not change that.
-bool prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
+// plan.apart: requests of one token are left to decode_attention.
+void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                        const int32_t* n_past, const int32_t* block_table, int table_width, const Rows& out, int n_seq,
                        int max_q_len, const AttentionPlan& plan, const AttentionShape& a);
 // How a step with prompt portions launches an attention (page_size, sink and so on of `a` are those of its launches): the cheapest of the launches that

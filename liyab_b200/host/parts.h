@@ -70,9 +70,9 @@ struct AttentionPlan {
     bool apart = false;        // bfloat16: requests of one token have a launch of their own, by the decode kernel
     bool tcgen05 = false;      // bfloat16: portions by the tcgen05 kernel where it takes the shape, else by the mma.sync one
     bool runs = false;         // float32: a tile of keys is read once for sixteen neighbouring tokens
-    bool joined = false;       // bfloat16, with tcgen05: that launch serves the requests of one token by blocks of their own, whatever `apart` says
-    int bits() const { return (apart ? 1 : 0) | (tcgen05 ? 2 : 0) | (runs ? 4 : 0); }
-    int key() const { return bits() | (joined ? 4 : 0); }      // what tells one step's launches from another's, in three bits: `runs` is float32's
+    bool joined = false;       // bfloat16, with tcgen05 and not apart: that launch serves the requests of one token by blocks of their own
+    int bits() const { return (apart ? 1 : 0) | (tcgen05 ? 2 : 0) | (runs ? 4 : 0) | (joined ? 8 : 0); }
+    int key() const { return (bits() & 7) | (joined ? 4 : 0); }      // what tells one step's launches from another's, in three bits: `runs` is float32's
 };
 
 // One cache group as a step sees it.

@@ -275,8 +275,8 @@ LB_API int32_t lb_replayer_step(lb_replayer* r, size_t n_entries, const int64_t*
  * memory (CUDA does not count it as page-locked: a copy out of it has read it when the call returns).  Making one costs as much as many steps: keep it. */
 LB_API int32_t lb_host_buffer_create(int32_t device, size_t bytes, void** out);
 LB_API void lb_host_buffer_destroy(void* buffer);
-/* How a step whose request i brings q_start[i + 1] - q_start[i] tokens on n_past[i] launches an attention: 1 single tokens by the decode kernel, 2 portions by
- * the tcgen05 kernel, 4 (float32) tiles of keys shared among neighbouring tokens.  mask: 0 all earlier keys, w > 0 a window, -c a chunk. */
+/* How a step whose request i brings q_start[i + 1] - q_start[i] tokens on n_past[i] launches an attention: 1 single tokens by a launch of the decode
+ * kernel, 2 portions by the tcgen05 kernel, 4 (float32) tiles of keys shared among neighbouring tokens, 8 single tokens by blocks of the tcgen05 kernel's launch.  mask: 0 all earlier keys, w > 0 a window, -c a chunk. */
 LB_API int32_t lb_attention_plan(const char* dtype, int32_t n_head, int32_t n_kv_head, int32_t head_dim, int32_t page_size, int32_t mask, int32_t sm_count,
                                  int32_t n_seq, const int32_t* q_start, const int32_t* n_past, int32_t max_q_len, int32_t* bits);
 /* Options at run time: "cuda_graphs" 0/1, "fused_decode" 0 (cannot be switched back on). */

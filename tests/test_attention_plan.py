@@ -8,7 +8,7 @@ import pytest
 
 from liyab_b200 import _capi
 
-APART, TCGEN05, RUNS = 1, 2, 4
+APART, TCGEN05, RUNS, JOINED = 1, 2, 4, 8
 
 
 def plan(requests, n_head, dtype="bfloat16", n_kv_head=None, head_dim=64, page_size=16, mask=0, sms=148):
@@ -31,9 +31,11 @@ def singles(n, lo, hi):
 @pytest.mark.parametrize("heads,requests,want", [
     # The launch for single tokens costs 3 to 5 us: not where they end before the portion does and all blocks run at once (0.93 to 0.98 of the speed) ...
     (12, singles(3, 50, 250) + [(0, 500)], TCGEN05), (12, singles(6, 300, 900) + [(700, 200)], TCGEN05), (12, singles(6, 50, 250) + [(300, 300)], TCGEN05),
-    # ... but where they reach further than the portion (1.05 to 1.10), or their blocks would fill the GPU several times (1.15 to 1.6).
-    (12, singles(6, 900, 1000) + [(0, 256)], APART | TCGEN05), (25, singles(12, 300, 900) + [(300, 500)], APART | TCGEN05), (12, singles(30, 900, 1000) + [(0, 500)], APART | TCGEN05),
-    (25, singles(16, 100, 300) + [(0, 700)], APART | TCGEN05),
+    # ... but where they reach further than the portion (1.05 to 1.10), or their blocks would fill the GPU several times (1.15 to 1.6): by blocks of the portion's
+    # launch (us in one launch / in two: 20.0 / 25.0 for twelve beside 500 on 300 with 25 heads) or, where those take longer (15.4 /
+    # 10.6 for one on 3000 beside 100), by a launch of their own.
+    (12, singles(6, 900, 1000) + [(0, 256)], TCGEN05 | JOINED), (25, singles(12, 300, 900) + [(300, 500)], TCGEN05 | JOINED), (12, singles(30, 900, 1000) + [(0, 500)], TCGEN05 | JOINED),
+    (25, singles(16, 100, 300) + [(0, 700)], APART | TCGEN05), (25, singles(1, 3000, 3000) + [(0, 100)], APART | TCGEN05),
     # Many blocks without rows: the mma.sync kernel for a short portion (the tcgen05 kernel has 0.82 of its speed there, 0.95 to 0.93 in two launches).
     (12, singles(30, 50, 250) + [(0, 130)], 0), (25, singles(30, 300, 900) + [(0, 130)], APART), (12, singles(60, 900, 1000) + [(0, 130)], APART),
     # Portions alone: the tcgen05 kernel for long ones (0.94 to 0.86 of its speed by the other), the other one for many short ones (0.87 to 0.94).
@@ -49,6 +51,7 @@ def test_only_kernels_that_take_the_shape():
     assert plan(mixed, 12, head_dim=32) == 0                     # the decode kernel on the tensor cores takes heads of 64 and 128
     assert plan(mixed, 12, head_dim=40) == 0 and plan(mixed, 34, n_kv_head=2) & APART == 0
     assert plan(mixed, 12, page_size=8) & APART == 0
+    assert plan(mixed, 12) & JOINED and plan(mixed, 12, n_kv_head=4) & JOINED == 0 and plan(mixed, 12, head_dim=128) & JOINED == 0     # blocks for single query heads of 64
     assert plan([(100, 1)], 12) in (0, APART, TCGEN05)           # a launch is chosen for any step
 
 
