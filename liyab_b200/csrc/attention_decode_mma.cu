@@ -14,18 +14,17 @@
 // where that fills the GPU's last wave of blocks better, or eight or sixteen in the
 // place of two to four ranges: see launch_for) takes every n-th 16-key
 // tile of the range (a tile lies inside one page: its keys, and its values, are
-// one contiguous run of the cache), brings it into its own two shared-memory
-// buffers with cp.async one tile ahead (16-byte chunks XOR-swizzled by the row, so
-// ldmatrix meets no bank twice and nothing is padded), and keeps its own running
+// one contiguous run of the cache), brings it into shared-memory buffers of its own
+// one or two tiles ahead (heads of 64: boxes of a tensor map; of 128: cp.async; 16-byte chunks
+// XOR-swizzled by the row either way, so ldmatrix meets no bank twice and nothing is padded), and keeps its own running
 // maximum, sum and output; the warps are merged at the end in warp order, the key
 // ranges in range order: two to eight ranges are the blocks of one cluster and
 // meet in its first block's shared memory (the launch carries the cluster size),
 // more than eight go through global memory to the block that finishes last.  Softmax, sums and
-// accumulators are 32-bit (exp2 of scores pre-scaled by log2 e).  Measured on
-// B200, 12 heads of 64 over 768 keys: 27 us for 64 requests and 51 us for 128
-// (5.5 and 5.9 TB/s of cache), where the scalar kernel takes 47 us for 64.
+// accumulators are 32-bit (exp2 of scores pre-scaled by log2 e).
 //
-// Heads of 64 with a key/value head each have their products on the 32-bit units instead (SINGLE below).
+// Heads of 64 with a key/value head each have their products on the 32-bit units instead (SINGLE below; launch_for has how many warps a block, blocks
+// an SM and tiles ahead).  Measured on B200, 64 requests x 12 heads on 1024 keys: 32.3 us (6.2 TB/s of cache; 33.3 on the tensor cores); 64 x 16 on 4096 154 us (7.0).
 //
 // Reference formulas: src/core/transformer.cpp:2303-2313, 2327-2341, 2344-2358, 2367-2385.
 #include "api.h"
@@ -532,20 +531,26 @@ struct Variant {
         return LB_OK;
     }
 
+    // at_once: no more blocks than these on an SM (0: as many as fit), by asking for more shared memory than the block needs, as little more as keeps another
+    // one out.
     static int launch(const CUtensorMap& map_kv, int kv_rows, int* status, const void* q, int64_t q_stride, const void* cache, const int32_t* q_start, const int32_t* positions, const int32_t* block_table,
                       int table_stride, void* out, int64_t out_stride, float* partial, int* counters, int n_seq, int n_head,
                       int n_kv_head, int page_shift, float scale, int window, int n_splits, const float* distance, const float* sink, float soft_cap,
-                      float bound, cudaStream_t s) {
+                      float bound, long at_once, cudaStream_t s) {
         dim3 grid(n_splits, n_kv_head, n_seq);
         // Two to eight key ranges: the ranges of a request and head form a cluster and merge in shared memory.
         const int group = n_head / n_kv_head;
         const bool cluster = n_splits > 1 && n_splits <= 8 && cluster_merge_enabled();
-        const size_t inbox = cluster ? (size_t)n_splits * group * (HD + 2) * sizeof(float) : 0;
+        size_t asked = smem + (cluster ? (size_t)n_splits * group * (HD + 2) * sizeof(float) : 0);
+        if (at_once > 0) {
+            const size_t alone = (size_t)228 * 1024 / (at_once + 1) / 128 * 128 - 1024;        // a block's kilobyte for the system and its barriers come on top
+            if (asked < alone && alone <= smem + kInboxMax) asked = alone;
+        }
         int per_sm = 0;
         const int rc = blocks_per_sm(&per_sm);              // sets the kernel's shared-memory limit
         if (rc != LB_OK) return rc;
         LB_CHECK_CUDA(lb_launch_overlapped_cluster(3, cluster ? n_splits : 1, decode_attention_mma_kernel<HD, kWarps, kStages, TMA, SINGLE>, grid,
-                                                   dim3(kWarps * 32), smem + inbox, s, map_kv, kv_rows, status, (const __nv_bfloat16*)q,
+                                                   dim3(kWarps * 32), asked, s, map_kv, kv_rows, status, (const __nv_bfloat16*)q,
                                                    q_stride, (const __nv_bfloat16*)cache, q_start, positions, block_table, table_stride,
                                                    (__nv_bfloat16*)out, out_stride, partial, counters, n_head, n_kv_head, page_shift,
                                                    scale, window, n_splits, cluster ? 1 : 0, distance, sink, soft_cap, bound));
@@ -562,17 +567,20 @@ int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* 
                int table_stride, void* out, int64_t out_stride, float* partial, int* counters, int n_seq, int n_head,
                int n_kv_head, int page_shift, float scale, int window, int n_splits, int max_keys, const float* distance, const float* sink, float soft_cap,
                       float bound, cudaStream_t s) {
-    // The 32-bit form is through with a tile sooner, and two tiles ahead of it pay: steps of GPT-2 medium with 64 requests 2.08 ms with one ahead, 1.98 with two;
-    // XL with 8 1.90 and 1.85; small level.  (With the tensor cores one is enough.)
-    constexpr int kDecodeStages = SINGLE ? 3 : 2;
-    using Wide = Variant<HD, 4, kDecodeStages, TMA, SINGLE>;
-    using Narrow = Variant<HD, 2, kDecodeStages, TMA, SINGLE>;
+    auto go = [&](auto variant, int ranges, long at_once) {
+        return decltype(variant)::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride, partial,
+                                         counters, n_seq, n_head, n_kv_head, page_shift, scale, window, ranges, distance, sink, soft_cap, bound, at_once, s);
+    };
+    // The 32-bit form is through with a tile sooner, and two tiles ahead of it pay while few blocks share an SM: steps of GPT-2 XL with 8 requests 1.90 ms with one
+    // ahead, 1.85 with two.  (With the tensor cores one is enough.)
+    constexpr int kAhead = SINGLE ? 3 : 2;
     static int n_sm = 0;
     if (n_sm == 0) {
         int dev = 0;
         LB_CHECK_CUDA(cudaGetDevice(&dev));
         LB_CHECK_CUDA(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
     }
+    const long pairs = (long)n_kv_head * n_seq, reach = max_keys > 0 ? max_keys : (long)table_stride << page_shift;
     // Two to four ranges of 64 or more (request, key/value head) pairs: one block of eight or sixteen warps a pair instead of a cluster of blocks of four.
     // The warps' states then meet in one merge, without the cluster's two barriers and the way through the first block's memory.  Fewer pairs would
     // leave SMs without a block.  Measured: GPT-2 small, 8 requests 369 -> 359 us a step; XL, 8 requests 1.98 -> 1.95 ms; medium, 9 requests 734 -> 706 us
@@ -581,16 +589,41 @@ int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* 
     // 150 pairs in two ranges, 2048 keys 1.00 to 1.07 times as fast with the wide block, 4096 0.97, 16384 0.88; 160 to 200 pairs 0.97 from 8192 on;
     // 144 pairs in three ranges 1.06 at 4096, 1.00 at 8192, 0.98 at 16384; up to 128 pairs 1.02 to 1.1 throughout.
     if constexpr (TMA) {
-        const long pairs = (long)n_kv_head * n_seq, reach = max_keys > 0 ? max_keys : (long)table_stride << page_shift;
         const long longest = n_splits == 2 ? (pairs < 160 ? 2048 : 6144) : pairs <= 128 ? reach : 8192;
         if (n_splits >= 2 && n_splits <= 4 && pairs >= 64 && reach <= longest && cluster_merge_enabled()) {
-            if (n_splits == 2)
-                return Variant<HD, 8, kDecodeStages, TMA, SINGLE>::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride,
-                                                      partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, 1, distance, sink, soft_cap, bound, s);
-            return Variant<HD, 16, kDecodeStages, TMA, SINGLE>::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride,
-                                                   partial, counters, n_seq, n_head, n_kv_head, page_shift, scale, window, 1, distance, sink, soft_cap, bound, s);
+            // Eight warps of the 32-bit form: one tile ahead, no more blocks on an SM than its share.  Two ahead take 99 KB a block, which keeps the next product out of an
+            // SM that has two (us a step with two ahead / so: XL, 8 requests on 20 to 60 1609 / 1566, on 900 to 1000 1964 / 1908; medium, 12 on 20 to 60 706 / 678, on 200 to 900
+            // 809 / 793; on 4096 192 pairs take 35.0 / 32.0 us alone).  Sixteen: two ahead until memory bounds them (96 pairs on 4096 17.4 / 18.1, on 16384 68 / 61).
+            if (SINGLE && n_splits == 2) return go(Variant<HD, 8, 2, TMA, SINGLE>{}, 1, (pairs + n_sm - 1) / n_sm);
+            if (SINGLE && reach > 4096) return go(Variant<HD, 16, 2, TMA, SINGLE>{}, 1, 0);
+            return n_splits == 2 ? go(Variant<HD, 8, 2, TMA, SINGLE>{}, 1, 0) : go(Variant<HD, 16, kAhead, TMA, SINGLE>{}, 1, 0);
         }
     }
+    if constexpr (SINGLE) {
+        // Blocks of single heads are through with their keys so fast that how evenly the SMs have them counts: where more fit an SM than its share of the pairs, the
+        // first SMs that the kernel before leaves take too many.  From a share of two on no SM takes more than that, and from four on the blocks keep one tile ahead, which
+        // is enough for the memory (us a launch, as many as fit and two tiles ahead / so: 384 pairs on 300 6.1 / 5.6, on 2048 34.9 / 31.3; 768 on 300 10.1 / 8.1, on 1024
+        // 35.3 / 32.3, on 4096 137 / 125; 1024 on 300 10.3 / 10.5, on 4096 164 / 154; the tensor cores' form 34, 33.3, 123 and 156 where those are bound by memory; us a
+        // step: medium, 14 requests on 20 to 60 719 / 705, on 200 to 900 931 / 868; XL, 10 requests 2250 / 2108 there, with one tile ahead as well 2437).
+        // More pairs than the SMs hold at once even in blocks of two warps: as many as fit (2048 pairs on 1024 79 us with two tiles ahead, 81 with one).
+        using Wide1 = Variant<HD, 4, 2, TMA, SINGLE>;
+        using Narrow1 = Variant<HD, 2, 2, TMA, SINGLE>;
+        const long share = (pairs + n_sm - 1) / n_sm;
+        if (n_splits == 1 && (share == 2 || share == 3)) return go(Variant<HD, 4, 3, TMA, SINGLE>{}, 1, share);
+        if (n_splits == 1 && share > 3) {
+            int per_wide = 1, per_narrow = 1;
+            if (int rc = Wide1::blocks_per_sm(&per_wide)) return rc;
+            if (int rc = Narrow1::blocks_per_sm(&per_narrow)) return rc;
+            if (share <= per_wide) return go(Wide1{}, 1, share);
+            // Blocks of two warps, all at once, unless those of four fill more than half of their last wave (us four / two warps: 1200 pairs on 1024 51.3 / 48.2, 1536 59.6 / 62.0).
+            const long slots = (long)per_wide * n_sm;
+            if (share <= per_narrow) return 2 * (pairs % slots) <= slots && pairs % slots != 0 ? go(Narrow1{}, 1, share) : go(Wide1{}, 1, 0);
+        }
+        // Ranges in a cluster, long contexts: one tile ahead as above (48 pairs in eight ranges on 16384 34.4 / 32.8).
+        if (n_splits > 1 && n_splits <= 8 && reach > 4096) return go(Wide1{}, n_splits, 0);
+    }
+    using Wide = Variant<HD, 4, kAhead, TMA, SINGLE>;
+    using Narrow = Variant<HD, 2, kAhead, TMA, SINGLE>;
     int per_wide = 1, per_narrow = 1;
     if (int rc = Wide::blocks_per_sm(&per_wide)) return rc;
     if (int rc = Narrow::blocks_per_sm(&per_narrow)) return rc;
@@ -599,11 +632,7 @@ int launch_for(const CUtensorMap& map_kv, int kv_rows, int* status, const void* 
     const long waves_wide = (blocks + slots_wide - 1) / slots_wide, waves_narrow = (blocks + slots_narrow - 1) / slots_narrow;
     // fill = blocks / (waves * slots); compared without division
     const bool narrow = blocks > slots_wide && waves_wide * slots_wide >= waves_narrow * slots_narrow;
-    if (narrow)
-        return Narrow::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride, partial, counters,
-                              n_seq, n_head, n_kv_head, page_shift, scale, window, n_splits, distance, sink, soft_cap, bound, s);
-    return Wide::launch(map_kv, kv_rows, status, q, q_stride, cache, q_start, positions, block_table, table_stride, out, out_stride, partial, counters, n_seq,
-                        n_head, n_kv_head, page_shift, scale, window, n_splits, distance, sink, soft_cap, bound, s);
+    return narrow ? go(Narrow{}, n_splits, 0) : go(Wide{}, n_splits, 0);
 }
 
 }  // namespace

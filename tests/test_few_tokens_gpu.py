@@ -39,3 +39,20 @@ def test_decode_attention_of_single_heads(dev, n_head, page_size, n_seq, window,
     ref = _attention_reference(refs, n_head, n_head, scale, window)
     # 32-bit weights and sums of up to 1024 values of order one (a rounding each), and the result in bfloat16.
     assert ((out.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1024 * 2.0 ** -23 * 4).all() and int(counters.abs().sum()) == 0
+
+
+@pytest.mark.parametrize("n_head,n_seq,splits,max_keys", [
+    (25, 9, 1, 0), (25, 16, 1, 0), (16, 32, 1, 0), (12, 64, 1, 0), (25, 48, 1, 0), (16, 96, 1, 0), (24, 80, 1, 0),         # two to thirteen pairs an SM
+    (25, 8, 2, 0), (12, 8, 4, 0), (12, 8, 4, 5000), (3, 9, 8, 5000)])                                                        # wide blocks, and ranges in a cluster
+def test_decode_attention_of_many_single_heads(dev, n_head, n_seq, splits, max_keys):
+    """Every form that the number of pairs chooses: tiles ahead, blocks held to an SM's share of them, blocks of two warps."""
+    from liyab_b200 import ops
+    lens, scale = ([1, 15, 16, 17, 31, 100, 250, 33, 600] * 11)[:n_seq], 0.125
+    q, cache, _, positions, table, refs = _paged_case(dev, torch.bfloat16, n_head, n_head, 64, 16, lens, [1] * n_seq, seed=n_seq, boost=(28, 4.0))
+    partial = torch.full((n_seq * n_head * splits * 66,), float("nan"), device=dev)
+    counters = torch.zeros(n_seq * n_head, dtype=torch.int32, device=dev)
+    out = torch.full_like(q, float("nan"))
+    ops.decode_attention(q, cache, positions, table, out, partial, counters, n_seq, n_head, n_head, 64, 16, scale, 0, splits, tensor_cores=True, max_keys=max_keys)
+    ref = _attention_reference(refs, n_head, n_head, scale, 0)
+    assert ((out.double().cpu() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1024 * 2.0 ** -23 * 4).all() and int(counters.abs().sum()) == 0
+    assert ops.device_status() == 0
