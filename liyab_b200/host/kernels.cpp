@@ -2,6 +2,7 @@
 
 #include <cstdlib>
 #include <algorithm>
+#include <cmath>
 
 #include "../csrc/api.h"
 
@@ -323,27 +324,24 @@ struct Tiles {
     }
 };
 
+// Two bounds of a launch that give way to each other: near the larger one where they are apart, above both where they are close.
+double both(double x, double y, double p) { return x > 0 && y > 0 ? std::pow(std::pow(x, p) + std::pow(y, p), 1 / p) : std::max(x, y); }
+
 // Microseconds of a launch of the tcgen05 kernel (128 rows and 128 keys a step, two blocks an SM), of the mma.sync kernel (64 and 64, several
-// blocks an SM) and of the decode kernel.  The last two were fitted to 813 steps of GPT-2 small, medium and XL (none to 60 single tokens on 50 to 1000 keys
-// beside portions of 40 to 700 tokens on 0 to 700, and one to twenty portions alone), the first to launches of one to sixteen portions of 37 to 1024 tokens on 0 to
-// 896 with 12 and 25 heads (us measured / estimated: 1 x 37 3.9 / 4.1, 16 x 128 6.5 / 6.3, 8 x 180 7.1 / 7.1, 1 x 453 8.8 / 9.0, 453 on 300 12.3 / 12.3,
-// 1 x 1024 15.4 / 15.6, 5 x 469 18.5 / 18.3, 2 x 1024 with 25 heads 22.1 / 21.4; the mma.sync kernel 4.1 to 62 there).
-// Steps of twenty requests and more were not timed again with this kernel: they keep the estimate, and so the choice, of the kernel
-// before it (one block an SM, which a block without rows cost half a microsecond a wave).
-double tcgen05_cost(const Tiles& t, double heads, double grid, double all_tiles, bool many, double sms) {
-    if (many) return 3.2 + std::max(1.7 * t.longest, 1.9 * (t.steps + 2.1 * t.count) * heads / sms) + 0.52 * (all_tiles - t.count * heads) / sms;
-    return 2.4 + std::max(1.65 * t.longest, 1.16 * (t.steps + 1.56 * t.count) * heads / sms) + 0.25 * (grid - t.count * heads) / sms;
+// blocks an SM) and of the decode kernel, alone and behind the tiles.  One model for any number of requests, fitted to 785 random steps of 4 to 32 heads (none to 80 single tokens on 20
+// to 6000 keys beside one to three portions of 2 to 700 tokens on 0 to 1200; one to 80 portions alone), each timed in every way it can be launched: half of the estimates are
+// within 5 % and nine of ten within 15 %, and the launches they choose are 0.9 % slower than the best ones on average.  The line between the two kernels' launches of portions lies
+// where many of them are shorter than a tile (us by tcgen05 / mma.sync: 20 of 100 with 25 heads 13.2 / 17.6, 40 of 64 21.2 / 14.8).
+double tcgen05_cost(const Tiles& t, double heads, double grid, double sms) {
+    return 2.53 + both(1.60 * t.longest, 1.31 * (t.steps + 0.85 * t.count) * heads / sms, 3.2) + 0.6 * (grid - t.count * heads) / sms;
 }
-// The tcgen05 launch with a block for each single token and head: such a block takes 1.5 us and 1 us for every 217 keys on an SM of its own, 7.5 us and 1 us for
-// every 95 keys where all SMs have two blocks, beside the tiles' work (us measured / estimated, us in two launches: 12 on 100 to 900 beside 453 on 300,
-// 25 heads 20.0 / 20.6, 25.0; 16 on 50 to 900 beside 100, 12 heads 8.5 / 10.8, 14.0; 6 on 300 to 900 beside 300 7.3 / 8.0, 15.2; 4 beside 200, 25 heads 6.9 / 8.0, 13.8;
-// 12 on 1000 beside 2000 on 4000, 16 heads 93.9 / 97, 105.5; not there: 40 on 500 beside 2, 12 heads 24.0 / 23.4, 16.1; 100 on 300 beside 64 44.6 / 45, 29.8; 30 on
-// 800 beside 600, 25 heads 46.4 / 47, 38.2; and by the keys' ranges of eight blocks, 4 on 6000 beside 200 29.9 / 31, 20.2; 1 on 3000 beside 100 15.4 / 17.7, 10.6).
+double mma_cost(const Tiles& t, double heads, double sms) { return 2.35 + both(1.78 * t.longest, 0.90 * (t.steps + 0.6 * t.count) * heads / sms, 1.7); }
+double decode_cost(double longest, double all, double heads, double sms) { return 3.1 + both(0.2 * longest / 128, 0.71 * all / 128 * heads / sms, 4); }
+// The tcgen05 launch with a block for each single token and head (us measured / estimated, us in two launches: 12 on 100 to 900 beside 500 on 300, 25 heads
+// 20.2 / 21.8, 26.0; six on 900 to 1000 beside 256, 12 heads 8.3 / 7.7, 11.7; thirty on 700 to 900 beside 600, 25 heads 46.0 / 44.4, 39.0; one on 3000 beside 100 16.0 / 16.4, 10.9).
 double joined_cost(const Tiles& t, double singles, double longest, double all, double heads, double sms) {
-    return 2.4 + std::max({1.65 * t.longest, 1.5 + longest / 217, 1.16 * (t.steps + 1.56 * t.count) * heads / sms + (7.5 * singles + all / 95) * heads / (2 * sms)});
+    return 2.4 + both(std::max(1.67 * t.longest, 0.13 + longest / 217), 1.54 * t.steps * heads / sms + (5.2 * singles + all / 80) * heads / (2 * sms), 5);
 }
-double mma_cost(const Tiles& t, double heads, double sms) { return 1.8 + std::max(2.15 * t.longest, 1.15 * (t.steps + 0.4 * t.count) * heads / sms); }
-double decode_cost(double longest, double all, double heads, double sms) { return 2.5 + std::max(0.35 * longest, 0.6 * all * heads / sms) / 128; }
 
 }  // namespace
 
@@ -389,26 +387,24 @@ AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const i
             n_single += 1;
         }
     }
-    const double never = 1e30, all_tiles = static_cast<double>(n_seq) * heads * ((max_q_len + 127) / 128);
-    const double grid = std::min(all_tiles, heads * (q_start[n_seq] / 128 + n_seq));
-    const bool tc = prefill_tc_supports(a), decode = longest_single > 0 && decode_mma_supports(a);
-    const double singles = decode ? decode_cost(longest_single, all_single, heads, sms) : never;
-    double best = never;
-    for (const bool apart : {false, true})
-        for (const bool tcgen05 : {true, false}) {
-            const int which = apart ? 0 : 1;
-            const double cost = (!tcgen05 ? mma_cost(narrow[which], heads, sms) : tc ? tcgen05_cost(wide[which], heads, grid, all_tiles, n_seq >= 20, sms) : never) + (apart ? singles : 0);
-            if (cost < best) {
-                best = cost;
-                plan.apart = apart;
-                plan.tcgen05 = tcgen05;
-            }
+    const double grid = heads * std::min(n_seq * ((max_q_len + 127) / 128), q_start[n_seq] / 128 + n_seq);
+    const bool tc = prefill_tc_supports(a), decode = n_single > 0 && decode_mma_supports(a);
+    const double singles = decode ? decode_cost(longest_single, all_single, heads, sms) : 0;
+    double best = 1e30;
+    auto way = [&](double cost, AttentionPlan as) {
+        if (cost < best) {
+            best = cost;
+            plan = as;
         }
-    // Behind the tiles the decode kernel's work takes half as long again as in a launch alone.
-    if (plan.tcgen05 && a.n_head == a.n_kv_head && n_single > 0 && wide[0].count > 0)
-        plan.joined = joined_cost(wide[0], n_single, longest_single, all_single, heads, sms) <
-                      tcgen05_cost(wide[plan.apart ? 0 : 1], heads, grid, all_tiles, false, sms) + (plan.apart ? decode_cost(longest_single, 1.5 * all_single, heads, sms) : 0);
-    if (plan.joined) plan.apart = false;
+    };
+    if (tc) way(tcgen05_cost(wide[1], heads, grid, sms), {.tcgen05 = true});
+    way(mma_cost(narrow[1], heads, sms), {});
+    if (decode) {          // behind the tiles, as those leave SMs free
+        if (tc) way(tcgen05_cost(wide[0], heads, grid, sms) + 0.9 * singles, {.apart = true, .tcgen05 = true});
+        way(mma_cost(narrow[0], heads, sms) + 1.1 * singles, {.apart = true});
+    }
+    if (tc && a.n_head == a.n_kv_head && n_single > 0 && wide[0].count > 0)
+        way(joined_cost(wide[0], n_single, longest_single, all_single, heads, sms), {.tcgen05 = true, .joined = true});
     return plan;
 }
 

@@ -28,18 +28,21 @@ def singles(n, lo, hi):
     return [(r.randint(lo, hi), 1) for _ in range(n)]
 
 
+# Measured in every way a step can be launched (us: with the chosen one, with the best of the others).
 @pytest.mark.parametrize("heads,requests,want", [
-    # The launch for single tokens costs 3 to 5 us: not where they end before the portion does and all blocks run at once (0.93 to 0.98 of the speed) ...
-    (12, singles(3, 50, 250) + [(0, 500)], TCGEN05), (12, singles(6, 300, 900) + [(700, 200)], TCGEN05), (12, singles(6, 50, 250) + [(300, 300)], TCGEN05),
-    # ... but where they reach further than the portion (1.05 to 1.10), or their blocks would fill the GPU several times (1.15 to 1.6): by blocks of the portion's
-    # launch (us in one launch / in two: 20.0 / 25.0 for twelve beside 500 on 300 with 25 heads) or, where those take longer (15.4 /
-    # 10.6 for one on 3000 beside 100), by a launch of their own.
+    # Single tokens among the portion's tiles, where they end before it does and all blocks run at once (14.9 / 14.9, 11.2 / 11.4) ...
+    (12, singles(6, 300, 900) + [(700, 200)], TCGEN05), (12, singles(6, 50, 250) + [(300, 300)], TCGEN05),
+    # ... by blocks of their own in that launch, where they reach further (8.3 / 11.7, 20.2 / 26.0, 23.5 / 23.0, 18.5 / 18.1, 4.4 / 7.6) ...
     (12, singles(6, 900, 1000) + [(0, 256)], TCGEN05 | JOINED), (25, singles(12, 300, 900) + [(300, 500)], TCGEN05 | JOINED), (12, singles(30, 900, 1000) + [(0, 500)], TCGEN05 | JOINED),
-    (25, singles(16, 100, 300) + [(0, 700)], APART | TCGEN05), (25, singles(1, 3000, 3000) + [(0, 100)], APART | TCGEN05),
-    # Many blocks without rows: the mma.sync kernel for a short portion (the tcgen05 kernel has 0.82 of its speed there, 0.95 to 0.93 in two launches).
-    (12, singles(30, 50, 250) + [(0, 130)], 0), (25, singles(30, 300, 900) + [(0, 130)], APART), (12, singles(60, 900, 1000) + [(0, 130)], APART),
-    # Portions alone: the tcgen05 kernel for long ones (0.94 to 0.86 of its speed by the other), the other one for many short ones (0.87 to 0.94).
-    (12, [(0, 1024)], TCGEN05), (12, [(0, 1000)] * 2, TCGEN05), (25, [(0, 1000)] * 2, TCGEN05), (25, [(0, 218), (0, 441), (0, 583), (0, 560), (0, 541)], TCGEN05), (25, [(0, 100)] * 20, 0), (25, [(350, 64)] * 20, 0), (16, [(350, 40)] * 20, 0)])
+    (25, singles(16, 100, 300) + [(0, 700)], TCGEN05 | JOINED), (12, [(300, 1)] * 6 + [(0, 64)], TCGEN05 | JOINED), (4, [(850, 1)] * 4 + [(0, 300)], TCGEN05 | JOINED),
+    # ... or by a launch of their own, where they are many or long (39.0 / 46.0, 10.9 / 16.0, 24.5 / 30.5, 35.0 / 39.1, 13.6 / 20.8, 19.3 / 44.1).
+    (25, singles(30, 700, 900) + [(0, 600)], APART | TCGEN05), (25, singles(1, 3000, 3000) + [(0, 100)], APART | TCGEN05), (25, singles(30, 300, 900) + [(0, 130)], APART | TCGEN05),
+    (12, singles(60, 900, 1000) + [(0, 130)], APART | TCGEN05), (12, singles(40, 400, 600) + [(0, 2)], APART | TCGEN05), (12, singles(100, 250, 350) + [(0, 64)], APART),
+    # Portions alone: the tcgen05 kernel for long ones (16.0 / 35.7 and the like) and, from nineteen requests to twenty, for short ones (13.0 / 16.9, 13.2 / 17.6, 22.5 / 34.0, 20.0 / 21.2,
+    # 25.5 / 41.1), the other one for many of less than a tile (14.8 / 21.2, 18.1 / 28.6, 5.3 / 5.7).
+    (12, [(0, 1024)], TCGEN05), (12, [(0, 1000)] * 2, TCGEN05), (25, [(0, 1000)] * 2, TCGEN05), (25, [(0, 218), (0, 441), (0, 583), (0, 560), (0, 541)], TCGEN05),
+    (25, [(0, 100)] * 19, TCGEN05), (25, [(0, 100)] * 20, TCGEN05), (25, [(350, 64)] * 20, TCGEN05), (16, [(350, 40)] * 20, TCGEN05), (12, [(500, 20)] * 40, TCGEN05),
+    (25, [(0, 64)] * 40, 0), (25, [(0, 30)] * 60, 0), (12, [(0, 8)] * 20, 0)])
 def test_choices_that_were_measured(heads, requests, want):
     assert plan(requests, heads) == want
     assert plan(requests[::-1], heads) == want          # whatever their order
