@@ -96,6 +96,7 @@ _SIGNATURES = {
     "lb_replayer_options_default": ([P(ReplayerOptionsC)], None), "lb_replayer_create": ([cp, cp, i64, P(ReplayerOptionsC), P(vp)], i32),
     "lb_replayer_destroy": ([vp], None), "lb_replayer_cache": ([vp], vp), "lb_replayer_describe": ([vp] + _TEXT, i32),
     "lb_attention_plan": ([cp, i32, i32, i32, i32, i32, i32, i32, P(i32), P(i32), i32, P(i32)], i32),
+    "lb_attention_plan_scores": ([cp, i32, i32, i32, i32, i32, i32, i32, i32, P(i32), P(i32), i32, P(i32)], i32),
     "lb_host_buffer_create": ([i32, sz, P(vp)], i32), "lb_host_buffer_destroy": ([vp], None),
     "lb_replayer_step": ([vp, sz, P(i64), P(i32), P(i32), P(i32), P(i32), P(f32), sz, P(i32)], i32),
     "lb_replayer_set": ([vp, cp, i32], i32), "lb_replayer_counters": ([vp] + _TEXT, i32),

@@ -527,11 +527,11 @@ int lb_prefill_attention_tc_portions(const void* q, int64_t q_stride, int n_toke
                                      const int32_t* n_past, const int32_t* block_table, int table_stride, void* out, int64_t out_stride, int n_seq,
                                      int max_q_len, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window,
                                      const float* distance, const float* sink, float soft_cap, float bound, int min_len, void* stream);
-/* The same; with `singles` non-zero (n_head == n_kv_head, min_len > 1) the requests of one token are served by the same launch, on the 32-bit units. */
+/* The same; flags: 1 (n_head == n_kv_head, min_len > 1) the requests of one token are served by the same launch, on the 32-bit units; 2 no two blocks share an SM. */
 int lb_prefill_attention_tc_mixed(const void* q, int64_t q_stride, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                                      const int32_t* n_past, const int32_t* block_table, int table_stride, void* out, int64_t out_stride, int n_seq,
                                      int max_q_len, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window,
-                                     const float* distance, const float* sink, float soft_cap, float bound, int min_len, int singles, void* stream);
+                                     const float* distance, const float* sink, float soft_cap, float bound, int min_len, int flags, void* stream);
 int lb_decode_attention_mma_mixed(const void* q, int64_t q_stride, const void* cache, int n_pages, const int32_t* q_start, const int32_t* positions,
                                   const int32_t* block_table, int table_stride, void* out, int64_t out_stride, float* partial, int* counters, int n_seq,
                                   int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window, int n_splits, int max_keys,

@@ -26,7 +26,8 @@
 // 1,024 cycles, its products some 500 of the tensor pipe, and a tile is a chain (scores,
 // maximum, exponentials, update).  So two blocks share an SM (256 columns of tensor
 // memory and 82 KB each): one block's chain and its start hide under the other's
-// exponentials.  Measured (us a launch, 20 a graph; one block of sixteen softmax warps an SM with the probabilities through shared memory /
+// exponentials, or one where the step's plan says so: where a few long blocks set the time, and above all with capped scores or a penalty by distance, whose two or three
+// special functions a score two blocks share (2 requests x 12 heads x 1,024 tokens capped 33.0 / 27.5 us, 1 x 16 x 2,048 70 / 52).  Measured (us a launch, 20 a graph; one block of sixteen softmax warps an SM with the probabilities through shared memory /
 // here / the mma.sync kernel): 2 requests x 12 heads x 1,024 tokens 21.1 / 17.4 / 40.3, 5 x 25 x 469 36.7 / 18.5 / 40.5, 1 x 25 x 453
 // 12.9 / 8.8 / 19.3, 8 x 12 x 180 14.9 / 7.1 / 10.7, 1 x 12 x 37 7.0 / 3.9 / 4.1.  Long contexts with few blocks are the chain: some 2,600 cycles
 // a tile.  On the way: issuing the products and the copies from a branch on the lane's number took 700 cycles for eight products and
@@ -88,6 +89,17 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// 1 / x for x >= 1 (0 above the normal range), log2 x for x in the normal range: the hardware approximations alone as well.
+__device__ __forceinline__ float rcp_approx(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float lg2_approx(float x) {
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 // The wait for a load, tied to its registers so that nothing is made of them before it.
@@ -491,6 +503,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
         // With a soft cap the scores are brought to base 2 as they are capped, so nothing is left to multiply.
         const lb_soft_cap capped(PLAIN ? 0.0f : soft_cap, bound);
         const float raw_sc = scale * kLog2e, sc = !PLAIN && capped.on ? 1.0f : raw_sc;
+        const float cap_in = raw_sc * capped.in;
         // The head's penalty by distance in the units of the raw scores (which are multiplied by sc later): a key d positions
         // back loses r1 ln(1 + r2 d) / scale = pen log2(1 + r2 d), or, with r2 < 0, r1 d / scale = pen d.
         const float r2 = !PLAIN && distance != nullptr ? distance[n_head + head] : 0.0f;
@@ -530,9 +543,14 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                 if (!seen[h]) continue;
                 tmem_ld32(t_row + (uint32_t)(part * kKeys + h * 32), v);
                 tmem_ld_wait32(v);
-                if (!PLAIN && capped.on) {
+                if (!PLAIN && capped.on && capped.series) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(capped(__uint_as_float(v[i]) * raw_sc));
+                } else if (!PLAIN && capped.on) {
+                    // The other form of lb_soft_cap, out - 2 out / (1 + 2^(in s)).
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        v[i] = __float_as_uint(fmaf(-2.0f * capped.out, rcp_approx(1.0f + ex2_approx(__uint_as_float(v[i]) * cap_in)), capped.out));
                 } else if (!PLAIN && distance != nullptr && r2 < 0.0f) {
                     // pen (pos - jh - i) = b0 - pen i.
                     const float b0 = pen * (float)(pos - jh);
@@ -543,7 +561,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __g
                     const float a0 = fmaf(r2, (float)(pos - jh), 1.0f);
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
-                        v[i] = __float_as_uint(fmaf(-pen, __log2f(fmaxf(fmaf(-r2, (float)i, a0), 1e-30f)), __uint_as_float(v[i])));
+                        v[i] = __float_as_uint(fmaf(-pen, lg2_approx(fmaxf(fmaf(-r2, (float)i, a0), 1e-30f)), __uint_as_float(v[i])));
                 }
                 const bool masked = jh + 31 > pos_lo || jh < first_hi;
                 if (masked) {
@@ -739,7 +757,9 @@ extern "C" int lb_prefill_attention_tc_portions(const void* q, int64_t q_stride,
 extern "C" int lb_prefill_attention_tc_mixed(const void* q, int64_t q_stride, int n_tokens, const void* cache, int n_pages, const int32_t* q_start,
                                               const int32_t* n_past, const int32_t* block_table, int table_stride, void* out, int64_t out_stride,
                                               int n_seq, int max_q_len, int n_head, int n_kv_head, int head_dim, int page_size, float scale, int window,
-                                              const float* distance, const float* sink, float soft_cap, float bound, int min_len, int singles, void* stream) {
+                                              const float* distance, const float* sink, float soft_cap, float bound, int min_len, int flags, void* stream) {
+    LB_CHECK_ARG((flags & ~3) == 0, "prefill attention (tcgen05): unknown flags %d", flags);
+    const int singles = flags & 1;
     LB_CHECK_ARG(singles == 0 || (min_len > 1 && n_head == n_kv_head), "prefill attention (tcgen05): single tokens beside the tiles need a key/value head to every query head and min_len above 1");
     LB_CHECK_ARG(soft_cap >= 0.0f && (soft_cap == 0.0f || distance == nullptr), "prefill attention (tcgen05): a soft cap is positive and goes without a penalty by distance");
     LB_CHECK_ARG(distance == nullptr || scale != 0.0f, "prefill attention (tcgen05): a penalty by distance needs a factor on the scores that is not zero");
@@ -767,13 +787,14 @@ extern "C" int lb_prefill_attention_tc_mixed(const void* q, int64_t q_stride, in
     int* status = nullptr;
     rc = lb_tc_status_word(&status);
     if (rc != LB_OK) return rc;
-    constexpr size_t smem = 1024 + (size_t)(1 + 2 * kStages) * kTileBytes + sizeof(Control);
+    constexpr size_t kTwo = 1024 + (size_t)(1 + 2 * kStages) * kTileBytes + sizeof(Control), kOne = 114 * 1024;      // the least that keeps a second block out of an SM's 228 KB
     static bool configured = false;
     if (!configured) {
         for (auto* kernel : {prefill_attention_tc_kernel<true>, prefill_attention_tc_kernel<false>})
-            LB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            LB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOne));
         configured = true;
     }
+    const size_t smem = (flags & 2) != 0 ? kOne : kTwo;
     dim3 grid((unsigned)blocks);
     auto* kernel = soft_cap == 0.0f && distance == nullptr ? prefill_attention_tc_kernel<true> : prefill_attention_tc_kernel<false>;
     LB_CHECK_CUDA(lb_launch_overlapped(kernel, dim3(grid), dim3(kThreads), smem, static_cast<cudaStream_t>(stream), 

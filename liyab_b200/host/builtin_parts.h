@@ -106,7 +106,7 @@ public:
     int64_t max_;
 };
 
-inline AttentionUse attention_use(const kernels::AttentionShape& a) { return {a.n_head, a.n_kv_head, a.head_dim, a.mask()}; }
+inline AttentionUse attention_use(const kernels::AttentionShape& a) { return {a.n_head, a.n_kv_head, a.head_dim, a.mask(), a.form()}; }
 
 // Chooses the attention kernel for queries q over a unit's pages.  bfloat16: a split-key decode kernel for steps of
 // single tokens (on the tensor cores where that one takes the shape, else scalar), the tensor-core prefill kernel for
@@ -136,7 +136,7 @@ inline void attend(StepContext& ctx, const Rows& q, void* cache, const GroupView
     // An attention that its mixer does not list is planned here; a captured step keeps to the plan of the step that it was recorded from.
     AttentionPlan plan;
     if (const AttentionPlan* p = ctx.attention_plan(attention_use(a)); p != nullptr) plan = *p;
-    else if (!ctx.decode_only) plan = kernels::attention_plan(ctx.runtime, a, ctx.host_q_start.data(), ctx.host_n_past.data(), S, ctx.max_q_len);
+    else if (!ctx.decode_only) plan = kernels::attention_plan(ctx.runtime, a, a.form(), ctx.host_q_start.data(), ctx.host_n_past.data(), S, ctx.max_q_len);
     plan.apart = plan.apart && kernels::decode_mma_supports(a);
     if (ctx.runtime.dtype == DType::BF16 && kernels::prefill_supports(a)) {
         kernels::prefill_attention(ctx.runtime, q, T, cache, n_pages, ctx.q_start, ctx.n_past, view.block_table, view.table_width, att, S, ctx.max_q_len,

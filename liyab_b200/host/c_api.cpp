@@ -729,7 +729,13 @@ void lb_host_buffer_destroy(void* buffer) {
 
 int32_t lb_attention_plan(const char* dtype, int32_t n_head, int32_t n_kv_head, int32_t head_dim, int32_t page_size, int32_t mask, int32_t sm_count, int32_t n_seq,
                           const int32_t* q_start, const int32_t* n_past, int32_t max_q_len, int32_t* bits) {
+    return lb_attention_plan_scores(dtype, n_head, n_kv_head, head_dim, page_size, mask, 0, sm_count, n_seq, q_start, n_past, max_q_len, bits);
+}
+
+int32_t lb_attention_plan_scores(const char* dtype, int32_t n_head, int32_t n_kv_head, int32_t head_dim, int32_t page_size, int32_t mask, int32_t scores, int32_t sm_count,
+                                 int32_t n_seq, const int32_t* q_start, const int32_t* n_past, int32_t max_q_len, int32_t* bits) {
     return guarded([&] {
+        if (scores < kernels::kPlainScores || scores > kernels::kDistanceScores) throw invalid_argument("attention plan: scores {} (0 plain to 3 with a penalty by distance)", scores);
         need(q_start, "q_start");
         need(n_past, "n_past");
         need(bits, "bits");
@@ -742,7 +748,7 @@ int32_t lb_attention_plan(const char* dtype, int32_t n_head, int32_t n_kv_head, 
         a.head_dim = head_dim;
         a.page_size = page_size;
         (mask < 0 ? a.chunk : a.window) = std::abs(mask);
-        *bits = kernels::attention_plan(rt, a, q_start, n_past, n_seq, max_q_len).bits();
+        *bits = kernels::attention_plan(rt, a, scores, q_start, n_past, n_seq, max_q_len).bits();
     });
 }
 

@@ -166,6 +166,7 @@ public:
             throw unsupported("gated_attention: capped scores go without a penalty by distance");
         if (s.options.get_bool("slopes", false)) {
             if (shape.distance != nullptr) throw unsupported("gated_attention: slopes or a learned penalty by distance, not both");
+            shape.straight = true;
             for (int h = 0; h < H; ++h) slopes.host.push_back(static_cast<float>(std::exp2(-8.0 * (h + 1) / H)));
             for (int h = 0; h < H; ++h) slopes.host.push_back(-1.0f);        // a negative second number: a straight line
         }

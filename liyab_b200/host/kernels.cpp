@@ -328,24 +328,46 @@ struct Tiles {
 double both(double x, double y, double p) { return x > 0 && y > 0 ? std::pow(std::pow(x, p) + std::pow(y, p), 1 / p) : std::max(x, y); }
 
 // Microseconds of a launch of the tcgen05 kernel (128 rows and 128 keys a step, two blocks an SM), of the mma.sync kernel (64 and 64, several
-// blocks an SM) and of the decode kernel, alone and behind the tiles.  One model for any number of requests, fitted to 785 random steps of 4 to 32 heads (none to 80 single tokens on 20
+// blocks an SM) and of the decode kernel, alone and behind the tiles.  One model for any number of requests, fitted to 2,100 random steps of 4 to 32 heads (none to 80 single tokens on 20
 // to 6000 keys beside one to three portions of 2 to 700 tokens on 0 to 1200; one to 80 portions alone), each timed in every way it can be launched: half of the estimates are
-// within 5 % and nine of ten within 15 %, and the launches they choose are 0.9 % slower than the best ones on average.  The line between the two kernels' launches of portions lies
+// within 5 % and nine of ten within 15 %, and the launches they choose are 1.2 % slower than the best of eight ways on average.  The line between the two kernels' launches of portions lies
 // where many of them are shorter than a tile (us by tcgen05 / mma.sync: 20 of 100 with 25 heads 13.2 / 17.6, 40 of 64 21.2 / 14.8).
-double tcgen05_cost(const Tiles& t, double heads, double grid, double sms) {
-    return 2.53 + both(1.60 * t.longest, 1.31 * (t.steps + 0.85 * t.count) * heads / sms, 3.2) + 0.6 * (grid - t.count * heads) / sms;
+// `form` (ScoreForm): what a tile's scores go through, which the SM's special-function units bound; `alone`: one block of the launch an SM.  Two share those units, so one is
+// faster where the longest blocks set the time (us two / one an SM, 16 heads, 2048 tokens: plain scores 33.9 / 30.6, capped 70 / 52, capped by the series 52.8 / 42.6, with a penalty
+// by distance 55.3 / 44.8; but 12 heads, eight of 180 tokens 7.3 / 11.6 and 10.3 / 14.8).
+struct PerTile {
+    double chain, step;        // us of a step of the longest block, and of any step while all SMs are busy
+};
+// The longest block's time.  Where two blocks share an SM it waits for steps of the other one, of a block of average length on as many SMs as have two.
+double longest_us(const Tiles& t, const PerTile& c, double heads, bool alone, int form, double sms) {
+    constexpr double kOther[4] = {0.5, 0.9, 0.6, 0.6};
+    const double two = alone || t.count == 0 ? 0.0 : std::clamp(t.count * heads / sms - 1.0, 0.0, 1.0);
+    return c.chain * (t.longest + (two > 0 ? kOther[form] * two * t.steps / t.count : 0.0));
 }
-double mma_cost(const Tiles& t, double heads, double sms) { return 2.35 + both(1.78 * t.longest, 0.90 * (t.steps + 0.6 * t.count) * heads / sms, 1.7); }
-double decode_cost(double longest, double all, double heads, double sms) { return 3.1 + both(0.2 * longest / 128, 0.71 * all / 128 * heads / sms, 4); }
-// The tcgen05 launch with a block for each single token and head (us measured / estimated, us in two launches: 12 on 100 to 900 beside 500 on 300, 25 heads
-// 20.2 / 21.8, 26.0; six on 900 to 1000 beside 256, 12 heads 8.3 / 7.7, 11.7; thirty on 700 to 900 beside 600, 25 heads 46.0 / 44.4, 39.0; one on 3000 beside 100 16.0 / 16.4, 10.9).
-double joined_cost(const Tiles& t, double singles, double longest, double all, double heads, double sms) {
-    return 2.4 + both(std::max(1.67 * t.longest, 0.13 + longest / 217), 1.54 * t.steps * heads / sms + (5.2 * singles + all / 80) * heads / (2 * sms), 5);
+double tcgen05_cost(const Tiles& t, double heads, double grid, int form, bool alone, double sms) {
+    constexpr PerTile kPer[2][4] = {{{1.58, 1.29}, {2.92, 1.74}, {2.42, 1.69}, {2.54, 1.63}}, {{1.61, 2.29}, {2.94, 3.32}, {2.43, 2.98}, {2.53, 3.01}}};
+    const PerTile& c = kPer[alone][form];
+    return (alone ? 2.43 : 2.57) + both(longest_us(t, c, heads, alone, form, sms), c.step * (t.steps + (alone ? 0.99 : 0.91) * t.count) * heads / sms, alone ? 12.9 : 2.9) +
+           0.57 * (grid - t.count * heads) / sms;
+}
+double mma_cost(const Tiles& t, double heads, int form, double sms) {
+    constexpr PerTile kPer[4] = {{1.77, 0.90}, {2.28, 1.10}, {2.00, 1.03}, {3.08, 1.28}};
+    return 2.37 + both(kPer[form].chain * t.longest, kPer[form].step * (t.steps + 0.56 * t.count) * heads / sms, 1.62);
+}
+double decode_cost(double longest, double all, double heads, double sms) { return 3.15 + both(0.206 * longest / 128, 0.70 * all / 128 * heads / sms, 4); }
+// The tcgen05 launch with a block for each single token and head (us measured, us in two launches: 12 on 100 to 900 beside 500 on 300, 25 heads 20.2, 26.0; six on 900 to 1000 beside
+// 256, 12 heads 8.3, 11.7; thirty on 700 to 900 beside 600, 25 heads 46.0, 39.0; one on 3000 beside 100 16.0, 10.9).
+double joined_cost(const Tiles& t, double singles, double longest, double all, double heads, int form, bool alone, double sms) {
+    constexpr PerTile kPer[2][4] = {{{1.65, 1.56}, {3.02, 2.84}, {2.52, 2.36}, {2.63, 2.53}}, {{1.63, 1.98}, {2.99, 3.20}, {2.45, 2.75}, {2.55, 2.97}}};
+    const PerTile& c = kPer[alone][form];
+    return (alone ? 2.30 : 2.44) + both(std::max(longest_us(t, c, heads, alone, form, sms), longest / (alone ? 207 : 217)),
+                                        c.step * (t.steps + (alone ? 0.98 : 0.0) * t.count) * heads / sms +
+                                            (alone ? 4.9 * singles + all / 70 : 5.0 * singles + all / 78) * heads / (2 * sms), alone ? 12.5 : 4.4);
 }
 
 }  // namespace
 
-AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const int32_t* q_start, const int32_t* n_past, int n_seq, int max_q_len) {
+AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, int form, const int32_t* q_start, const int32_t* n_past, int n_seq, int max_q_len) {
     AttentionPlan plan;
     const double heads = a.n_head, sms = rt.sm_count;
     const int64_t span = a.chunk > 0 ? a.chunk : a.window;
@@ -397,14 +419,15 @@ AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const i
             plan = as;
         }
     };
-    if (tc) way(tcgen05_cost(wide[1], heads, grid, sms), {.tcgen05 = true});
-    way(mma_cost(narrow[1], heads, sms), {});
-    if (decode) {          // behind the tiles, as those leave SMs free
-        if (tc) way(tcgen05_cost(wide[0], heads, grid, sms) + 0.9 * singles, {.apart = true, .tcgen05 = true});
-        way(mma_cost(narrow[0], heads, sms) + 1.1 * singles, {.apart = true});
+    way(mma_cost(narrow[1], heads, form, sms), {});
+    if (decode) way(mma_cost(narrow[0], heads, form, sms) + 1.1 * singles, {.apart = true});          // behind the tiles, as those leave SMs free
+    for (const bool alone : {false, true}) {
+        if (!tc) break;
+        way(tcgen05_cost(wide[1], heads, grid, form, alone, sms), {.tcgen05 = true, .alone = alone});
+        if (decode) way(tcgen05_cost(wide[0], heads, grid, form, alone, sms) + 0.9 * singles, {.apart = true, .tcgen05 = true, .alone = alone});
+        if (a.n_head == a.n_kv_head && n_single > 0 && wide[0].count > 0)
+            way(joined_cost(wide[0], n_single, longest_single, all_single, heads, form, alone, sms), {.tcgen05 = true, .joined = true, .alone = alone});
     }
-    if (tc && a.n_head == a.n_kv_head && n_single > 0 && wide[0].count > 0)
-        way(joined_cost(wide[0], n_single, longest_single, all_single, heads, sms), {.tcgen05 = true, .joined = true});
     return plan;
 }
 
@@ -419,7 +442,7 @@ void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const voi
     if (tc)
         check(lb_prefill_attention_tc_mixed(q.data, q.stride, n_tokens, cache, n_pages, q_start, n_past, block_table, table_width,
                                            out.data, out.stride, n_seq, max_q_len, a.n_head, a.n_kv_head, a.head_dim, a.page_size,
-                                           a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, singles ? 1 : 0, rt.stream), "prefill_attention_tc");
+                                           a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, (singles ? 1 : 0) | (plan.alone ? 2 : 0), rt.stream), "prefill_attention_tc");
     else
         check(lb_prefill_attention_portions(q.data, q.stride, cache, q_start, n_past, block_table, table_width, out.data, out.stride, n_seq,
                                         max_q_len, a.n_head, a.n_kv_head, a.head_dim, a.page_size, a.scale, a.mask(), a.distance, a.sink, a.soft_cap, a.score_bound, min_len, rt.stream),

@@ -90,6 +90,7 @@ void linear(const Runtime& rt, Workspace* ws, const Rows& a, const Tensor& w, co
 bool linear_with_cache(const Runtime& rt, Workspace* ws, const Rows& a, const Tensor& w, const float* bias, const Rows& out, int m,
                        const KvDestination& kv);
 
+enum ScoreForm : int { kPlainScores = 0, kCappedScores = 1, kSeriesScores = 2, kDistanceScores = 3 };
 struct AttentionShape {
     int n_head = 0, n_kv_head = 0, head_dim = 0, page_size = 0;
     float scale = 1.0f;
@@ -101,6 +102,12 @@ struct AttentionShape {
     const float* sink = nullptr;
     // A soft cap on the scores, s <- soft_cap tanh(s / soft_cap) (0: none), and the largest |s| before it that can occur (0: unknown).
     float soft_cap = 0.0f, score_bound = 0.0f;
+    // What the scores go through (ScoreForm); the cap's two forms are those of lb_soft_cap.
+    int form() const {
+        if (soft_cap > 0.0f) return score_bound > 0.0f && score_bound <= 0.25f * soft_cap ? kSeriesScores : kCappedScores;
+        return distance != nullptr && !straight ? kDistanceScores : kPlainScores;
+    }
+    bool straight = false;   // the penalty by distance is a straight line, which needs no logarithm
     // One number for the kernels: 0 all earlier keys, w > 0 a window, -c a chunk (a shape has one of the two at most).
     int mask() const { return chunk > 0 ? -chunk : window; }
 };
@@ -122,8 +129,8 @@ void prefill_attention(const Runtime& rt, const Rows& q, int n_tokens, const voi
                        int max_q_len, const AttentionPlan& plan, const AttentionShape& a);
 // How a step with prompt portions launches an attention (page_size, sink and so on of `a` are those of its launches): the cheapest of the launches that
 // take it, by estimates from the requests' tokens (q_start, n_past: n_seq + 1 and n_seq numbers on the host) and the longest portion that
-// the launches have room for.
-AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, const int32_t* q_start, const int32_t* n_past, int n_seq, int max_q_len);
+// the launches have room for; form: that of the scores (ScoreForm).
+AttentionPlan attention_plan(const Runtime& rt, const AttentionShape& a, int form, const int32_t* q_start, const int32_t* n_past, int n_seq, int max_q_len);
 
 // ---- row-wise pieces between the products: RMS norm in groups, token shift, xIELU, gated side input ----
 // out[r] = x[rows ? rows[r] : r] cut into `groups` equal parts, each over its own root mean square, times weight.

@@ -63,7 +63,7 @@ struct CacheUnit {
 
 // An attention that `attend` (builtin_parts.h) launches, and how it is launched in a step with prompt portions (see kernels::attention_plan).
 struct AttentionUse {
-    int n_head = 0, n_kv_head = 0, head_dim = 0, mask = 0;
+    int n_head = 0, n_kv_head = 0, head_dim = 0, mask = 0, form = 0;       // form: kernels::ScoreForm
     auto operator<=>(const AttentionUse&) const = default;
 };
 struct AttentionPlan {
@@ -71,8 +71,10 @@ struct AttentionPlan {
     bool tcgen05 = false;      // bfloat16: portions by the tcgen05 kernel where it takes the shape, else by the mma.sync one
     bool runs = false;         // float32: a tile of keys is read once for sixteen neighbouring tokens
     bool joined = false;       // bfloat16, with tcgen05 and not apart: that launch serves the requests of one token by blocks of their own
-    int bits() const { return (apart ? 1 : 0) | (tcgen05 ? 2 : 0) | (runs ? 4 : 0) | (joined ? 8 : 0); }
-    int key() const { return (bits() & 7) | (joined ? 4 : 0); }      // what tells one step's launches from another's, in three bits: `runs` is float32's
+    bool alone = false;        // bfloat16, with tcgen05: one block of that launch an SM
+    int bits() const { return (apart ? 1 : 0) | (tcgen05 ? 2 : 0) | (runs ? 4 : 0) | (joined ? 8 : 0) | (alone ? 16 : 0); }
+    // What tells one step's launches from another's, in three bits: two ways with mma.sync (float32: with `runs` and without), six with tcgen05.
+    int key() const { return tcgen05 ? 2 + (joined ? 2 : apart ? 1 : 0) + (alone ? 3 : 0) : apart || runs ? 1 : 0; }
 };
 
 // One cache group as a step sees it.

@@ -139,7 +139,7 @@ void Stepper::plan_attention(const std::vector<int>& rows, const std::vector<int
     }
     for (const AttentionUse& use : attention_uses_) {
         if (longest == 1 && decode_covers(use)) continue;
-        const AttentionPlan plan = kernels::attention_plan(model.runtime, attention_shape(use), q_start.data(), n_past.data(), static_cast<int>(rows.size()),
+        const AttentionPlan plan = kernels::attention_plan(model.runtime, attention_shape(use), use.form, q_start.data(), n_past.data(), static_cast<int>(rows.size()),
                                                            static_cast<int>((longest + 63) / 64 * 64));
         attention_bits_ |= static_cast<uint64_t>(plan.key()) << (3 * attention_plan_.size());
         attention_plan_.emplace_back(use, plan);

@@ -276,9 +276,13 @@ LB_API int32_t lb_replayer_step(lb_replayer* r, size_t n_entries, const int64_t*
 LB_API int32_t lb_host_buffer_create(int32_t device, size_t bytes, void** out);
 LB_API void lb_host_buffer_destroy(void* buffer);
 /* How a step whose request i brings q_start[i + 1] - q_start[i] tokens on n_past[i] launches an attention: 1 single tokens by a launch of the decode
- * kernel, 2 portions by the tcgen05 kernel, 4 (float32) tiles of keys shared among neighbouring tokens, 8 single tokens by blocks of the tcgen05 kernel's launch.  mask: 0 all earlier keys, w > 0 a window, -c a chunk. */
+ * kernel, 2 portions by the tcgen05 kernel, 4 (float32) tiles of keys shared among neighbouring tokens, 8 single tokens by blocks of the tcgen05 kernel's launch, 16 that
+ * launch with one block an SM.  mask: 0 all earlier keys, w > 0 a window, -c a chunk. */
 LB_API int32_t lb_attention_plan(const char* dtype, int32_t n_head, int32_t n_kv_head, int32_t head_dim, int32_t page_size, int32_t mask, int32_t sm_count,
                                  int32_t n_seq, const int32_t* q_start, const int32_t* n_past, int32_t max_q_len, int32_t* bits);
+/* The same for scores that are 1 capped, 2 capped with a bound that allows the series, 3 lowered by a learned function of the distance (0: plain, as above). */
+LB_API int32_t lb_attention_plan_scores(const char* dtype, int32_t n_head, int32_t n_kv_head, int32_t head_dim, int32_t page_size, int32_t mask, int32_t scores,
+                                        int32_t sm_count, int32_t n_seq, const int32_t* q_start, const int32_t* n_past, int32_t max_q_len, int32_t* bits);
 /* Options at run time: "cuda_graphs" 0/1, "fused_decode" 0 (cannot be switched back on). */
 LB_API int32_t lb_replayer_set(lb_replayer* r, const char* option, int32_t value);
 /* {"steps", "graph_steps", "fused_steps", "eager_steps", "graphs_captured", "tokens_run", "kernel_launches"} */

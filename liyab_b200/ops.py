@@ -529,10 +529,11 @@ def prefill_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tenso
                       block_table: torch.Tensor, out: torch.Tensor, n_seq: int, max_q_len: int, n_head: int,
                       n_kv_head: int, head_dim: int, page_size: int, scale: float, window: int = 0,
                       tcgen05: Optional[bool] = None, distance: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None,
-                      soft_cap: float = 0.0, score_bound: float = 0.0, min_len: int = 1, singles: bool = False) -> torch.Tensor:
+                      soft_cap: float = 0.0, score_bound: float = 0.0, min_len: int = 1, singles: bool = False, alone: bool = False) -> torch.Tensor:
     """Attention of the step's prompt portions of at least `min_len` tokens over their pages (bfloat16, tensor cores).  `tcgen05`: None picks
     the tcgen05 kernel where it takes the shape and the rows are 16-byte aligned, else the mma.sync one.  `distance`: as for
-    paged_attention_generic; `score_bound`: as for decode_attention.  `singles`: the tcgen05 launch serves the requests of one token as well."""
+    paged_attention_generic; `score_bound`: as for decode_attention.  `singles`: the tcgen05 launch serves the requests of one token as well;
+    `alone`: no two of its blocks share an SM."""
     if q.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or out.dtype != torch.bfloat16:
         raise invalid_argument("prefill attention takes bfloat16 only")
     if q.stride(1) != 1 or out.stride(1) != 1:
@@ -552,7 +553,7 @@ def prefill_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tenso
             _dev(q_start, "q_start", torch.int32), _dev(n_past, "n_past", torch.int32),
             _dev(block_table, "block_table", torch.int32), block_table.stride(0), _dev(out, "out"), out.stride(0), n_seq,
             max_q_len, n_head, n_kv_head, head_dim, page_size, float(scale), int(window), _distance(distance, n_head), _sink(sink, n_head), float(soft_cap), float(score_bound),
-            min_len, 1 if singles else 0, stream_ptr()), "prefill_attention_tc")
+            min_len, (1 if singles else 0) | (2 if alone else 0), stream_ptr()), "prefill_attention_tc")
         return out
     check(lib().lb_prefill_attention_portions(
         _dev(q, "q"), q.stride(0), _dev(cache, "cache"), _dev(q_start, "q_start", torch.int32),

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import plain_gpt2 as plain
-from test_attention_plan import APART, JOINED, TCGEN05, plan
+from test_attention_plan import ALONE, APART, JOINED, TCGEN05, plan
 from tiny_models import random_tokens
 
 pytestmark = pytest.mark.gpu
@@ -53,7 +53,7 @@ def test_a_captured_step_serves_every_arrangement(model, route):
                 rows = list(range(n)) if n < 50 else [0, n // 2] + [n - 1] * (9 - sum(m for m in lens if m < 50))
                 entries.append(StepEntry(name, fresh[:n], rows))
                 wants += [want_fresh[i] for i in rows]
-        assert plan([(held if n == 1 else 0, n) for n in lens], RAW["n_head"]) == bits
+        assert plan([(held if n == 1 else 0, n) for n in lens], RAW["n_head"]) & ~ALONE == bits
         counted = r.counters()
         got = r.step(entries).logits
         after = r.counters()

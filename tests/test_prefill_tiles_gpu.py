@@ -2,6 +2,7 @@
 tiles (where warps without rows run ahead of the others), and more requests than one look finds."""
 from __future__ import annotations
 
+import numpy as np
 import pytest
 import torch
 
@@ -61,3 +62,40 @@ def test_single_tokens_in_the_launch(dev, new, past, window, soft_cap, slopes):
     assert ops.device_status() == 0
     # As above; the single tokens' weights stay in 32 bits, their result has one rounding.
     assert (out.float() - want.float()).abs().max().item() < 1.5e-2
+
+
+@pytest.mark.parametrize("form", [{}, {"soft_cap": 3.0}, {"soft_cap": 40.0, "score_bound": 8.0}, {"distance": True}])
+def test_one_block_an_sm_has_the_bits_of_two(dev, form):
+    """The launch that keeps its blocks apart, alone and with the single tokens: the same sums; capped and biased scores against 64 bits."""
+    from liyab_b200 import ops
+    lens, q_lens, H, scale = [400, 300, 17, 129, 700], [400, 130, 1, 2, 1], 3, 0.125
+    q, cache, _, positions, table, refs = _paged_case(dev, torch.bfloat16, H, H, 64, 16, lens, q_lens, seed=77)
+    start = torch.tensor([0] + np.cumsum(q_lens).tolist(), dtype=torch.int32, device=dev)
+    past = torch.tensor([l - n for l, n in zip(lens, q_lens)], dtype=torch.int32, device=dev)
+    kw = dict(form)
+    if kw.pop("distance", False):
+        kw["distance"] = torch.tensor([0.4, 0.2, 0.9, 0.5, 2.0, 0.1], device=dev)
+    outs = {}
+    for singles in (False, True):
+        for alone in (False, True):
+            out = torch.full_like(q, float("nan"))
+            ops.prefill_attention(q, cache, start, past, table, out, len(lens), 448, H, H, 64, 16, scale, 0, tcgen05=True, min_len=2 if singles else 1, singles=singles, alone=alone, **kw)
+            outs[singles, alone] = out
+    assert ops.device_status() == 0
+    assert torch.equal(outs[False, False], outs[False, True]) and torch.equal(outs[True, False], outs[True, True])
+    at = 0
+    for (qs, k, v, first), n in zip(refs, q_lens):
+        back = (torch.arange(n)[:, None] + first - torch.arange(k.shape[0])[None]).double()
+        for h in range(H):
+            s = qs[:, h] @ k[:, h].t() * scale
+            if "soft_cap" in kw:
+                s = kw["soft_cap"] * torch.tanh(s / kw["soft_cap"])
+            if "distance" in kw:
+                d = kw["distance"].double().cpu()
+                s = s - d[h] * torch.log1p(d[H + h] * back.clamp(min=0))
+            ref = s.masked_fill(back < 0, -float("inf")).softmax(-1) @ v[:, h]
+            for out in (outs[False, False], outs[True, False]):
+                got = out[at:at + n, h * 64:(h + 1) * 64].double().cpu()
+                # Probabilities rounded to bfloat16 (2^-9 of values of up to four), and the result.
+                assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -9 * 4).all()
+        at += n
