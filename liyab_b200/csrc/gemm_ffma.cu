@@ -558,7 +558,7 @@ inline StreamShape stream_shape(int K, int most) {
     const int n_chunks = (K + kChunk - 1) / kChunk, G = chunks_per_group(K), n_groups = (n_chunks + G - 1) / G;
     constexpr int kFinishing = kStreamTokens * kStreamFeatures / 32;          // a thread an element at the end
     StreamShape s{(n_groups + 3) / 4 > kFinishing ? (n_groups + 3) / 4 : kFinishing, 0, 0};
-    const size_t fixed = ((size_t)kStreamTokens * n_chunks * kStreamChunkPitch + (size_t)2 * s.warps * 4 * kStreamTokens * kStreamFeatures) * sizeof(float) + 64;
+    const size_t fixed = ((size_t)kStreamTokens * n_chunks * kStreamChunkPitch + (size_t)2 * s.warps * 4 * kStreamTokens * kStreamFeatures) * sizeof(float) + 80;
     const size_t stage = (size_t)kStreamFeatures * stream_row_pitch(K) * sizeof(float), half = 113 * 1024, whole = 227 * 1024;
     if (fixed + stage > whole) return s;
     const int in_half = fixed < half ? (int)((half - fixed) / stage) : 0, in_whole = (int)((whole - fixed) / stage);
@@ -568,6 +568,8 @@ inline StreamShape stream_shape(int K, int most) {
     s.smem = fixed + s.stages * stage;
     return s;
 }
+
+int g_withhold_next = 0;      // the next launch's blocks leave their first stage's barrier one arrival short (tests)
 
 // Whether a product goes that way: a block has at least two stages or no second group of features.  Short reductions (one chunk a group, which the kernel of
 // eight features a block brings in one go as well) stay with that one where they have no more groups than SMs, and where the last round of blocks would be less
@@ -590,7 +592,7 @@ __device__ __forceinline__ uint32_t ffma_smem(const void* p) { return (uint32_t)
 
 __global__ void __launch_bounds__(256)
 gemm_ffma_stream_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ W, int64_t ldw, const float* __restrict__ bias,
-                        const float* residual, int64_t ldr, float* out, int64_t ldo, int M, int N, int K, int act, int stages, int* status) {
+                        const float* residual, int64_t ldr, float* out, int64_t ldo, int M, int N, int K, int act, int stages, int withhold, int* status) {
     constexpr int TOKENS = kStreamTokens;
     extern __shared__ __align__(16) float stream_smem[];
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
@@ -602,9 +604,11 @@ gemm_ffma_stream_kernel(const float* __restrict__ A, int64_t lda, const float* _
     float* red = a_s + (size_t)TOKENS * a_pitch;                         // [2][group][token][8]
     const int red_floats = n_warps * 4 * TOKENS * kStreamFeatures;
     uint64_t* full = reinterpret_cast<uint64_t*>(red + 2 * red_floats);
+    volatile int* gave_up = reinterpret_cast<int*>(full + 8);             // a wait ran out: the later ones end at once
     const int n_feature_groups = (N + kStreamFeatures - 1) / kStreamFeatures, step = gridDim.x;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < stages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ffma_smem(full + i)));
+        *gave_up = 0;
+        for (int i = 0; i < stages; ++i) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(ffma_smem(full + i)), "r"(i == 0 && withhold != 0 ? 2 : 1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -643,14 +647,11 @@ gemm_ffma_stream_kernel(const float* __restrict__ A, int64_t lda, const float* _
         const bool finishes = threadIdx.x < TOKENS * kStreamFeatures && er < M && ef < N;
         const float early_b = finishes && bias != nullptr ? __ldg(bias + ef) : 0.0f, early_r = finishes && residual != nullptr ? __ldcg(residual + (size_t)er * ldr + ef) : 0.0f;
         {
-            // Bounded: a copy that never lands leaves a code in the status word and wrong results instead of a hang.
-            const uint32_t bar = ffma_smem(full + stage), parity = (uint32_t)(it / stages) & 1u;
-            uint32_t ok = 0;
-            const long long t0 = clock64();
-            while (!ok) {
-                asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-                if (!ok && clock64() - t0 > 4000000000ll) atomicCAS(status, 0, (0x9 << 12) | 1);
-                if (!ok && clock64() - t0 > 8000000000ll) break;              // the copy has had its time again: the block may leave
+            // Bounded, once for the block: a copy that never lands leaves a code in the status word and wrong results instead of a hang, and the groups
+            // after it are not waited for.
+            if (!lb_tc::mbar_wait(full + stage, (uint32_t)(it / stages) & 1u, gave_up)) {
+                atomicCAS(status, 0, (0x9 << 12) | 1);
+                *gave_up = 1;
             }
         }
         const float* w_row = w_s + ((size_t)stage * kStreamFeatures + fi) * w_pitch;
@@ -683,7 +684,7 @@ gemm_ffma_stream_kernel(const float* __restrict__ A, int64_t lda, const float* _
 #pragma unroll
         for (int r = 0; r < TOKENS; ++r) here[(group * TOKENS + r) * kStreamFeatures + fi] = grp[r];
         __syncthreads();                                                 // the group sums are there, and the stage has been read
-        if (warp == 0 && fg + stages * step < n_feature_groups) rows(fg + stages * step, stage);
+        if (warp == 0 && fg + stages * step < n_feature_groups && __shfl_sync(0xffffffffu, *gave_up, 0) == 0) rows(fg + stages * step, stage);
         if (finishes) {
             float v = here[threadIdx.x];
             for (int g2 = 1; g2 < n_groups; ++g2) v += here[g2 * TOKENS * kStreamFeatures + threadIdx.x];
@@ -692,6 +693,12 @@ gemm_ffma_stream_kernel(const float* __restrict__ A, int64_t lda, const float* _
             if (residual != nullptr) v += early_r;
             out[(size_t)er * ldo + ef] = v;
         }
+    }
+    // Leave no copy in flight: what was asked for has its time once more.  (Before the limit nothing is: every stage asked for was waited for.)
+    __syncthreads();
+    if (warp == 0 && *gave_up != 0) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 2000000) {}              // a millisecond, hundreds of times what a copy takes
     }
 }
 
@@ -702,7 +709,8 @@ int launch_stream(const void* A, int64_t lda, const void* W, int64_t ldw, const 
     if (rc != LB_OK) return rc;
     LB_CHECK_CUDA(cudaFuncSetAttribute(gemm_ffma_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     LB_CHECK_CUDA(lb_launch_overlapped(gemm_ffma_stream_kernel, dim3(grid), dim3(shape.warps * 32), shape.smem, s, (const float*)A, lda,
-                                       (const float*)W, ldw, bias, residual, ldr, (float*)out, ldo, M, N, K, act, shape.stages, status));
+                                       (const float*)W, ldw, bias, residual, ldr, (float*)out, ldo, M, N, K, act, shape.stages, g_withhold_next, status));
+    g_withhold_next = 0;
     LB_CHECK_LAUNCH();
     return LB_OK;
 }
@@ -799,4 +807,9 @@ extern "C" int lb_gemm_ffma(int in_dtype, int out_dtype, const void* A, int64_t 
     if (in_dtype == LB_BF16 && out_dtype == LB_F32)
         return launch<__nv_bfloat16, float>(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, s);
     return lb_fail(LB_ERR_INVALID_ARGUMENT, "gemm: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
+}
+
+extern "C" int lb_gemm_ffma_withhold_next(int on) {
+    g_withhold_next = on != 0 ? 1 : 0;
+    return LB_OK;
 }

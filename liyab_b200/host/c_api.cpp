@@ -861,7 +861,8 @@ int32_t lb_debug_withhold_next(int32_t which, int32_t on) {
         if (which == 0) kernels::check(lb_gemm_tcgen05_withhold_next(on), "withhold_next");
         else if (which == 1) kernels::check(lb_decode_stack_withhold_next(on), "withhold_next");
         else if (which == 2) kernels::check(lb_gemm_pair_withhold_next(on), "withhold_next");
-        else throw invalid_argument("wait {} does not exist (0: the tcgen05 product's accumulator barrier, 1: the fused step's grid barrier, 2: the two-SM product's accumulator barriers)", which);
+        else if (which == 3) kernels::check(lb_gemm_ffma_withhold_next(on), "withhold_next");
+        else throw invalid_argument("wait {} does not exist (0: the tcgen05 product's accumulator barrier, 1: the fused step's grid barrier, 2: the two-SM product's accumulator barriers, 3: the float32 product's first rows of weights)", which);
     });
 }
 

@@ -31,6 +31,7 @@ def no_order_left_behind():
     withhold_next(0, False)
     withhold_next(1, False)
     withhold_next(2, False)
+    withhold_next(3, False)
     device_status()
 
 
@@ -84,6 +85,32 @@ def test_two_sm_product_whose_accumulator_is_never_reported_stops_both_blocks(M,
         ops.gemm_pair(a, w, None, out, M, residual=res)
         torch.cuda.synchronize()
         assert (out.double() - want).abs().max().item() <= 1e-5 * max(1.0, want.abs().max().item())
+    assert device_status() == (0, 0)
+
+
+def test_float32_product_whose_rows_never_land_waits_for_them_once():
+    """50 groups of features a block, each with a stage to wait for: the limit runs out at the first, not at every one of them."""
+    import time
+    from liyab_b200 import ops
+    from liyab_b200.engine import device_status, withhold_next
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(7)
+    M, N, K = 8, 50 * 296 * 8, 132
+    a, w = torch.randn((M, K), generator=g).to(dev), torch.randn((N, K), generator=g).to(dev)
+    want = a.double() @ w.double().t()
+    out = torch.zeros((M, N), device=dev)
+    assert device_status() == (0, 0)
+    withhold_next(3)
+    t0 = time.monotonic()
+    ops.gemm_ffma(a, w, None, out, M)
+    torch.cuda.synchronize()
+    took = time.monotonic() - t0
+    assert device_status() == ((0x9 << 12) | 1, 0) and 1.0 < took < 8.0, took
+    for _ in range(2):
+        out.fill_(float("nan"))
+        ops.gemm_ffma(a, w, None, out, M)
+        torch.cuda.synchronize()
+        assert (out.double() - want).abs().max().item() <= 1e-4
     assert device_status() == (0, 0)
 
 
