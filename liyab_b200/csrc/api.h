@@ -342,12 +342,14 @@ int lb_gemm_tcgen05_status_set(int value);
 int lb_decode_stack_status_set(int value);
 /* Makes the NEXT launch meet a wait that nothing ends, once: the one-tile tcgen05 product leaves its
  * accumulator-ready barrier unsignalled; the fused step's block 0 is not counted at its first grid barrier; the pairs of the two-SM product leave their
- * first accumulator's barriers unsignalled; the blocks of the float32 product of up to 8 tokens leave their first stage's barrier one arrival short.
+ * first accumulator's barriers unsignalled; the blocks of the float32 product of up to 8 tokens leave their first stage's barrier one arrival short; those of the
+ * product for some dozens of tokens leave their accumulators' barriers unsignalled.
  * The waits run to their limit (about two seconds), set the status word and the kernel returns. */
 int lb_gemm_tcgen05_withhold_next(int on);
 int lb_decode_stack_withhold_next(int on);
 int lb_gemm_pair_withhold_next(int on);
 int lb_gemm_ffma_withhold_next(int on);
+int lb_gemm_narrow_withhold_next(int on);
 
 /* lb_gemm_rows_normed with the kind of norm as an argument: rms != 0: y = x / sqrt(mean(x^2) + eps) * (gain + gain_offset) + offset. */
 int lb_gemm_rows_normed_kind(int out_dtype, const float* x, int64_t ldx, const float* gain, const float* offset, float eps, int rms, float gain_offset,

@@ -396,7 +396,8 @@ def device_status() -> Tuple[int, int]:
 
 def withhold_next(which: int, on: bool = True) -> None:
     """The next launch of kernel family `which` (0: the one-tile tcgen05 product, 1: the one-kernel decode step, 2: the
-    product whose tiles two SMs make together, 3: the float32 product of up to 8 tokens) meets a wait that nothing ends, once: its bounded wait runs to its limit (about two seconds), sets the status word and
+    product whose tiles two SMs make together, 3: the float32 product of up to 8 tokens, 4: the product
+    for some dozens of tokens) meets a wait that nothing ends, once: its bounded wait runs to its limit (about two seconds), sets the status word and
     the kernel returns.  `on=False` takes back an order that no launch has used.  For tests of that path; the device
     stays usable."""
     _capi.check(_capi.lib().lb_debug_withhold_next(which, 1 if on else 0))

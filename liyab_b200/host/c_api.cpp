@@ -862,7 +862,8 @@ int32_t lb_debug_withhold_next(int32_t which, int32_t on) {
         else if (which == 1) kernels::check(lb_decode_stack_withhold_next(on), "withhold_next");
         else if (which == 2) kernels::check(lb_gemm_pair_withhold_next(on), "withhold_next");
         else if (which == 3) kernels::check(lb_gemm_ffma_withhold_next(on), "withhold_next");
-        else throw invalid_argument("wait {} does not exist (0: the tcgen05 product's accumulator barrier, 1: the fused step's grid barrier, 2: the two-SM product's accumulator barriers, 3: the float32 product's first rows of weights)", which);
+        else if (which == 4) kernels::check(lb_gemm_narrow_withhold_next(on), "withhold_next");
+        else throw invalid_argument("wait {} does not exist (0: the tcgen05 product's accumulator barrier, 1: the fused step's grid barrier, 2: the two-SM product's accumulator barriers, 3: the float32 product's first rows of weights, 4: the accumulator barriers of the product for some dozens of tokens)", which);
     });
 }
 

@@ -305,7 +305,8 @@ LB_API int32_t lb_device_status(int32_t* words2);
  * switched off, the engine goes on). */
 LB_API int32_t lb_debug_set_device_status(int32_t which, int32_t value);
 /* With `on`, the next launch of kernel family `which` (0: the one-tile tcgen05 product, 1: the one-kernel decode
- * step, 2: the product whose tiles two SMs make together, 3: the float32 product of up to 8 tokens) meets a wait that nothing ends, once.  Its bounded wait runs to its limit (about two seconds), sets the
+ * step, 2: the product whose tiles two SMs make together, 3: the float32 product of up to 8 tokens, 4: the product for
+ * some dozens of tokens) meets a wait that nothing ends, once.  Its bounded wait runs to its limit (about two seconds), sets the
  * status word and the kernel returns; the context stays usable.  Without `on`, takes an order back that no launch
  * has used yet.  For tests of that path. */
 LB_API int32_t lb_debug_withhold_next(int32_t which, int32_t on);

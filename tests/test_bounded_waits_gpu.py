@@ -32,6 +32,7 @@ def no_order_left_behind():
     withhold_next(1, False)
     withhold_next(2, False)
     withhold_next(3, False)
+    withhold_next(4, False)
     device_status()
 
 
@@ -83,6 +84,31 @@ def test_two_sm_product_whose_accumulator_is_never_reported_stops_both_blocks(M,
     for _ in range(3):
         out.fill_(float("nan"))
         ops.gemm_pair(a, w, None, out, M, residual=res)
+        torch.cuda.synchronize()
+        assert (out.double() - want).abs().max().item() <= 1e-5 * max(1.0, want.abs().max().item())
+    assert device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("M,N,K,features,splits", [(40, 64, 320, 32, 1), (100, 512, 2048, 64, 4), (40, 2048, 6400, 256, 8)])
+def test_product_of_some_dozens_of_tokens_gives_up_in_every_block(M, N, K, features, splits):
+    """One block a tile; clusters whose blocks wait for one another twice, with the sums beside the stages and over them."""
+    from liyab_b200 import ops
+    from liyab_b200.engine import device_status, withhold_next
+    dev = torch.device("cuda:0")
+    g = torch.Generator().manual_seed(8)
+    a = torch.randn((M, K), generator=g).to(torch.bfloat16).to(dev)
+    w = (torch.randn((N, K), generator=g) * 0.2).to(torch.bfloat16).to(dev)
+    want = a.double() @ w.double().t()
+    out = torch.zeros((M, N), dtype=torch.float32, device=dev)
+    assert device_status() == (0, 0)
+    withhold_next(4)
+    ops.gemm_narrow(a, w, None, out, M, features=features, splits=splits)
+    torch.cuda.synchronize()
+    word, barrier = device_status()
+    assert word >> 12 == 0xF and (word >> 8 & 0xF) in (1, 3) and barrier == 0, f"a role of the product reports itself: {word:#x}"
+    for _ in range(3):
+        out.fill_(float("nan"))
+        ops.gemm_narrow(a, w, None, out, M, features=features, splits=splits)
         torch.cuda.synchronize()
         assert (out.double() - want).abs().max().item() <= 1e-5 * max(1.0, want.abs().max().item())
     assert device_status() == (0, 0)

@@ -65,3 +65,41 @@ def test_refusals(dev):
                 lambda: ops.gemm_narrow(a, w[:16].clone(), None, torch.zeros((40, 16), device=dev), 40, features=16, splits=2)):
         with pytest.raises(LiyabError):
             bad()
+
+
+@pytest.mark.parametrize("activation", ["gelu_tanh", "gelu_erf", "xielu", "relu2"])
+@pytest.mark.parametrize("features,splits", [(64, 1), (64, 4)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_activations(dev, activation, features, splits, dtype):
+    """Every activation on sums around zero, beside the kernel of the float32 units on the same operands."""
+    from liyab_b200 import ops
+    M, N, K = 70, 328, 1536
+    a, w = _rand((M, K), 100, dev, torch.bfloat16), _rand((N, K), 101, dev, torch.bfloat16, 0.05)
+    bias = _rand((N + 2,), 102, dev)                                          # xIELU keeps its two numbers behind the bias
+    bias[N:] = torch.tensor([0.8, 0.4], device=dev)
+    out, want = (torch.empty((M, N), dtype=t, device=dev) for t in (dtype, torch.float32))
+    ops.gemm_narrow(a, w, bias[:N], out, M, activation, features=features, splits=splits)
+    ops.gemm_ffma(a, w, bias[:N], want, M, activation)
+    assert ops.device_status() == 0
+    # The sums' roundings (see test_products) through slopes of up to 2.4 |x| + 1, and the result's own; GELU of bfloat16 results leaves 2^-12 of its argument.
+    sums = (K / 16 + 16) * 2.0 ** -23 * (a.double().abs() @ w.double().abs().t() + bias[:N].double().abs())
+    x = a.double() @ w.double().t() + bias[:N].double()
+    slope = 3 * x.abs().max() + 2
+    bound = slope * sums + (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20) * want.double().abs() + (2.0 ** -12 * x.abs() if dtype == torch.bfloat16 else 0)
+    assert ((out.double() - want.double()).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("features,splits", [(48, 1), (64, 4), (256, 8)])
+def test_special_values_stay_in_their_rows_and_columns(dev, features, splits):
+    """Infinities and NaN among activations and weights: the places they reach and no others, like the products of 64-bit numbers."""
+    from liyab_b200 import ops
+    M, N, K = 70, 512, 2048
+    a, w = _rand((M, K), 103, dev, torch.bfloat16), _rand((N, K), 104, dev, torch.bfloat16, 0.1)
+    a[3, 5], a[64, K - 1], a[9, 700] = float("inf"), float("nan"), -float("inf")
+    w[17, 5], w[511, 40], w[200, 700] = 0.0, float("-inf"), float("nan")
+    out = torch.empty((M, N), device=dev)
+    ops.gemm_narrow(a, w, None, out, M, features=features, splits=splits)
+    ref = a.double() @ w.double().t()
+    assert torch.equal(out.isnan(), ref.isnan()) and torch.equal(out == float("inf"), ref == float("inf")) and torch.equal(out == -float("inf"), ref == -float("inf"))
+    finite = ref.isfinite()
+    assert ((out.double() - ref)[finite].abs() <= 1e-3).all() and ops.device_status() == 0
