@@ -48,6 +48,8 @@ int lb_gemm_ffma(int in_dtype, int out_dtype, const void* A, int64_t lda, const 
                  void* stream);
 /* Which of its kernels takes a float32 product of 9 to 16 rows: features a block (16 or 8) of the one whose weights come by whole rows, 0 the other one. */
 int lb_gemm_ffma_row_features(int M, int N, int K);
+/* The stages of a block, and the blocks, of the kernel whose weights come by whole rows and bulk copies (up to 8 tokens, float32); 0 where another one takes the product. */
+int lb_gemm_ffma_stream_stages(int M, int N, int K, int n_sm, int* blocks);
 
 /* The same product for bfloat16 operands on the tcgen05 tensor cores (TMA-fed,
  * accumulator in tensor memory).  Needs K, lda and ldw to be multiples of 8 and

@@ -574,11 +574,7 @@ int g_withhold_next = 0;      // the next launch's blocks leave their first stag
 // Whether a product goes that way: a block has at least two stages or no second group of features.  Short reductions (one chunk a group, which the kernel of
 // eight features a block brings in one go as well) stay with that one where they have no more groups than SMs, and where the last round of blocks would be less
 // than two fifths full.
-inline bool stream_takes(int N, int K, StreamShape* shape, int* grid) {
-    static const int n_sm = [] {
-        int dev = 0, n = 0;
-        return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 148;
-    }();
+inline bool stream_takes(int N, int K, int n_sm, StreamShape* shape, int* grid) {
     const int groups = (N + kStreamFeatures - 1) / kStreamFeatures;
     *shape = stream_shape(K, (groups + n_sm - 1) / n_sm);
     if (shape->stages < 1 || (shape->stages < 2 && groups > n_sm)) return false;
@@ -731,7 +727,11 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
         if constexpr (sizeof(TI) == 4 && sizeof(TO) == 4) {
             StreamShape shape;
             int grid = 0;
-            if (M <= kStreamTokens && stream_takes(N, K, &shape, &grid)) return launch_stream(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, shape, grid, s);
+            static const int n_sm = [] {
+                int dev = 0, n = 0;
+                return cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess ? n : 148;
+            }();
+            if (M <= kStreamTokens && stream_takes(N, K, n_sm, &shape, &grid)) return launch_stream(A, lda, W, ldw, bias, residual, ldr, out, ldo, M, N, K, act, shape, grid, s);
         }
         if constexpr (sizeof(TI) == 4) {
             if (M > 8) {
@@ -782,7 +782,8 @@ int launch(const void* A, int64_t lda, const void* W, int64_t ldw, const float* 
 // 256 and two rounds of blocks), enough blocks to fill the GPU, and with four warps, whose blocks of sixteen features have an SM each, rounds over the SMs
 // that are at least two thirds full (3072 x 1024: 11.5 / 12.0).  Fewer features than a wave of such blocks go by rows, eight a block, from 768 on, with 11 to 16
 // chunks, or 33 to 48 below 1536 features: alone such a product is level (768 x 3072 13.4 / 13.0), within a step it is not (GPT-2 small, 12
-// requests: 878 / 803 us with its down products by rows; medium, 9 requests: 1677 / 1647 with its output products).  Up to eight tokens the other kernel is the faster one throughout (a step of 8 requests 615 against 632 us).
+// requests: 878 / 803 us with its down products by rows; medium, 9 requests: 1677 / 1647 with its output products).  Up to eight tokens it was behind
+// throughout (a step of 8 requests 615 against 632 us); most of those products have bulk copies now (stream_takes).
 extern "C" int lb_gemm_ffma_row_features(int M, int N, int K) {
     const int n_chunks = (K + kChunk - 1) / kChunk, warps = (n_chunks + 3) / 4;
     const int round = 16 * 148, rounds = (N + round - 1) / round;
@@ -790,6 +791,16 @@ extern "C" int lb_gemm_ffma_row_features(int M, int N, int K) {
     if (N < round) return (N >= 768 && n_chunks > 10 && n_chunks <= 16) || (N >= 768 && N < 1536 && n_chunks > 32 && n_chunks <= 48) ? 8 : 0;
     if (warps == 1) return N >= 2 * round ? 16 : 0;
     return warps < 4 || (warps == 4 && 3ll * N >= 2ll * rounds * round) ? 16 : 0;
+}
+
+// The stages of a block in the kernel whose weights come by whole rows and bulk copies, for float32 products of whole 16-byte pieces on n_sm SMs; 0 where another kernel
+// takes the product.  *blocks: the launch's.
+extern "C" int lb_gemm_ffma_stream_stages(int M, int N, int K, int n_sm, int* blocks) {
+    StreamShape shape{};
+    int grid = 0;
+    if (M < 1 || M > kStreamTokens || N < 1 || K < 4 || K % 4 != 0 || n_sm < 1 || !stream_takes(N, K, n_sm, &shape, &grid)) return 0;
+    if (blocks != nullptr) *blocks = grid;
+    return shape.stages;
 }
 
 extern "C" int lb_gemm_ffma(int in_dtype, int out_dtype, const void* A, int64_t lda, const void* W, int64_t ldw,

@@ -74,6 +74,7 @@ _SIGNATURES = {
     "lb_gemm_rows_kind": [_i, _i, _i, _i, _i],
     "lb_gemm_rows_normed_pays": [_i, _i],
     "lb_gemm_ffma_row_features": [_i, _i, _i],
+    "lb_gemm_ffma_stream_stages": [_i, _i, _i, _i, _p],
     "lb_paged_attention_f32_runs": [_p, _l, _p, _p, _p, _p, _i, _p, _l, _i, _i, _i, _i, _f, _i, _p, _p],
     "lb_qkv_rotary_store_scaled": [_i, _p, _l, _i, _i, _i, _p, _p, _p, _l, _p, _p, _i, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p, _i, _p, _p, _l, _p, _i, _f, _p],
     "lb_row_norm_gate": [_i, _p, _l, _p, _l, _p, _p, _l, _i, _i, _i, _f, _p],

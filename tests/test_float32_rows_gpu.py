@@ -12,10 +12,12 @@ EPS = 2.0 ** -24          # chains of 64 products, then up to 32 + K / 2048 sums
 
 
 @pytest.mark.parametrize("M", [1, 5, 8])
-@pytest.mark.parametrize("N,K", [(2304, 768), (2301, 772), (11000, 132), (9999, 4), (768, 3072), (1184, 3072), (9, 2052), (3300, 1600), (1187, 4160), (300, 1092), (30, 8000)])
-def test_products_of_up_to_eight_rows(dev, M, N, K):
+@pytest.mark.parametrize("N,K,stages", [(2304, 768, 2), (2301, 772, 2), (11000, 132, 8), (9999, 4, 8), (768, 3072, 1), (1184, 3072, 1), (9, 2052, 1), (3300, 1600, 3), (1187, 4160, 0),
+                                        (300, 1092, 1), (30, 8000, 0)])
+def test_products_of_up_to_eight_rows(dev, M, N, K, stages):
     """One group of features a block or many, a ring that wraps, chunks and rows with remainders, one to three chunks a group, a row that does not fit."""
     from liyab_b200 import ops
+    assert torch.cuda.get_device_properties(dev).multi_processor_count != 148 or ops.lib().lb_gemm_ffma_stream_stages(M, N, K, 148, None) == stages      # which kernel this is
     a, w, bias, res = _rand((24, K + 4), 65, dev)[:, :K], _rand((N, K), 66, dev), _rand((N,), 67, dev), _rand((24, N), 68, dev)
     out, whole = res[:M].clone(), res.clone()
     ops.gemm_ffma(a[:M], w, bias, out, M, "none", residual=out)

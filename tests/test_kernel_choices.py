@@ -180,3 +180,29 @@ def test_single_tokens_beside_portions_are_not_left_out(head_dim, tcgen05):
     with pytest.raises(LiyabError, match="single tokens"):
         ops.prefill_attention(rows, torch.zeros((1, 2, 2, 16, head_dim), dtype=torch.bfloat16), ints, ints, ints.view(1, 4), rows, 3, 64, 2, 2, head_dim, 16, 0.125,
                               tcgen05=tcgen05, min_len=2, singles=True)
+
+
+def test_float32_products_of_up_to_eight_rows_by_bulk_copies():
+    """(stages, blocks) on 148 SMs: rows that fit a ring, or one group of features a block; short reductions where their last round of blocks is full enough."""
+    blocks = C.c_int(0)
+
+    def f(m, n, k, n_sm=148):
+        stages = ops.lib().lb_gemm_ffma_stream_stages(m, n, k, n_sm, C.addressof(blocks))
+        return (stages, blocks.value) if stages else 0
+
+    for m in (1, 8):
+        assert [f(m, n, 768) for n in (768, 1184, 1192, 2304, 2368, 3072, 3312, 3320, 9472, 50257)] == [0, 0, (2, 149), (2, 288), (2, 296), 0, 0, (3, 296), (3, 296), (3, 296)]
+        assert [f(m, n, 1600) for n in (1600, 4800, 6400)] == [(2, 148), (3, 148), (3, 148)]
+        assert [f(m, n, 3072) for n in (768, 1184, 1192, 2304)] == [(1, 96), (1, 148), 0, 0]           # one stage: one group a block
+        assert f(m, 1600, 6400) == 0 and f(m, 2304, 770) == 0                                           # a row that does not fit; no whole pieces
+    assert f(9, 2304, 768) == 0 and f(8, 2304, 768, 74) == (3, 148)
+
+
+@pytest.mark.parametrize("N,K,bf16,f32", [
+    (768, 768, range(33, 257), range(33, 257)), (2304, 768, range(33, 257), ()), (1024, 4096, range(17, 257), range(17, 513)), (6400, 1600, range(17, 257), range(17, 33)),
+    (1280, 1280, range(17, 257), range(17, 129)), (10248, 1600, (), ()), (768, 248, (), ()), (764, 768, (), ()), (248, 768, (), ())])
+def test_products_of_some_dozens_of_tokens(N, K, bf16, f32):
+    """From where to where the kernel of one launch is the faster one: few tokens with short reductions, wide float32 results and more than 256 tokens are others'."""
+    pays = ops.lib().lb_gemm_narrow_pays
+    for m in (1, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 2000):
+        assert bool(pays(ops.BF16, m, N, K)) == (m in bf16) and bool(pays(ops.F32, m, N, K)) == (m in f32), m
