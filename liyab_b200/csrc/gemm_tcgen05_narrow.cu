@@ -347,10 +347,13 @@ extern "C" int lb_gemm_narrow_plan(int M, int N, int K, int n_sm, int* splits_ou
 // 14.2 / 8.6, 128 x 768 x 3072 10.3 / 6.0, 128 x 1600 x 6400 16.5 / 10.0; 256 x 768 x 768 5.4 / 4.7, 256 x 6400 x 1600 10.5 / 10.1, but 256 x 1280 x 1280 with float32
 // results 7.7 / 8.1 (a thread stores 32 bytes of a row at a time, which many float32 results feel: 128 x 2560 x 768 5.7 / 7.0); beyond 256 only long reductions
 // gain: 465 x 1024 x 4096 14.0 / 11.1, 330 x 1600 x 6400 20.1 / 16.7, but 465 x 1600 x 6400 20.5 / 20.1 and slower within a step, level or slower at 640.  Up to 32 tokens 20 x 3072 x 768 4.1 / 4.5 but 20 x 1600 x 6400 9.2 / 7.7.
+// Up to 48 tokens with reductions of up to 512 and up to 2048 features the kernel for single tokens is through while this one has hardly begun: 40 x 256 x 256 2.5 / 2.8,
+// 40 x 1000 x 264 3.6 / 3.9, 33 x 2048 x 512 4.1 / 4.2, but 56 x 1000 x 264 4.2 / 3.8, 48 x 768 x 640 4.4 / 3.6.
 // Reductions under 256 and more than 10240 features were not measured.
 extern "C" int lb_gemm_narrow_pays(int out_dtype, int M, int N, int K) {
     if (M <= 16 || M > 512 || K < 256 || N < 256 || N > 10240 || N % 8 != 0 || K % 8 != 0) return 0;
     if (M <= 32) return K > 1024;
+    if (M <= 48 && K <= 512 && N <= 2048) return 0;
     const bool wide = out_dtype == LB_F32 && N > 2048;
     if (M <= 128) return !wide;
     const bool deep = out_dtype == LB_F32 && K >= 3 * N && K >= 2048 && (M <= 256 || (long)M * N <= 600000);

@@ -200,9 +200,10 @@ def test_float32_products_of_up_to_eight_rows_by_bulk_copies():
 
 @pytest.mark.parametrize("N,K,bf16,f32", [
     (768, 768, range(33, 257), range(33, 257)), (2304, 768, range(33, 257), ()), (1024, 4096, range(17, 257), range(17, 513)), (6400, 1600, range(17, 257), range(17, 33)),
-    (1280, 1280, range(17, 257), range(17, 129)), (10248, 1600, (), ()), (768, 248, (), ()), (764, 768, (), ()), (248, 768, (), ())])
+    (1280, 1280, range(17, 257), range(17, 129)), (512, 256, range(49, 257), range(49, 129)), (2048, 512, range(49, 257), range(49, 129)),
+    (2056, 512, range(33, 257), ()), (10248, 1600, (), ()), (768, 248, (), ()), (764, 768, (), ()), (248, 768, (), ())])
 def test_products_of_some_dozens_of_tokens(N, K, bf16, f32):
     """From where to where the kernel of one launch is the faster one: few tokens with short reductions, wide float32 results and more than 256 tokens are others'."""
     pays = ops.lib().lb_gemm_narrow_pays
-    for m in (1, 16, 17, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 2000):
+    for m in (1, 16, 17, 32, 33, 48, 49, 64, 65, 128, 129, 256, 257, 512, 513, 2000):
         assert bool(pays(ops.BF16, m, N, K)) == (m in bf16) and bool(pays(ops.F32, m, N, K)) == (m in f32), m
