@@ -66,6 +66,7 @@ _SIGNATURES = {
     "lb_gemm_pair": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
     "lb_gemm_narrow": [_i, _p, _l, _p, _l, _p, _p, _l, _p, _l, _i, _i, _i, _i, _i, _i, _p, _p, _i, _i, _i, _i, _p],
     "lb_gemm_narrow_pays": [_i, _i, _i, _i],
+    "lb_gemm_narrow_supports": [_i, _p, _l, _p, _l, _p, _l, _p, _l, _i, _i, _i],
     "lb_gemm_narrow_block": [_i, _i, _i, _i, _p],
     "lb_gemm_narrow_plan": [_i, _i, _i, _i, _p, _p],
     "lb_gemm_pair_tile": [_i, _i, _i, _i, _p],
@@ -338,6 +339,14 @@ def gemm_narrow(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], 
     return out
 
 
+def gemm_narrow_takes(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, m: int, residual: Optional[torch.Tensor] = None) -> bool:
+    """Whether the product goes that way in a step: the kernel is the faster one for its sizes and takes its operands."""
+    code, (n, k) = _code(out.dtype, "out"), w.shape
+    return bool(lib().lb_gemm_narrow_pays(code, m, n, k)) and bool(lib().lb_gemm_narrow_supports(
+        code, _dev(a, "a"), a.stride(0), _dev(w, "w"), w.stride(0), _opt(residual, "residual", torch.float32), residual.stride(0) if residual is not None else 0,
+        _dev(out, "out"), out.stride(0), m, n, k))
+
+
 def gemm_persistent_tile(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, m: int,
                          residual: Optional[torch.Tensor] = None) -> int:
     """The feature tile the persistent tensor-core product would use for these operands, 0 where it does not take them."""
@@ -386,15 +395,16 @@ def device_status() -> int:
 
 def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor, m: int,
            activation: str = "none", residual: Optional[torch.Tensor] = None, workspace=None) -> torch.Tensor:
-    """out[:m] = act(a[:m] @ w.T + bias) + residual: the kernel is chosen by type and size.  With a workspace
+    """out[:m] = act(a[:m] @ w.T + bias) + residual: the kernel is chosen by type and size, as in the engine's steps.  With a workspace
     (scratch buffers) a product of few tokens splits K over blocks."""
     if tcgen05_accepts(a, w):
+        if gemm_narrow_takes(a, w, out, m, residual):
+            return gemm_narrow(a, w, bias, out, m, activation, residual)
         if m > 64 and gemm_persistent_tile(a, w, out, m, residual) > 0:
             return gemm_persistent(a, w, bias, out, m, activation, residual)
-        # Up to 64 tokens: one launch on mma.sync where every block can afford to fetch all activations (measured on
-        # B200, 64 tokens: 6-7 us against 8-9 us for K = 768; for K = 3072 the 393 KB of activations per block cost
-        # more than the split of K saves: 13 us against 8 us; 8 tokens with K = 1600 or 3072 lose to the split too).
-        if m <= 64 and w.shape[1] <= 1024 and gemm_rows_supports(a, w, m):
+        # Few tokens, or shapes that the kernels above decline: one launch on mma.sync where every block can afford to fetch all activations, up to 16 tokens
+        # also with longer reductions.
+        if m <= 64 and (w.shape[1] <= 1024 or m <= 16) and gemm_rows_supports(a, w, m):
             return gemm_rows(a, w, bias, out, m, activation, residual)
         splits = gemm_splits(m, w.shape[0], w.shape[1]) if workspace is not None else 1
         if splits > 1:

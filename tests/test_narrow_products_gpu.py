@@ -103,3 +103,17 @@ def test_special_values_stay_in_their_rows_and_columns(dev, features, splits):
     assert torch.equal(out.isnan(), ref.isnan()) and torch.equal(out == float("inf"), ref == float("inf")) and torch.equal(out == -float("inf"), ref == -float("inf"))
     finite = ref.isfinite()
     assert ((out.double() - ref)[finite].abs() <= 1e-3).all() and ops.device_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,narrow", [(40, 768, 768, True), (20, 1600, 6400, True), (20, 768, 768, False), (40, 512, 256, False), (300, 768, 768, False)])
+def test_linear_goes_where_a_step_goes(dev, M, N, K, narrow):
+    from liyab_b200 import ops
+    a, w, bias = _rand((M, K), 105, dev, torch.bfloat16), _rand((N, K), 106, dev, torch.bfloat16, 0.1), _rand((N,), 107, dev)
+    out, same = (torch.empty((M, N), dtype=torch.bfloat16, device=dev) for _ in range(2))
+    assert ops.gemm_narrow_takes(a, w, out, M) == narrow
+    ops.linear(a, w, bias, out, M, "gelu_tanh")
+    if narrow:
+        ops.gemm_narrow(a, w, bias, same, M, "gelu_tanh")
+        assert torch.equal(out, same)
+    ref = torch.nn.functional.gelu(a.double() @ w.double().t() + bias.double(), approximate="tanh")
+    assert ((out.double() - ref).abs() <= 2.0 ** -7 * ref.abs() + 2e-3).all()
