@@ -87,7 +87,7 @@ int lb_gemm_rows_normed(int out_dtype, const float* x, int64_t ldx, const float*
  * one that holds them in registers, 0 none. */
 int lb_gemm_rows_kind(int M, int N, int K, int n_sm, int normed);
 /* The same product for 1 to 64 tokens in one launch on mma.sync (weights streamed once, no split of K over blocks,
- * no second kernel): lb_gemm_rows_supports tells whether it takes the product.  With kv_cache given (bfloat16 pages
+ * no second kernel): lb_gemm_rows_supports tells whether it takes the product, lb_gemm_narrow_pays where that kernel is faster.  With kv_cache given (bfloat16 pages
  * of one layer), features from q_dim on are the keys and values of a fused projection and are also written to the
  * tokens' cache slots (as lb_kv_append would). */
 int lb_gemm_rows_supports(const void* A, int64_t lda, const void* W, int64_t ldw, int M, int N, int K);

@@ -85,7 +85,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
           "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
         : "memory");
 }
-// 2^x for x <= 8 or so: the hardware approximation alone (results below the normal range become zero).
+// 2^x (the exponentials' arguments are at most 0 up to rounding): the hardware approximation alone (results below the normal range become zero).
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

@@ -55,9 +55,8 @@ void gemm_ffma(cudaStream_t s, const Rows& a, const Tensor& w, const float* bias
                const Rows* residual);
 void gemm_tcgen05(cudaStream_t s, const Rows& a, const Tensor& w, const float* bias, const Rows& out, int m, int act,
                   const Rows* residual, float* partial, int n_splits);
-// Products of up to 64 tokens take the one-launch kernel on mma.sync while every block can afford to fetch all
-// activations: a reduction length of up to 1024 (measured at 17 to 64 tokens: with K = 1600 or 3072 the tcgen05 kernel with K split
-// over blocks and a second half wins).
+// Products of up to 64 tokens that gemm_narrow does not take (lb_gemm_narrow_pays: most of 33 tokens and more, long reductions from 17 on) go to the one-launch
+// kernel on mma.sync while every block can afford to fetch all activations: a reduction length of up to 1024.
 inline constexpr int kRowsMaxK = 1024;
 // Up to 16 tokens a longer reduction (up to 8192) is worth it too while a block has at most eight groups of eight features: in one pass where
 // its registers hold the weights (up to 4096), else through a ring in shared memory (GPT-2 XL's projections: 1.05 to 1.7 times as fast as the split
