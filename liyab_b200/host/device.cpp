@@ -47,10 +47,15 @@ void cuda_check(cudaError_t err, const char* what) {
     throw Error(code, std::format("{} failed: {}", what, cudaGetErrorString(err)));
 }
 
+void finish_default_stream() { LIYAB_CUDA(cudaStreamSynchronize(cudaStreamLegacy)); }
+
 DeviceBuffer::DeviceBuffer(size_t bytes, bool zero) : bytes_(bytes) {
     if (bytes == 0) return;
     LIYAB_CUDA(cudaMalloc(&ptr_, bytes));
-    if (zero) LIYAB_CUDA(cudaMemset(ptr_, 0, bytes));
+    if (zero) {
+        LIYAB_CUDA(cudaMemset(ptr_, 0, bytes));
+        finish_default_stream();
+    }
 }
 DeviceBuffer::~DeviceBuffer() {
     if (ptr_ != nullptr) cudaFree(ptr_);

@@ -27,6 +27,10 @@ DType compute_dtype_from_name(const std::string& name);      // bfloat16/bf16, f
 void cuda_check(cudaError_t err, const char* what);
 #define LIYAB_CUDA(expr) ::liyab::cuda_check((expr), #expr)
 
+// cudaMemset returns before it has run, and so may cudaMemcpy from ordinary memory (the last piece is then still on its way to the device): both are work of the default
+// stream, for which the engine's own streams do not wait.  What they fill is there, and stays as a later kernel or copy leaves it, only after this.
+void finish_default_stream();
+
 class DeviceBuffer {
 public:
     DeviceBuffer() = default;

@@ -87,6 +87,7 @@ std::unique_ptr<FusedDecodeStack> FusedDecodeStack::try_build(const DecoderModel
     const size_t T = kMaxTokens;
     s->layers_ = DeviceBuffer(records.size() * sizeof(LayerRecord));
     LIYAB_CUDA(cudaMemcpy(s->layers_.data(), records.data(), records.size() * sizeof(LayerRecord), cudaMemcpyHostToDevice));
+    finish_default_stream();
     s->x_ = DeviceBuffer(T * static_cast<size_t>(spec.hidden()) * 4);
     s->q_ = DeviceBuffer(T * static_cast<size_t>(s->max_qd_) * 2);
     s->att_ = DeviceBuffer(T * static_cast<size_t>(s->max_qd_) * 2);

@@ -310,6 +310,7 @@ WeightStore::WeightStore(const std::map<std::string, HostTensor>& host) {
         params_.add(name, Tensor{dst, t.dtype, t.shape});
         at += (t.bytes.size() + 255) / 256 * 256;
     }
+    finish_default_stream();
 }
 
 namespace {
