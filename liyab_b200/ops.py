@@ -536,6 +536,13 @@ def prefill_attention_tc_supports(n_head: int, n_kv_head: int, head_dim: int, pa
     return bool(lib().lb_prefill_attention_tc_supports(n_head, n_kv_head, head_dim, page_size))
 
 
+def prefill_tcgen05_pays(n_seq: int, n_head: int, max_q_len: int, n_sm: int) -> bool:
+    """Whether portions of up to `max_q_len` tokens are better left to the tcgen05 kernel, by what is known without their lengths (the engine, which has them, estimates
+    both kernels: lb_attention_plan).  The mma.sync kernel is the faster one for many portions shorter than a tile (40 of 64 with 25 heads 14.8 us against 21.2; 8 of 1,024
+    with 12 heads 99 against 40): over 1,191 random steps of portions this is 2.5 % behind the better kernel on average."""
+    return max_q_len > 64 or n_seq * n_head * -(-max_q_len // 128) <= 2 * n_sm
+
+
 def prefill_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tensor, n_past: torch.Tensor,
                       block_table: torch.Tensor, out: torch.Tensor, n_seq: int, max_q_len: int, n_head: int,
                       n_kv_head: int, head_dim: int, page_size: int, scale: float, window: int = 0,
@@ -550,12 +557,9 @@ def prefill_attention(q: torch.Tensor, cache: torch.Tensor, q_start: torch.Tenso
     if q.stride(1) != 1 or out.stride(1) != 1:
         raise invalid_argument("prefill attention: q and out must be dense within a row")
     if tcgen05 is None:
-        # The tcgen05 kernel is the faster one up to about four blocks per SM.  The engine knows the requests' lengths and estimates both
-        # (lb_attention_plan); here they are on the device.
-        blocks = n_seq * n_head * -(-max_q_len // 128)
         tcgen05 = (prefill_attention_tc_supports(n_head, n_kv_head, head_dim, page_size) and q.stride(0) % 8 == 0
                    and out.stride(0) % 8 == 0 and q.data_ptr() % 16 == 0 and out.data_ptr() % 16 == 0
-                   and (singles or blocks <= 4 * _sm_count(q.device)))
+                   and (singles or prefill_tcgen05_pays(n_seq, n_head, max_q_len, _sm_count(q.device))))
     if singles and not tcgen05:
         raise invalid_argument("prefill attention: only the tcgen05 launch serves single tokens beside the portions")
     if tcgen05:

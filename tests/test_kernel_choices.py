@@ -207,3 +207,8 @@ def test_products_of_some_dozens_of_tokens(N, K, bf16, f32):
     pays = ops.lib().lb_gemm_narrow_pays
     for m in (1, 16, 17, 32, 33, 48, 49, 64, 65, 128, 129, 256, 257, 512, 513, 2000):
         assert bool(pays(ops.BF16, m, N, K)) == (m in bf16) and bool(pays(ops.F32, m, N, K)) == (m in f32), m
+
+
+@pytest.mark.parametrize("n_seq,heads,longest,tcgen05", [(8, 12, 1024, True), (16, 12, 512, True), (20, 25, 100, True), (40, 25, 64, False), (60, 25, 30, False), (8, 12, 64, True), (1, 12, 8, True)])
+def test_portions_of_unknown_lengths(n_seq, heads, longest, tcgen05):
+    assert ops.prefill_tcgen05_pays(n_seq, heads, longest, 148) == tcgen05
